@@ -414,6 +414,7 @@ int setup(f8_ctx *c) {
     API_CUDA(c, c->alloc(&d.red, 4096));
     API_CUDA(c, c->alloc(&d.scal, 64));
     API_CUDA(c, c->alloc(&d.flag, 4));
+    API_CUDA(c, c->alloc(&d.code_count, 4));
     c->res_bytes = sizeof(StepCounters) + c->cyl.size() * 3 * sizeof(double);
     static_assert(sizeof(StepCounters) % sizeof(double) == 0, "drag slot alignment");
     API_CUDA(c, c->alloc(&c->res_dev, c->res_bytes));

@@ -85,6 +85,7 @@ struct Dev {
     double *red;                           // scratch partial sums (>= 4096)
     double *scal;                          // small scalar results
     int *flag;                             // SOR convergence flag / iteration
+    int *code_count;                       // FP64 3D: cells queued for the FP64 eigen test, per direction
     StepCounters *cnt;
 };
 
@@ -119,6 +120,14 @@ constexpr int NKERNEL = 6;   // enum f8_kernel
 
 // FP64 step (f8_step_fp64.cu).  Returns a cudaError_t of the launches; SOR
 // iteration count in *sor_iters.
+// SPD candidate choice of the FP64 3D step (f8_codes_fp64.cu): the codes that
+// rounding cannot change, and the queue of the others per direction (entry:
+// i - 1 + nx * (row + rows * (k - 1)), rows of the polymer update)
+cudaError_t codes3_filter(Dev &d, cudaStream_t s);
+inline unsigned *codes3_queue(const Dev &d, int dir) {
+    const size_t cap = (size_t)d.g.nx * (d.g.ny + 2) * d.g.nz;
+    return dir == 2 ? reinterpret_cast<unsigned *>(d.H2) : reinterpret_cast<unsigned *>(d.H) + (dir == 1 ? cap : 0);
+}
 cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_iters, cudaStream_t s);
 cudaError_t bc_all_state_fp64(Dev &d, cudaStream_t s);
 cudaError_t init_kernels_fp64();

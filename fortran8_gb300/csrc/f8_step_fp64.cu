@@ -273,6 +273,62 @@ __global__ void __launch_bounds__(128) k_polymer_codes3(const double *__restrict
     else codes_g[gcix(g, i, j, k)] = (uint8_t)code;
 }
 
+// The queue of k_codes3_filter: the FP64 evaluation of the (cell, direction)
+// pairs whose choice rounding might change.  Two lanes per entry, one for each
+// face of a candidate, so that a short queue's FP64 chain (three Vieta
+// evaluations, ~170 FP64 slots each) is half as long.
+__global__ void __launch_bounds__(128) k_codes3_exact(const double *__restrict__ C, uint8_t *codes, uint8_t *codes_g,
+                                                      Geo g, int cs, const unsigned *__restrict__ q0,
+                                                      const unsigned *__restrict__ q1, const unsigned *__restrict__ q2,
+                                                      const int *__restrict__ count) {
+    const int n0 = count[0], n1 = count[1], n = n0 + n1 + count[2];
+    const int face = threadIdx.x & 1;
+    // whole warps stay in the loop together for the shuffles
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 1; (w & ~15) < n; w += (gridDim.x * blockDim.x) >> 1) {
+        const bool active = w < n;
+        int d = 0, code = 0;
+        unsigned e = 0;
+        double v[3] = {0.0, 0.0, 0.0};
+        int i = 1, j = 1, k = 1;
+        if (active) {
+            d = w < n0 ? 0 : (w < n0 + n1 ? 1 : 2);
+            e = d == 0 ? q0[w] : (d == 1 ? q1[w - n0] : q2[w - n0 - n1]);
+            i = (int)(e % g.nx) + 1;
+            const int r = (int)(e / g.nx);
+            j = r % prows(g) + prow0(g);
+            k = r / prows(g) + 1;
+            const int h = hix(g, i, j, k), od = d == 0 ? 1 : (d == 1 ? g.sx : g.sx * g.sy);
+            const bool lo = !(d == 1 && j == 0), hi = !(d == 1 && j == g.ny + 1);   // zero beyond the ghost rows
+            double c0[6], cm[6], cp[6];
+            for (int m = 0; m < 6; ++m) {
+                const double *Cm = C + (size_t)m * cs + h;
+                c0[m] = Cm[0];
+                cm[m] = lo ? Cm[-od] : 0.0;
+                cp[m] = hi ? Cm[od] : 0.0;
+            }
+#pragma unroll 1
+            for (int l = 1; l <= 3; ++l) {
+                double f[6];
+                for (int m = 0; m < 6; ++m)
+                    f[m] = face ? face_n(l, cm[m], c0[m], cp[m]) : face_p(l, cm[m], c0[m], cp[m]);
+                v[l - 1] = vieta(f);
+            }
+        }
+        double minlist[4];
+        for (int l = 0; l < 3; ++l) {
+            const double o = __shfl_xor_sync(0xffffffffu, v[l], 1);
+            minlist[l] = face ? nanmin2(o, v[l]) : nanmin2(v[l], o);
+        }
+        minlist[3] = 0.0;
+        code = (maxloc4(minlist) - 1) << (2 * d);
+        if (active && face == 0 && code) {
+            uint8_t *dst = (j >= 1 && j <= g.ny) ? codes + qix(g, i, j, k) : codes_g + gcix(g, i, j, k);
+            const size_t a = reinterpret_cast<size_t>(dst);
+            atomicOr(reinterpret_cast<unsigned *>(a & ~(size_t)3), (unsigned)code << (8 * (a & 3)));
+        }
+    }
+}
+
 // fenep.f90:588-605
 __device__ inline void lyap_func3(const double A0[3][3], const double *b, const double *x, double *l, double lp2,
                                   double dt, double wi) {
@@ -1359,7 +1415,14 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
         dim3 blk(32, 4);
         // the rows of the polymer update (with walls the ghost rows too)
         dim3 grd((g.nx + blk.x - 1) / blk.x, (prows(g) + blk.y - 1) / blk.y, g.nz);
-        if (d3) { k_polymer_codes3<<<grd, blk, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs, d.ph.eigen_test); count_launch(); }
+        if (d3 && d.ph.eigen_test == 0) {
+            F8_CUDA_RET(codes3_filter(d, s));
+            // at most two lanes for each (cell, direction); grid-stride beyond the chip
+            const long most = 2L * 3 * g.nx * prows(g) * g.nz;
+            const unsigned nb = (unsigned)std::min((most + 127) / 128, 16L * device_sm_count());
+            k_codes3_exact<<<nb, 128, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs, codes3_queue(d, 0), codes3_queue(d, 1),
+                                              codes3_queue(d, 2), d.code_count); count_launch();
+        } else if (d3) { k_polymer_codes3<<<grd, blk, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs, d.ph.eigen_test); count_launch(); }
         else { k_polymer_codes2<<<grd, blk, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs); count_launch(); }
         mark(1);
         if (d3) { k_polymer_update3<<<grd, blk, 0, s>>>(d.C, d.Cn, d.fpet, d.codes, d.codes_g, d.U, d.V, d.W, g, d.ph, d.cs, d.cnt); count_launch(); }

@@ -329,26 +329,233 @@ __global__ void __launch_bounds__(128) k_codes3_exact(const double *__restrict__
     }
 }
 
-// fenep.f90:588-605
-__device__ inline void lyap_func3(const double A0[3][3], const double *b, const double *x, double *l, double lp2,
-                                  double dt, double wi) {
-    double A[3][3];
-    for (int r = 0; r < 3; ++r)
-        for (int q = 0; q < 3; ++q) A[r][q] = A0[r][q];
-    double fx = (lp2 - 3) / (lp2 - x[0] - x[3] - x[5]);
-    double dd = (1.0 + fx * dt / wi) / 2.0;
-    A[0][0] = A[0][0] + dd;
-    A[1][1] = A[1][1] + dd;
-    A[2][2] = A[2][2] + dd;
-    l[0] = (A[0][0] + A[0][0]) * x[0] + A[0][1] * x[1] + A[0][2] * x[2] + A[0][1] * x[1] + A[0][2] * x[2] - b[0];
-    l[1] = A[1][0] * x[0] + (A[1][1] + A[0][0]) * x[1] + A[1][2] * x[2] + A[0][1] * x[3] + A[0][2] * x[4] - b[1];
-    l[2] = A[2][0] * x[0] + A[2][1] * x[1] + (A[2][2] + A[0][0]) * x[2] + A[0][1] * x[4] + A[0][2] * x[5] - b[2];
-    l[3] = A[1][0] * x[1] + A[1][0] * x[1] + (A[1][1] + A[1][1]) * x[3] + A[1][2] * x[4] + A[1][2] * x[4] - b[3];
-    l[4] = A[1][0] * x[2] + A[2][0] * x[1] + A[2][1] * x[3] + (A[2][2] + A[1][1]) * x[4] + A[1][2] * x[5] - b[4];
-    l[5] = A[2][0] * x[2] + A[2][1] * x[4] + A[2][0] * x[2] + A[2][1] * x[4] + (A[2][2] + A[2][2]) * x[5] - b[5];
+// ---------------------------------------------------------------------------
+// Division by a divisor that is known in advance, from its reciprocal as the
+// unevaluated sum h + l of two doubles: RN(x h + RN(x l)) (Brisebarre, Muller and
+// Raina, IEEE Trans. Comput. 53 (2004) 1069).  The sum is within 2^-105 of x/d
+// before its one rounding, so it is the correctly rounded quotient unless x/d
+// lies that close to a rounding boundary (for a given d, a few x at most).  Two
+// FP64 slots where a division takes 7.2 (measured).
+struct Recip {
+    double h, l;
+};
+__host__ __device__ inline Recip recip(double d) {
+    const double h = 1.0 / d;
+    return Recip{h, fma(-d, h, 1.0) / d};
+}
+// on the device the second part only needs a few bits: its division is a product
+__device__ __forceinline__ Recip recip_dev(double d) {
+    const double h = 1.0 / d;
+    return Recip{h, __dmul_rn(__fma_rn(-d, h, 1.0), h)};
+}
+__device__ __forceinline__ double div_by(double x, Recip r) { return __fma_rn(x, r.h, __dmul_rn(x, r.l)); }
+
+// Divisors of the polymer update: the reference's expressions with their
+// divisions by constants.
+struct PolyConst {
+    Recip d2[3], d1[3], d4[3];   // 2 dX, dX, 4 dX, ... of the three directions
+    Recip wi, dc2;               // Wi, 2 dc
+    double dtwi;                 // dt / Wi
+    double eps2_lo, eps2_hi;     // bounds of the step test (below)
+};
+
+PolyConst poly_const(const Geo &g, const Phys &ph) {
+    PolyConst c;
+    const double d[3] = {g.dx, g.dy, g.dz};
+    for (int q = 0; q < 3; ++q) {
+        c.d1[q] = recip(d[q]);
+        c.d2[q] = recip(2 * d[q]);
+        c.d4[q] = recip(4 * d[q]);
+    }
+    c.wi = recip(ph.wi);
+    c.dc2 = recip(2.0 * ph.newton_dc);
+    c.dtwi = ph.dt / ph.wi;
+    c.eps2_lo = ph.newton_eps * ph.newton_eps * (1.0 - 1.0e-12);
+    c.eps2_hi = ph.newton_eps * ph.newton_eps * (1.0 + 1.0e-12);
+    return c;
 }
 
-// Gauss-Jordan with partial pivoting (fenep.f90:608-643)
+// The Newton step test sqrt(sr / sx) < eps (fenep.f90:575).  Squared, away from
+// the boundary by more than the rounding of either form; the reference's
+// expression within it (or for NaN).
+__device__ __forceinline__ bool newton_small(double sr, double sx, double eps, const PolyConst &c) {
+    if (sr < sx * c.eps2_lo) return true;
+    if (sr > sx * c.eps2_hi) return false;
+    return sqrt(sr / sx) < eps;
+}
+
+// A candidate face of fenep.f90:179-184 as w * t, with w a power of two and t
+// two rounded operations that give the reference's value scaled by 1/w exactly
+// (a scaling by a power of two commutes with rounding): t = RN(RN(a c0 + e) + f).
+//   plus face:  1: 3 c0/2 - cp/2 = (RN(3 c0) - cp)/2;  2: cm/2 + c0/2 = (c0 + cm)/2;
+//               3: cm/4 + c0 - cp/4 = (RN(4 c0 + cm) - cp)/4;  4: c0
+//   minus face: 1: (c0 + cp)/2;  2: (RN(3 c0) - cm)/2;  3: (RN(4 c0 - cm) + cp)/4;  4: c0
+// The candidate differs from lane to lane; a switch over the reference's
+// expressions costs every lane all of them (11 FP64 slots), this form two.
+struct FaceSel {
+    double a;        // factor of c0
+    double w;        // scale
+    int idx;
+};
+__device__ __forceinline__ FaceSel face_sel(int idx, bool minus) {
+    FaceSel s;
+    s.a = idx == 3 ? 4.0 : (idx == (minus ? 2 : 1) ? 3.0 : 1.0);
+    s.w = idx == 3 ? 0.25 : (idx == 4 ? 1.0 : 0.5);
+    s.idx = idx;
+    return s;
+}
+__device__ __forceinline__ double face_pt(const FaceSel &s, double cm, double c0, double cp) {
+    const double e = s.idx == 2 || s.idx == 3 ? cm : 0.0, f = s.idx == 1 || s.idx == 3 ? cp : 0.0;
+    return __dsub_rn(__fma_rn(c0, s.a, e), f);
+}
+__device__ __forceinline__ double face_nt(const FaceSel &s, double cm, double c0, double cp) {
+    const double e = s.idx == 1 ? cp : (s.idx == 3 ? -cm : 0.0), f = s.idx == 2 ? -cm : (s.idx == 3 ? cp : 0.0);
+    return __dadd_rn(__fma_rn(c0, s.a, e), f);
+}
+
+// Lyapunov_func (fenep.f90:588-605) and its central-difference Jacobian
+// (fenep.f90:540-572): the sums in the reference's order, every product and
+// partial sum that a perturbed column leaves unchanged taken from the base point
+// (the same operations on the same operands give the same double).
+//  * the off-diagonal columns (x1, x2, x4) do not change f(X): the diagonal of A
+//    is the base one, one row does not hold the variable (its entry is 0), and
+//    the sums before the variable's first term are the base ones;
+//  * the diagonal columns (x0, x3, x5) change f(X), so each row from its first
+//    diagonal term on.
+// About 1,000 FP64 slots an iteration where 13 full evaluations, the divisions
+// and the elimination took 1,700.
+struct Lyap3 {
+    double a01, a02, a10, a12, a20, a21, a00, a11, a22;
+};
+
+struct LyapSums {
+    double d00, d10, d20, d11, d21, d22;   // (A00+A00), (A11+A00), (A22+A00), ...
+};
+
+__device__ __forceinline__ LyapSums lyap_sums(const Lyap3 &A, double x0, double x3, double x5, double lp2, double dt,
+                                              const PolyConst &pc) {
+    const double fx = (lp2 - 3) / (lp2 - x0 - x3 - x5);
+    const double dd = (1.0 + div_by(fx * dt, pc.wi)) * 0.5;
+    const double a0 = A.a00 + dd, a1 = A.a11 + dd, a2 = A.a22 + dd;
+    return LyapSums{a0 + a0, a1 + a0, a2 + a0, a1 + a1, a2 + a1, a2 + a2};
+}
+
+// the products that do not hold a diagonal element of A
+struct LyapProd {
+    double p01x1, p02x2, p10x0, p12x2, p01x3, p02x4, p20x0, p21x1, p01x4, p02x5, p10x1, p12x4, p10x2, p20x1, p21x3,
+        p12x5, p20x2, p21x4;
+};
+
+// residuals of all rows with the diagonal sums D and the given diagonal
+// variables (x0, x3, x5 may be perturbed; p10x0, p20x0, p01x3, p21x3, p02x5 and
+// p12x5 are their products)
+__device__ __forceinline__ void lyap_rows(const LyapSums &D, const LyapProd &P, const double (&x)[6], double x0,
+                                          double x3, double x5, double p10x0, double p20x0, double p01x3, double p21x3,
+                                          double p02x5, double p12x5, const double (&b)[6], double r3, double r5,
+                                          double (&l)[6]) {
+    l[0] = D.d00 * x0 + P.p01x1 + P.p02x2 + P.p01x1 + P.p02x2 - b[0];
+    l[1] = p10x0 + D.d10 * x[1] + P.p12x2 + p01x3 + P.p02x4 - b[1];
+    l[2] = p20x0 + P.p21x1 + D.d20 * x[2] + P.p01x4 + p02x5 - b[2];
+    l[3] = r3 + D.d11 * x3 + P.p12x4 + P.p12x4 - b[3];
+    l[4] = P.p10x2 + P.p20x1 + p21x3 + D.d21 * x[4] + p12x5 - b[4];
+    l[5] = r5 + D.d22 * x5 - b[5];
+}
+
+// the residual at x in Ah[.][6] and the Jacobian in Ah[.][0..5]
+__device__ __forceinline__ void lyap_system(const Lyap3 &A, const double (&b)[6], const double (&x)[6], double lp2,
+                                            double dt, double dc, const PolyConst &pc, double (&Ah)[6][7]) {
+    LyapProd P;
+    P.p01x1 = A.a01 * x[1]; P.p02x2 = A.a02 * x[2]; P.p10x0 = A.a10 * x[0]; P.p12x2 = A.a12 * x[2];
+    P.p01x3 = A.a01 * x[3]; P.p02x4 = A.a02 * x[4]; P.p20x0 = A.a20 * x[0]; P.p21x1 = A.a21 * x[1];
+    P.p01x4 = A.a01 * x[4]; P.p02x5 = A.a02 * x[5]; P.p10x1 = A.a10 * x[1]; P.p12x4 = A.a12 * x[4];
+    P.p10x2 = A.a10 * x[2]; P.p20x1 = A.a20 * x[1]; P.p21x3 = A.a21 * x[3]; P.p12x5 = A.a12 * x[5];
+    P.p20x2 = A.a20 * x[2]; P.p21x4 = A.a21 * x[4];
+    const LyapSums D = lyap_sums(A, x[0], x[3], x[5], lp2, dt, pc);
+    const double r3 = P.p10x1 + P.p10x1, r5 = P.p20x2 + P.p21x4 + P.p20x2 + P.p21x4;
+    {
+        double l[6];
+        lyap_rows(D, P, x, x[0], x[3], x[5], P.p10x0, P.p20x0, P.p01x3, P.p21x3, P.p02x5, P.p12x5, b, r3, r5, l);
+#pragma unroll
+        for (int r = 0; r < 6; ++r) Ah[r][6] = l[r];
+    }
+    // columns 0, 3, 5
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int col = c == 0 ? 0 : (c == 1 ? 3 : 5);
+        double l1[6], l2[6];
+#pragma unroll
+        for (int sg = 0; sg < 2; ++sg) {
+            const double xv = sg == 0 ? x[col] + dc : x[col] - dc;
+            const double x0 = col == 0 ? xv : x[0], x3 = col == 3 ? xv : x[3], x5 = col == 5 ? xv : x[5];
+            const LyapSums Dp = lyap_sums(A, x0, x3, x5, lp2, dt, pc);
+            lyap_rows(Dp, P, x, x0, x3, x5, col == 0 ? A.a10 * xv : P.p10x0, col == 0 ? A.a20 * xv : P.p20x0,
+                      col == 3 ? A.a01 * xv : P.p01x3, col == 3 ? A.a21 * xv : P.p21x3, col == 5 ? A.a02 * xv : P.p02x5,
+                      col == 5 ? A.a12 * xv : P.p12x5, b, r3, r5, sg == 0 ? l1 : l2);
+        }
+#pragma unroll
+        for (int r = 0; r < 6; ++r) Ah[r][col] = div_by(l1[r] - l2[r], pc.dc2);
+    }
+    // columns 1, 2, 4: rows in the reference's order from the variable's first term
+    const double q0x0 = D.d00 * x[0], q1x1 = D.d10 * x[1], q2x2 = D.d20 * x[2], q3x3 = D.d11 * x[3],
+                 q4x4 = D.d21 * x[4], q5x5 = D.d22 * x[5];
+    double v1[5], v2[5];
+#pragma unroll
+    for (int sg = 0; sg < 2; ++sg) {
+        const double y = sg == 0 ? x[1] + dc : x[1] - dc;
+        double *v = sg == 0 ? v1 : v2;
+        const double t0 = A.a01 * y, t3 = A.a10 * y;
+        v[0] = q0x0 + t0 + P.p02x2 + t0 + P.p02x2 - b[0];
+        v[1] = P.p10x0 + D.d10 * y + P.p12x2 + P.p01x3 + P.p02x4 - b[1];
+        v[2] = P.p20x0 + A.a21 * y + q2x2 + P.p01x4 + P.p02x5 - b[2];
+        v[3] = t3 + t3 + q3x3 + P.p12x4 + P.p12x4 - b[3];
+        v[4] = P.p10x2 + A.a20 * y + P.p21x3 + q4x4 + P.p12x5 - b[4];
+    }
+#pragma unroll
+    for (int r = 0; r < 5; ++r) Ah[r][1] = div_by(v1[r] - v2[r], pc.dc2);
+    Ah[5][1] = 0.0;
+    const double s1 = P.p10x0 + q1x1, s2 = P.p20x0 + P.p21x1, s0 = q0x0 + P.p01x1;
+#pragma unroll
+    for (int sg = 0; sg < 2; ++sg) {
+        const double y = sg == 0 ? x[2] + dc : x[2] - dc;
+        double *v = sg == 0 ? v1 : v2;
+        const double t0 = A.a02 * y, t5 = A.a20 * y;
+        v[0] = s0 + t0 + P.p01x1 + t0 - b[0];
+        v[1] = s1 + A.a12 * y + P.p01x3 + P.p02x4 - b[1];
+        v[2] = s2 + D.d20 * y + P.p01x4 + P.p02x5 - b[2];
+        v[3] = A.a10 * y + P.p20x1 + P.p21x3 + q4x4 + P.p12x5 - b[4];
+        v[4] = t5 + P.p21x4 + t5 + P.p21x4 + q5x5 - b[5];
+    }
+    Ah[0][2] = div_by(v1[0] - v2[0], pc.dc2);
+    Ah[1][2] = div_by(v1[1] - v2[1], pc.dc2);
+    Ah[2][2] = div_by(v1[2] - v2[2], pc.dc2);
+    Ah[3][2] = 0.0;
+    Ah[4][2] = div_by(v1[3] - v2[3], pc.dc2);
+    Ah[5][2] = div_by(v1[4] - v2[4], pc.dc2);
+    const double e1 = s1 + P.p12x2 + P.p01x3, e2 = s2 + q2x2, e3 = r3 + q3x3, e4 = P.p10x2 + P.p20x1 + P.p21x3;
+#pragma unroll
+    for (int sg = 0; sg < 2; ++sg) {
+        const double y = sg == 0 ? x[4] + dc : x[4] - dc;
+        double *v = sg == 0 ? v1 : v2;
+        const double t3 = A.a12 * y, t5 = A.a21 * y;
+        v[0] = e1 + A.a02 * y - b[1];
+        v[1] = e2 + A.a01 * y + P.p02x5 - b[2];
+        v[2] = e3 + t3 + t3 - b[3];
+        v[3] = e4 + D.d21 * y + P.p12x5 - b[4];
+        v[4] = P.p20x2 + t5 + P.p20x2 + t5 + q5x5 - b[5];
+    }
+    Ah[0][4] = 0.0;
+#pragma unroll
+    for (int r = 0; r < 5; ++r) Ah[r + 1][4] = div_by(v1[r] - v2[r], pc.dc2);
+}
+
+// magnitude order of two doubles from their high words (sign dropped): true
+// only when |a| > |b| whatever the low words are
+__device__ __forceinline__ bool surely_larger(double a, double b) {
+    return (__double2hiint(a) & 0x7fffffff) > (__double2hiint(b) & 0x7fffffff);
+}
+
+// Gauss-Jordan with partial pivoting (fenep.f90:608-643); the pivot row is
+// divided through its reciprocal (div_by)
 template <int N>
 __device__ inline void gauss(double (&Ah)[N][N + 1], double *x) {
     for (int k = 0; k < N; ++k) {
@@ -363,8 +570,8 @@ __device__ inline void gauss(double (&Ah)[N][N + 1], double *x) {
         }
         if (k != maxidx)
             for (int q = k; q <= N; ++q) { double tmp = Ah[k][q]; Ah[k][q] = Ah[maxidx][q]; Ah[maxidx][q] = tmp; }
-        double piv = Ah[k][k];
-        for (int q = k + 1; q <= N; ++q) Ah[k][q] = Ah[k][q] / piv;
+        const Recip piv = recip_dev(Ah[k][k]);
+        for (int q = k + 1; q <= N; ++q) Ah[k][q] = div_by(Ah[k][q], piv);
         Ah[k][k] = 1.0;
         for (int r = 0; r < N; ++r) {
             if (r == k) continue;
@@ -376,15 +583,54 @@ __device__ inline void gauss(double (&Ah)[N][N + 1], double *x) {
     for (int r = 0; r < N; ++r) x[r] = Ah[r][N];
 }
 
+// The same elimination where every pivot is the diagonal element, as nearly
+// always (the Lyapunov system is dominated by it): in registers, the pivot
+// search as integer comparisons of the high words.  Returns false, with x
+// unusable, when some pivot might be another row's.
+template <int N>
+__device__ __forceinline__ bool gauss_diagonal(double (&Ah)[N][N + 1], double *x) {
+    bool plain = true;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+#pragma unroll
+        for (int r = k + 1; r < N; ++r) plain = plain && surely_larger(Ah[k][k], Ah[r][k]);
+        const Recip piv = recip_dev(Ah[k][k]);
+#pragma unroll
+        for (int q = k + 1; q <= N; ++q) Ah[k][q] = div_by(Ah[k][q], piv);
+#pragma unroll
+        for (int r = 0; r < N; ++r)
+            if (r != k) {
+                const double f = Ah[r][k];
+#pragma unroll
+                for (int q = k + 1; q <= N; ++q) Ah[r][q] = Ah[r][q] - f * Ah[k][q];
+            }
+    }
+#pragma unroll
+    for (int r = 0; r < N; ++r) x[r] = Ah[r][N];
+    return plain && surely_larger(Ah[N - 1][N - 1], 0.0);
+}
+
+// The Newton step with the pivoting elimination, out of line
+__device__ __noinline__ void lyap_step_pivoting(const Lyap3 &A, const double (&b)[6], const double (&x)[6], double lp2,
+                                                double dt, double dc, const PolyConst &pc, double (&r)[6]) {
+    double Ah[6][7];
+    lyap_system(A, b, x, lp2, dt, dc, pc, Ah);
+    gauss<6>(Ah, r);
+}
+
 // Cstar (fenep.f90:464-507) + Lyapunov Newton (fenep.f90:518-585) for one
 // cell.  The face states Cp/Cn of the three cells along each direction are
-// rebuilt from their selection codes, so no face arrays are stored.
-__global__ void __launch_bounds__(128) k_polymer_update3(const double *__restrict__ C, double *__restrict__ Cn,
+// rebuilt from their selection codes, so no face arrays are stored.  Bound by
+// the FP64 pipe: one warp instruction holds its sub-partition's pipe for 64
+// cycles (as long as its latency), so what counts is the number of FP64 slots,
+// not the occupancy; integer selects are free beside it.
+template <bool WALLS>
+__global__ void __launch_bounds__(128, 2) k_polymer_update3(const double *__restrict__ C, double *__restrict__ Cn,
                                                          double *__restrict__ fpet, const uint8_t *__restrict__ codes,
                                                          const uint8_t *__restrict__ codes_g,
                                                          const double *__restrict__ U, const double *__restrict__ V,
-                                                         const double *__restrict__ W, Geo g, Phys ph, int cs,
-                                                         StepCounters *cnt) {
+                                                         const double *__restrict__ W, Geo g, Phys ph, PolyConst pc,
+                                                         int cs, StepCounters *cnt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + prow0(g);
     const int k = blockIdx.z + 1;
@@ -392,126 +638,122 @@ __global__ void __launch_bounds__(128) k_polymer_update3(const double *__restric
     unsigned long long my_itr = 0, my_unconv = 0;
     if (active) {
         const int h = hix(g, i, j, k);
-        const double dt = ph.dt, dX = g.dx, dY = g.dy, dZ = g.dz;
+        const double dt = ph.dt;
         // selection codes of the cell and its neighbours (with walls the rows
         // beyond the ghost rows are outside: their faces are multiplied by
         // exactly zero in Cstar, the code there is the cell value's)
-        const int cself = code_at(codes, codes_g, g, i, j, k);
-        const int cxm = code_at(codes, codes_g, g, wrapx(g, i - 1), j, k) & 3;
-        const int cxp = code_at(codes, codes_g, g, wrapx(g, i + 1), j, k) & 3;
-        const int czm = (code_at(codes, codes_g, g, i, j, wrapz(g, k - 1)) >> 4) & 3;
-        const int czp = (code_at(codes, codes_g, g, i, j, wrapz(g, k + 1)) >> 4) & 3;
-        int cym, cyp;
+        const int xm = wrapx(g, i - 1), xp = wrapx(g, i + 1), zm = wrapz(g, k - 1), zp = wrapz(g, k + 1);
         int jm = j - 1, jp = j + 1;
-        if (!g.walls) { jm = wrapy(g, jm); jp = wrapy(g, jp); }
-        cym = (jm < 0) ? 3 : (code_at(codes, codes_g, g, i, jm, k) >> 2) & 3;
-        cyp = (jp > g.ny + 1) ? 3 : (code_at(codes, codes_g, g, i, jp, k) >> 2) & 3;
-        const int isx = (cself & 3) + 1, isy = ((cself >> 2) & 3) + 1, isz = ((cself >> 4) & 3) + 1;
-        // centres of the neighbour cells along each direction (wrapped)
-        const int xm = wrapx(g, i - 1), xp = wrapx(g, i + 1);
-        const int zm = wrapz(g, k - 1), zp = wrapz(g, k + 1);
-        const int hxm = hix(g, xm, j, k), hxp = hix(g, xp, j, k);
-        const int hzm = hix(g, i, j, zm), hzp = hix(g, i, j, zp);
-        const int ox = 1, oz = g.sx * g.sy;
-
-        double u1 = U[hix(g, i - 1, j, k)], u2 = U[h];
-        double v1 = crow(V, g, i, j - 1, k), v2 = V[h];
-        double w1 = W[hix(g, i, j, k - 1)], w2 = W[h];
-        double s1 = (-u2 + fabs(u2)) * dt / (2 * dX);
-        double s2 = 1.0 / 6 + (-u2 - fabs(u2)) * dt / (2 * dX);
-        double s3 = 1.0 / 6 + (u1 - fabs(u1)) * dt / (2 * dX);
-        double s4 = (u1 + fabs(u1)) * dt / (2 * dX);
-        double s5 = (-v2 + fabs(v2)) * dt / (2 * dY);
-        double s6 = 1.0 / 6 + (-v2 - fabs(v2)) * dt / (2 * dY);
-        double s7 = 1.0 / 6 + (v1 - fabs(v1)) * dt / (2 * dY);
-        double s8 = (v1 + fabs(v1)) * dt / (2 * dY);
-        double s9 = (-w2 + fabs(w2)) * dt / (2 * dZ);
-        double s10 = 1.0 / 6 + (-w2 - fabs(w2)) * dt / (2 * dZ);
-        double s11 = 1.0 / 6 + (w1 - fabs(w1)) * dt / (2 * dZ);
-        double s12 = (w1 + fabs(w1)) * dt / (2 * dZ);
-
+        if (!WALLS) { jm = wrapy(g, jm); jp = wrapy(g, jp); }
+        const int cself = code_at(codes, codes_g, g, i, j, k);
+        const int cym = (WALLS && jm < 0) ? 3 : (code_at(codes, codes_g, g, i, jm, k) >> 2) & 3;
+        const int cyp = (WALLS && jp > g.ny + 1) ? 3 : (code_at(codes, codes_g, g, i, jp, k) >> 2) & 3;
+        const int ox = 1, oy = g.sx, oz = g.sx * g.sy;
         double b[6], x[6];
-        for (int m = 0; m < 6; ++m) {
-            const double *Cm = C + (size_t)m * cs;
-            const double c0 = Cm[h];
-            // x
-            double pxm = face_p(isx, Cm[h - ox], c0, Cm[h + ox]);
-            double nxp = face_n(isx, Cm[h - ox], c0, Cm[h + ox]);
-            double pxp = face_p(cxp + 1, Cm[hxp - ox], Cm[hxp], Cm[hxp + ox]);
-            double nxm = face_n(cxm + 1, Cm[hxm - ox], Cm[hxm], Cm[hxm + ox]);
-            // y
-            double pym, nyp, pyp, nym;
-            if (!g.walls) {   // jm, jp wrapped; rows read around them through the halo
-                const int hym = hix(g, i, jm, k), hyp = hix(g, i, jp, k), oy = g.sx;
-                pym = face_p(isy, Cm[h - oy], c0, Cm[h + oy]);
-                nyp = face_n(isy, Cm[h - oy], c0, Cm[h + oy]);
-                pyp = face_p(cyp + 1, Cm[hyp - oy], Cm[hyp], Cm[hyp + oy]);
-                nym = face_n(cym + 1, Cm[hym - oy], Cm[hym], Cm[hym + oy]);
-            } else {          // zero beyond the ghost rows
-                const double ym2 = crow(Cm, g, i, j - 2, k), ym1 = crow(Cm, g, i, j - 1, k);
-                const double yp1 = crow(Cm, g, i, j + 1, k), yp2 = crow(Cm, g, i, j + 2, k);
-                pym = face_p(isy, ym1, c0, yp1);
-                nyp = face_n(isy, ym1, c0, yp1);
-                pyp = face_p(cyp + 1, c0, yp1, yp2);   // the p face of cell j+1
-                nym = face_n(cym + 1, ym2, ym1, c0);   // the n face of cell j-1
+#pragma unroll
+        for (int m = 0; m < 6; ++m) { x[m] = C[(size_t)m * cs + h]; b[m] = 0.0; }
+        // The directions in the reference's order of the sum: per direction the
+        // plus face of this cell's minus side, the plus face of the plus
+        // neighbour, the minus face of the minus neighbour and this cell's minus
+        // face (s3 Cpxm + s1 Cpxp + s4 Cnxm + s2 Cnxp + ...).
+        double u00, u11, u22;
+#pragma unroll 1
+        for (int d = 0; d < 3; ++d) {
+            const double *Vd = d == 0 ? U : (d == 1 ? V : W);
+            const int od = d == 0 ? ox : (d == 1 ? oy : oz);
+            const int self = ((cself >> (2 * d)) & 3) + 1;
+            const int cm_ = d == 0 ? code_at(codes, codes_g, g, xm, j, k) & 3
+                                   : (d == 1 ? cym : (code_at(codes, codes_g, g, i, j, zm) >> 4) & 3);
+            const int cp_ = d == 0 ? code_at(codes, codes_g, g, xp, j, k) & 3
+                                   : (d == 1 ? cyp : (code_at(codes, codes_g, g, i, j, zp) >> 4) & 3);
+            const bool ywall = WALLS && d == 1;
+            const double v1 = ywall && j == 0 ? 0.0 : Vd[h - od], v2 = Vd[h];
+            const Recip r2 = pc.d2[d];
+            const double a1 = fabs(v1), a2 = fabs(v2);
+            // s1 s2 s3 s4 of fenep.f90:481-492, scaled by the faces' powers of two
+            const double t1 = div_by((-v2 + a2) * dt, r2), t2 = 1.0 / 6 + div_by((-v2 - a2) * dt, r2);
+            const double t3 = 1.0 / 6 + div_by((v1 - a1) * dt, r2), t4 = div_by((v1 + a1) * dt, r2);
+            const FaceSel fps = face_sel(self, false), fns = face_sel(self, true), fpp = face_sel(cp_ + 1, false),
+                          fnm = face_sel(cm_ + 1, true);
+            const double s3 = t3 * fps.w, s2 = t2 * fns.w, s1 = t1 * fpp.w, s4 = t4 * fnm.w;
+            // the neighbours' centres and the cells beyond them (through the
+            // periodic image; zero beyond the ghost rows of a wall channel)
+            int hm, hp;
+            if (d == 0) { hm = hix(g, xm, j, k); hp = hix(g, xp, j, k); }
+            else if (d == 1) { hm = ywall ? h - od : hix(g, i, jm, k); hp = ywall ? h + od : hix(g, i, jp, k); }
+            else { hm = hix(g, i, j, zm); hp = hix(g, i, j, zp); }
+            const bool m1 = !(ywall && j < 1), m2 = !(ywall && j < 2), p1 = !(ywall && j > g.ny), p2 = !(ywall && j > g.ny - 1);
+#pragma unroll
+            for (int m = 0; m < 6; ++m) {
+                const double *Cm = C + (size_t)m * cs;
+                const double c0 = x[m];
+                const double cm = m1 ? Cm[h - od] : 0.0, cp = p1 ? Cm[h + od] : 0.0;
+                const double nm = ywall ? cm : Cm[hm], np = ywall ? cp : Cm[hp];      // neighbours' own values
+                const double mm = m2 ? Cm[hm - od] : 0.0, pp = p2 ? Cm[hp + od] : 0.0;
+                const double mc = ywall ? c0 : Cm[hm + od], pm = ywall ? c0 : Cm[hp - od];
+                const double f3 = s3 * face_pt(fps, cm, c0, cp);
+                b[m] = d == 0 ? f3 : b[m] + f3;
+                b[m] = b[m] + s1 * face_pt(fpp, pm, np, pp);
+                b[m] = b[m] + s4 * face_nt(fnm, mm, nm, mc);
+                b[m] = b[m] + s2 * face_nt(fns, cm, c0, cp);
             }
-            // z
-            double pzm = face_p(isz, Cm[h - oz], c0, Cm[h + oz]);
-            double nzp = face_n(isz, Cm[h - oz], c0, Cm[h + oz]);
-            double pzp = face_p(czp + 1, Cm[hzp - oz], Cm[hzp], Cm[hzp + oz]);
-            double nzm = face_n(czm + 1, Cm[hzm - oz], Cm[hzm], Cm[hzm + oz]);
-            b[m] = s3 * pxm + s1 * pxp + s4 * nxm + s2 * nxp + s7 * pym + s5 * pyp + s8 * nym + s6 * nyp
-                   + s11 * pzm + s9 * pzp + s12 * nzm + s10 * nzp;
-            x[m] = c0;
+            const double du = div_by(-dt * (-v1 + v2), pc.d1[d]);
+            if (d == 0) u00 = du;
+            else if (d == 1) u11 = du;
+            else u22 = du;
         }
-        const double wi = ph.wi;
-        b[0] = b[0] + dt / wi;
-        b[3] = b[3] + dt / wi;
-        b[5] = b[5] + dt / wi;
-        auto u = [&](int a, int bb, int cc) { return crow(U, g, a, bb, cc); };
-        auto v = [&](int a, int bb, int cc) { return crow(V, g, a, bb, cc); };
-        auto w = [&](int a, int bb, int cc) { return crow(W, g, a, bb, cc); };
-        double A0[3][3];
-        A0[0][0] = -dt * (-u(i - 1, j, k) + u(i, j, k)) / dX;
-        A0[0][1] = -dt * (-v(i - 1, j - 1, k) + v(i + 1, j - 1, k) - v(i - 1, j, k) + v(i + 1, j, k)) / (4 * dX);
-        A0[0][2] = -dt * (-w(i - 1, j, k - 1) + w(i + 1, j, k - 1) - w(i - 1, j, k) + w(i + 1, j, k)) / (4 * dX);
-        A0[1][0] = -dt * (-u(i - 1, j - 1, k) - u(i, j - 1, k) + u(i - 1, j + 1, k) + u(i, j + 1, k)) / (4 * dY);
-        A0[1][1] = -dt * (-v(i, j - 1, k) + v(i, j, k)) / dY;
-        A0[1][2] = -dt * (-w(i, j - 1, k - 1) + w(i, j + 1, k - 1) - w(i, j - 1, k) + w(i, j + 1, k)) / (4 * dY);
-        A0[2][0] = -dt * (-u(i - 1, j, k - 1) - u(i, j, k - 1) + u(i - 1, j, k + 1) + u(i, j, k + 1)) / (4 * dZ);
-        A0[2][1] = -dt * (-v(i, j - 1, k - 1) - v(i, j, k - 1) + v(i, j - 1, k + 1) + v(i, j, k + 1)) / (4 * dZ);
-        A0[2][2] = -dt * (-w(i, j, k - 1) + w(i, j, k)) / dZ;
-        double AT[3][3];
-        for (int r = 0; r < 3; ++r)
-            for (int q = 0; q < 3; ++q) AT[r][q] = A0[q][r];
-        const double dc = ph.newton_dc, eps = ph.newton_eps;
+        b[0] = b[0] + pc.dtwi;
+        b[3] = b[3] + pc.dtwi;
+        b[5] = b[5] + pc.dtwi;
+        // A = transpose of the velocity gradient (fenep.f90:541-550), zero
+        // velocity beyond the ghost rows of a wall channel
+        Lyap3 A;
+        {
+            const bool rm = !(WALLS && j == 0), rp = !(WALLS && j == g.ny + 1);
+            auto at = [&](const double *F, int di, int dj, int dk) {
+                if (WALLS && ((dj < 0 && !rm) || (dj > 0 && !rp))) return 0.0;
+                return F[h + di * ox + dj * oy + dk * oz];
+            };
+            A.a00 = u00;
+            A.a11 = u11;
+            A.a22 = u22;
+            A.a10 = div_by(-dt * (-at(V, -1, -1, 0) + at(V, 1, -1, 0) - at(V, -1, 0, 0) + at(V, 1, 0, 0)), pc.d4[0]);
+            A.a20 = div_by(-dt * (-at(W, -1, 0, -1) + at(W, 1, 0, -1) - at(W, -1, 0, 0) + at(W, 1, 0, 0)), pc.d4[0]);
+            A.a01 = div_by(-dt * (-at(U, -1, -1, 0) - at(U, 0, -1, 0) + at(U, -1, 1, 0) + at(U, 0, 1, 0)), pc.d4[1]);
+            A.a21 = div_by(-dt * (-at(W, 0, -1, -1) + at(W, 0, 1, -1) - at(W, 0, -1, 0) + at(W, 0, 1, 0)), pc.d4[1]);
+            A.a02 = div_by(-dt * (-at(U, -1, 0, -1) - at(U, 0, 0, -1) + at(U, -1, 0, 1) + at(U, 0, 0, 1)), pc.d4[2]);
+            A.a12 = div_by(-dt * (-at(V, 0, -1, -1) - at(V, 0, 0, -1) + at(V, 0, -1, 1) + at(V, 0, 0, 1)), pc.d4[2]);
+        }
         int itr;
+#pragma unroll 1
         for (itr = 1; itr <= ph.newton_itrmax; ++itr) {
-            double Ah[6][7], x1[6], x2[6], l1[6], l2[6], l[6], r[6];
-            for (int col = 0; col < 6; ++col) {
-                for (int m = 0; m < 6; ++m) { x1[m] = x[m]; x2[m] = x[m]; }
-                x1[col] = x1[col] + dc;
-                x2[col] = x2[col] - dc;
-                lyap_func3(AT, b, x1, l1, ph.lp2, dt, wi);
-                lyap_func3(AT, b, x2, l2, ph.lp2, dt, wi);
-                for (int row = 0; row < 6; ++row) Ah[row][col] = (l1[row] - l2[row]) / (2.0 * dc);
+            double Ah[6][7], r[6];
+            lyap_system(A, b, x, ph.lp2, dt, ph.newton_dc, pc, Ah);
+            if (!gauss_diagonal<6>(Ah, r)) {
+                // copies, so that the operands of the usual path stay in registers
+                const Lyap3 A2 = A;
+                double b2[6], x2[6], r2[6];
+#pragma unroll
+                for (int m = 0; m < 6; ++m) { b2[m] = b[m]; x2[m] = x[m]; }
+                lyap_step_pivoting(A2, b2, x2, ph.lp2, dt, ph.newton_dc, pc, r2);
+#pragma unroll
+                for (int m = 0; m < 6; ++m) r[m] = r2[m];
             }
-            lyap_func3(AT, b, x, l, ph.lp2, dt, wi);
-            for (int row = 0; row < 6; ++row) Ah[row][6] = l[row];
-            gauss<6>(Ah, r);
+#pragma unroll
             for (int m = 0; m < 6; ++m) x[m] = x[m] - r[m];
             double sr = 0, sx = 0;
+#pragma unroll
             for (int m = 0; m < 6; ++m) sr = sr + r[m] * r[m];
+#pragma unroll
             for (int m = 0; m < 6; ++m) sx = sx + x[m] * x[m];
-            if (sqrt(sr / sx) < eps) break;
+            if (newton_small(sr, sx, ph.newton_eps, pc)) break;
         }
         my_itr = (unsigned long long)itr;
         my_unconv = itr > ph.newton_itrmax ? 1ull : 0ull;
+#pragma unroll
         for (int m = 0; m < 6; ++m) Cn[(size_t)m * cs + h] = x[m];
         fpet[h] = (ph.lp2 - 3) / (ph.lp2 - x[0] - x[3] - x[5]);
     }
-    const int lane_flat = threadIdx.x + blockDim.x * threadIdx.y;
-    (void)lane_flat;
     unsigned long long a = my_itr, b2 = my_unconv;
     for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_down_sync(0xffffffffu, a, o);
@@ -585,10 +827,10 @@ __global__ void k_polymer_codes2(const double *__restrict__ C, uint8_t *__restri
 }
 
 __device__ inline void lyap_func2(const double A0[2][2], const double *b, const double *x, double *l, double lp2,
-                                  double dt, double wi) {
+                                  double dt, Recip wi) {
     double A[2][2] = {{A0[0][0], A0[0][1]}, {A0[1][0], A0[1][1]}};
     double fx = (lp2 - 2) / (lp2 - x[0] - x[2]);
-    double dd = (1.0 + fx * dt / wi) / 2.0;
+    double dd = (1.0 + div_by(fx * dt, wi)) * 0.5;
     A[0][0] = A[0][0] + dd;
     A[1][1] = A[1][1] + dd;
     l[0] = (A[0][0] + A[0][0]) * x[0] + A[0][1] * x[1] + A[0][1] * x[1] - b[0];
@@ -598,8 +840,8 @@ __device__ inline void lyap_func2(const double A0[2][2], const double *b, const 
 
 __global__ void k_polymer_update2(const double *__restrict__ C, double *__restrict__ Cn, double *__restrict__ fpet,
                                   const uint8_t *__restrict__ codes, const uint8_t *__restrict__ codes_g,
-                                  const double *__restrict__ U, const double *__restrict__ V, Geo g, Phys ph, int cs,
-                                  StepCounters *cnt) {
+                                  const double *__restrict__ U, const double *__restrict__ V, Geo g, Phys ph, PolyConst pc,
+                                  int cs, StepCounters *cnt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + prow0(g);
     const int k = 1;
@@ -607,7 +849,7 @@ __global__ void k_polymer_update2(const double *__restrict__ C, double *__restri
     unsigned long long my_itr = 0, my_unconv = 0;
     if (active) {
         const int h = hix(g, i, j, k);
-        const double dt = ph.dt, dX = g.dx, dY = g.dy;
+        const double dt = ph.dt;
         const int cself = code_at(codes, codes_g, g, i, j, k);
         const int cxm = code_at(codes, codes_g, g, wrapx(g, i - 1), j, k) & 3;
         const int cxp = code_at(codes, codes_g, g, wrapx(g, i + 1), j, k) & 3;
@@ -620,14 +862,14 @@ __global__ void k_polymer_update2(const double *__restrict__ C, double *__restri
         const int ox = 1;
         double u1 = U[hix(g, i - 1, j, k)], u2 = U[h];
         double v1 = crow(V, g, i, j - 1, k), v2 = V[h];
-        double s1 = (-u2 + fabs(u2)) * dt / (2 * dX);
-        double s2 = 1.0 / 4 + (-u2 - fabs(u2)) * dt / (2 * dX);
-        double s3 = 1.0 / 4 + (u1 - fabs(u1)) * dt / (2 * dX);
-        double s4 = (u1 + fabs(u1)) * dt / (2 * dX);
-        double s5 = (-v2 + fabs(v2)) * dt / (2 * dY);
-        double s6 = 1.0 / 4 + (-v2 - fabs(v2)) * dt / (2 * dY);
-        double s7 = 1.0 / 4 + (v1 - fabs(v1)) * dt / (2 * dY);
-        double s8 = (v1 + fabs(v1)) * dt / (2 * dY);
+        double s1 = div_by((-u2 + fabs(u2)) * dt, pc.d2[0]);
+        double s2 = 1.0 / 4 + div_by((-u2 - fabs(u2)) * dt, pc.d2[0]);
+        double s3 = 1.0 / 4 + div_by((u1 - fabs(u1)) * dt, pc.d2[0]);
+        double s4 = div_by((u1 + fabs(u1)) * dt, pc.d2[0]);
+        double s5 = div_by((-v2 + fabs(v2)) * dt, pc.d2[1]);
+        double s6 = 1.0 / 4 + div_by((-v2 - fabs(v2)) * dt, pc.d2[1]);
+        double s7 = 1.0 / 4 + div_by((v1 - fabs(v1)) * dt, pc.d2[1]);
+        double s8 = div_by((v1 + fabs(v1)) * dt, pc.d2[1]);
         double b[3], x[3];
         for (int m = 0; m < 3; ++m) {
             const double *Cm = C + (size_t)m * cs;
@@ -654,18 +896,17 @@ __global__ void k_polymer_update2(const double *__restrict__ C, double *__restri
             b[m] = s3 * pxm + s1 * pxp + s4 * nxm + s2 * nxp + s7 * pym + s5 * pyp + s8 * nym + s6 * nyp;
             x[m] = c0;
         }
-        const double wi = ph.wi;
-        b[0] = b[0] + dt / wi;
-        b[2] = b[2] + dt / wi;
+        b[0] = b[0] + pc.dtwi;
+        b[2] = b[2] + pc.dtwi;
         auto u = [&](int a, int bb) { return crow(U, g, a, bb, k); };
         auto v = [&](int a, int bb) { return crow(V, g, a, bb, k); };
         double A0[2][2];
-        A0[0][0] = -dt * (-u(i - 1, j) + u(i, j)) / dX;
-        A0[0][1] = -dt * (-v(i - 1, j - 1) + v(i + 1, j - 1) - v(i - 1, j) + v(i + 1, j)) / (4 * dX);
-        A0[1][0] = -dt * (-u(i - 1, j - 1) - u(i, j - 1) + u(i - 1, j + 1) + u(i, j + 1)) / (4 * dY);
-        A0[1][1] = -dt * (-v(i, j - 1) + v(i, j)) / dY;
+        A0[0][0] = div_by(-dt * (-u(i - 1, j) + u(i, j)), pc.d1[0]);
+        A0[0][1] = div_by(-dt * (-v(i - 1, j - 1) + v(i + 1, j - 1) - v(i - 1, j) + v(i + 1, j)), pc.d4[0]);
+        A0[1][0] = div_by(-dt * (-u(i - 1, j - 1) - u(i, j - 1) + u(i - 1, j + 1) + u(i, j + 1)), pc.d4[1]);
+        A0[1][1] = div_by(-dt * (-v(i, j - 1) + v(i, j)), pc.d1[1]);
         double AT[2][2] = {{A0[0][0], A0[1][0]}, {A0[0][1], A0[1][1]}};
-        const double dc = ph.newton_dc, eps = ph.newton_eps;
+        const double dc = ph.newton_dc;
         int itr;
         for (itr = 1; itr <= ph.newton_itrmax; ++itr) {
             double Ah[3][4], x1[3], x2[3], l1[3], l2[3], l[3], r[3];
@@ -673,18 +914,21 @@ __global__ void k_polymer_update2(const double *__restrict__ C, double *__restri
                 for (int m = 0; m < 3; ++m) { x1[m] = x[m]; x2[m] = x[m]; }
                 x1[col] = x1[col] + dc;
                 x2[col] = x2[col] - dc;
-                lyap_func2(AT, b, x1, l1, ph.lp2, dt, wi);
-                lyap_func2(AT, b, x2, l2, ph.lp2, dt, wi);
-                for (int row = 0; row < 3; ++row) Ah[row][col] = (l1[row] - l2[row]) / (2.0 * dc);
+                lyap_func2(AT, b, x1, l1, ph.lp2, dt, pc.wi);
+                lyap_func2(AT, b, x2, l2, ph.lp2, dt, pc.wi);
+                for (int row = 0; row < 3; ++row) Ah[row][col] = div_by(l1[row] - l2[row], pc.dc2);
             }
-            lyap_func2(AT, b, x, l, ph.lp2, dt, wi);
+            lyap_func2(AT, b, x, l, ph.lp2, dt, pc.wi);
             for (int row = 0; row < 3; ++row) Ah[row][3] = l[row];
-            gauss<3>(Ah, r);
+            double Ag[3][4];
+            for (int row = 0; row < 3; ++row)
+                for (int q = 0; q < 4; ++q) Ag[row][q] = Ah[row][q];
+            if (!gauss_diagonal<3>(Ah, r)) gauss<3>(Ag, r);
             for (int m = 0; m < 3; ++m) x[m] = x[m] - r[m];
             double sr = 0, sx = 0;
             for (int m = 0; m < 3; ++m) sr = sr + r[m] * r[m];
             for (int m = 0; m < 3; ++m) sx = sx + x[m] * x[m];
-            if (sqrt(sr / sx) < eps) break;
+            if (newton_small(sr, sx, ph.newton_eps, pc)) break;
         }
         my_itr = (unsigned long long)itr;
         my_unconv = itr > ph.newton_itrmax ? 1ull : 0ull;
@@ -1425,8 +1669,11 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
         } else if (d3) { k_polymer_codes3<<<grd, blk, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs, d.ph.eigen_test); count_launch(); }
         else { k_polymer_codes2<<<grd, blk, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs); count_launch(); }
         mark(1);
-        if (d3) { k_polymer_update3<<<grd, blk, 0, s>>>(d.C, d.Cn, d.fpet, d.codes, d.codes_g, d.U, d.V, d.W, g, d.ph, d.cs, d.cnt); count_launch(); }
-        else { k_polymer_update2<<<grd, blk, 0, s>>>(d.C, d.Cn, d.fpet, d.codes, d.codes_g, d.U, d.V, g, d.ph, d.cs, d.cnt); count_launch(); }
+        const PolyConst pc = poly_const(g, d.ph);
+        if (d3) {
+            auto update = g.walls ? k_polymer_update3<true> : k_polymer_update3<false>;
+            update<<<grd, blk, 0, s>>>(d.C, d.Cn, d.fpet, d.codes, d.codes_g, d.U, d.V, d.W, g, d.ph, pc, d.cs, d.cnt); count_launch();
+        } else { k_polymer_update2<<<grd, blk, 0, s>>>(d.C, d.Cn, d.fpet, d.codes, d.codes_g, d.U, d.V, g, d.ph, pc, d.cs, d.cnt); count_launch(); }
         std::swap(d.C, d.Cn);
         long n = halo_count(g);
         if (g.walls) { k_bc_c_pet_xz<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d.C, d.fpet, g, d.ncomp, d.cs, d.ph.lp2); count_launch(); }

@@ -93,7 +93,7 @@ cudaError_t step_mixed_adjoint(Dev &d, AdjStateF &A, const MixTape &t, const dou
         k_pack3<float><<<adj_cells(g, blk), blk, 0, s>>>(A.lUp[0], A.lUp[1], A.lUp[2], pk[0], pk[1], pk[2], g);
         count_launch();
         const float *src[3] = {pk[0], pk[1], pk[2]};
-        F8_CUDA_RET(mixed_helmholtz3(d, src, A.lQ, s));
+        F8_CUDA_RET(mixed_helmholtz(d, 3, src, A.lQ, s));
     }
     // 3. IBM
     for (int c = 0; c < 3; ++c) F8_CUDA_RET(cudaMemsetAsync(A.lUa[c], 0, hb, s));

@@ -378,6 +378,7 @@ int setup(f8_ctx *c) {
     API_CUDA(c, c->alloc(&d.codes_g, 2 * (size_t)g.nx * g.nz));
     const size_t nxh = g.nx / 2 + 1;
     const size_t nspec = 2 * nxh * (size_t)(g.ny + 2) * g.nz;
+    d.nspec = nspec;
     if (!mixed) {
         for (double **p : {&d.fpet, &d.Ua, &d.Va, &d.Wa}) API_CUDA(c, c->alloc(p, cs));
         API_CUDA(c, c->alloc(&d.C, cs * d.ncomp));
@@ -385,8 +386,8 @@ int setup(f8_ctx *c) {
         for (double **p : {&d.Ax0, &d.Ay0, &d.Az0, &d.Tx0, &d.Ty0, &d.Tz0, &d.Fx, &d.Fy, &d.Fz, &d.Bx, &d.By, &d.Bz,
                            &d.Q[0], &d.Q[1], &d.Q[2], &d.E})
             API_CUDA(c, c->alloc(p, ni));
-        API_CUDA(c, c->alloc(&d.H, nspec));
-        API_CUDA(c, c->alloc(&d.H2, nspec));
+        API_CUDA(c, c->alloc(&d.H, 3 * nspec));
+        API_CUDA(c, c->alloc(&d.H2, (g.walls ? 3 : 1) * nspec));
     } else {
         API_CUDA(c, c->alloc(&d.Cf, cs * d.ncomp));
         for (float **p : {&d.Uf, &d.Vf, &d.Wf, &d.Ul, &d.Vl, &d.Wl, &d.Pf, &d.Pl, &d.Phif, &d.Phil,
@@ -408,8 +409,6 @@ int setup(f8_ctx *c) {
         API_CUDA(c, c->alloc(&d.Rhf, ni));
         API_CUDA(c, c->alloc(&d.Rlf, ni));
         API_CUDA(c, c->alloc(&d.Rdf, ni));
-        API_CUDA(c, c->alloc(&d.Hf, nspec));
-        API_CUDA(c, c->alloc(&d.H2f, nspec));
     }
     API_CUDA(c, c->alloc(&d.red, 4096));
     API_CUDA(c, c->alloc(&d.scal, 64));
@@ -453,6 +452,10 @@ int setup(f8_ctx *c) {
     if (int st = upload(c, &d.kx2, kx2)) return st;
     if (int st = upload(c, &d.ky2, ky2)) return st;
     if (int st = upload(c, &d.kz2, kz2)) return st;
+    if (!mixed && g.walls) {
+        for (double *&t : d.walltab) API_CUDA(c, c->alloc(&t, 3 * nxh * (size_t)g.nz * (g.ny + 2)));
+        API_CUDA(c, wall_tables_fp64(d, c->s));
+    }
     if (mixed) {
         if (int st = upload_f(c, &d.kx2f, kx2)) return st;
         if (int st = upload_f(c, &d.ky2f, ky2)) return st;
@@ -467,6 +470,12 @@ int setup(f8_ctx *c) {
         if (g.walls) d.fused_planes = (d.plane_cl > 0 || (size_t)12 * ((g.ny + 2) | 1) * g.nz <= (size_t)optin) ? 1 : 0;
         else d.fused_planes = (size_t)8 * (g.ny + 1) * g.nz <= (size_t)optin ? 1 : 0;
         if (g.dim == 2) d.fused_planes = 0;   // 2D: the line transforms and tridiagonal sweeps
+        API_CUDA(c, c->alloc(&d.Hf, (d.fused_planes ? 1 : 3) * nspec));
+        if (!d.fused_planes && g.walls) {
+            API_CUDA(c, c->alloc(&d.H2f, 3 * nspec));
+            for (float *&t : d.walltabf) API_CUDA(c, c->alloc(&t, 3 * nxh * (size_t)g.nz * (g.ny + 2)));
+            API_CUDA(c, wall_tables_mixed(d, c->s));
+        }
         if (d.fused_planes) {
             // side streams and spectra of the V and W Helmholtz solves
             for (int b = 0; b < 2; ++b) {

@@ -474,26 +474,10 @@ cudaError_t device_spectrum(Dev &d, bool mixed, const double *const mean[3], Spe
     const double inv_n2 = 1.0 / ((double)ni * (double)ni);
     for (int c = 0; c < 3; ++c) {
         k_pack_fluct<<<(unsigned)((ni + 255) / 256), 256, 0, s>>>(in, g, c, w.pack); count_launch();
-        {
-            const int tpp = std::max(nx / 2, 1), ppc = std::max(1, 256 / tpp);
-            const int npp = ny / 2, total = npp * nz;
-            const size_t smem = (size_t)ppc * 2 * nx * sizeof(Cx<double>);
-            k_fft_x_fwd<double, double><<<(total + ppc - 1) / ppc, ppc * tpp, smem, s>>>(w.pack, w.H, nx, ny, 1, ny, npp, nz,
-                                                                                         w.twr[0], w.twi[0]); count_launch();
-        }
-        DivideSpec none{};
-        {
-            const int tx = std::max(1, std::min(32, 2048 / ny));
-            const size_t smem = (size_t)2 * ny * tx * sizeof(Cx<double>);
-            k_fft_lines<double><<<dim3((nxh + tx - 1) / tx, nz), 256, smem, s>>>(w.H, ny, nxh, nxh, nxh * ny, tx, w.twr[1],
-                                                                                  w.twi[1], -1, 0, none); count_launch();
-        }
-        {
-            const int tx = std::max(1, std::min(32, 2048 / nz));
-            const size_t smem = (size_t)2 * nz * tx * sizeof(Cx<double>);
-            k_fft_lines<double><<<dim3((nxh + tx - 1) / tx, ny), 256, smem, s>>>(w.H, nz, nxh * ny, nxh, nxh, tx, w.twr[2],
-                                                                                  w.twi[2], -1, 0, none); count_launch();
-        }
+        const DivideSpec none{};
+        fft_x_fwd<double, double>(1, Batch<const double *>{{w.pack}}, w.H, 0, nx, ny, 1, ny, ny / 2, nz, w.twr[0], w.twi[0], s);
+        fft_lines<double>(1, w.H, 0, ny, nxh, nxh, nz, nxh * ny, w.twr[1], w.twi[1], -1, 0, none, s);
+        fft_lines<double>(1, w.H, 0, nz, nxh * ny, nxh, ny, nxh, w.twr[2], w.twi[2], -1, 0, none, s);
         k_spec_bin<<<diag_blocks(), DIAG_THREADS, (size_t)nbins * sizeof(double), s>>>(w.H, g, nbins, inv_n2, w.hist,
                                                                                     c > 0 ? 1 : 0); count_launch();
     }

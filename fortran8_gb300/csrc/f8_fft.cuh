@@ -9,6 +9,7 @@
 // Spectral layout: complex values interleaved (re, im), [k][j][kx] with
 // kx = 0..NX/2 (NXH = NX/2+1 values per row).
 #pragma once
+#include <algorithm>
 #include "f8_common.cuh"
 #include "f8_df64.cuh"
 
@@ -17,44 +18,88 @@ namespace f8 {
 template <typename T>
 struct Cx { T r, i; };
 
-// One Stockham pass set over a line held in shared memory.  x and y are two
-// buffers of n complex values; t is the butterfly index (0..n/2-1) owned by the
-// calling thread; nthr threads cooperate on several lines: the caller passes
-// line-local pointers.  Returns the buffer that holds the result.
+__host__ __device__ inline int ilog2_pow2(int n) {
+    int l = 0;
+    while ((1 << l) < n) ++l;
+    return l;
+}
+
+// One butterfly (index j of 2^(lg-1)) of the Stockham stage of span 2^ls on a
+// line of 2^lg complex values in shared memory, x -> y.
 //   tw: forward twiddles exp(-2 pi i t/n), t < n/2 (re, im arrays)
+// The first stage's twiddle is 1.
 template <typename T>
-__device__ inline void stockham_stage(const Cx<T> *x, Cx<T> *y, int n, int ns, int j, const T *twr, const T *twi,
-                                      int sign) {
-    const int half = n >> 1;
-    const int kk = j % ns;
-    const int stride = n / (2 * ns);
-    T wr = twr[kk * stride];
-    T wi = sign < 0 ? twi[kk * stride] : -twi[kk * stride];
-    Cx<T> a = x[j], b = x[j + half];
-    T tr = b.r * wr - b.i * wi;
-    T ti = b.r * wi + b.i * wr;
-    int o = (j / ns) * 2 * ns + kk;
+__device__ __forceinline__ void stockham_stage(const Cx<T> *x, Cx<T> *y, int lg, int ls, int j, const T *twr,
+                                               const T *twi, int sign) {
+    const int half = 1 << (lg - 1), ns = 1 << ls;
+    const int kk = j & (ns - 1);
+    const Cx<T> a = x[j], b = x[j + half];
+    T tr = b.r, ti = b.i;
+    if (ls > 0) {
+        const int t = kk << (lg - 1 - ls);
+        const T wr = twr[t];
+        const T wi = sign < 0 ? twi[t] : -twi[t];
+        tr = b.r * wr - b.i * wi;
+        ti = b.r * wi + b.i * wr;
+    }
+    const int o = ((j >> ls) << (ls + 1)) + kk;
     y[o].r = a.r + tr; y[o].i = a.i + ti;
     y[o + ns].r = a.r - tr; y[o + ns].i = a.i - ti;
 }
+
+// Shapes of the transform launches.  A block takes up to 256 butterflies of a
+// stage (one per thread).  A small problem is bound by the chain of its stages
+// (an FP64 butterfly holds a sub-partition's pipe for 640 cycles), not by
+// memory, so its lines are spread over the chip: fewer lines per block until
+// there are two blocks per SM (304).  2D 128^2, FP64: 19 us a pass with 16
+// columns in each of 5 blocks, 4 us with one in each of 65.
+constexpr long FFT_MIN_BLOCKS = 304;
+
+// lines (row pairs) per block of an x pass over `pairs` row pairs
+inline int fft_pairs_per_block(int n, long pairs) {
+    int p = std::max(1, 512 / n);
+    while (p > 1 && p * n > 64 && (pairs + p - 1) / p < FFT_MIN_BLOCKS) p >>= 1;
+    return p;
+}
+
+// columns per block of a line pass; segments of at least 32 bytes where the
+// problem is large enough for memory to matter
+template <typename T>
+inline int fft_cols_per_block(int n, int ncols, long sets) {
+    int tx = std::max(512 / n, (int)(32 / sizeof(Cx<T>)));
+    while (tx > 1 && tx * n > 64 && (ncols + tx - 1) / tx * sets < FFT_MIN_BLOCKS) tx >>= 1;
+    return tx;
+}
+template <typename T>
+inline int fft_line_threads(int n, int tx) {
+    return std::min(256, std::max(32, n / 2 * tx));
+}
+
+// Up to three transforms of the same shape in one launch (blockIdx.z; their
+// spectra lie hstride values apart).
+template <typename P>
+struct Batch {
+    P p[3];
+};
 
 // ---------------------------------------------------------------------------
 // x direction, real <-> half spectrum, two rows per complex transform.
 //
 // Forward: rows (j0 + jj, j0 + jj + 1) of plane k of the interior-ordered
 // source src (row length n, nrow_src rows per plane) become spectral rows
-// jj, jj+1 of H (nrow_h rows per plane).  One CTA handles ppc row pairs with
-// n/2 threads each.
+// jj, jj+1 of H (nrow_h rows per plane).  One CTA handles blockDim.x / (n/2) row
+// pairs with n/2 threads each.
 template <typename T, typename TS>
-__global__ void k_fft_x_fwd(const TS *__restrict__ src, T *__restrict__ H, int n, int nrow_src, int j0, int nrow_h,
-                            int npairs_per_plane, int nplanes, const T *__restrict__ twr, const T *__restrict__ twi) {
+__global__ void k_fft_x_fwd(Batch<const TS *> srcs, T *__restrict__ H, size_t hstride, int lg, int nrow_src, int j0,
+                            int nrow_h, int npairs_per_plane, int nplanes, const T *__restrict__ twr,
+                            const T *__restrict__ twi) {
     extern __shared__ unsigned char smem_raw[];
     Cx<T> *sm = reinterpret_cast<Cx<T> *>(smem_raw);
-    const int half = n >> 1;
-    const int tpp = half > 0 ? half : 1;
-    const int ppc = blockDim.x / tpp;
-    const int p = threadIdx.x / tpp, t = threadIdx.x % tpp;
-    const long pair = (long)blockIdx.x * ppc + p;
+    const int n = 1 << lg, half = n >> 1, tpp = half;
+    const TS *__restrict__ src = srcs.p[blockIdx.z];
+    H += (size_t)blockIdx.z * hstride;
+    const int p = threadIdx.x >> (lg - 1), t = threadIdx.x & (half - 1);
+    const long pair = (long)blockIdx.x * (blockDim.x >> (lg - 1)) + p;
     const bool active = pair < (long)npairs_per_plane * nplanes;
     Cx<T> *x = sm + (size_t)p * 2 * n, *y = x + n;
     int k = 0, jj = 0;
@@ -66,8 +111,8 @@ __global__ void k_fft_x_fwd(const TS *__restrict__ src, T *__restrict__ H, int n
         for (int e = t; e < n; e += tpp) { x[e].r = T(ra[e]); x[e].i = T(rb[e]); }
     }
     __syncthreads();
-    for (int ns = 1; ns < n; ns *= 2) {
-        if (active && t < half) stockham_stage(x, y, n, ns, t, twr, twi, -1);
+    for (int ls = 0; ls < lg; ++ls) {
+        if (active) stockham_stage(x, y, lg, ls, t, twr, twi, -1);
         __syncthreads();
         Cx<T> *tmp = x; x = y; y = tmp;
     }
@@ -76,8 +121,7 @@ __global__ void k_fft_x_fwd(const TS *__restrict__ src, T *__restrict__ H, int n
     T *ha = H + 2 * ((size_t)nxh * ((size_t)jj + (size_t)nrow_h * k));
     T *hb = ha + 2 * nxh;
     for (int kx = t; kx < nxh; kx += tpp) {
-        int m = (n - kx) % n;
-        Cx<T> zk = x[kx], zm = x[m];
+        const Cx<T> zk = x[kx], zm = x[(n - kx) & (n - 1)];
         ha[2 * kx] = (zk.r + zm.r) * T(0.5);
         ha[2 * kx + 1] = (zk.i - zm.i) * T(0.5);
         hb[2 * kx] = (zk.i + zm.i) * T(0.5);
@@ -85,13 +129,23 @@ __global__ void k_fft_x_fwd(const TS *__restrict__ src, T *__restrict__ H, int n
     }
 }
 
-// Destinations of an inverse x pass.  XOutD: an FP64 field, optionally the
-// sum base + value (FP64 path and stand-alone solve).  XOutF: the FP32 /
-// double-float fields of the mixed path (modes below).
+template <typename T, typename TS>
+inline void fft_x_fwd(int nb, Batch<const TS *> src, T *H, size_t hstride, int n, int nrow_src, int j0, int nrow_h,
+                      int npairs, int nplanes, const T *twr, const T *twi, cudaStream_t s) {
+    const int ppc = fft_pairs_per_block(n, (long)npairs * nplanes * nb);
+    const size_t smem = (size_t)ppc * 2 * n * sizeof(Cx<T>);
+    const dim3 grid((unsigned)(((long)npairs * nplanes + ppc - 1) / ppc), 1, nb);
+    k_fft_x_fwd<T, TS><<<grid, ppc * (n / 2), smem, s>>>(src, H, hstride, ilog2_pow2(n), nrow_src, j0, nrow_h, npairs,
+                                                         nplanes, twr, twi);
+    count_launch();
+}
+
+// Destinations of an inverse x pass.  XOutD: an FP64 field (FP64 path and
+// stand-alone solve).  XOutF: the FP32 / double-float fields of the mixed path
+// (modes below).
 struct XOutD {
     double *dst;
-    const double *base;
-    __device__ __forceinline__ void put(size_t o, double v) const { dst[o] = base ? base[o] + v : v; }
+    __device__ __forceinline__ void put(size_t o, double v) const { dst[o] = v; }
 };
 
 struct XOutF {
@@ -115,16 +169,16 @@ struct XOutF {
 // jdst0 + jj + 1 of a halo-layout field (x written at 1..n) through the
 // destination functor.
 template <typename T, typename Out>
-__global__ void k_fft_x_inv(const T *__restrict__ H, Out out, int n, int nrow_h, int npairs_per_plane,
-                            int nplanes, int jdst0, int sx, int sy, const T *__restrict__ twr, const T *__restrict__ twi,
-                            int plain = 0) {
+__global__ void k_fft_x_inv(const T *__restrict__ H, size_t hstride, Batch<Out> outs, int lg, int nrow_h,
+                            int npairs_per_plane, int nplanes, int jdst0, int sx, int sy, const T *__restrict__ twr,
+                            const T *__restrict__ twi, int plain) {
     extern __shared__ unsigned char smem_raw[];
     Cx<T> *sm = reinterpret_cast<Cx<T> *>(smem_raw);
-    const int half = n >> 1;
-    const int tpp = half > 0 ? half : 1;
-    const int ppc = blockDim.x / tpp;
-    const int p = threadIdx.x / tpp, t = threadIdx.x % tpp;
-    const long pair = (long)blockIdx.x * ppc + p;
+    const int n = 1 << lg, half = n >> 1, tpp = half;
+    const Out out = outs.p[blockIdx.z];
+    H += (size_t)blockIdx.z * hstride;
+    const int p = threadIdx.x >> (lg - 1), t = threadIdx.x & (half - 1);
+    const long pair = (long)blockIdx.x * (blockDim.x >> (lg - 1)) + p;
     const bool active = pair < (long)npairs_per_plane * nplanes;
     Cx<T> *x = sm + (size_t)p * 2 * n, *y = x + n;
     int k = 0, jj = 0;
@@ -146,8 +200,8 @@ __global__ void k_fft_x_inv(const T *__restrict__ H, Out out, int n, int nrow_h,
         }
     }
     __syncthreads();
-    for (int ns = 1; ns < n; ns *= 2) {
-        if (active && t < half) stockham_stage(x, y, n, ns, t, twr, twi, +1);
+    for (int ls = 0; ls < lg; ++ls) {
+        if (active) stockham_stage(x, y, lg, ls, t, twr, twi, +1);
         __syncthreads();
         Cx<T> *tmp = x; x = y; y = tmp;
     }
@@ -160,9 +214,20 @@ __global__ void k_fft_x_inv(const T *__restrict__ H, Out out, int n, int nrow_h,
     for (int e = t; e < n; e += tpp) { out.put(oa + e, x[e].r); out.put(ob + e, x[e].i); }
 }
 
+template <typename T, typename Out>
+inline void fft_x_inv(int nb, const T *H, size_t hstride, Batch<Out> out, int n, int nrow_h, int npairs, int nplanes,
+                      int jdst0, int sx, int sy, const T *twr, const T *twi, int plain, cudaStream_t s) {
+    const int ppc = fft_pairs_per_block(n, (long)npairs * nplanes * nb);
+    const size_t smem = (size_t)ppc * 2 * n * sizeof(Cx<T>);
+    const dim3 grid((unsigned)(((long)npairs * nplanes + ppc - 1) / ppc), 1, nb);
+    k_fft_x_inv<T, Out><<<grid, ppc * (n / 2), smem, s>>>(H, hstride, out, ilog2_pow2(n), nrow_h, npairs, nplanes, jdst0,
+                                                          sx, sy, twr, twi, plain);
+    count_launch();
+}
+
 // ---------------------------------------------------------------------------
 // Strided complex transforms along y or z of the half spectrum.  A CTA owns tx
-// consecutive kx columns of one line set and keeps [n][tx] complex values in
+// consecutive kx columns of one line set and keeps [tx][n] complex values in
 // shared memory (so global reads are row segments of tx complex values).
 //   line element e of column c: H[base + e*lstride + c]  (complex units)
 //   base = set*sstride + kx0
@@ -171,63 +236,95 @@ __global__ void k_fft_x_inv(const T *__restrict__ H, Out out, int n, int nrow_h,
 // modified-wavenumber tables and the line index of the other axes.
 struct DivideSpec {
     const double *kx2, *ky2, *kz2;  // tables (FP64)
-    double lhs0, lhs1, ntot;        // LHS = lhs0 + lhs1*((kx2+ky2)+kz2); Q/ntot/LHS
+    double lhs0, lhs1;              // LHS = lhs0 + lhs1*((kx2+ky2)+kz2); Q/ntot/LHS
+    double inv_ntot;                // 1/(nx ny nz), a power of two: the product is the quotient
     int line_is_z;                  // 1: line along z (set = j); 0: along y (set = k)
 };
 
 template <typename T>
-__global__ void k_fft_lines(T *__restrict__ H, int n, int lstride, int ncols, int sstride, int tx,
-                            const T *__restrict__ twr, const T *__restrict__ twi, int sign, int mode, DivideSpec dv) {
+__global__ void __launch_bounds__(256) k_fft_lines(T *__restrict__ H, size_t hstride, int lg, int lstride, int ncols,
+                                                   int sstride, int tx, const T *__restrict__ twr,
+                                                   const T *__restrict__ twi, int sign, int mode, DivideSpec dv) {
     extern __shared__ unsigned char smem_raw[];
+    const int n = 1 << lg;
     Cx<T> *bufA = reinterpret_cast<Cx<T> *>(smem_raw);
     Cx<T> *bufB = bufA + (size_t)n * tx;
     const int set = blockIdx.y;
     const int kx0 = blockIdx.x * tx;
     const int ncol = min(tx, ncols - kx0);
-    Cx<T> *Hc = reinterpret_cast<Cx<T> *>(H);
+    const int ltx = 31 - __clz(tx);     // tx is a power of two
+    Cx<T> *Hc = reinterpret_cast<Cx<T> *>(H + (size_t)blockIdx.z * hstride);
     const size_t base = (size_t)set * sstride + kx0;
     // load: element (e, c) -> buf[c*n + e]
     for (int q = threadIdx.x; q < n * tx; q += blockDim.x) {
-        int e = q / tx, c = q % tx;
-        if (c < ncol) bufA[(size_t)c * n + e] = Hc[base + (size_t)e * lstride + c];
+        const int e = q >> ltx, c = q & (tx - 1);
+        if (c < ncol) bufA[(c << lg) + e] = Hc[base + (size_t)e * lstride + c];
     }
     __syncthreads();
-    const int half = n >> 1;
-    const int nbfly = half * tx;
-    int passes = mode == 1 ? 2 : 1;
+    const int nbfly = ncol << (lg - 1);
+    const int passes = mode == 1 ? 2 : 1;
     Cx<T> *x = bufA, *y = bufB;
     for (int ps = 0; ps < passes; ++ps) {
         const int sg = mode == 1 ? (ps == 0 ? -1 : +1) : sign;
-        for (int ns = 1; ns < n; ns *= 2) {
+        for (int ls = 0; ls < lg; ++ls) {
             for (int q = threadIdx.x; q < nbfly; q += blockDim.x) {
-                int c = q / half, j = q % half;
-                if (c < ncol) stockham_stage(x + (size_t)c * n, y + (size_t)c * n, n, ns, j, twr, twi, sg);
+                const int c = q >> (lg - 1), j = q & ((n >> 1) - 1);
+                stockham_stage(x + (c << lg), y + (c << lg), lg, ls, j, twr, twi, sg);
             }
             __syncthreads();
             Cx<T> *tmp = x; x = y; y = tmp;
         }
         if (mode == 1 && ps == 0) {
-            for (int q = threadIdx.x; q < n * tx; q += blockDim.x) {
-                int c = q / n, e = q % n;
-                if (c >= ncol) continue;
-                int kx = kx0 + c;
+            for (int q = threadIdx.x; q < ncol << lg; q += blockDim.x) {
+                const int c = q >> lg, e = q & (n - 1);
                 // element e of the line: along z -> kz = e, ky = set; along y -> ky = e, kz = set
-                int jy = dv.line_is_z ? set : e;
-                int kz = dv.line_is_z ? e : set;
-                double lhs = dv.lhs0 + dv.lhs1 * (dv.kx2[kx] + dv.ky2[jy] + dv.kz2[kz]);
-                Cx<T> v = x[(size_t)c * n + e];
-                T qr = v.r / T(dv.ntot), qi = v.i / T(dv.ntot);
+                const int jy = dv.line_is_z ? set : e;
+                const int kz = dv.line_is_z ? e : set;
+                const double lhs = dv.lhs0 + dv.lhs1 * (dv.kx2[kx0 + c] + dv.ky2[jy] + dv.kz2[kz]);
+                Cx<T> v = x[q];
+                const T qr = v.r * T(dv.inv_ntot), qi = v.i * T(dv.inv_ntot);
                 if (fabs(lhs) < 1.0e-16) { v.r = T(0); v.i = T(0); }
                 else { v.r = qr / T(lhs); v.i = qi / T(lhs); }
-                x[(size_t)c * n + e] = v;
+                x[q] = v;
             }
             __syncthreads();
         }
     }
     for (int q = threadIdx.x; q < n * tx; q += blockDim.x) {
-        int e = q / tx, c = q % tx;
-        if (c < ncol) Hc[base + (size_t)e * lstride + c] = x[(size_t)c * n + e];
+        const int e = q >> ltx, c = q & (tx - 1);
+        if (c < ncol) Hc[base + (size_t)e * lstride + c] = x[(c << lg) + e];
     }
+}
+
+template <typename T>
+inline void fft_lines(int nb, T *H, size_t hstride, int n, int lstride, int ncols, int sets, int sstride, const T *twr,
+                      const T *twi, int sign, int mode, const DivideSpec &dv, cudaStream_t s) {
+    const int tx = fft_cols_per_block<T>(n, ncols, (long)sets * nb);
+    const size_t smem = (size_t)2 * n * tx * sizeof(Cx<T>);
+    k_fft_lines<T><<<dim3((ncols + tx - 1) / tx, sets, nb), fft_line_threads<T>(n, tx), smem, s>>>(
+        H, hstride, ilog2_pow2(n), lstride, ncols, sstride, tx, twr, twi, sign, mode, dv);
+    count_launch();
+}
+
+// The periodic solve (fft_solve, fenep.f90:1400-1428) of nb right-hand sides
+// (interior order) through their spectra H: five passes in 3D; in 2D (nz = 1)
+// the y lines transform, divide and transform back in one of three.
+template <typename T, typename TS, typename Out>
+inline void fft_solve_passes(int nb, Batch<const TS *> src, T *H, size_t hstride, Batch<Out> out, int nx, int ny, int nz,
+                             int jdst0, int sx, int sy, int plain, const T *twx_r, const T *twx_i, const T *twy_r,
+                             const T *twy_i, const T *twz_r, const T *twz_i, const double *kx2, const double *ky2,
+                             const double *kz2, double lhs0, double lhs1, cudaStream_t s) {
+    const int nxh = nx / 2 + 1;
+    const DivideSpec dv{kx2, ky2, kz2, lhs0, lhs1, 1.0 / ((double)nx * ny * nz), nz > 1 ? 1 : 0};
+    fft_x_fwd<T, TS>(nb, src, H, hstride, nx, ny, 1, ny, ny / 2, nz, twx_r, twx_i, s);
+    if (nz == 1) {
+        fft_lines<T>(nb, H, hstride, ny, nxh, nxh, 1, nxh * ny, twy_r, twy_i, -1, 1, dv, s);
+    } else {
+        fft_lines<T>(nb, H, hstride, ny, nxh, nxh, nz, nxh * ny, twy_r, twy_i, -1, 0, dv, s);
+        fft_lines<T>(nb, H, hstride, nz, nxh * ny, nxh, ny, nxh, twz_r, twz_i, -1, 1, dv, s);
+        fft_lines<T>(nb, H, hstride, ny, nxh, nxh, nz, nxh * ny, twy_r, twy_i, +1, 0, dv, s);
+    }
+    fft_x_inv<T, Out>(nb, H, hstride, out, nx, ny, ny / 2, nz, jdst0, sx, sy, twx_r, twx_i, plain, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -243,12 +340,23 @@ struct WallSpec {
     const double *kx2, *kz2;
     double dt, beta, re, dy;
     double nxz;     // NX*NZ normalisation of the forward transforms
-    double uwall;   // 2*uwall on the top ghost row of mode (0,0) for SYS_U
+};
+
+inline WallSpec wall_spec(const Geo &g, const Phys &ph, const double *kx2, const double *kz2) {
+    return WallSpec{kx2, kz2, ph.dt, ph.beta, ph.re, g.dy, (double)g.nx * g.nz};
+}
+
+// One system of a batched wall solve: the tables of its kind, and the value of
+// the top ghost row of mode (0, 0) (2*uwall for U)
+template <typename T>
+struct WallItem {
     int sys;
+    const T *tab;
+    double top;
 };
 
 template <typename T>
-__device__ inline void wall_coef(const WallSpec &w, int sys, int j, int ny, double lam, T &a, T &b, T &c) {
+__host__ __device__ inline void wall_coef(const WallSpec &w, int sys, int j, int ny, double lam, T &a, T &b, T &c) {
     const int n = ny + 2;
     if (sys == SYS_U) {
         if (j == 0) { a = T(1.0); b = T(1.0); c = T(0.0); }
@@ -276,68 +384,111 @@ __device__ inline void wall_coef(const WallSpec &w, int sys, int j, int ny, doub
     }
 }
 
+// Tables of the Thomas recurrence of every (kx, kz) system: per row and mode
+// P = -b/den and 1/den as the sum of two T (Brisebarre, Muller and Raina's
+// division by a known divisor); all three zero where tdma's guard sets P = Q = 0
+// (fenep_2d.f90:1157-1160).  The recurrence runs in FP64 for either T, so the
+// singular mean mode of the pressure is pinned exactly.  Layout [row][kz][kx].
 template <typename T>
-__global__ void k_wall_tdma(const T *__restrict__ Hin, T *__restrict__ Hout, int ny, int nxh, int tx, WallSpec w) {
-    extern __shared__ unsigned char smem_raw[];
+__global__ void k_wall_table(T *__restrict__ P, T *__restrict__ rh, T *__restrict__ rl, int ny, int nxh, int nz,
+                             WallSpec w, int sys) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= nxh * nz) return;
+    const double lam = w.kx2[q % nxh] + w.kz2[q / nxh];
+    double p = 0.0;
+    for (int j = 0; j < ny + 2; ++j) {
+        double a, b, cc;
+        wall_coef<double>(w, sys, j, ny, lam, a, b, cc);
+        const double den = j == 0 ? a : a + cc * p;
+        const size_t o = (size_t)j * nxh * nz + q;
+        const bool guard = j > 0 && fabs(den) < 1.0e-16;
+        p = guard ? 0.0 : -b / den;
+        const double r = 1.0 / den;
+        P[o] = T(p);
+        rh[o] = guard ? T(0) : T(r);
+        rl[o] = guard ? T(0) : (sizeof(T) == 8 ? T(fma(-den, r, 1.0) / den) : T(r - (double)T(r)));
+    }
+}
+
+// The wall-normal solves (tdma, fenep_2d.f90:1145-1177) of every mode with
+// those tables.  A thread runs the recurrence of the real or the imaginary part
+// of one mode (the coefficients are real), neighbouring threads neighbouring
+// values of a row, so the rows stream through without a tile; the forward
+// values wait in the output.  In FP64 the chain is 5 slots a row forward and 2
+// back, where forming the coefficients and dividing took about 60 in a
+// half-filled warp.
+template <typename T>
+__global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *Hout, size_t hstride, int ny, int nxh,
+                                                  int nz, T inv_nxz, Batch<WallItem<T>> items, Batch<T> off) {
     const int n = ny + 2;
-    Cx<T> *q = reinterpret_cast<Cx<T> *>(smem_raw);       // [n][tx] rhs, then Q
-    T *P = reinterpret_cast<T *>(q + (size_t)n * tx);       // [n][tx]
+    const WallItem<T> it = items.p[blockIdx.z];
+    const int sys = it.sys;
+    const T ci = off.p[blockIdx.z];                         // the interior rows' off-diagonal
+    const size_t modes = (size_t)nxh * nz;
+    const T *__restrict__ P = it.tab, *__restrict__ rh = P + modes * n, *__restrict__ rl = rh + modes * n;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;   // kx * 2 + part
     const int kz = blockIdx.y;
-    const int kx0 = blockIdx.x * tx;
-    const int ncol = min(tx, nxh - kx0);
-    const Cx<T> *Hi = reinterpret_cast<const Cx<T> *>(Hin);
-    Cx<T> *Ho = reinterpret_cast<Cx<T> *>(Hout);
-    for (int e = threadIdx.x; e < n * tx; e += blockDim.x) {
-        int j = e / tx, c = e % tx;
-        if (c >= ncol) continue;
-        Cx<T> v;
-        if (j >= 1 && j <= ny && !(w.sys == SYS_V && j == ny)) {
-            Cx<T> h = Hi[(size_t)nxh * ((size_t)(j - 1) + (size_t)ny * kz) + kx0 + c];
-            v.r = h.r / T(w.nxz); v.i = h.i / T(w.nxz);
-        } else {
-            v.r = T(0); v.i = T(0);
-            if (w.sys == SYS_U && j == n - 1 && kx0 + c == 0 && kz == 0) v.r = T(2 * w.uwall);
-        }
-        q[(size_t)j * tx + c] = v;
+    if (c >= 2 * nxh) return;
+    const size_t mode = (size_t)nxh * kz + (c >> 1);
+    const T *__restrict__ hin = Hin + blockIdx.z * hstride + (size_t)2 * nxh * ny * kz + c;
+    T *hout = Hout + blockIdx.z * hstride + (size_t)2 * nxh * n * kz + c;
+    T q = T(0);
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+        T d = T(0);
+        if (j >= 1 && j <= ny && !(sys == SYS_V && j == ny)) d = hin[(size_t)2 * nxh * (j - 1)] * inv_nxz;
+        else if (j == n - 1 && mode == 0 && c == 0) d = T(it.top);
+        const T cc = j == 0 ? T(0) : (j == n - 1 ? (sys == SYS_U ? T(1) : (sys == SYS_V ? T(0) : T(-1)))
+                                                 : (sys == SYS_V && j >= ny ? T(0) : ci));
+        const size_t o = (size_t)j * modes + mode;
+        const T t = d - cc * q;
+        q = fma(t, rh[o], t * rl[o]);
+        hout[(size_t)2 * nxh * j] = q;
     }
-    __syncthreads();
-    const int c = threadIdx.x;
-    if (c < ncol) {
-        const double lam = w.kx2[kx0 + c] + w.kz2[kz];
-        T a, b, cc;
-        wall_coef<T>(w, w.sys, 0, ny, lam, a, b, cc);
-        Cx<T> d = q[c];
-        T p = -b / a;
-        Cx<T> Q; Q.r = d.r / a; Q.i = d.i / a;
-        P[c] = p; q[c] = Q;
-        for (int j = 1; j < n; ++j) {
-            wall_coef<T>(w, w.sys, j, ny, lam, a, b, cc);
-            d = q[(size_t)j * tx + c];
-            T den = a + cc * p;
-            if (fabs(den) < T(1.0e-16)) { p = T(0); Q.r = T(0); Q.i = T(0); }
-            else {
-                p = -b / den;
-                Q.r = (d.r - cc * Q.r) / den;
-                Q.i = (d.i - cc * Q.i) / den;
-            }
-            P[(size_t)j * tx + c] = p;
-            q[(size_t)j * tx + c] = Q;
-        }
-        Cx<T> x = q[(size_t)(n - 1) * tx + c];
-        for (int j = n - 2; j >= 0; --j) {
-            T pj = P[(size_t)j * tx + c];
-            Cx<T> qj = q[(size_t)j * tx + c];
-            x.r = pj * x.r + qj.r;
-            x.i = pj * x.i + qj.i;
-            q[(size_t)j * tx + c] = x;
-        }
+    T x = q;
+#pragma unroll 8
+    for (int j = n - 2; j >= 0; --j) {
+        x = P[(size_t)j * modes + mode] * x + hout[(size_t)2 * nxh * j];
+        hout[(size_t)2 * nxh * j] = x;
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < n * tx; e += blockDim.x) {
-        int j = e / tx, cc2 = e % tx;
-        if (cc2 >= ncol) continue;
-        Ho[(size_t)nxh * ((size_t)j + (size_t)n * kz) + kx0 + cc2] = q[(size_t)j * tx + cc2];
+}
+
+inline size_t wall_table_size(int ny, int nxh, int nz) { return (size_t)3 * (ny + 2) * nxh * nz; }
+
+template <typename T>
+inline void wall_table(T *tab, int ny, int nxh, int nz, const WallSpec &w, int sys, cudaStream_t s) {
+    const size_t m = (size_t)(ny + 2) * nxh * nz;
+    k_wall_table<T><<<(nxh * nz + 127) / 128, 128, 0, s>>>(tab, tab + m, tab + 2 * m, ny, nxh, nz, w, sys);
+    count_launch();
+}
+
+template <typename T>
+inline void wall_tdma(int nb, const T *Hin, T *Hout, size_t hstride, int ny, int nxh, int nz, const WallSpec &w,
+                      Batch<WallItem<T>> items, cudaStream_t s) {
+    Batch<T> off{};
+    for (int q = 0; q < nb; ++q) {
+        T a, b;
+        wall_coef<T>(w, items.p[q].sys, 1, ny, 0.0, a, b, off.p[q]);
     }
+    k_wall_tdma<T><<<dim3((2 * nxh + 63) / 64, nz, nb), 64, 0, s>>>(Hin, Hout, hstride, ny, nxh, nz, T(1.0 / w.nxz), items,
+                                                                    off);
+    count_launch();
+}
+
+// The wall-bounded solves of nb systems: FFT(x, z) of rows 1..NY, the
+// tridiagonal systems in y over rows 0..NY+1, inverse FFT of all NY+2 rows into
+// the halo rows of out.  H holds nb spectra of ny rows, H2 of ny + 2.
+template <typename T, typename TS, typename Out>
+inline void wall_solve_passes(int nb, Batch<const TS *> src, T *H, T *H2, size_t hstride, Batch<Out> out, const Geo &g,
+                              const T *twx_r, const T *twx_i, const T *twz_r, const T *twz_i, const WallSpec &w,
+                              Batch<WallItem<T>> items, cudaStream_t s) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz, nxh = nx / 2 + 1, n = ny + 2;
+    const DivideSpec none{};
+    fft_x_fwd<T, TS>(nb, src, H, hstride, nx, ny, 1, ny, ny / 2, nz, twx_r, twx_i, s);
+    if (nz > 1) fft_lines<T>(nb, H, hstride, nz, nxh * ny, nxh, ny, nxh, twz_r, twz_i, -1, 0, none, s);
+    wall_tdma<T>(nb, H, H2, hstride, ny, nxh, nz, w, items, s);
+    if (nz > 1) fft_lines<T>(nb, H2, hstride, nz, nxh * n, nxh, n, nxh, twz_r, twz_i, +1, 0, none, s);
+    fft_x_inv<T, Out>(nb, H2, hstride, out, nx, n, n / 2, nz, 0, g.sx, g.sy, twx_r, twx_i, 0, s);
 }
 
 }  // namespace f8

@@ -47,8 +47,9 @@ __global__ void k_xfwd_t(const TS *__restrict__ src, float2 *__restrict__ S, int
         for (int e = t; e < nx; e += half) { x[e].r = (float)ra[e]; x[e].i = (float)rbp[e]; }
     }
     __syncthreads();
-    for (int ns = 1; ns < nx; ns *= 2) {
-        if (active) stockham_stage(x, y, nx, ns, t, twr, twi, -1);
+    const int lg = ilog2_pow2(nx);
+    for (int ls = 0; ls < lg; ++ls) {
+        if (active) stockham_stage(x, y, lg, ls, t, twr, twi, -1);
         __syncthreads();
         Cx<float> *tmp = x; x = y; y = tmp;
     }
@@ -112,8 +113,9 @@ __global__ void k_xinv_t(const float2 *__restrict__ S, Out out, int nx, int nrow
         }
     }
     __syncthreads();
-    for (int ns = 1; ns < nx; ns *= 2) {
-        if (active) stockham_stage(x, y, nx, ns, t, twr, twi, +1);
+    const int lg = ilog2_pow2(nx);
+    for (int ls = 0; ls < lg; ++ls) {
+        if (active) stockham_stage(x, y, lg, ls, t, twr, twi, +1);
         __syncthreads();
         Cx<float> *tmp = x; x = y; y = tmp;
     }

@@ -48,31 +48,16 @@ SolveTables make_tables(int nx, int ny, int nz, double lx, double ly, double lz)
     return t;
 }
 
-// The five passes of the periodic solve on device buffers: q (dense
+// The passes of the periodic solve on device buffers: q (dense
 // nx*ny*nz) -> phi (dense), spectrum workspace H of 2*(nx/2+1)*ny*nz doubles,
 // tables as laid out by make_tables at dtab.
 cudaError_t run_solve(const double *q, double *phi, double *H, const double *dtab, const SolveTables &t, int nx,
                       int ny, int nz, double lhs0, double lhs1, cudaStream_t s) {
     using namespace f8;
-    const int nxh = nx / 2 + 1;
-    const double *twx_r = dtab + t.twx_r, *twx_i = dtab + t.twx_i;
-    const double *twy_r = dtab + t.twy_r, *twy_i = dtab + t.twy_i;
-    const double *twz_r = dtab + t.twz_r, *twz_i = dtab + t.twz_i;
-    const int tpp = std::max(nx / 2, 1), ppc = std::max(1, 256 / tpp);
-    const int npp = ny / 2, total = npp * nz;
-    const size_t smx = (size_t)ppc * 2 * nx * sizeof(Cx<double>);
-    k_fft_x_fwd<double, double><<<(total + ppc - 1) / ppc, ppc * tpp, smx, s>>>(q, H, nx, ny, 1, ny, npp, nz, twx_r, twx_i); count_launch();
-    DivideSpec none{};
-    const int txy = std::max(1, std::min(32, 2048 / ny));
-    const size_t smy = (size_t)2 * ny * txy * sizeof(Cx<double>);
-    k_fft_lines<double><<<dim3((nxh + txy - 1) / txy, nz), 256, smy, s>>>(H, ny, nxh, nxh, nxh * ny, txy, twy_r, twy_i, -1, 0, none); count_launch();
-    DivideSpec dv{dtab + t.kx2, dtab + t.ky2, dtab + t.kz2, lhs0, lhs1, (double)nx * ny * nz, 1};
-    const int txz = std::max(1, std::min(32, 2048 / nz));
-    const size_t smz = (size_t)2 * nz * txz * sizeof(Cx<double>);
-    k_fft_lines<double><<<dim3((nxh + txz - 1) / txz, ny), 256, smz, s>>>(H, nz, nxh * ny, nxh, nxh, txz, twz_r, twz_i, -1, 1, dv); count_launch();
-    k_fft_lines<double><<<dim3((nxh + txy - 1) / txy, nz), 256, smy, s>>>(H, ny, nxh, nxh, nxh * ny, txy, twy_r, twy_i, +1, 0, none); count_launch();
-    k_fft_x_inv<double, XOutD><<<(total + ppc - 1) / ppc, ppc * tpp, smx, s>>>(H, XOutD{phi, nullptr}, nx, ny, npp, nz, 0, nx, ny,
-                                                                            twx_r, twx_i, 1); count_launch();
+    fft_solve_passes<double, double, XOutD>(1, Batch<const double *>{{q}}, H, 0, Batch<XOutD>{{XOutD{phi}}}, nx, ny, nz, 0,
+                                            nx, ny, 1, dtab + t.twx_r, dtab + t.twx_i, dtab + t.twy_r, dtab + t.twy_i,
+                                            dtab + t.twz_r, dtab + t.twz_i, dtab + t.kx2, dtab + t.ky2, dtab + t.kz2,
+                                            lhs0, lhs1, s);
     return cudaGetLastError();
 }
 

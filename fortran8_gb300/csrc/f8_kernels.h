@@ -25,7 +25,10 @@ struct Dev {
     double *Bx, *By, *Bz;                  // interior
     double *Q[3];                          // interior right-hand sides
     double *E;                             // interior SOR residual
-    double *H, *H2;                        // spectral scratch
+    double *H, *H2;                        // spectral scratch: up to three spectra of nspec values each
+    size_t nspec;
+    double *walltab[3];                    // FP64 walls: Thomas tables of the U, V, P systems (k_wall_table)
+    float *walltabf[3];                    // the same in FP32 (mixed contexts without a fused plane kernel)
     double *twx_r, *twx_i, *twy_r, *twy_i, *twz_r, *twz_i;
     double *kx2, *ky2, *kz2;
     // IBM
@@ -131,6 +134,7 @@ inline unsigned *codes3_queue(const Dev &d, int dir) {
 cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_iters, cudaStream_t s);
 cudaError_t bc_all_state_fp64(Dev &d, cudaStream_t s);
 cudaError_t init_kernels_fp64();
+cudaError_t wall_tables_fp64(Dev &d, cudaStream_t s);
 cudaError_t aos_to_soa(const double *aos, double *soa, int ncomp, int cs, cudaStream_t s);
 cudaError_t soa_to_aos(const double *soa, double *aos, int ncomp, int cs, cudaStream_t s);
 cudaError_t count_nonfinite(const double *a, int n, unsigned long long *out, cudaStream_t s);
@@ -242,7 +246,7 @@ struct AdjStateF {
 cudaError_t mixed_solve_periodic(Dev &d, const float *src, float *dst, float *lo, int mode, double lhs0, double lhs1,
                                  cudaStream_t s);
 cudaError_t mixed_solve_walls(Dev &d, const float *src, float *dst, float *lo, int mode, int sys, cudaStream_t s);
-cudaError_t mixed_helmholtz3(Dev &d, const float *const src[3], float *const dst[3], cudaStream_t s);
+cudaError_t mixed_helmholtz(Dev &d, int n, const float *const src[3], float *const dst[3], cudaStream_t s);
 cudaError_t mixed_defect(Dev &d, const float *phi, const float *rh, const float *rl, float *rd, cudaStream_t s);
 cudaError_t setup_staged_projection(Dev &d);
 cudaError_t step_mixed_adjoint(Dev &d, AdjStateF &A, const MixTape &t, const double *drag_w, bool ab2_first,
@@ -251,6 +255,7 @@ cudaError_t adjoint_fold_state_f(AdjStateF &A, const Dev &d, cudaStream_t s);
 cudaError_t take_interior_f(const float *src, float *dst, const Geo &g, int n, cudaStream_t s);
 // Mixed path (f8_step_mixed.cu)
 cudaError_t init_kernels_mixed();
+cudaError_t wall_tables_mixed(Dev &d, cudaStream_t s);
 cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_iters, cudaStream_t s);
 cudaError_t bc_all_state_mixed(Dev &d, cudaStream_t s);
 cudaError_t mixed_state_to_fp64(Dev &d, cudaStream_t s);

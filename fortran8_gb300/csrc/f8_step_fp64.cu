@@ -41,19 +41,36 @@ __device__ inline double halo_value(const Geo &g, const double *A, int kind, int
     }
 }
 
-__global__ void k_bc_scalar(double *A, Geo g, int kind) {
+// Boundary values of up to four fields in one launch, and V = 0 on the upper
+// wall face (V(:,NB) = 0, fenep_2d.f90:1114)
+struct BcSetD {
+    double *A[4];
+    int kind[4];
+    int n;
+};
+
+__global__ void k_bc_set64(BcSetD b, Geo g) {
     long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     int i, j, k;
     if (halo_cell(g, t, i, j, k)) {
-        A[hix(g, i, j, k)] = halo_value(g, A, kind, i, j, k);
+        const int h = hix(g, i, j, k);
+        // every field's source value before the first store
+        double v[4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+            if (f < b.n) v[f] = halo_value(g, b.A[f], b.kind[f], i, j, k);
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+            if (f < b.n) b.A[f][h] = v[f];
         return;
     }
-    // V on the upper wall face (V(:,NB) = 0, fenep_2d.f90:1114)
-    if (kind == BC_V && g.walls) {
+    if (g.walls) {
         t -= halo_count(g);
         if (t >= 0 && t < (long)g.nx * g.nz) {
             i = 1 + (int)(t % g.nx); k = 1 + (int)(t / g.nx);
-            A[hix(g, i, g.ny, k)] = 0.0;
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+                if (f < b.n && b.kind[f] == BC_V) b.A[f][hix(g, i, g.ny, k)] = 0.0;
         }
     }
 }
@@ -372,6 +389,24 @@ PolyConst poly_const(const Geo &g, const Phys &ph) {
     c.dtwi = ph.dt / ph.wi;
     c.eps2_lo = ph.newton_eps * ph.newton_eps * (1.0 - 1.0e-12);
     c.eps2_hi = ph.newton_eps * ph.newton_eps * (1.0 + 1.0e-12);
+    return c;
+}
+
+// The same for the stencils of the momentum, projection and IBM kernels
+struct GridRecip {
+    Recip d1[3], d4[3], dd[3];   // dX, 4 dX, dX^2, ...
+    Recip dt;
+};
+
+GridRecip grid_recip(const Geo &g) {
+    GridRecip c;
+    const double d[3] = {g.dx, g.dy, g.dz};
+    for (int q = 0; q < 3; ++q) {
+        c.d1[q] = recip(d[q]);
+        c.d4[q] = recip(4 * d[q]);
+        c.dd[q] = recip(d[q] * d[q]);
+    }
+    c.dt = recip(g.dt);
     return c;
 }
 
@@ -965,12 +1000,12 @@ struct MomArgs {
 };
 
 template <int DIM>
-__global__ void __launch_bounds__(256) k_momentum(MomArgs a, Geo g) {
+__global__ void __launch_bounds__(256) k_momentum(MomArgs a, Geo g, GridRecip kc) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z + 1;
     if (i > g.nx || j > g.ny) return;
-    const double dX = g.dx, dY = g.dy, dZ = g.dz, dt = g.dt;
+    const double dt = g.dt;
     const double *U = a.U, *V = a.V, *W = a.W;
     auto u = [&](int x, int y, int z) { return U[hix(g, x, y, z)]; };
     auto v = [&](int x, int y, int z) { return V[hix(g, x, y, z)]; };
@@ -988,15 +1023,15 @@ __global__ void __launch_bounds__(256) k_momentum(MomArgs a, Geo g) {
                 int hh = hix(g, x, y, z);
                 return fp[hh] * C[(size_t)(m - 1) * cs + hh] - E[m - 1];
             };
-            double sx = (-c0(1, i, j, k) + c0(1, i + 1, j, k)) / dX
-                      + (-c0(2, i, j - 1, k) - c0(2, i + 1, j - 1, k) + c0(2, i, j + 1, k) + c0(2, i + 1, j + 1, k)) / (4 * dY)
-                      + (-c0(3, i, j, k - 1) - c0(3, i + 1, j, k - 1) + c0(3, i, j, k + 1) + c0(3, i + 1, j, k + 1)) / (4 * dZ);
-            double sy = (-c0(2, i - 1, j, k) + c0(2, i + 1, j, k) - c0(2, i - 1, j + 1, k) + c0(2, i + 1, j + 1, k)) / (4 * dX)
-                      + (-c0(4, i, j, k) + c0(4, i, j + 1, k)) / dY
-                      + (-c0(5, i, j, k - 1) - c0(5, i, j + 1, k - 1) + c0(5, i, j, k + 1) + c0(5, i, j + 1, k + 1)) / (4 * dZ);
-            double sz = (-c0(3, i - 1, j, k) + c0(3, i + 1, j, k) - c0(3, i - 1, j, k + 1) + c0(3, i + 1, j, k + 1)) / (4 * dX)
-                      + (-c0(5, i, j - 1, k) + c0(5, i, j + 1, k) - c0(5, i, j - 1, k + 1) + c0(5, i, j + 1, k + 1)) / (4 * dY)
-                      + (-c0(6, i, j, k) + c0(6, i, j, k + 1)) / dZ;
+            double sx = div_by(-c0(1, i, j, k) + c0(1, i + 1, j, k), kc.d1[0])
+                      + div_by(-c0(2, i, j - 1, k) - c0(2, i + 1, j - 1, k) + c0(2, i, j + 1, k) + c0(2, i + 1, j + 1, k), kc.d4[1])
+                      + div_by(-c0(3, i, j, k - 1) - c0(3, i + 1, j, k - 1) + c0(3, i, j, k + 1) + c0(3, i + 1, j, k + 1), kc.d4[2]);
+            double sy = div_by(-c0(2, i - 1, j, k) + c0(2, i + 1, j, k) - c0(2, i - 1, j + 1, k) + c0(2, i + 1, j + 1, k), kc.d4[0])
+                      + div_by(-c0(4, i, j, k) + c0(4, i, j + 1, k), kc.d1[1])
+                      + div_by(-c0(5, i, j, k - 1) - c0(5, i, j + 1, k - 1) + c0(5, i, j, k + 1) + c0(5, i, j + 1, k + 1), kc.d4[2]);
+            double sz = div_by(-c0(3, i - 1, j, k) + c0(3, i + 1, j, k) - c0(3, i - 1, j, k + 1) + c0(3, i + 1, j, k + 1), kc.d4[0])
+                      + div_by(-c0(5, i, j - 1, k) + c0(5, i, j + 1, k) - c0(5, i, j - 1, k + 1) + c0(5, i, j + 1, k + 1), kc.d4[1])
+                      + div_by(-c0(6, i, j, k) + c0(6, i, j, k + 1), kc.d1[2]);
             tx = a.coef_t * sx; ty = a.coef_t * sy; tz = a.coef_t * sz;
         } else {
             const double E[3] = {1.0, 0.0, 1.0};
@@ -1004,43 +1039,43 @@ __global__ void __launch_bounds__(256) k_momentum(MomArgs a, Geo g) {
                 int hh = hix(g, x, y, k);
                 return fp[hh] * C[(size_t)(m - 1) * cs + hh] - E[m - 1];
             };
-            double sx = (-c0(1, i, j) + c0(1, i + 1, j)) / dX
-                      + (-c0(2, i, j - 1) - c0(2, i + 1, j - 1) + c0(2, i, j + 1) + c0(2, i + 1, j + 1)) / (4 * dY);
-            double sy = (-c0(2, i - 1, j) + c0(2, i + 1, j) - c0(2, i - 1, j + 1) + c0(2, i + 1, j + 1)) / (4 * dX)
-                      + (-c0(3, i, j) + c0(3, i, j + 1)) / dY;
+            double sx = div_by(-c0(1, i, j) + c0(1, i + 1, j), kc.d1[0])
+                      + div_by(-c0(2, i, j - 1) - c0(2, i + 1, j - 1) + c0(2, i, j + 1) + c0(2, i + 1, j + 1), kc.d4[1]);
+            double sy = div_by(-c0(2, i - 1, j) + c0(2, i + 1, j) - c0(2, i - 1, j + 1) + c0(2, i + 1, j + 1), kc.d4[0])
+                      + div_by(-c0(3, i, j) + c0(3, i, j + 1), kc.d1[1]);
             tx = a.coef_t * sx; ty = a.coef_t * sy;
         }
     }
     // convection and viscous terms
     double t1 = (u(i - 1, j, k) + u(i, j, k)) / 2, t2 = (u(i, j, k) + u(i + 1, j, k)) / 2;
-    double ax = (-(t1 * t1) + t2 * t2) / dX
-              + (-(v(i, j - 1, k) + v(i + 1, j - 1, k)) / 2 * (u(i, j - 1, k) + u(i, j, k)) / 2
-                 + (v(i, j, k) + v(i + 1, j, k)) / 2 * (u(i, j, k) + u(i, j + 1, k)) / 2) / dY;
+    double ax = div_by(-(t1 * t1) + t2 * t2, kc.d1[0])
+              + div_by(-(v(i, j - 1, k) + v(i + 1, j - 1, k)) / 2 * (u(i, j - 1, k) + u(i, j, k)) / 2
+                 + (v(i, j, k) + v(i + 1, j, k)) / 2 * (u(i, j, k) + u(i, j + 1, k)) / 2, kc.d1[1]);
     double t3 = (v(i, j - 1, k) + v(i, j, k)) / 2, t4 = (v(i, j, k) + v(i, j + 1, k)) / 2;
-    double ay = (-(u(i - 1, j, k) + u(i - 1, j + 1, k)) / 2 * (v(i - 1, j, k) + v(i, j, k)) / 2
-                 + (u(i, j, k) + u(i, j + 1, k)) / 2 * (v(i, j, k) + v(i + 1, j, k)) / 2) / dX
-              + (-(t3 * t3) + t4 * t4) / dY;
-    double bx = (u(i - 1, j, k) - 2 * u(i, j, k) + u(i + 1, j, k)) / (dX * dX)
-              + (u(i, j - 1, k) - 2 * u(i, j, k) + u(i, j + 1, k)) / (dY * dY);
-    double by = (v(i - 1, j, k) - 2 * v(i, j, k) + v(i + 1, j, k)) / (dX * dX)
-              + (v(i, j - 1, k) - 2 * v(i, j, k) + v(i, j + 1, k)) / (dY * dY);
+    double ay = div_by(-(u(i - 1, j, k) + u(i - 1, j + 1, k)) / 2 * (v(i - 1, j, k) + v(i, j, k)) / 2
+                 + (u(i, j, k) + u(i, j + 1, k)) / 2 * (v(i, j, k) + v(i + 1, j, k)) / 2, kc.d1[0])
+              + div_by(-(t3 * t3) + t4 * t4, kc.d1[1]);
+    double bx = div_by(u(i - 1, j, k) - 2 * u(i, j, k) + u(i + 1, j, k), kc.dd[0])
+              + div_by(u(i, j - 1, k) - 2 * u(i, j, k) + u(i, j + 1, k), kc.dd[1]);
+    double by = div_by(v(i - 1, j, k) - 2 * v(i, j, k) + v(i + 1, j, k), kc.dd[0])
+              + div_by(v(i, j - 1, k) - 2 * v(i, j, k) + v(i, j + 1, k), kc.dd[1]);
     double az = 0, bz = 0;
     if (DIM == 3) {
-        ax = ax + (-(w(i, j, k - 1) + w(i + 1, j, k - 1)) / 2 * (u(i, j, k - 1) + u(i, j, k)) / 2
-                   + (w(i, j, k) + w(i + 1, j, k)) / 2 * (u(i, j, k) + u(i, j, k + 1)) / 2) / dZ;
-        ay = ay + (-(w(i, j, k - 1) + w(i, j + 1, k - 1)) / 2 * (v(i, j, k - 1) + v(i, j, k)) / 2
-                   + (w(i, j, k) + w(i, j + 1, k)) / 2 * (v(i, j, k) + v(i, j, k + 1)) / 2) / dZ;
+        ax = ax + div_by(-(w(i, j, k - 1) + w(i + 1, j, k - 1)) / 2 * (u(i, j, k - 1) + u(i, j, k)) / 2
+                   + (w(i, j, k) + w(i + 1, j, k)) / 2 * (u(i, j, k) + u(i, j, k + 1)) / 2, kc.d1[2]);
+        ay = ay + div_by(-(w(i, j, k - 1) + w(i, j + 1, k - 1)) / 2 * (v(i, j, k - 1) + v(i, j, k)) / 2
+                   + (w(i, j, k) + w(i, j + 1, k)) / 2 * (v(i, j, k) + v(i, j, k + 1)) / 2, kc.d1[2]);
         double t5 = (w(i, j, k - 1) + w(i, j, k)) / 2, t6 = (w(i, j, k) + w(i, j, k + 1)) / 2;
-        az = (-(u(i - 1, j, k) + u(i - 1, j, k + 1)) / 2 * (w(i - 1, j, k) + w(i, j, k)) / 2
-              + (u(i, j, k) + u(i, j, k + 1)) / 2 * (w(i, j, k) + w(i + 1, j, k)) / 2) / dX
-           + (-(v(i, j - 1, k) + v(i, j - 1, k + 1)) / 2 * (w(i, j - 1, k) + w(i, j, k)) / 2
-              + (v(i, j, k) + v(i, j, k + 1)) / 2 * (w(i, j, k) + w(i, j + 1, k)) / 2) / dY
-           + (-(t5 * t5) + t6 * t6) / dZ;
-        bx = bx + (u(i, j, k - 1) - 2 * u(i, j, k) + u(i, j, k + 1)) / (dZ * dZ);
-        by = by + (v(i, j, k - 1) - 2 * v(i, j, k) + v(i, j, k + 1)) / (dZ * dZ);
-        bz = (w(i - 1, j, k) - 2 * w(i, j, k) + w(i + 1, j, k)) / (dX * dX)
-           + (w(i, j - 1, k) - 2 * w(i, j, k) + w(i, j + 1, k)) / (dY * dY)
-           + (w(i, j, k - 1) - 2 * w(i, j, k) + w(i, j, k + 1)) / (dZ * dZ);
+        az = div_by(-(u(i - 1, j, k) + u(i - 1, j, k + 1)) / 2 * (w(i - 1, j, k) + w(i, j, k)) / 2
+              + (u(i, j, k) + u(i, j, k + 1)) / 2 * (w(i, j, k) + w(i + 1, j, k)) / 2, kc.d1[0])
+           + div_by(-(v(i, j - 1, k) + v(i, j - 1, k + 1)) / 2 * (w(i, j - 1, k) + w(i, j, k)) / 2
+              + (v(i, j, k) + v(i, j, k + 1)) / 2 * (w(i, j, k) + w(i, j + 1, k)) / 2, kc.d1[1])
+           + div_by(-(t5 * t5) + t6 * t6, kc.d1[2]);
+        bx = bx + div_by(u(i, j, k - 1) - 2 * u(i, j, k) + u(i, j, k + 1), kc.dd[2]);
+        by = by + div_by(v(i, j, k - 1) - 2 * v(i, j, k) + v(i, j, k + 1), kc.dd[2]);
+        bz = div_by(w(i - 1, j, k) - 2 * w(i, j, k) + w(i + 1, j, k), kc.dd[0])
+           + div_by(w(i, j - 1, k) - 2 * w(i, j, k) + w(i, j + 1, k), kc.dd[1])
+           + div_by(w(i, j, k - 1) - 2 * w(i, j, k) + w(i, j, k + 1), kc.dd[2]);
     }
     const double A[3] = {-ax, -ay, -az};
     const double B[3] = {a.vis * bx, a.vis * by, a.vis * bz};
@@ -1049,13 +1084,12 @@ __global__ void __launch_bounds__(256) k_momentum(MomArgs a, Geo g) {
     double *T0p[3] = {a.Tx0, a.Ty0, a.Tz0};
     const double *Fp[3] = {a.Fx, a.Fy, a.Fz};
     const double *Us[3] = {U, V, W};
-    const double d[3] = {dX, dY, dZ};
     const int hp[3] = {hix(g, i + 1, j, k), hix(g, i, j + 1, k), hix(g, i, j, k + 1)};
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
         double a0 = a.ab2_first ? A[c] : A0p[c][o];
         double t0 = a.ab2_first ? T[c] : T0p[c][o];
-        double gp = -dt * (-a.P[h] + a.P[hp[c]]) / d[c];
+        double gp = div_by(-dt * (-a.P[h] + a.P[hp[c]]), kc.d1[c]);
         double val;
         if (!a.ibm)
             val = Us[c][h] + gp + dt * (3.0 * A[c] - a0) / 2.0 + dt * B[c] / 2.0 + dt * (T[c] + t0) / 2.0 + dt * Fp[c][o];
@@ -1096,7 +1130,8 @@ struct IbmArgs {
     const double *mx, *my, *mu, *mv;
     const int *mcyl;
     int nm, ncomp, d3;
-    double dvol, dxn;
+    Recip dvol;                // cell volume
+    double dxn;
     const double *mvol;        // per marker: spreading volume (dX^3, or the ring's arc element)
     int accumulate;            // forcing iteration > 1: Fc += (Uc - Ub)/dt (smac.f90:1345-1353)
     const double *Uf[3];
@@ -1145,8 +1180,8 @@ __global__ void k_plane_weights(int comp, Geo g, double *wz) {
 
 // delta(x_e - X_m) of stencil cell (a, b, c) of marker m on plane n
 __device__ inline double ibm_delta(const IbmArgs &a, int comp, int m, int n, int ia, int jb, int kc) {
-    return a.d3 ? a.wx[comp][3 * m + ia] * a.wy[comp][3 * m + jb] * a.wz[comp][3 * (n - 1) + kc] / a.dvol
-                : a.wx[comp][3 * m + ia] * a.wy[comp][3 * m + jb] / a.dvol;
+    const double xy = a.wx[comp][3 * m + ia] * a.wy[comp][3 * m + jb];
+    return div_by(a.d3 ? xy * a.wz[comp][3 * (n - 1) + kc] : xy, a.dvol);
 }
 
 // interpolation at the markers and the marker force Fc = (Uc - Ub)/dt
@@ -1191,37 +1226,36 @@ __device__ inline double spread_at(const IbmArgs &a, const Geo &g, int comp, int
 
 // Spread the marker forces (with the periodic fold of ibm_PBM,
 // fenep.f90:2195-2205) and form Q = Ua + dt*f - dt*B/2 (ibm_predict,
-// fenep.f90:2229) for every interior cell.
+// fenep.f90:2229) for every interior cell; a thread per cell and component (the
+// few cells under a cylinder sum tens of entries each, in a serial FP64 chain).
 __global__ void k_ibm_spread_q(IbmArgs a, Geo g) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z + 1;
+    const int comp = blockIdx.z / g.nz, k = blockIdx.z - comp * g.nz + 1;
     if (i > g.nx || j > g.ny) return;
     const int o = qix(g, i, j, k), h = hix(g, i, j, k);
     int xs[2] = {i, -1}, ys[2] = {j, -1}, zs[2] = {k, -1};
     if (i == 1) xs[1] = g.nx + 1; else if (i == g.nx) xs[1] = 0;
     if (!g.walls) { if (j == 1) ys[1] = g.ny + 1; else if (j == g.ny) ys[1] = 0; }
     if (a.d3) { if (k == 1) zs[1] = g.nz + 1; else if (k == g.nz) zs[1] = 0; }
-    for (int comp = 0; comp < a.ncomp; ++comp) {
-        double fz = 0.0;
-        for (int zz = 0; zz < 2; ++zz) {
-            if (zs[zz] < 0) continue;
-            double fy = 0.0;
-            for (int yy = 0; yy < 2; ++yy) {
-                if (ys[yy] < 0) continue;
-                double fx = 0.0;
-                for (int xx = 0; xx < 2; ++xx) {
-                    if (xs[xx] < 0) continue;
-                    double v = spread_at(a, g, comp, xs[xx], ys[yy], zs[zz]);
-                    fx = xx == 0 ? v : fx + v;
-                }
-                fy = yy == 0 ? fx : fy + fx;
+    double fz = 0.0;
+    for (int zz = 0; zz < 2; ++zz) {
+        if (zs[zz] < 0) continue;
+        double fy = 0.0;
+        for (int yy = 0; yy < 2; ++yy) {
+            if (ys[yy] < 0) continue;
+            double fx = 0.0;
+            for (int xx = 0; xx < 2; ++xx) {
+                if (xs[xx] < 0) continue;
+                double v = spread_at(a, g, comp, xs[xx], ys[yy], zs[zz]);
+                fx = xx == 0 ? v : fx + v;
             }
-            fz = zz == 0 ? fy : fz + fy;
+            fy = yy == 0 ? fx : fy + fx;
         }
-        const double dt = g.dt;
-        a.Q[comp][o] = a.Ua[comp][h] + dt * fz - dt * a.B[comp][o] / 2;
+        fz = zz == 0 ? fy : fz + fy;
     }
+    const double dt = g.dt;
+    a.Q[comp][o] = a.Ua[comp][h] + dt * fz - dt * a.B[comp][o] / 2;
 }
 
 // drag of each cylinder: -sum(Fc) * dv per component.  Stage 1: block
@@ -1269,31 +1303,31 @@ __global__ void k_drag_final(const double *part, int nz, int ncomp, const double
 // ---------------------------------------------------------------------------
 // Poisson right-hand side (fenep.f90:1547-1555) and projection (1562-1604).
 
-__global__ void k_poisson_rhs(const double *Up, const double *Vp, const double *Wp, double *Q, Geo g) {
+__global__ void k_poisson_rhs(const double *Up, const double *Vp, const double *Wp, double *Q, Geo g, GridRecip kc) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z + 1;
     if (i > g.nx || j > g.ny) return;
-    double s = (-Up[hix(g, i - 1, j, k)] + Up[hix(g, i, j, k)]) / g.dx + (-Vp[hix(g, i, j - 1, k)] + Vp[hix(g, i, j, k)]) / g.dy;
-    if (g.dim == 3) s = s + (-Wp[hix(g, i, j, k - 1)] + Wp[hix(g, i, j, k)]) / g.dz;
-    Q[qix(g, i, j, k)] = s / g.dt;
+    double s = div_by(-Up[hix(g, i - 1, j, k)] + Up[hix(g, i, j, k)], kc.d1[0]) + div_by(-Vp[hix(g, i, j - 1, k)] + Vp[hix(g, i, j, k)], kc.d1[1]);
+    if (g.dim == 3) s = s + div_by(-Wp[hix(g, i, j, k - 1)] + Wp[hix(g, i, j, k)], kc.d1[2]);
+    Q[qix(g, i, j, k)] = div_by(s, kc.dt);
 }
 
 __global__ void k_march(double *U, double *V, double *W, double *P, const double *Up, const double *Vp,
-                        const double *Wp, const double *Phi, Geo g, double pc) {
+                        const double *Wp, const double *Phi, Geo g, GridRecip kc, double pc) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z + 1;
     if (i > g.nx || j > g.ny) return;
     const int h = hix(g, i, j, k);
-    const double dt = g.dt, dX = g.dx, dY = g.dy, dZ = g.dz;
+    const double dt = g.dt;
     const double ph = Phi[h];
-    U[h] = Up[h] - dt * (-ph + Phi[hix(g, i + 1, j, k)]) / dX;
-    V[h] = Vp[h] - dt * (-ph + Phi[hix(g, i, j + 1, k)]) / dY;
-    if (g.dim == 3) W[h] = Wp[h] - dt * (-ph + Phi[hix(g, i, j, k + 1)]) / dZ;
-    double lap = (Phi[hix(g, i - 1, j, k)] - 2 * ph + Phi[hix(g, i + 1, j, k)]) / (dX * dX)
-               + (Phi[hix(g, i, j - 1, k)] - 2 * ph + Phi[hix(g, i, j + 1, k)]) / (dY * dY);
-    if (g.dim == 3) lap = lap + (Phi[hix(g, i, j, k - 1)] - 2 * ph + Phi[hix(g, i, j, k + 1)]) / (dZ * dZ);
+    U[h] = Up[h] - div_by(dt * (-ph + Phi[hix(g, i + 1, j, k)]), kc.d1[0]);
+    V[h] = Vp[h] - div_by(dt * (-ph + Phi[hix(g, i, j + 1, k)]), kc.d1[1]);
+    if (g.dim == 3) W[h] = Wp[h] - div_by(dt * (-ph + Phi[hix(g, i, j, k + 1)]), kc.d1[2]);
+    double lap = div_by(Phi[hix(g, i - 1, j, k)] - 2 * ph + Phi[hix(g, i + 1, j, k)], kc.dd[0])
+               + div_by(Phi[hix(g, i, j - 1, k)] - 2 * ph + Phi[hix(g, i, j + 1, k)], kc.dd[1]);
+    if (g.dim == 3) lap = lap + div_by(Phi[hix(g, i, j, k - 1)] - 2 * ph + Phi[hix(g, i, j, k + 1)], kc.dd[2]);
     P[h] = P[h] + ph - pc * lap;
 }
 
@@ -1411,94 +1445,59 @@ inline dim3 cell_grid(const Geo &g, dim3 blk) {
     return dim3((g.nx + blk.x - 1) / blk.x, (g.ny + blk.y - 1) / blk.y, g.nz);
 }
 
-cudaError_t bc(double *A, const Geo &g, int kind, cudaStream_t s) {
-    long n = halo_count(g) + ((kind == BC_V && g.walls) ? (long)g.nx * g.nz : 0);
-    k_bc_scalar<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(A, g, kind); count_launch();
+cudaError_t bc_set(const Geo &g, int n, double *const *A, const int *kind, cudaStream_t s) {
+    BcSetD b{};
+    b.n = n;
+    bool v = false;
+    for (int f = 0; f < n; ++f) {
+        b.A[f] = A[f];
+        b.kind[f] = kind[f];
+        v = v || kind[f] == BC_V;
+    }
+    const long t = halo_count(g) + (v && g.walls ? (long)g.nx * g.nz : 0);
+    k_bc_set64<<<(unsigned)((t + 255) / 256), 256, 0, s>>>(b, g); count_launch();
     return cudaGetLastError();
 }
 
-// Periodic spectral solve (fft_solve): src interior -> dst halo interior.
-cudaError_t fft_solve_periodic(Dev &d, const double *src, double *dst, double lhs0, double lhs1, cudaStream_t s) {
+cudaError_t bc(double *A, const Geo &g, int kind, cudaStream_t s) { return bc_set(g, 1, &A, &kind, s); }
+
+// U, V, (W,) P
+cudaError_t bc_state(Dev &d, cudaStream_t s) {
+    double *A3[4] = {d.U, d.V, d.W, d.P}, *A2[3] = {d.U, d.V, d.P};
+    const int k3[4] = {BC_U, BC_V, BC_W, BC_P}, k2[3] = {BC_U, BC_V, BC_P};
+    return d.g.dim == 3 ? bc_set(d.g, 4, A3, k3, s) : bc_set(d.g, 3, A2, k2, s);
+}
+
+// The spectral solves of nb systems (interior right-hand sides -> halo fields)
+// in one launch per pass: periodic (fft_solve), or with walls FFT(x, z) of rows
+// 1..NY, the tridiagonal systems in y over rows 0..NY+1 and the inverse FFT of
+// all NY+2 rows.  sys: 0 U/W, 1 V, 2 P; top: the top ghost value of mode (0, 0).
+cudaError_t solve_batch(Dev &d, int nb, const double *const *src, double *const *dst, const int *sys, const double *top,
+                        cudaStream_t s) {
     const Geo &g = d.g;
-    const int nx = g.nx, ny = g.ny, nz = g.nz, nxh = nx / 2 + 1;
-    // x forward
-    {
-        int tpp = std::max(nx / 2, 1), ppc = std::max(1, 256 / tpp);
-        int npp = ny / 2, total = npp * nz;
-        size_t smem = (size_t)ppc * 2 * nx * sizeof(Cx<double>);
-        k_fft_x_fwd<double, double><<<(total + ppc - 1) / ppc, ppc * tpp, smem, s>>>(src, d.H, nx, ny, 1, ny, npp, nz, d.twx_r, d.twx_i); count_launch();
+    Batch<const double *> in{};
+    Batch<XOutD> out{};
+    Batch<WallItem<double>> items{};
+    for (int q = 0; q < nb; ++q) {
+        in.p[q] = src[q];
+        out.p[q] = XOutD{dst[q]};
+        items.p[q] = WallItem<double>{sys[q], d.walltab[sys[q]], top[q]};
     }
-    DivideSpec none{};
-    // y forward (line along y: stride nxh, sets = k planes)
-    {
-        int tx = std::max(1, std::min(32, 2048 / ny));
-        size_t smem = (size_t)2 * ny * tx * sizeof(Cx<double>);
-        dim3 grid((nxh + tx - 1) / tx, nz);
-        k_fft_lines<double><<<grid, 256, smem, s>>>(d.H, ny, nxh, nxh, nxh * ny, tx, d.twy_r, d.twy_i, -1, 0, none); count_launch();
-    }
-    // z forward + divide + z inverse (line along z: stride nxh*ny, sets = j)
-    {
-        DivideSpec dv{d.kx2, d.ky2, d.kz2, lhs0, lhs1, (double)nx * ny * nz, 1};
-        int tx = std::max(1, std::min(32, 2048 / nz));
-        size_t smem = (size_t)2 * nz * tx * sizeof(Cx<double>);
-        dim3 grid((nxh + tx - 1) / tx, ny);
-        k_fft_lines<double><<<grid, 256, smem, s>>>(d.H, nz, nxh * ny, nxh, nxh, tx, d.twz_r, d.twz_i, -1, 1, dv); count_launch();
-    }
-    // y inverse
-    {
-        int tx = std::max(1, std::min(32, 2048 / ny));
-        size_t smem = (size_t)2 * ny * tx * sizeof(Cx<double>);
-        dim3 grid((nxh + tx - 1) / tx, nz);
-        k_fft_lines<double><<<grid, 256, smem, s>>>(d.H, ny, nxh, nxh, nxh * ny, tx, d.twy_r, d.twy_i, +1, 0, none); count_launch();
-    }
-    // x inverse
-    {
-        int tpp = std::max(nx / 2, 1), ppc = std::max(1, 256 / tpp);
-        int npp = ny / 2, total = npp * nz;
-        size_t smem = (size_t)ppc * 2 * nx * sizeof(Cx<double>);
-        k_fft_x_inv<double, XOutD><<<(total + ppc - 1) / ppc, ppc * tpp, smem, s>>>(d.H, XOutD{dst, nullptr}, nx, ny, npp, nz, 1, g.sx, g.sy, d.twx_r, d.twx_i); count_launch();
+    if (!g.walls) {
+        const bool p = sys[0] == SYS_P;
+        fft_solve_passes<double, double, XOutD>(nb, in, d.H, d.nspec, out, g.nx, g.ny, g.nz, 1, g.sx, g.sy, 0, d.twx_r,
+                                                d.twx_i, d.twy_r, d.twy_i, d.twz_r, d.twz_i, d.kx2, d.ky2, d.kz2,
+                                                p ? 0.0 : 1.0, p ? -1.0 : d.ph.dt * d.ph.beta / d.ph.re / 2.0, s);
+    } else {
+        wall_solve_passes<double, double, XOutD>(nb, in, d.H, d.H2, d.nspec, out, g, d.twx_r, d.twx_i, d.twz_r, d.twz_i,
+                                                 wall_spec(g, d.ph, d.kx2, d.kz2), items, s);
     }
     return cudaGetLastError();
 }
 
-// Wall-bounded solve: FFT(x, z) of rows 1..NY, tridiagonal in y over rows
-// 0..NY+1, inverse FFT of all NY+2 rows into dst (halo rows 0..NY+1).
-cudaError_t wall_solve(Dev &d, const double *src, double *dst, int sys, double uwall, cudaStream_t s) {
-    const Geo &g = d.g;
-    const int nx = g.nx, ny = g.ny, nz = g.nz, nxh = nx / 2 + 1, n = ny + 2;
-    DivideSpec none{};
-    {
-        int tpp = std::max(nx / 2, 1), ppc = std::max(1, 256 / tpp);
-        int npp = ny / 2, total = npp * nz;
-        size_t smem = (size_t)ppc * 2 * nx * sizeof(Cx<double>);
-        k_fft_x_fwd<double, double><<<(total + ppc - 1) / ppc, ppc * tpp, smem, s>>>(src, d.H, nx, ny, 1, ny, npp, nz, d.twx_r, d.twx_i); count_launch();
-    }
-    if (nz > 1) {
-        int tx = std::max(1, std::min(32, 2048 / nz));
-        size_t smem = (size_t)2 * nz * tx * sizeof(Cx<double>);
-        dim3 grid((nxh + tx - 1) / tx, ny);
-        k_fft_lines<double><<<grid, 256, smem, s>>>(d.H, nz, nxh * ny, nxh, nxh, tx, d.twz_r, d.twz_i, -1, 0, none); count_launch();
-    }
-    {
-        WallSpec w{d.kx2, d.kz2, d.ph.dt, d.ph.beta, d.ph.re, g.dy, (double)nx * nz, uwall, sys};
-        int tx = 16;
-        size_t smem = (size_t)n * tx * (sizeof(Cx<double>) + sizeof(double));
-        dim3 grid((nxh + tx - 1) / tx, nz);
-        k_wall_tdma<double><<<grid, 128, smem, s>>>(d.H, d.H2, ny, nxh, tx, w); count_launch();
-    }
-    if (nz > 1) {
-        int tx = std::max(1, std::min(32, 2048 / nz));
-        size_t smem = (size_t)2 * nz * tx * sizeof(Cx<double>);
-        dim3 grid((nxh + tx - 1) / tx, n);
-        k_fft_lines<double><<<grid, 256, smem, s>>>(d.H2, nz, nxh * n, nxh, nxh, tx, d.twz_r, d.twz_i, +1, 0, none); count_launch();
-    }
-    {
-        int tpp = std::max(nx / 2, 1), ppc = std::max(1, 256 / tpp);
-        int npp = n / 2, total = npp * nz;
-        size_t smem = (size_t)ppc * 2 * nx * sizeof(Cx<double>);
-        k_fft_x_inv<double, XOutD><<<(total + ppc - 1) / ppc, ppc * tpp, smem, s>>>(d.H2, XOutD{dst, nullptr}, nx, n, npp, nz, 0, g.sx, g.sy, d.twx_r, d.twx_i); count_launch();
-    }
-    return cudaGetLastError();
+cudaError_t solve_one(Dev &d, const double *src, double *dst, int sys, cudaStream_t s) {
+    const double top = 0.0;
+    return solve_batch(d, 1, &src, &dst, &sys, &top, s);
 }
 
 cudaError_t reduce_sumsq(const double *A, int n, double *part, double *scal, int slot, int mode, int *flag, double eps,
@@ -1567,7 +1566,6 @@ cudaError_t remove_mean(Dev &d, double *A, int n, cudaStream_t s) {
 cudaError_t init_kernels_fp64() {
     const int big = 200 * 1024;
     F8_CUDA_RET(cudaFuncSetAttribute(k_fft_lines<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    F8_CUDA_RET(cudaFuncSetAttribute(k_wall_tdma<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     F8_CUDA_RET(cudaFuncSetAttribute(k_fft_x_fwd<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     F8_CUDA_RET(cudaFuncSetAttribute(k_fft_x_inv<double, XOutD>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     return cudaSuccess;
@@ -1575,10 +1573,7 @@ cudaError_t init_kernels_fp64() {
 
 cudaError_t bc_all_state_fp64(Dev &d, cudaStream_t s) {
     cudaError_t e;
-    if ((e = bc(d.U, d.g, BC_U, s))) return e;
-    if ((e = bc(d.V, d.g, BC_V, s))) return e;
-    if (d.g.dim == 3 && (e = bc(d.W, d.g, BC_W, s))) return e;
-    if ((e = bc(d.P, d.g, BC_P, s))) return e;
+    if ((e = bc_state(d, s))) return e;
     long n = halo_count(d.g);
     k_bc_c_pet<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d.C, d.fpet, d.g, d.ncomp, d.cs, d.ph.lp2); count_launch();
     k_pet_all<<<(d.cs + 255) / 256, 256, 0, s>>>(d.C, d.fpet, d.ncomp, d.cs, d.ph.lp2); count_launch();
@@ -1588,8 +1583,7 @@ cudaError_t bc_all_state_fp64(Dev &d, cudaStream_t s) {
 cudaError_t bc_field(double *A, const Geo &g, int kind, cudaStream_t s) { return bc(A, g, kind, s); }
 
 cudaError_t helmholtz_solve_fp64(Dev &d, int comp, const double *src, double *dst, cudaStream_t s) {
-    if (!d.g.walls) return fft_solve_periodic(d, src, dst, 1.0, d.ph.dt * d.ph.beta / d.ph.re / 2.0, s);
-    return wall_solve(d, src, dst, comp == 1 ? SYS_V : SYS_U, 0.0, s);
+    return solve_one(d, src, dst, comp == 1 ? SYS_V : SYS_U, s);
 }
 
 cudaError_t sor_solve_fp64(Dev &d, const double *Q, double *Phi, double *E, double omega, double eps, int itrmax,
@@ -1600,19 +1594,25 @@ cudaError_t sor_solve_fp64(Dev &d, const double *Q, double *Phi, double *E, doub
 cudaError_t remove_mean_fp64(Dev &d, double *A, int n, cudaStream_t s) { return remove_mean(d, A, n, s); }
 
 cudaError_t poisson_solve_fp64(Dev &d, const double *src, double *dst, cudaStream_t s) {
-    if (!d.g.walls) return fft_solve_periodic(d, src, dst, 0.0, -1.0, s);
-    return wall_solve(d, src, dst, SYS_P, 0.0, s);
+    return solve_one(d, src, dst, SYS_P, s);
+}
+
+cudaError_t wall_tables_fp64(Dev &d, cudaStream_t s) {
+    const Geo &g = d.g;
+    for (int sys = 0; sys < 3; ++sys)
+        wall_table<double>(d.walltab[sys], g.ny, g.nx / 2 + 1, g.nz, wall_spec(g, d.ph, d.kx2, d.kz2), sys, s);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_poisson_rhs(Dev &d, double *out, cudaStream_t s) {
     dim3 blk(32, 8);
-    k_poisson_rhs<<<cell_grid(d.g, blk), blk, 0, s>>>(d.Up, d.Vp, d.Wp, out, d.g); count_launch();
+    k_poisson_rhs<<<cell_grid(d.g, blk), blk, 0, s>>>(d.Up, d.Vp, d.Wp, out, d.g, grid_recip(d.g)); count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_march(Dev &d, cudaStream_t s) {
     dim3 blk(32, 8);
-    k_march<<<cell_grid(d.g, blk), blk, 0, s>>>(d.U, d.V, d.W, d.P, d.Up, d.Vp, d.Wp, d.Phi, d.g,
+    k_march<<<cell_grid(d.g, blk), blk, 0, s>>>(d.U, d.V, d.W, d.P, d.Up, d.Vp, d.Wp, d.Phi, d.g, grid_recip(d.g),
                                                 d.ph.dt * d.ph.beta / d.ph.re / 2.0); count_launch();
     return cudaGetLastError();
 }
@@ -1697,8 +1697,8 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
     {
         dim3 blk(32, 8);
         dim3 grd = cell_grid(g, blk);
-        if (d3) { k_momentum<3><<<grd, blk, 0, s>>>(ma, g); count_launch(); }
-        else { k_momentum<2><<<grd, blk, 0, s>>>(ma, g); count_launch(); }
+        if (d3) { k_momentum<3><<<grd, blk, 0, s>>>(ma, g, grid_recip(g)); count_launch(); }
+        else { k_momentum<2><<<grd, blk, 0, s>>>(ma, g, grid_recip(g)); count_launch(); }
         if ((e = cudaGetLastError())) return e;
     }
     mark(3);
@@ -1706,16 +1706,14 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
     // forcing iterations (smac.f90:1607-1611) each further iteration
     // interpolates from the last Helmholtz solution, adds to the marker
     // forces, spreads them and solves again
-    double *outs[3] = {d.Up, d.Vp, d.Wp};
-    const double lhs1 = d.ph.dt * d.ph.beta / d.ph.re / 2.0;
+    double *outs[3] = {d.Up, d.Vp, d.Wp}, *ua[3] = {d.Ua, d.Va, d.Wa};
+    const int nv = d3 ? 3 : 2, kinds[3] = {BC_U, BC_V, BC_W};
     IbmArgs ia{};
     if (o.ibm) {
-        if ((e = bc(d.Ua, g, BC_U, s))) return e;
-        if ((e = bc(d.Va, g, BC_V, s))) return e;
-        if (d3 && (e = bc(d.Wa, g, BC_W, s))) return e;
+        if ((e = bc_set(g, nv, ua, kinds, s))) return e;
         ia.mx = d.mx; ia.my = d.my; ia.mu = d.mu; ia.mv = d.mv; ia.mcyl = d.mcyl;
         ia.nm = d.nm; ia.ncomp = d3 ? 3 : 2; ia.d3 = d3;
-        ia.dvol = d3 ? (g.dx * g.dy) * g.dz : g.dx * g.dy;
+        ia.dvol = recip(d3 ? (g.dx * g.dy) * g.dz : g.dx * g.dy);
         ia.dxn = d3 ? g.dx * g.dx * g.dx : g.dx * g.dx;
         ia.mvol = d.mvol;
         for (int c = 0; c < 3; ++c) {
@@ -1738,30 +1736,26 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
             dim3 gi((d.nm + 127) / 128, g.nz, ia.ncomp);
             k_ibm_interp<<<gi, 128, 0, s>>>(ia, g); count_launch();
             dim3 blk(32, 8);
-            k_ibm_spread_q<<<cell_grid(g, blk), blk, 0, s>>>(ia, g); count_launch();
+            dim3 gs = cell_grid(g, blk);
+            gs.z *= ia.ncomp;
+            k_ibm_spread_q<<<gs, blk, 0, s>>>(ia, g); count_launch();
             if (r == repeats - 1 && drag_out_dev) F8_CUDA_RET(launch_drag(d, drag_out_dev, s));
             if ((e = cudaGetLastError())) return e;
         }
         if (r == 0) mark(4);
-        for (int c = 0; c < (d3 ? 3 : 2); ++c) {
-            if (!g.walls) e = fft_solve_periodic(d, d.Q[c], outs[c], 1.0, lhs1, s);
-            else e = wall_solve(d, d.Q[c], outs[c], c == 1 ? SYS_V : SYS_U, c == 0 ? g.uwall : 0.0, s);
-            if (e) return e;
-        }
-        if ((e = bc(d.Up, g, BC_U, s))) return e;
-        if ((e = bc(d.Vp, g, BC_V, s))) return e;
-        if (d3 && (e = bc(d.Wp, g, BC_W, s))) return e;
+        const int sys[3] = {SYS_U, SYS_V, SYS_U};
+        const double top[3] = {2 * g.uwall, 0.0, 0.0};
+        if ((e = solve_batch(d, nv, d.Q, outs, sys, top, s))) return e;
+        if ((e = bc_set(g, nv, outs, kinds, s))) return e;
     }
     mark(5);
     // 5. Poisson
     {
         dim3 blk(32, 8);
-        k_poisson_rhs<<<cell_grid(g, blk), blk, 0, s>>>(d.Up, d.Vp, d.Wp, d.Q[0], g); count_launch();
+        k_poisson_rhs<<<cell_grid(g, blk), blk, 0, s>>>(d.Up, d.Vp, d.Wp, d.Q[0], g, grid_recip(g)); count_launch();
     }
     if (o.poisson == 0) {
-        if (!g.walls) e = fft_solve_periodic(d, d.Q[0], d.Phi, 0.0, -1.0, s);
-        else e = wall_solve(d, d.Q[0], d.Phi, SYS_P, 0.0, s);
-        if (e) return e;
+        if ((e = solve_one(d, d.Q[0], d.Phi, SYS_P, s))) return e;
         if ((e = bc(d.Phi, g, BC_P, s))) return e;
         *sor_iters = -1;
     } else {
@@ -1771,14 +1765,11 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
     // 6. projection and pressure update
     {
         dim3 blk(32, 8);
-        k_march<<<cell_grid(g, blk), blk, 0, s>>>(d.U, d.V, d.W, d.P, d.Up, d.Vp, d.Wp, d.Phi, g,
+        k_march<<<cell_grid(g, blk), blk, 0, s>>>(d.U, d.V, d.W, d.P, d.Up, d.Vp, d.Wp, d.Phi, g, grid_recip(g),
                                                   d.ph.dt * d.ph.beta / d.ph.re / 2.0); count_launch();
         if ((e = cudaGetLastError())) return e;
     }
-    if ((e = bc(d.U, g, BC_U, s))) return e;
-    if ((e = bc(d.V, g, BC_V, s))) return e;
-    if (d3 && (e = bc(d.W, g, BC_W, s))) return e;
-    if ((e = bc(d.P, g, BC_P, s))) return e;
+    if ((e = bc_state(d, s))) return e;
     if (o.c_mid) F8_CUDA_RET(cudaMemcpyAsync(o.c_mid, d.C, (size_t)d.ncomp * d.cs * sizeof(double),
                                              cudaMemcpyDeviceToDevice, s));
     if (o.polymer && g.walls) {

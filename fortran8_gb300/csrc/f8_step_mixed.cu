@@ -1880,76 +1880,26 @@ inline dim3 cell_grid_m(const Geo &g, dim3 blk) {
 }
 
 // ---------------------------------------------------------------------------
-// FP32 spectral solves.  src (interior, FP32 or FP64) -> dst (FP64 halo
-// interior; dst = base + result when base is given).
-template <typename TS>
-cudaError_t solve_periodic_mp(Dev &d, const TS *src, XOutF out, double lhs0, double lhs1, cudaStream_t s) {
+// FP32 spectral solves of up to three right-hand sides (interior order) by the
+// line passes of f8_fft.cuh: 2D, and the 3D grids without a fused plane kernel.
+cudaError_t solve_periodic_mp(Dev &d, int nb, Batch<const float *> src, Batch<XOutF> out, double lhs0, double lhs1,
+                              cudaStream_t s) {
     const Geo &g = d.g;
-    const int nx = g.nx, ny = g.ny, nz = g.nz, nxh = nx / 2 + 1;
-    const int tpp = std::max(nx / 2, 1), ppc = std::max(1, 256 / tpp);
-    const size_t smx = (size_t)ppc * 2 * nx * sizeof(Cx<float>);
-    {
-        int npp = ny / 2, total = npp * nz;
-        k_fft_x_fwd<float, TS><<<(total + ppc - 1) / ppc, ppc * tpp, smx, s>>>(src, d.Hf, nx, ny, 1, ny, npp, nz, d.twxf_r, d.twxf_i); count_launch();
-    }
-    DivideSpec none{};
-    const int txy = std::max(1, std::min(32, 4096 / ny));
-    const size_t smy = (size_t)2 * ny * txy * sizeof(Cx<float>);
-    if (nz == 1) {
-        // 2D: the y lines transform, divide and transform back in one pass
-        DivideSpec dv{d.kx2, d.ky2, d.kz2, lhs0, lhs1, (double)nx * ny * nz, 0};
-        k_fft_lines<float><<<dim3((nxh + txy - 1) / txy, nz), 256, smy, s>>>(d.Hf, ny, nxh, nxh, nxh * ny, txy, d.twyf_r, d.twyf_i, -1, 1, dv); count_launch();
-        int npp = ny / 2, total = npp * nz;
-        k_fft_x_inv<float, XOutF><<<(total + ppc - 1) / ppc, ppc * tpp, smx, s>>>(d.Hf, out, nx, ny, npp, nz, 1, g.sx, g.sy, d.twxf_r, d.twxf_i); count_launch();
-        return cudaGetLastError();
-    }
-    k_fft_lines<float><<<dim3((nxh + txy - 1) / txy, nz), 256, smy, s>>>(d.Hf, ny, nxh, nxh, nxh * ny, txy, d.twyf_r, d.twyf_i, -1, 0, none); count_launch();
-    {
-        DivideSpec dv{d.kx2, d.ky2, d.kz2, lhs0, lhs1, (double)nx * ny * nz, 1};
-        const int txz = std::max(1, std::min(32, 4096 / nz));
-        const size_t smz = (size_t)2 * nz * txz * sizeof(Cx<float>);
-        k_fft_lines<float><<<dim3((nxh + txz - 1) / txz, ny), 256, smz, s>>>(d.Hf, nz, nxh * ny, nxh, nxh, txz, d.twzf_r, d.twzf_i, -1, 1, dv); count_launch();
-    }
-    k_fft_lines<float><<<dim3((nxh + txy - 1) / txy, nz), 256, smy, s>>>(d.Hf, ny, nxh, nxh, nxh * ny, txy, d.twyf_r, d.twyf_i, +1, 0, none); count_launch();
-    {
-        int npp = ny / 2, total = npp * nz;
-        k_fft_x_inv<float, XOutF><<<(total + ppc - 1) / ppc, ppc * tpp, smx, s>>>(d.Hf, out, nx, ny, npp, nz, 1, g.sx, g.sy, d.twxf_r, d.twxf_i); count_launch();
-    }
+    fft_solve_passes<float, float, XOutF>(nb, src, d.Hf, d.nspec, out, g.nx, g.ny, g.nz, 1, g.sx, g.sy, 0, d.twxf_r,
+                                          d.twxf_i, d.twyf_r, d.twyf_i, d.twzf_r, d.twzf_i, d.kx2, d.ky2, d.kz2, lhs0,
+                                          lhs1, s);
     return cudaGetLastError();
 }
 
-template <typename TS>
-cudaError_t solve_walls_mp(Dev &d, const TS *src, XOutF out, int sys, cudaStream_t s) {
+cudaError_t solve_walls_mp(Dev &d, int nb, Batch<const float *> src, Batch<XOutF> out, const int (&sys)[3],
+                           cudaStream_t s) {
     const Geo &g = d.g;
-    const int nx = g.nx, ny = g.ny, nz = g.nz, nxh = nx / 2 + 1, n = ny + 2;
-    const int tpp = std::max(nx / 2, 1), ppc = std::max(1, 256 / tpp);
-    const size_t smx = (size_t)ppc * 2 * nx * sizeof(Cx<float>);
-    {
-        int npp = ny / 2, total = npp * nz;
-        k_fft_x_fwd<float, TS><<<(total + ppc - 1) / ppc, ppc * tpp, smx, s>>>(src, d.Hf, nx, ny, 1, ny, npp, nz, d.twxf_r, d.twxf_i); count_launch();
-    }
-    DivideSpec none{};
-    const int txz = std::max(1, std::min(32, 4096 / nz));
-    const size_t smz = (size_t)2 * nz * txz * sizeof(Cx<float>);
-    if (nz > 1) {
-        k_fft_lines<float><<<dim3((nxh + txz - 1) / txz, ny), 256, smz, s>>>(d.Hf, nz, nxh * ny, nxh, nxh, txz, d.twzf_r, d.twzf_i, -1, 0, none); count_launch();
-    }
-    {
-        WallSpec w{d.kx2, d.kz2, d.ph.dt, d.ph.beta, d.ph.re, g.dy, (double)nx * nz, 0.0, sys};
-        const int tx = 32;
-        const size_t sm = (size_t)n * tx * (sizeof(Cx<float>) + sizeof(float));
-        k_wall_tdma<float><<<dim3((nxh + tx - 1) / tx, nz), 128, sm, s>>>(d.Hf, d.H2f, ny, nxh, tx, w); count_launch();
-    }
-    if (nz > 1) {
-        k_fft_lines<float><<<dim3((nxh + txz - 1) / txz, n), 256, smz, s>>>(d.H2f, nz, nxh * n, nxh, nxh, txz, d.twzf_r, d.twzf_i, +1, 0, none); count_launch();
-    }
-    {
-        int npp = n / 2, total = npp * nz;
-        k_fft_x_inv<float, XOutF><<<(total + ppc - 1) / ppc, ppc * tpp, smx, s>>>(d.H2f, out, nx, n, npp, nz, 0, g.sx, g.sy, d.twxf_r, d.twxf_i); count_launch();
-    }
+    Batch<WallItem<float>> items{};
+    for (int q = 0; q < nb; ++q) items.p[q] = WallItem<float>{sys[q], d.walltabf[sys[q]], 0.0};
+    wall_solve_passes<float, float, XOutF>(nb, src, d.Hf, d.H2f, d.nspec, out, g, d.twxf_r, d.twxf_i, d.twzf_r, d.twzf_i,
+                                           wall_spec(g, d.ph, d.kx2, d.kz2), items, s);
     return cudaGetLastError();
 }
-
 
 // Fused path: transposing x pass, one CTA per kx for the (z, y) plane,
 // transposing inverse x pass.
@@ -2072,12 +2022,12 @@ cudaError_t solve_walls_fused(Dev &d, const TS *src, XOutF out, int sys, cudaStr
 
 cudaError_t solve_periodic_f(Dev &d, const float *src, XOutF out, double lhs0, double lhs1, cudaStream_t s) {
     if (d.fused_planes) return solve_periodic_fused<float>(d, src, out, (float)lhs0, (float)lhs1, s);
-    return solve_periodic_mp<float>(d, src, out, lhs0, lhs1, s);
+    return solve_periodic_mp(d, 1, {{src}}, {{out}}, lhs0, lhs1, s);
 }
 
 cudaError_t solve_walls_f(Dev &d, const float *src, XOutF out, int sys, cudaStream_t s) {
     if (d.fused_planes) return solve_walls_fused<float>(d, src, out, sys, s);
-    return solve_walls_mp<float>(d, src, out, sys, s);
+    return solve_walls_mp(d, 1, {{src}}, {{out}}, {sys}, s);
 }
 
 cudaError_t sor_solve_m(Dev &d, const StepOpts &o, int *iters, cudaStream_t s) {
@@ -2128,40 +2078,39 @@ cudaError_t mixed_solve_walls(Dev &d, const float *src, float *dst, float *lo, i
     return solve_walls_f(d, src, XOutF{dst, lo, mode}, sys, s);
 }
 
-// the three Helmholtz solves of one step (dst[c] = v of component c, mode 0),
-// the V and W solves forked onto the side streams with their own spectra on
-// the fused spectral path, as in the forward step
-cudaError_t mixed_helmholtz3(Dev &d, const float *const src[3], float *const dst[3], cudaStream_t s) {
+// The Helmholtz solves of n velocity components (dst[c] = v, mode 0).  On the
+// fused spectral path they are independent branches: V and W run on side
+// streams with their own spectra, forked from and joined to the stream
+// (parallel branches of the captured graph), so their x transforms fill the SMs
+// that one solve's kernels leave idle.  The line passes take all components in
+// one launch each.
+cudaError_t mixed_helmholtz(Dev &d, int n, const float *const src[3], float *const dst[3], cudaStream_t s) {
     const Geo &g = d.g;
     const double lhs1 = d.ph.dt * d.ph.beta / d.ph.re / 2.0;
-    const bool branches = d.fused_planes && d.aux[0] && d.aux[1];
-    if (branches) {
-        F8_CUDA_RET(cudaEventRecord(d.ev_fork, s));
-        for (int b = 0; b < 2; ++b) F8_CUDA_RET(cudaStreamWaitEvent(d.aux[b], d.ev_fork, 0));
+    if (!d.fused_planes) {
+        Batch<const float *> in{};
+        Batch<XOutF> out{};
+        for (int c = 0; c < n; ++c) {
+            in.p[c] = src[c];
+            out.p[c] = XOutF{dst[c], nullptr, 0};
+        }
+        if (!g.walls) return solve_periodic_mp(d, n, in, out, 1.0, lhs1, s);
+        return solve_walls_mp(d, n, in, out, {SYS_U, SYS_V, SYS_U}, s);
     }
-    for (int c = 0; c < 3; ++c) {
+    F8_CUDA_RET(cudaEventRecord(d.ev_fork, s));
+    for (int b = 0; b < 2; ++b) F8_CUDA_RET(cudaStreamWaitEvent(d.aux[b], d.ev_fork, 0));
+    for (int c = 0; c < n; ++c) {
         const XOutF out{dst[c], nullptr, 0};
-        const int sys = c == 1 ? SYS_V : SYS_U;
-        cudaError_t e;
-        if (branches) {
-            cudaStream_t sc = c == 0 ? s : d.aux[c - 1];
-            float *spec = c == 0 ? d.Hf : d.HfB[c - 1];
-            if (!g.walls) e = solve_periodic_fused<float>(d, src[c], out, 1.0f, (float)lhs1, sc, spec);
-            else e = solve_walls_fused<float>(d, src[c], out, sys, sc, spec);
-        } else if (!g.walls) {
-            e = solve_periodic_f(d, src[c], out, 1.0, lhs1, s);
-        } else {
-            e = solve_walls_f(d, src[c], out, sys, s);
-        }
-        if (e) return e;
+        cudaStream_t sc = c == 0 ? s : d.aux[c - 1];
+        float *spec = c == 0 ? d.Hf : d.HfB[c - 1];
+        if (!g.walls) F8_CUDA_RET(solve_periodic_fused<float>(d, src[c], out, 1.0f, (float)lhs1, sc, spec));
+        else F8_CUDA_RET(solve_walls_fused<float>(d, src[c], out, c == 1 ? SYS_V : SYS_U, sc, spec));
     }
-    if (branches) {
-        for (int b = 0; b < 2; ++b) {
-            F8_CUDA_RET(cudaEventRecord(d.ev_join[b], d.aux[b]));
-            F8_CUDA_RET(cudaStreamWaitEvent(s, d.ev_join[b], 0));
-        }
+    for (int b = 0; b < 2; ++b) {
+        F8_CUDA_RET(cudaEventRecord(d.ev_join[b], d.aux[b]));
+        F8_CUDA_RET(cudaStreamWaitEvent(s, d.ev_join[b], 0));
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 // defect rd = (rh + rl) - L_h phi of an FP32 pressure-type field in df64, the
@@ -2221,10 +2170,16 @@ cudaError_t setup_staged_projection(Dev &d) {
     return cudaSuccess;
 }
 
+cudaError_t wall_tables_mixed(Dev &d, cudaStream_t s) {
+    const Geo &g = d.g;
+    for (int sys = 0; sys < 3; ++sys)
+        wall_table<float>(d.walltabf[sys], g.ny, g.nx / 2 + 1, g.nz, wall_spec(g, d.ph, d.kx2, d.kz2), sys, s);
+    return cudaGetLastError();
+}
+
 cudaError_t init_kernels_mixed() {
     const int big = 200 * 1024;
     F8_CUDA_RET(cudaFuncSetAttribute(k_fft_lines<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    F8_CUDA_RET(cudaFuncSetAttribute(k_wall_tdma<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     F8_CUDA_RET(cudaFuncSetAttribute(k_fft_x_fwd<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     F8_CUDA_RET(cudaFuncSetAttribute(k_fft_x_inv<float, XOutF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     int dev = 0, optin = 0;
@@ -2576,37 +2531,8 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
                                                 cudaMemcpyDeviceToDevice, s));
         }
         if (r == 0) mark(4);
-        // Helmholtz solves for the FP32 increments dU (U* = U^n + dU).  On the
-        // fused spectral path the three solves are independent branches: V and W
-        // run on side streams with their own spectra, forked from and joined to
-        // the step's stream (parallel branches of the captured graph), so their
-        // x transforms fill the SMs that one solve's kernels leave idle.
-        const double lhs1 = d.ph.dt * d.ph.beta / d.ph.re / 2.0;
-        const bool branches = d.fused_planes && d.aux[0] && d.aux[1];
-        if (branches) {
-            F8_CUDA_RET(cudaEventRecord(d.ev_fork, s));
-            for (int b = 0; b < 2; ++b) F8_CUDA_RET(cudaStreamWaitEvent(d.aux[b], d.ev_fork, 0));
-        }
-        for (int c = 0; c < nvc; ++c) {
-            const XOutF out{d.dUf[c], nullptr, 0};
-            if (branches) {
-                cudaStream_t sc = c == 0 ? s : d.aux[c - 1];
-                float *spec = c == 0 ? d.Hf : d.HfB[c - 1];
-                if (!g.walls) e = solve_periodic_fused<float>(d, d.Qf[c], out, 1.0f, (float)lhs1, sc, spec);
-                else e = solve_walls_fused<float>(d, d.Qf[c], out, c == 1 ? SYS_V : SYS_U, sc, spec);
-            } else if (!g.walls) {
-                e = solve_periodic_f(d, d.Qf[c], out, 1.0, lhs1, s);
-            } else {
-                e = solve_walls_f(d, d.Qf[c], out, c == 1 ? SYS_V : SYS_U, s);
-            }
-            if (e) return e;
-        }
-        if (branches) {
-            for (int b = 0; b < 2; ++b) {
-                F8_CUDA_RET(cudaEventRecord(d.ev_join[b], d.aux[b]));
-                F8_CUDA_RET(cudaStreamWaitEvent(s, d.ev_join[b], 0));
-            }
-        }
+        // Helmholtz solves for the FP32 increments dU (U* = U^n + dU)
+        if ((e = mixed_helmholtz(d, nvc, d.Qf, d.dUf, s))) return e;
         if (tp) {
             const TapeUp a{{d.Uf, d.Vf, d.Wf}, {d.dUf[0], d.dUf[1], d.dUf[2]}, {tp->Up[0], tp->Up[1], tp->Up[2]}};
             k_tape_up<<<dim3(tnb, 3), 256, 0, s>>>(a, g); count_launch();

@@ -45,7 +45,7 @@ cudaError_t step_fp64_adjoint(Dev &d, AdjState &A, const TapeStep &t, const doub
     if (A.sor) {
         F8_CUDA_RET(remove_mean_fp64(d, A.pack, d.ni, s));
         int it = 0;
-        F8_CUDA_RET(sor_solve_fp64(d, A.pack, A.lsor, A.work, A.sor_omega, A.sor_eps, A.sor_itrmax, &it, s));
+        F8_CUDA_RET(sor_solve_fp64(d, A.pack, A.lsor, A.sor_omega, A.sor_eps, A.sor_itrmax, &it, s));
         if (it > A.sor_itrmax) ++A.sor_capped;
         lq = A.lsor;
     } else {
@@ -501,7 +501,7 @@ cudaError_t step_fp64_adjoint2(Dev &d, AdjState &A, const TapeStep &t, const dou
     if (A.sor) {
         F8_CUDA_RET(remove_mean_fp64(d, A.pack, d.ni, s));
         int it = 0;
-        F8_CUDA_RET(sor_solve_fp64(d, A.pack, A.lsor, A.work, A.sor_omega, A.sor_eps, A.sor_itrmax, &it, s));
+        F8_CUDA_RET(sor_solve_fp64(d, A.pack, A.lsor, A.sor_omega, A.sor_eps, A.sor_itrmax, &it, s));
         if (it > A.sor_itrmax) ++A.sor_capped;
         lq = A.lsor;
     } else {

@@ -371,6 +371,7 @@ int setup(f8_ctx *c) {
     const size_t cs = d.cs, ni = d.ni;
     const bool mixed = c->precision == F8_MIXED;
     if (mixed) API_CUDA(c, init_kernels_mixed());
+    if (mixed && c->poisson == F8_POISSON_SOR) API_CUDA(c, setup_sor_mixed(d));
     for (double **p : {&d.U, &d.V, &d.W, &d.P, &d.Phi, &d.Up, &d.Vp, &d.Wp})
         API_CUDA(c, c->alloc(p, cs));
     API_CUDA(c, c->alloc(&c->scratch_aos, cs * d.ncomp));
@@ -384,7 +385,7 @@ int setup(f8_ctx *c) {
         API_CUDA(c, c->alloc(&d.C, cs * d.ncomp));
         API_CUDA(c, c->alloc(&d.Cn, cs * d.ncomp));
         for (double **p : {&d.Ax0, &d.Ay0, &d.Az0, &d.Tx0, &d.Ty0, &d.Tz0, &d.Fx, &d.Fy, &d.Fz, &d.Bx, &d.By, &d.Bz,
-                           &d.Q[0], &d.Q[1], &d.Q[2], &d.E})
+                           &d.Q[0], &d.Q[1], &d.Q[2]})
             API_CUDA(c, c->alloc(p, ni));
         API_CUDA(c, c->alloc(&d.H, 3 * nspec));
         API_CUDA(c, c->alloc(&d.H2, (g.walls ? 3 : 1) * nspec));

@@ -24,7 +24,6 @@ struct Dev {
     double *Up, *Vp, *Wp, *Ua, *Va, *Wa;   // halo
     double *Bx, *By, *Bz;                  // interior
     double *Q[3];                          // interior right-hand sides
-    double *E;                             // interior SOR residual
     double *H, *H2;                        // spectral scratch: up to three spectra of nspec values each
     size_t nspec;
     double *walltab[3];                    // FP64 walls: Thomas tables of the U, V, P systems (k_wall_table)
@@ -87,7 +86,8 @@ struct Dev {
     // reductions
     double *red;                           // scratch partial sums (>= 4096)
     double *scal;                          // small scalar results
-    int *flag;                             // SOR convergence flag / iteration
+    int *flag;                             // SOR: converged, iteration, barrier time-out, barrier arrivals
+    int sor_cluster;                       // mixed SOR: CTAs of a cluster that the device can hold
     int *code_count;                       // FP64 3D: cells queued for the FP64 eigen test, per direction
     StepCounters *cnt;
 };
@@ -150,9 +150,9 @@ cudaError_t marker_weights_fp64(Dev &d, cudaStream_t s);
 // pressure Poisson L x = q; src interior, dst halo layout (interior written)
 cudaError_t helmholtz_solve_fp64(Dev &d, int comp, const double *src, double *dst, cudaStream_t s);
 cudaError_t poisson_solve_fp64(Dev &d, const double *src, double *dst, cudaStream_t s);
-// red-black SOR of Q (interior) into the halo field Phi (start value), residuals in E (interior)
-cudaError_t sor_solve_fp64(Dev &d, const double *Q, double *Phi, double *E, double omega, double eps, int itrmax,
-                           int *iters, cudaStream_t s);
+// red-black SOR of Q (interior) into the halo field Phi (start value)
+cudaError_t sor_solve_fp64(Dev &d, const double *Q, double *Phi, double omega, double eps, int itrmax, int *iters,
+                           cudaStream_t s);
 cudaError_t remove_mean_fp64(Dev &d, double *A, int n, cudaStream_t s);
 // On-device diagnostics (f8_diag.cu)
 struct DiagValues {
@@ -256,6 +256,7 @@ cudaError_t take_interior_f(const float *src, float *dst, const Geo &g, int n, c
 // Mixed path (f8_step_mixed.cu)
 cudaError_t init_kernels_mixed();
 cudaError_t wall_tables_mixed(Dev &d, cudaStream_t s);
+cudaError_t setup_sor_mixed(Dev &d);
 cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_iters, cudaStream_t s);
 cudaError_t bc_all_state_mixed(Dev &d, cudaStream_t s);
 cudaError_t mixed_state_to_fp64(Dev &d, cudaStream_t s);

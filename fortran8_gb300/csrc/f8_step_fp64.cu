@@ -10,6 +10,7 @@
 #include "f8_common.cuh"
 #include "f8_fft.cuh"
 #include "f8_kernels.h"
+#include "f8_sor.cuh"
 
 namespace f8 {
 
@@ -1332,42 +1333,14 @@ __global__ void k_march(double *U, double *V, double *W, double *P, const double
 }
 
 // ---------------------------------------------------------------------------
-// Red-black SOR (the reference's sweep, fenep.f90:885-896, is lexicographic in
-// k and j; the GPU colours by (i+j+k) parity, so it matches the reference
-// only at the converged tolerance).  A device flag stops the remaining
-// launched iterations once the tolerance is met.
-
-__global__ void k_sor_color(double *Phi, double *E, const double *Q, Geo g, int color, double om, const int *flag) {
-    if (flag[0]) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z + 1;
-    if (i > g.nx || j > g.ny) return;
-    if (((i + j + k) & 1) != color) return;
-    const bool d3 = g.dim == 3;
-    const double BXM = 1.0 / (g.dx * g.dx), BXP = BXM, BYM = 1.0 / (g.dy * g.dy), BYP = BYM;
-    const double BZM = d3 ? 1.0 / (g.dz * g.dz) : 0.0, BZP = BZM;
-    const double B0 = BXM + BXP + BYM + BYP + BZM + BZP;
-    const int h = hix(g, i, j, k);
-    double e = BZM * Phi[hix(g, i, j, k - 1)] + BYM * Phi[hix(g, i, j - 1, k)] + BXM * Phi[hix(g, i - 1, j, k)]
-               - B0 * Phi[h] + BXP * Phi[hix(g, i + 1, j, k)] + BYP * Phi[hix(g, i, j + 1, k)]
-               + BZP * Phi[hix(g, i, j, k + 1)] - Q[qix(g, i, j, k)];
-    E[qix(g, i, j, k)] = e;
-    Phi[h] = Phi[h] + om * e / B0;
-}
-
-__global__ void k_bc_scalar_flag(double *A, Geo g, int kind, const int *flag) {
-    if (flag[0]) return;
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    int i, j, k;
-    if (halo_cell(g, t, i, j, k)) A[hix(g, i, j, k)] = halo_value(g, A, kind, i, j, k);
-}
+// Reductions.  The red-black SOR itself is in f8_sor.cuh (the reference's
+// sweep, fenep.f90:885-896, is lexicographic in k and j; the GPU colours by
+// (i+j+k) parity, so it matches the reference only at the converged tolerance).
 
 // Deterministic two-level reductions: partial sums per block in a fixed order,
 // then one block sums the partials.
 template <int OP>  // 0: sum of squares, 1: sum of interior values of a halo field, 2: sum of values
-__global__ void k_reduce_part(const double *A, int n, double *part, Geo g, const int *flag) {
-    if (flag && flag[0]) return;
+__global__ void k_reduce_part(const double *A, int n, double *part, Geo g) {
     __shared__ double sh[256];
     double s = 0.0;
     for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
@@ -1387,11 +1360,9 @@ __global__ void k_reduce_part(const double *A, int n, double *part, Geo g, const
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-// finish: scal[slot] = sum(part); mode 1 (SOR check): compare with er0 and set
-// the flag (flag[0] = 1 when converged, flag[1] = iteration count)
-__global__ void k_reduce_final(const double *part, int nparts, double *scal, int slot, int mode, int *flag, double eps,
-                               int itr) {
-    if (mode == 1 && flag[0]) return;
+// finish: scal[slot] = sum(part), with the reference's guard for a zero sum
+// when it becomes the SOR's er0
+__global__ void k_reduce_final(const double *part, int nparts, double *scal, int slot, int guard) {
     __shared__ double sh[256];
     double s = 0.0;
     for (int q = threadIdx.x; q < nparts; q += blockDim.x) s += part[q];
@@ -1401,17 +1372,7 @@ __global__ void k_reduce_final(const double *part, int nparts, double *scal, int
         if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        scal[slot] = sh[0];
-        if (mode == 1) {
-            flag[1] = itr;
-            double er0 = scal[0];
-            if (sqrt(sh[0] / er0) < eps) flag[0] = 1;
-        }
-        if (mode == 2) {  // er0 with the reference's zero guard
-            if (sh[0] == 0.0) scal[slot] = 1.0e-16;
-        }
-    }
+    if (threadIdx.x == 0) scal[slot] = guard && sh[0] == 0.0 ? 1.0e-16 : sh[0];
 }
 
 __global__ void k_shift(double *A, int n, const double *scal, int slot, double inv_n) {
@@ -1500,63 +1461,49 @@ cudaError_t solve_one(Dev &d, const double *src, double *dst, int sys, cudaStrea
     return solve_batch(d, 1, &src, &dst, &sys, &top, s);
 }
 
-cudaError_t reduce_sumsq(const double *A, int n, double *part, double *scal, int slot, int mode, int *flag, double eps,
-                         int itr, const Geo &g, cudaStream_t s) {
-    int nb = std::min(1024, (n + 255) / 256);
-    k_reduce_part<0><<<nb, 256, 0, s>>>(A, n, part, g, mode == 1 ? flag : nullptr); count_launch();
-    k_reduce_final<<<1, 256, 0, s>>>(part, nb, scal, slot, mode, flag, eps, itr); count_launch();
-    return cudaGetLastError();
-}
-
-// Red-black SOR (the reference's poisson, fenep.f90:848-905) of the
+// Red-black SOR (f8_sor.cuh; the reference's poisson, fenep.f90:848-905) of the
 // right-hand side Q (interior) into the halo field Phi, which holds the start
-// value; E (interior) receives the residuals.  Stops when
-// sqrt(sum E^2 / sum Q^2) < eps or after itrmax sweeps (*iters = itrmax + 1),
-// then shifts Phi to zero mean (fenep_2d.f90:577-579).
-cudaError_t sor_solve_on(Dev &d, const double *Q, double *Phi, double *E, double omega, double eps, int itrmax,
-                         int *iters, cudaStream_t s) {
+// value.  Stops when sqrt(sum E^2 / sum Q^2) < eps, E the residuals of a sweep,
+// or after itrmax sweeps (*iters = itrmax + 1), then shifts Phi to zero mean
+// (fenep_2d.f90:577-579).
+cudaError_t sor_solve_on(Dev &d, const double *Q, double *Phi, double omega, double eps, int itrmax, int *iters,
+                         cudaStream_t s) {
     const Geo &g = d.g;
-    dim3 blk(32, 8);
-    dim3 grd = cell_grid(g, blk);
-    // er0 = sum(Q^2) (+1e-16 guard); flag reset
-    F8_CUDA_RET(cudaMemsetAsync(d.flag, 0, 2 * sizeof(int), s));
-    F8_CUDA_RET(reduce_sumsq(Q, d.ni, d.red, d.scal, 0, 2, d.flag, 0.0, 0, g, s));
-    const long nh = halo_count(g);
-    const unsigned hb = (unsigned)((nh + 255) / 256);
-    int done = 0, it_host[2] = {0, 0};
-    const int chunk = 25;
-    for (int it0 = 1; it0 <= itrmax && !done; it0 += chunk) {
-        int last = std::min(itrmax, it0 + chunk - 1);
-        for (int it = it0; it <= last; ++it) {
-            for (int color = 0; color < 2; ++color) {
-                k_sor_color<<<grd, blk, 0, s>>>(Phi, E, Q, g, color, omega, d.flag); count_launch();
-                k_bc_scalar_flag<<<hb, 256, 0, s>>>(Phi, g, BC_P, d.flag); count_launch();
-            }
-            k_bc_scalar_flag<<<hb, 256, 0, s>>>(Phi, g, BC_P, d.flag); count_launch();
-            F8_CUDA_RET(reduce_sumsq(E, d.ni, d.red, d.scal, 1, 1, d.flag, eps, it, g, s));
-        }
-        F8_CUDA_RET(cudaMemcpyAsync(it_host, d.flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-        F8_CUDA_RET(cudaStreamSynchronize(s));
-        done = it_host[0];
-    }
-    *iters = done ? it_host[1] : itrmax + 1;
+    const int nb = std::min(1024, (d.ni + 255) / 256);
+    // er0 = sum(Q^2) (+1e-16 guard)
+    k_reduce_part<0><<<nb, 256, 0, s>>>(Q, d.ni, d.red, g); count_launch();
+    k_reduce_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 0, 1); count_launch();
+    SorArgs<double> a{};
+    a.Phi = Phi; a.R = Q; a.er0 = d.scal; a.part = reinterpret_cast<SorSum<double> *>(d.red); a.flag = d.flag;
+    a.om = omega;
+    a.bx = 1.0 / (g.dx * g.dx); a.by = 1.0 / (g.dy * g.dy); a.bz = g.dim == 3 ? 1.0 / (g.dz * g.dz) : 0.0;
+    a.b0 = a.bx + a.bx + a.by + a.by + a.bz + a.bz;
+    const Recip r = recip(a.b0);
+    a.b0h = r.h; a.b0l = r.l;
+    a.eps = eps; a.itrmax = itrmax;
+    F8_CUDA_RET(sor_sweeps(a, g, device_sm_count(), 1, s));
+    int it_host[3] = {0, 0, 0};
+    F8_CUDA_RET(cudaMemcpyAsync(it_host, d.flag, sizeof(it_host), cudaMemcpyDeviceToHost, s));
+    F8_CUDA_RET(cudaStreamSynchronize(s));
+    if (it_host[2]) return cudaErrorLaunchTimeout;
+    *iters = it_host[0] ? it_host[1] : itrmax + 1;
+    F8_CUDA_RET(bc(Phi, g, BC_P, s));
     // zero-mean shift (fenep_2d.f90:577-579)
-    int nb = std::min(1024, (d.ni + 255) / 256);
-    k_reduce_part<1><<<nb, 256, 0, s>>>(Phi, d.ni, d.red, g, nullptr); count_launch();
-    k_reduce_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 2, 0, d.flag, 0.0, 0); count_launch();
+    k_reduce_part<1><<<nb, 256, 0, s>>>(Phi, d.ni, d.red, g); count_launch();
+    k_reduce_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 2, 0); count_launch();
     k_shift<<<(d.cs + 255) / 256, 256, 0, s>>>(Phi, d.cs, d.scal, 2, 1.0 / ((double)g.nx * g.ny * g.nz)); count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t sor_solve(Dev &d, const StepOpts &o, int *iters, cudaStream_t s) {
-    return sor_solve_on(d, d.Q[0], d.Phi, d.E, o.sor_omega, o.sor_eps, o.sor_itrmax, iters, s);
+    return sor_solve_on(d, d.Q[0], d.Phi, o.sor_omega, o.sor_eps, o.sor_itrmax, iters, s);
 }
 
 // subtract the mean of an interior field (n values)
 cudaError_t remove_mean(Dev &d, double *A, int n, cudaStream_t s) {
     int nb = std::min(1024, (n + 255) / 256);
-    k_reduce_part<2><<<nb, 256, 0, s>>>(A, n, d.red, d.g, nullptr); count_launch();
-    k_reduce_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 3, 0, d.flag, 0.0, 0); count_launch();
+    k_reduce_part<2><<<nb, 256, 0, s>>>(A, n, d.red, d.g); count_launch();
+    k_reduce_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 3, 0); count_launch();
     k_shift<<<(n + 255) / 256, 256, 0, s>>>(A, n, d.scal, 3, 1.0 / n); count_launch();
     return cudaGetLastError();
 }
@@ -1586,9 +1533,9 @@ cudaError_t helmholtz_solve_fp64(Dev &d, int comp, const double *src, double *ds
     return solve_one(d, src, dst, comp == 1 ? SYS_V : SYS_U, s);
 }
 
-cudaError_t sor_solve_fp64(Dev &d, const double *Q, double *Phi, double *E, double omega, double eps, int itrmax,
-                           int *iters, cudaStream_t s) {
-    return sor_solve_on(d, Q, Phi, E, omega, eps, itrmax, iters, s);
+cudaError_t sor_solve_fp64(Dev &d, const double *Q, double *Phi, double omega, double eps, int itrmax, int *iters,
+                           cudaStream_t s) {
+    return sor_solve_on(d, Q, Phi, omega, eps, itrmax, iters, s);
 }
 
 cudaError_t remove_mean_fp64(Dev &d, double *A, int n, cudaStream_t s) { return remove_mean(d, A, n, s); }

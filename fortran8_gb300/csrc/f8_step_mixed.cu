@@ -29,6 +29,7 @@
 #include "f8_fft.cuh"
 #include "f8_fft_fused.cuh"
 #include "f8_kernels.h"
+#include "f8_sor.cuh"
 #include "f8_tma.cuh"
 
 namespace f8 {
@@ -1761,37 +1762,9 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_march_tma(MarchTmaArgs a, Geo
     }
 }
 
-// ---------------------------------------------------------------------------
-// Red-black SOR variant of the pressure solve (the reference's poisson,
-// fenep.f90:848-905; the GPU colours by (i+j+k) parity as the FP64 step does)
-// on the FP32 pressure correction: Phi (hi part) warm-started from the
-// previous step, sweeps until sqrt(sum E^2 / sum R^2) < eps with the sums in
-// FP64, then the zero-mean shift (fenep_2d.f90:577-579).  The reference's
-// tolerance (1e-5) is far above FP32 rounding.  Halo-free: periodic wrap and
-// the Neumann copy at the walls, which is what the halo pass between the
-// colour sweeps of the FP64 step provides.
-__global__ void k_sor_color_f(float *Phi, float *E, const float *R, Geo g, int color, float om, float bx, float by,
-                              float bz, const int *flag) {
-    if (flag[0]) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z + 1;
-    if (i > g.nx || j > g.ny) return;
-    if (((i + j + k) & 1) != color) return;
-    const int h = hix(g, i, j, k);
-    const float b0 = 2.0f * (bx + by + bz);
-    const int q = qix(g, i, j, k);
-    const float e = bz * Phi[nbr_p(g, i, j, k, 2, -1)] + by * Phi[nbr_p(g, i, j, k, 1, -1)]
-                  + bx * Phi[nbr_p(g, i, j, k, 0, -1)] - b0 * Phi[h] + bx * Phi[nbr_p(g, i, j, k, 0, 1)]
-                  + by * Phi[nbr_p(g, i, j, k, 1, 1)] + bz * Phi[nbr_p(g, i, j, k, 2, 1)] - R[q];
-    E[q] = e;
-    Phi[h] = Phi[h] + om * e / b0;
-}
-
 // block partials of sum(a^2) (mode 0) or of the interior sum of a halo field
 // (mode 1), in FP64, fixed order
-__global__ void k_sum_part_f(const float *a, int n, int mode, double *part, Geo g, const int *flag) {
-    if (flag && flag[0]) return;
+__global__ void k_sum_part_f(const float *a, int n, int mode, double *part, Geo g) {
     __shared__ double sh[256];
     double s = 0.0;
     for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
@@ -1812,12 +1785,9 @@ __global__ void k_sum_part_f(const float *a, int n, int mode, double *part, Geo 
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-// mode 0: scal[slot] = sum (er0, the reference's zero guard); mode 1: the
-// convergence test against scal[0] (flag[0] = 1, flag[1] = iteration);
-// mode 2: scal[slot] = sum
-__global__ void k_sum_final(const double *part, int nparts, double *scal, int slot, int mode, int *flag, double eps,
-                            int itr) {
-    if (mode == 1 && flag[0]) return;
+// scal[slot] = sum, with the reference's guard for a zero sum when it becomes
+// the SOR's er0
+__global__ void k_sum_final(const double *part, int nparts, double *scal, int slot, int guard) {
     __shared__ double sh[256];
     double s = 0.0;
     for (int q = threadIdx.x; q < nparts; q += blockDim.x) s += part[q];
@@ -1827,13 +1797,7 @@ __global__ void k_sum_final(const double *part, int nparts, double *scal, int sl
         if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        scal[slot] = (mode == 0 && sh[0] == 0.0) ? 1.0e-16 : sh[0];
-        if (mode == 1) {
-            flag[1] = itr;
-            if (sqrt(sh[0] / scal[0]) < eps) flag[0] = 1;
-        }
-    }
+    if (threadIdx.x == 0) scal[slot] = guard && sh[0] == 0.0 ? 1.0e-16 : sh[0];
 }
 
 __global__ void k_shift_f(float *a, Geo g, const double *scal, int slot) {
@@ -2030,34 +1994,29 @@ cudaError_t solve_walls_f(Dev &d, const float *src, XOutF out, int sys, cudaStre
     return solve_walls_mp(d, 1, {{src}}, {{out}}, {sys}, s);
 }
 
+// Red-black SOR of the right-hand side's high part into Phi (f8_sor.cuh), then
+// the zero-mean shift
 cudaError_t sor_solve_m(Dev &d, const StepOpts &o, int *iters, cudaStream_t s) {
     const Geo &g = d.g;
     const dim3 blk(32, 8), grd = cell_grid_m(g, blk);
     const int nb = std::min(1024, (d.ni + 255) / 256);
-    F8_CUDA_RET(cudaMemsetAsync(d.flag, 0, 2 * sizeof(int), s));
     F8_CUDA_RET(cudaMemsetAsync(d.Phil, 0, (size_t)d.cs * sizeof(float), s));
-    k_sum_part_f<<<nb, 256, 0, s>>>(d.Rhf, d.ni, 0, d.red, g, nullptr); count_launch();
-    k_sum_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 0, 0, d.flag, 0.0, 0); count_launch();
-    const float bx = (float)(1.0 / (g.dx * g.dx)), by = (float)(1.0 / (g.dy * g.dy)), bz = (float)(1.0 / (g.dz * g.dz));
-    int done = 0, it_host[2] = {0, 0};
-    const int chunk = 25;
-    for (int it0 = 1; it0 <= o.sor_itrmax && !done; it0 += chunk) {
-        const int last = std::min(o.sor_itrmax, it0 + chunk - 1);
-        for (int it = it0; it <= last; ++it) {
-            for (int color = 0; color < 2; ++color) {
-                k_sor_color_f<<<grd, blk, 0, s>>>(d.Phif, d.Rdf, d.Rhf, g, color, (float)o.sor_omega, bx, by, bz,
-                                                  d.flag); count_launch();
-            }
-            k_sum_part_f<<<nb, 256, 0, s>>>(d.Rdf, d.ni, 0, d.red, g, d.flag); count_launch();
-            k_sum_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 1, 1, d.flag, o.sor_eps, it); count_launch();
-        }
-        F8_CUDA_RET(cudaMemcpyAsync(it_host, d.flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-        F8_CUDA_RET(cudaStreamSynchronize(s));
-        done = it_host[0];
-    }
-    *iters = done ? it_host[1] : o.sor_itrmax + 1;
-    k_sum_part_f<<<nb, 256, 0, s>>>(d.Phif, d.ni, 1, d.red, g, nullptr); count_launch();
-    k_sum_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 2, 2, d.flag, 0.0, 0); count_launch();
+    k_sum_part_f<<<nb, 256, 0, s>>>(d.Rhf, d.ni, 0, d.red, g); count_launch();
+    k_sum_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 0, 1); count_launch();
+    SorArgs<float> a{};
+    a.Phi = d.Phif; a.R = d.Rhf; a.er0 = d.scal; a.part = reinterpret_cast<SorSum<float> *>(d.red); a.flag = d.flag;
+    a.om = (float)o.sor_omega;
+    a.bx = (float)(1.0 / (g.dx * g.dx)); a.by = (float)(1.0 / (g.dy * g.dy)); a.bz = (float)(1.0 / (g.dz * g.dz));
+    a.b0 = 2.0f * (a.bx + a.by + a.bz);
+    a.eps = o.sor_eps; a.itrmax = o.sor_itrmax;
+    F8_CUDA_RET(sor_sweeps(a, g, device_sm_count(), d.sor_cluster, s));
+    int it_host[3] = {0, 0, 0};
+    F8_CUDA_RET(cudaMemcpyAsync(it_host, d.flag, sizeof(it_host), cudaMemcpyDeviceToHost, s));
+    F8_CUDA_RET(cudaStreamSynchronize(s));
+    if (it_host[2]) return cudaErrorLaunchTimeout;
+    *iters = it_host[0] ? it_host[1] : o.sor_itrmax + 1;
+    k_sum_part_f<<<nb, 256, 0, s>>>(d.Phif, d.ni, 1, d.red, g); count_launch();
+    k_sum_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 2, 0); count_launch();
     k_shift_f<<<grd, blk, 0, s>>>(d.Phif, g, d.scal, 2); count_launch();
     return cudaGetLastError();
 }
@@ -2169,6 +2128,8 @@ cudaError_t setup_staged_projection(Dev &d) {
     d.march_depth = depth;
     return cudaSuccess;
 }
+
+cudaError_t setup_sor_mixed(Dev &d) { return sor_cluster_size(&d.sor_cluster); }
 
 cudaError_t wall_tables_mixed(Dev &d, cudaStream_t s) {
     const Geo &g = d.g;

@@ -433,23 +433,50 @@ __global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *
     const T *__restrict__ hin = Hin + blockIdx.z * hstride + (size_t)2 * nxh * ny * kz + c;
     T *hout = Hout + blockIdx.z * hstride + (size_t)2 * nxh * n * kz + c;
     T q = T(0);
-#pragma unroll 4
-    for (int j = 0; j < n; ++j) {
-        T d = T(0);
-        if (j >= 1 && j <= ny && !(sys == SYS_V && j == ny)) d = hin[(size_t)2 * nxh * (j - 1)] * inv_nxz;
-        else if (j == n - 1 && mode == 0 && c == 0) d = T(it.top);
-        const T cc = j == 0 ? T(0) : (j == n - 1 ? (sys == SYS_U ? T(1) : (sys == SYS_V ? T(0) : T(-1)))
-                                                 : (sys == SYS_V && j >= ny ? T(0) : ci));
-        const size_t o = (size_t)j * modes + mode;
-        const T t = d - cc * q;
-        q = fma(t, rh[o], t * rl[o]);
-        hout[(size_t)2 * nxh * j] = q;
+    // in groups of 8 rows: the loads do not depend on the recurrence, so a group's
+    // are all in flight before its chain begins
+    constexpr int G = 8;
+    for (int j0 = 0; j0 < n; j0 += G) {
+        T d[G], h[G], l[G];
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            const int j = j0 + u;
+            d[u] = h[u] = l[u] = T(0);
+            if (j >= n) continue;
+            if (j >= 1 && j <= ny && !(sys == SYS_V && j == ny)) d[u] = hin[(size_t)2 * nxh * (j - 1)] * inv_nxz;
+            else if (j == n - 1 && mode == 0 && c == 0) d[u] = T(it.top);
+            h[u] = rh[(size_t)j * modes + mode];
+            l[u] = rl[(size_t)j * modes + mode];
+        }
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            const int j = j0 + u;
+            if (j >= n) continue;
+            const T cc = j == 0 ? T(0) : (j == n - 1 ? (sys == SYS_U ? T(1) : (sys == SYS_V ? T(0) : T(-1)))
+                                                     : (sys == SYS_V && j >= ny ? T(0) : ci));
+            const T t = d[u] - cc * q;
+            q = fma(t, h[u], t * l[u]);
+            hout[(size_t)2 * nxh * j] = q;
+        }
     }
     T x = q;
-#pragma unroll 8
-    for (int j = n - 2; j >= 0; --j) {
-        x = P[(size_t)j * modes + mode] * x + hout[(size_t)2 * nxh * j];
-        hout[(size_t)2 * nxh * j] = x;
+    for (int j0 = n - 2; j0 >= 0; j0 -= G) {
+        T p[G], r[G];
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            const int j = j0 - u;
+            p[u] = r[u] = T(0);
+            if (j < 0) continue;
+            p[u] = P[(size_t)j * modes + mode];
+            r[u] = hout[(size_t)2 * nxh * j];
+        }
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            const int j = j0 - u;
+            if (j < 0) continue;
+            x = p[u] * x + r[u];
+            hout[(size_t)2 * nxh * j] = x;
+        }
     }
 }
 

@@ -8,6 +8,7 @@
 // transform as the time step's periodic solves.
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <vector>
 #include "../../include/f8.h"
 #include "f8_common.cuh"
@@ -80,6 +81,21 @@ cudaError_t set_smem_attrs() {
 
 }  // namespace
 
+// Fixed device arrays, one set per GPU: a spectrum of up to 135168 complex
+// values (65 * 64 * 32 = 33 * 64 * 64) and the tables of any grid (twiddles and
+// wavenumbers, N <= 1024).  Both entry points use them, one call at a time
+// (g_solve_mutex): a pair of cudaMalloc / cudaFree takes 62 us on this part, and
+// two of them were most of a small solve (128 x 128: 239 us with them).
+#define F8_NOALLOC_MAX_SPECTRUM 135168
+#define F8_NOALLOC_MAX_TABLE 8192
+
+static __device__ __align__(256) double g_noalloc_spectrum[2 * F8_NOALLOC_MAX_SPECTRUM];
+static __device__ __align__(256) double g_noalloc_table[F8_NOALLOC_MAX_TABLE];
+
+namespace {
+std::mutex g_solve_mutex;
+}
+
 extern "C" int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double lz, const double *q, double *phi,
                             double lhs0, double lhs1) {
     if (int st = check_args(nx, ny, nz, lx, ly, lz, q, phi)) return st;
@@ -90,19 +106,26 @@ extern "C" int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double
     }
     if (set_smem_attrs() != cudaSuccess) return F8_ERR_CUDA;
     const SolveTables t = make_tables(nx, ny, nz, lx, ly, lz);
-    double *H = nullptr, *dtab = nullptr;
-    const size_t nspec = 2 * (size_t)(nx / 2 + 1) * ny * nz;
+    const size_t nspec = (size_t)(nx / 2 + 1) * ny * nz;
+    std::lock_guard<std::mutex> lock(g_solve_mutex);
+    // the arrays of the current device, looked up on every call (a device reset
+    // between calls may move them)
+    void *tab = nullptr, *fixed = nullptr;
+    double *own = nullptr;
     int st = F8_OK;
-    if (cudaMalloc(&H, nspec * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&dtab, t.buf.size() * sizeof(double)) != cudaSuccess) {
-        st = F8_ERR_NOMEM;
-    } else if (cudaMemcpy(dtab, t.buf.data(), t.buf.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-               run_solve(q, phi, H, dtab, t, nx, ny, nz, lhs0, lhs1, 0) != cudaSuccess ||
-               cudaStreamSynchronize(0) != cudaSuccess) {
+    if (t.buf.size() > (size_t)F8_NOALLOC_MAX_TABLE || cudaGetSymbolAddress(&tab, g_noalloc_table) != cudaSuccess ||
+        cudaGetSymbolAddress(&fixed, g_noalloc_spectrum) != cudaSuccess) {
         st = F8_ERR_CUDA;
+    } else if (nspec > (size_t)F8_NOALLOC_MAX_SPECTRUM && cudaMalloc(&own, 2 * nspec * sizeof(double)) != cudaSuccess) {
+        st = F8_ERR_NOMEM;
+    } else {
+        double *H = own ? own : static_cast<double *>(fixed), *dtab = static_cast<double *>(tab);
+        if (cudaMemcpyAsync(dtab, t.buf.data(), t.buf.size() * sizeof(double), cudaMemcpyHostToDevice, 0) != cudaSuccess ||
+            run_solve(q, phi, H, dtab, t, nx, ny, nz, lhs0, lhs1, 0) != cudaSuccess ||
+            cudaStreamSynchronize(0) != cudaSuccess)
+            st = F8_ERR_CUDA;
     }
-    if (H) cudaFree(H);
-    if (dtab) cudaFree(dtab);
+    if (own) cudaFree(own);
     cudaGetLastError();
     return st;
 }
@@ -125,24 +148,16 @@ extern "C" int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double
 //  * the spectrum of the grid must fit in F8_NOALLOC_MAX_SPECTRUM complex
 //    values, (nx/2+1)*ny*nz <= 135168 (for example 64^3, 128 x 64 x 32 or a
 //    2D 512 x 256 field); larger grids get F8_ERR_TOO_LARGE;
-//  * the arrays are shared by every call in the process on a device and keep
-//    the last call's contents; each call overwrites all it reads (the forward
-//    transform fills the whole spectrum and the tables are rewritten), so
-//    nothing has to start at zero, but calls that overlap on the GPU (from
-//    several host threads, or other streams) race on the arrays;
+//  * the arrays are shared by every call in the process on a device, of
+//    f8_fft_solve too, and keep the last call's contents; each call overwrites
+//    all it reads (the forward transform fills the whole spectrum and the
+//    tables are rewritten), so nothing has to start at zero; the calls of
+//    several host threads take turns;
 //  * the first call on a device looks up the device addresses of the arrays
 //    (cudaGetSymbolAddress, with that device current); make that first call
 //    before any stream capture on that device.  The addresses are kept for
 //    the life of the process: after a cudaDeviceReset the library has to be
 //    unloaded and loaded again before this entry point is used there.
-
-#include <mutex>
-
-#define F8_NOALLOC_MAX_SPECTRUM 135168   /* complex values: 65 * 64 * 32 = 33 * 64 * 64 */
-#define F8_NOALLOC_MAX_TABLE 8192        /* doubles: twiddles and wavenumbers, N <= 1024 */
-
-static __device__ __align__(256) double g_noalloc_spectrum[2 * F8_NOALLOC_MAX_SPECTRUM];
-static __device__ __align__(256) double g_noalloc_table[F8_NOALLOC_MAX_TABLE];
 
 namespace {
 
@@ -198,6 +213,7 @@ extern "C" int f8_fft_solve_noalloc(int nx, int ny, int nz, double lx, double ly
     if (int st = noalloc_setup(p)) return st;
     const SolveTables t = make_tables(nx, ny, nz, lx, ly, lz);
     if (t.buf.size() > (size_t)F8_NOALLOC_MAX_TABLE) return F8_ERR_TOO_LARGE;
+    std::lock_guard<std::mutex> lock(g_solve_mutex);
     if (cudaMemcpyAsync(p.tab, t.buf.data(), t.buf.size() * sizeof(double), cudaMemcpyHostToDevice, 0) != cudaSuccess ||
         run_solve(q, phi, p.spec, p.tab, t, nx, ny, nz, lhs0, lhs1, 0) != cudaSuccess ||
         cudaStreamSynchronize(0) != cudaSuccess) {

@@ -343,9 +343,10 @@ int f8_kernel_timing(f8_ctx *ctx, double *kernel_ms, long long *steps_timed);
  * is the CN Helmholtz solve of fft_navier (fenep.f90:1458-1479); lhs0 = 0,
  * lhs1 = -1 the Poisson solve of fft_poisson (fenep.f90:1539-1557).
  * q and phi are DEVICE pointers to dense nx*ny*nz arrays (x fastest, no halo;
- * nz = 1 for a 2D field).  Sizes are powers of two.  FP64.  Allocates its
- * workspace on the device for the duration of the call; runs on the default
- * stream and returns when the result is complete. */
+ * nz = 1 for a 2D field).  Sizes are powers of two.  FP64.  Grids within the
+ * fixed workspace of f8_fft_solve_noalloc use it, larger ones allocate theirs
+ * on the device for the duration of the call; runs on the default stream and
+ * returns when the result is complete.  Calls from several threads take turns. */
 int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double lz,
                  const double *q, double *phi, double lhs0, double lhs1);
 
@@ -358,9 +359,9 @@ int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double lz,
  * until the process exits.  Limits and rules:
  *   - (nx/2+1)*ny*nz <= 135168 complex values (e.g. 64^3); larger grids return
  *     F8_ERR_TOO_LARGE;
- *   - every call shares that workspace and leaves its contents behind; each
- *     call overwrites what it reads, but calls that overlap on the GPU (from
- *     several threads or streams) race;
+ *   - every call, of f8_fft_solve too, shares that workspace and leaves its
+ *     contents behind; each call overwrites what it reads, and calls from
+ *     several threads take turns;
  *   - the first call on a device looks up the workspace address on that
  *     device (the device must be current); make it before any stream capture;
  *   - with CUDA's lazy module loading, the fixed arrays are placed in device

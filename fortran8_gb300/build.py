@@ -1,8 +1,8 @@
 """Build the in-tree CUDA library ``fortran8_gb300/libf8.so`` for sm_103a.
 
 Each translation unit is compiled by nvcc in parallel and linked into one
-shared object that exports the C ABI of include/f8.h.  The FP64 kernels are
-compiled with ``--fmad=false`` so that their arithmetic keeps the reference's
+shared object that exports the C ABI of include/f8.h.  The kernels of the FP64
+step are compiled with ``--fmad=false`` so that their arithmetic keeps the reference's
 operation order (no fused multiply-add contraction).
 """
 from __future__ import annotations
@@ -28,7 +28,7 @@ UNITS = {
     "f8_step_mixed.cu": [],
     "f8_fftsolve.cu": ["--fmad=false"],
     "f8_diag.cu": ["--fmad=false"],
-    "f8_adjoint.cu": ["--fmad=false"],
+    "f8_adjoint.cu": [],
     "f8_adjoint_mixed.cu": [],
 }
 

@@ -1,7 +1,9 @@
 // f8_adjoint.cu — discrete adjoint of the FP64 3D step (the gradient of
 // f8_grad on an F8_FP64 context).  The kernels, their conventions and the
-// stage order are in f8_adjoint_kernels.cuh (instantiated here for double,
-// compiled without FMA contraction like the FP64 step).
+// stage order are in f8_adjoint_kernels.cuh (instantiated here for double).  The
+// forward it linearises is the FP64 step bit for bit; the transposes themselves
+// have no reference order to keep and are compiled with FMA contraction (their
+// kernels are bound by the FP64 pipe, and a fused product rounds once).
 #include <algorithm>
 #include <cstdio>
 #include "f8_adjoint_kernels.cuh"
@@ -54,9 +56,12 @@ cudaError_t step_fp64_adjoint(Dev &d, AdjState &A, const TapeStep &t, const doub
     k_div_adj<double><<<nb, 256, 0, s>>>(A.lU, A.lV, A.lW, lq, A.lUp[0], A.lUp[1], A.lUp[2], g); count_launch();
     F8_CUDA_RET(fold(fold_set<double>({{A.lUp[0], BC_U}, {A.lUp[1], BC_V}, {A.lUp[2], BC_W}}), g, s));
     // 4. Helmholtz
-    for (int c = 0; c < 3; ++c) {
-        k_pack<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lUp[c], A.pack, g); count_launch();
-        F8_CUDA_RET(helmholtz_solve_fp64(d, c, A.pack, A.lQ[c], s));
+    {
+        double *pk[3];
+        for (int c = 0; c < 3; ++c) pk[c] = A.pack + (size_t)c * d.ni;
+        k_pack3<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lUp[0], A.lUp[1], A.lUp[2], pk[0], pk[1], pk[2], g);
+        count_launch();
+        F8_CUDA_RET(helmholtz_solves_fp64(d, 3, pk, A.lQ, s));
     }
     // 3. IBM
     for (int c = 0; c < 3; ++c) F8_CUDA_RET(cudaMemsetAsync(A.lUa[c], 0, hb, s));
@@ -71,7 +76,9 @@ cudaError_t step_fp64_adjoint(Dev &d, AdjState &A, const TapeStep &t, const doub
         ia.grad = A.grad;
         ia.d3 = 1;
         k_ibm_adj<double><<<dim3((d.nm + 127) / 128, g.nz, 3), 128, 0, s>>>(ia, g); count_launch();
-        F8_CUDA_RET(fold(fold_set<double>({{A.lUa[0], BC_U}, {A.lUa[1], BC_V}, {A.lUa[2], BC_W}}), g, s));
+        // the y and x passes only where a stencil reaches a ghost column or row
+        const FoldSet<double> fa = fold_set<double>({{A.lUa[0], BC_U}, {A.lUa[1], BC_V}, {A.lUa[2], BC_W}});
+        F8_CUDA_RET(d.ibm_edge ? fold(fa, g, s) : fold_z_only(fa, g, s));
     }
     // 2. momentum right-hand side: per-cell sources, then the gather of the
     // velocity, pressure and (with the polymer) C0 / C adjoints
@@ -510,9 +517,13 @@ cudaError_t step_fp64_adjoint2(Dev &d, AdjState &A, const TapeStep &t, const dou
     k_div_adj<double><<<nb, 256, 0, s>>>(A.lU, A.lV, A.lW, lq, A.lUp[0], A.lUp[1], A.lUp[2], g); count_launch();
     F8_CUDA_RET(fold(fold_set<double>({{A.lUp[0], BC_U}, {A.lUp[1], BC_V}}), g, s));
     // 4. Helmholtz
-    for (int c = 0; c < 2; ++c) {
-        k_pack<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lUp[c], A.pack, g); count_launch();
-        F8_CUDA_RET(helmholtz_solve_fp64(d, c, A.pack, A.lQ[c], s));
+    {
+        double *pk[2];
+        for (int c = 0; c < 2; ++c) {
+            pk[c] = A.pack + (size_t)c * d.ni;
+            k_pack<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lUp[c], pk[c], g); count_launch();
+        }
+        F8_CUDA_RET(helmholtz_solves_fp64(d, 2, pk, A.lQ, s));
     }
     // 3. IBM
     for (int c = 0; c < 2; ++c) F8_CUDA_RET(cudaMemsetAsync(A.lUa[c], 0, hb, s));

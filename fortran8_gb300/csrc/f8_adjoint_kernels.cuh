@@ -1,6 +1,6 @@
 // f8_adjoint_kernels.cuh — kernels of the discrete adjoint of the 3D step,
 // templated on the arithmetic type T of the adjoint fields and of the tape:
-// double for the FP64 step (f8_adjoint.cu, compiled without FMA contraction),
+// double for the FP64 step (f8_adjoint.cu),
 // float for the FP32-mixed step (f8_adjoint_mixed.cu).  The gradient with
 // respect to the parameters is accumulated in FP64 in both (per-block sums
 // added to one FP64 array).

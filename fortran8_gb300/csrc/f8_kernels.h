@@ -146,9 +146,9 @@ cudaError_t launch_drag(Dev &d, double *out, cudaStream_t s);
 // the FP64 IBM weight tables (mwxd, mwyd, mwzd, mi0d, mj0d) from the marker positions
 cudaError_t marker_weights_fp64(Dev &d, cudaStream_t s);
 // the linear solves of the step without their inhomogeneous boundary terms:
-// Helmholtz (I - dt beta/(2 Re) L) x = q of velocity component comp, and the
+// Helmholtz (I - dt beta/(2 Re) L) x = q of the first ncomp velocity components, and the
 // pressure Poisson L x = q; src interior, dst halo layout (interior written)
-cudaError_t helmholtz_solve_fp64(Dev &d, int comp, const double *src, double *dst, cudaStream_t s);
+cudaError_t helmholtz_solves_fp64(Dev &d, int ncomp, const double *const *src, double *const *dst, cudaStream_t s);
 cudaError_t poisson_solve_fp64(Dev &d, const double *src, double *dst, cudaStream_t s);
 // red-black SOR of Q (interior) into the halo field Phi (start value)
 cudaError_t sor_solve_fp64(Dev &d, const double *Q, double *Phi, double omega, double eps, int itrmax, int *iters,
@@ -201,7 +201,7 @@ struct AdjState {
     double *lC, *lC2;                      // C and a second C buffer (6 fields each)
     double *lA0[3], *lT0[3];               // AB2 histories (interior)
     double *lUa[3], *lUp[3], *lQ[3];       // explicit velocity, Helmholtz solution, right-hand side
-    double *pack;                          // one packed interior field
+    double *pack;                          // packed interior fields (3 * ni)
     double *work;                          // per-cell sources of the gather kernels (ADJ_WORK_FIELDS halo fields)
     double *grad;                          // dJ/d(Wi, beta, L^2, (xc, yc) per cylinder), accumulated
     // SOR variant: the adjoint pressure solve by the same red-black SOR, warm

@@ -1529,8 +1529,10 @@ cudaError_t bc_all_state_fp64(Dev &d, cudaStream_t s) {
 
 cudaError_t bc_field(double *A, const Geo &g, int kind, cudaStream_t s) { return bc(A, g, kind, s); }
 
-cudaError_t helmholtz_solve_fp64(Dev &d, int comp, const double *src, double *dst, cudaStream_t s) {
-    return solve_one(d, src, dst, comp == 1 ? SYS_V : SYS_U, s);
+cudaError_t helmholtz_solves_fp64(Dev &d, int ncomp, const double *const *src, double *const *dst, cudaStream_t s) {
+    const int sys[3] = {SYS_U, SYS_V, SYS_U};
+    const double top[3] = {0.0, 0.0, 0.0};
+    return solve_batch(d, ncomp, src, dst, sys, top, s);
 }
 
 cudaError_t sor_solve_fp64(Dev &d, const double *Q, double *Phi, double omega, double eps, int itrmax, int *iters,

@@ -461,15 +461,15 @@ int setup(f8_ctx *c) {
         if (int st = upload_f(c, &d.kx2f, kx2)) return st;
         if (int st = upload_f(c, &d.ky2f, ky2)) return st;
         if (int st = upload_f(c, &d.kz2f, kz2)) return st;
-        // shared memory of one (z, y) plane: walls 12 B x (NY+2 | 1) x NZ,
-        // periodic 8 B x (NY+1) x NZ; opt-in limit 227 KB
+        // the (z, y) plane of one kx in shared memory (opt-in limit 227 KB); other
+        // grids take the line passes
         int dev = 0, optin = 0;
         API_CUDA(c, cudaGetDevice(&dev));
         API_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         d.plane_cl = g.walls ? cached_wall_plane(g.ny, g.nz, optin, &d.plane_wl) : 0;
         API_CUDA(c, setup_staged_projection(d));
         if (g.walls) d.fused_planes = (d.plane_cl > 0 || (size_t)12 * ((g.ny + 2) | 1) * g.nz <= (size_t)optin) ? 1 : 0;
-        else d.fused_planes = (size_t)8 * (g.ny + 1) * g.nz <= (size_t)optin ? 1 : 0;
+        else d.fused_planes = periodic_plane_fits(g.ny, g.nz, (size_t)optin) ? 1 : 0;
         if (g.dim == 2) d.fused_planes = 0;   // 2D: the line transforms and tridiagonal sweeps
         API_CUDA(c, c->alloc(&d.Hf, (d.fused_planes ? 1 : 3) * nspec));
         if (!d.fused_planes && g.walls) {
@@ -477,15 +477,16 @@ int setup(f8_ctx *c) {
             for (float *&t : d.walltabf) API_CUDA(c, c->alloc(&t, 3 * nxh * (size_t)g.nz * (g.ny + 2)));
             API_CUDA(c, wall_tables_mixed(d, c->s));
         }
-        if (d.fused_planes) {
-            // side streams and spectra of the V and W Helmholtz solves
+        // side streams (the V and W Helmholtz solves, the wall ghost rows, the drag)
+        // and the spectra of those solves
+        if (g.dim == 3) {
             for (int b = 0; b < 2; ++b) {
-                API_CUDA(c, c->alloc(&d.HfB[b], nspec));
+                if (d.fused_planes) API_CUDA(c, c->alloc(&d.HfB[b], nspec));
                 API_CUDA(c, cudaStreamCreateWithFlags(&d.aux[b], cudaStreamNonBlocking));
                 API_CUDA(c, cudaEventCreateWithFlags(&d.ev_join[b], cudaEventDisableTiming));
             }
             API_CUDA(c, cudaEventCreateWithFlags(&d.ev_fork, cudaEventDisableTiming));
-            for (int q = 0; q < 4; ++q) API_CUDA(c, cudaEventCreateWithFlags(&d.ev_g[q], cudaEventDisableTiming));
+            for (int q = 0; q < 6; ++q) API_CUDA(c, cudaEventCreateWithFlags(&d.ev_g[q], cudaEventDisableTiming));
         }
         {
             // stage-major twiddles of the warp transforms: stage span m holds
@@ -500,7 +501,9 @@ int setup(f8_ctx *c) {
                     }
                 return t;
             };
-            const std::vector<float2> t2 = stage_table(g.nz), tx = stage_table(g.nx);
+            const std::vector<float2> t2 = stage_table(g.nz), ty = stage_table(g.ny), tx = stage_table(g.nx);
+            API_CUDA(c, c->alloc(&d.twy2, ty.size()));
+            API_CUDA(c, cudaMemcpyAsync(d.twy2, ty.data(), ty.size() * sizeof(float2), cudaMemcpyHostToDevice, c->s));
             API_CUDA(c, c->alloc(&d.twz2, t2.size()));
             API_CUDA(c, cudaMemcpyAsync(d.twz2, t2.data(), t2.size() * sizeof(float2), cudaMemcpyHostToDevice, c->s));
             API_CUDA(c, c->alloc(&d.twx2, tx.size()));
@@ -593,6 +596,8 @@ int setup(f8_ctx *c) {
             if (int st = upload_i(c, &d.mperm, perm)) return st;
             if (int st = upload_i(c, &d.moff, off)) return st;
             API_CUDA(c, c->alloc(&d.dragpart, c->cyl.size() * (size_t)g.nz * 3));
+            API_CUDA(c, c->alloc(&d.dragcnt, c->cyl.size()));
+            API_CUDA(c, cudaMemsetAsync(d.dragcnt, 0, c->cyl.size() * sizeof(unsigned), c->s));
         }
         const int ncomp = g.dim == 3 ? 3 : 2;
         const int ncol = g.sx * g.sy;

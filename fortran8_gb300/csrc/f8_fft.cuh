@@ -24,27 +24,37 @@ __host__ __device__ inline int ilog2_pow2(int n) {
     return l;
 }
 
+// b * (wr, wi).  FP64: rounded products and sum, as the oracle forms them.  FP32:
+// one product fused into the sum, in a fixed order so that every form of a
+// transform gives the same bits; INV: the order of a conjugated twiddle.
+template <bool INV>
+__device__ __forceinline__ Cx<double> twiddle_mul(Cx<double> b, double wr, double wi) {
+    return Cx<double>{__dsub_rn(__dmul_rn(b.r, wr), __dmul_rn(b.i, wi)), __dadd_rn(__dmul_rn(b.r, wi), __dmul_rn(b.i, wr))};
+}
+template <bool INV>
+__device__ __forceinline__ Cx<float> twiddle_mul(Cx<float> b, float wr, float wi) {
+    return Cx<float>{__fmaf_rn(b.r, wr, -__fmul_rn(b.i, wi)),
+                     INV ? __fmaf_rn(b.i, wr, __fmul_rn(b.r, wi)) : __fmaf_rn(b.r, wi, __fmul_rn(b.i, wr))};
+}
+
 // One butterfly (index j of 2^(lg-1)) of the Stockham stage of span 2^ls on a
 // line of 2^lg complex values in shared memory, x -> y.
 //   tw: forward twiddles exp(-2 pi i t/n), t < n/2 (re, im arrays)
 // The first stage's twiddle is 1.
-template <typename T>
+template <bool INV, typename T>
 __device__ __forceinline__ void stockham_stage(const Cx<T> *x, Cx<T> *y, int lg, int ls, int j, const T *twr,
                                                const T *twi, int sign) {
     const int half = 1 << (lg - 1), ns = 1 << ls;
     const int kk = j & (ns - 1);
     const Cx<T> a = x[j], b = x[j + half];
-    T tr = b.r, ti = b.i;
+    Cx<T> t = b;
     if (ls > 0) {
-        const int t = kk << (lg - 1 - ls);
-        const T wr = twr[t];
-        const T wi = sign < 0 ? twi[t] : -twi[t];
-        tr = b.r * wr - b.i * wi;
-        ti = b.r * wi + b.i * wr;
+        const int q = kk << (lg - 1 - ls);
+        t = twiddle_mul<INV>(b, twr[q], sign < 0 ? twi[q] : -twi[q]);
     }
     const int o = ((j >> ls) << (ls + 1)) + kk;
-    y[o].r = a.r + tr; y[o].i = a.i + ti;
-    y[o + ns].r = a.r - tr; y[o + ns].i = a.i - ti;
+    y[o].r = a.r + t.r; y[o].i = a.i + t.i;
+    y[o + ns].r = a.r - t.r; y[o + ns].i = a.i - t.i;
 }
 
 // Shapes of the transform launches.  A block takes up to 256 butterflies of a
@@ -112,7 +122,7 @@ __global__ void k_fft_x_fwd(Batch<const TS *> srcs, T *__restrict__ H, size_t hs
     }
     __syncthreads();
     for (int ls = 0; ls < lg; ++ls) {
-        if (active) stockham_stage(x, y, lg, ls, t, twr, twi, -1);
+        if (active) stockham_stage<false>(x, y, lg, ls, t, twr, twi, -1);
         __syncthreads();
         Cx<T> *tmp = x; x = y; y = tmp;
     }
@@ -201,7 +211,7 @@ __global__ void k_fft_x_inv(const T *__restrict__ H, size_t hstride, Batch<Out> 
     }
     __syncthreads();
     for (int ls = 0; ls < lg; ++ls) {
-        if (active) stockham_stage(x, y, lg, ls, t, twr, twi, +1);
+        if (active) stockham_stage<true>(x, y, lg, ls, t, twr, twi, +1);
         __syncthreads();
         Cx<T> *tmp = x; x = y; y = tmp;
     }
@@ -269,7 +279,8 @@ __global__ void __launch_bounds__(256) k_fft_lines(T *__restrict__ H, size_t hst
         for (int ls = 0; ls < lg; ++ls) {
             for (int q = threadIdx.x; q < nbfly; q += blockDim.x) {
                 const int c = q >> (lg - 1), j = q & ((n >> 1) - 1);
-                stockham_stage(x + (c << lg), y + (c << lg), lg, ls, j, twr, twi, sg);
+                if (sg < 0) stockham_stage<false>(x + (c << lg), y + (c << lg), lg, ls, j, twr, twi, sg);
+                else stockham_stage<true>(x + (c << lg), y + (c << lg), lg, ls, j, twr, twi, sg);
             }
             __syncthreads();
             Cx<T> *tmp = x; x = y; y = tmp;
@@ -385,30 +396,38 @@ __host__ __device__ inline void wall_coef(const WallSpec &w, int sys, int j, int
 }
 
 // Tables of the Thomas recurrence of every (kx, kz) system: per row and mode
-// P = -b/den and 1/den as the sum of two T (Brisebarre, Muller and Raina's
-// division by a known divisor); all three zero where tdma's guard sets P = Q = 0
-// (fenep_2d.f90:1157-1160).  The recurrence runs in FP64 for either T, so the
-// singular mean mode of the pressure is pinned exactly.  Layout [row][kz][kx].
+// P = -b/den and den, in FP64 1/den as the sum of two doubles (Brisebarre, Muller
+// and Raina's division by a known divisor) in the second and third table, in
+// FP32 den itself (an FP32 division is cheap).  Where tdma's guard sets P = Q = 0
+// (fenep_2d.f90:1157-1160): P = 1/den = 0, den = inf.  Layout [row][kz][kx].
 template <typename T>
 __global__ void k_wall_table(T *__restrict__ P, T *__restrict__ rh, T *__restrict__ rl, int ny, int nxh, int nz,
                              WallSpec w, int sys) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nxh * nz) return;
     const double lam = w.kx2[q % nxh] + w.kz2[q / nxh];
-    double p = 0.0;
+    T p = T(0);
     for (int j = 0; j < ny + 2; ++j) {
-        double a, b, cc;
-        wall_coef<double>(w, sys, j, ny, lam, a, b, cc);
-        const double den = j == 0 ? a : a + cc * p;
+        T a, b, cc;
+        wall_coef<T>(w, sys, j, ny, lam, a, b, cc);
+        const T den = j == 0 ? a : a + cc * p;
         const size_t o = (size_t)j * nxh * nz + q;
-        const bool guard = j > 0 && fabs(den) < 1.0e-16;
-        p = guard ? 0.0 : -b / den;
-        const double r = 1.0 / den;
-        P[o] = T(p);
-        rh[o] = guard ? T(0) : T(r);
-        rl[o] = guard ? T(0) : (sizeof(T) == 8 ? T(fma(-den, r, 1.0) / den) : T(r - (double)T(r)));
+        const bool guard = j > 0 && fabs(den) < T(1.0e-16);
+        p = guard ? T(0) : -b / den;
+        P[o] = p;
+        if constexpr (sizeof(T) == 8) {
+            const double r = 1.0 / den;
+            rh[o] = guard ? 0.0 : r;
+            rl[o] = guard ? 0.0 : fma(-den, r, 1.0) / den;
+        } else {
+            rh[o] = guard ? __int_as_float(0x7f800000) : den;
+        }
     }
 }
+
+// t / den with those tables
+__device__ __forceinline__ double wall_div(double t, double h, double l) { return __fma_rn(t, h, __dmul_rn(t, l)); }
+__device__ __forceinline__ float wall_div(float t, float den, float) { return t / den; }
 
 // The wall-normal solves (tdma, fenep_2d.f90:1145-1177) of every mode with
 // those tables.  A thread runs the recurrence of the real or the imaginary part
@@ -446,7 +465,7 @@ __global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *
             if (j >= 1 && j <= ny && !(sys == SYS_V && j == ny)) d[u] = hin[(size_t)2 * nxh * (j - 1)] * inv_nxz;
             else if (j == n - 1 && mode == 0 && c == 0) d[u] = T(it.top);
             h[u] = rh[(size_t)j * modes + mode];
-            l[u] = rl[(size_t)j * modes + mode];
+            if (sizeof(T) == 8) l[u] = rl[(size_t)j * modes + mode];
         }
 #pragma unroll
         for (int u = 0; u < G; ++u) {
@@ -455,7 +474,7 @@ __global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *
             const T cc = j == 0 ? T(0) : (j == n - 1 ? (sys == SYS_U ? T(1) : (sys == SYS_V ? T(0) : T(-1)))
                                                      : (sys == SYS_V && j >= ny ? T(0) : ci));
             const T t = d[u] - cc * q;
-            q = fma(t, h[u], t * l[u]);
+            q = wall_div(t, h[u], l[u]);
             hout[(size_t)2 * nxh * j] = q;
         }
     }

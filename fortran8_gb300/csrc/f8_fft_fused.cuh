@@ -8,12 +8,11 @@
 //   k_xfwd_t   real rows -> S: two rows per complex FFT of length NX (the
 //              same pairing as the FP64 kernels), transposed through shared
 //              memory so that each kx receives RB consecutive rows.
-//   k_plane_*  one CTA per kx: in-place radix-2 transforms along z (and y when
-//              periodic), the spectral divide (fft_solve, fenep.f90:1400-1428)
-//              or the Thomas solve along y (tdma, fenep_2d.f90:1145-1177), and
-//              the inverse transforms.  Forward transforms are decimation in
-//              time (bit-reversed load), inverse ones decimation in frequency
-//              (bit-reversed store), so no reordering pass is needed.
+//   k_plane_*  one CTA (or a cluster) per kx: warp transforms along z (and y
+//              when periodic), the spectral divide (fft_solve, fenep.f90:1400-
+//              1428) or the Thomas solve along y (tdma, fenep_2d.f90:1145-1177),
+//              and the inverse transforms.  Forward transforms leave their
+//              values in bit-reversed order, inverse ones take them so.
 //   k_xinv_t   S -> real rows through a destination functor (XOutF).
 #pragma once
 #include <cooperative_groups.h>
@@ -23,6 +22,11 @@
 namespace f8 {
 
 __device__ inline int bitrev(int v, int lg) { return lg ? (int)(__brev((unsigned)v) >> (32 - lg)) : 0; }
+
+// a * w in packed FP32x2: (fma(ax, wx, -(ay wy)), fma(ax, wy, ay wx))
+__device__ __forceinline__ float2 cmul_p(float2 a, float2 w) {
+    return __ffma2_rn(make_float2(a.x, a.x), w, __fmul2_rn(make_float2(a.y, a.y), make_float2(-w.y, w.x)));
+}
 
 // ---------------------------------------------------------------------------
 // x forward, transposing.  Block b handles RB rows (RB/2 pairs) of plane k.
@@ -49,7 +53,7 @@ __global__ void k_xfwd_t(const TS *__restrict__ src, float2 *__restrict__ S, int
     __syncthreads();
     const int lg = ilog2_pow2(nx);
     for (int ls = 0; ls < lg; ++ls) {
-        if (active) stockham_stage(x, y, lg, ls, t, twr, twi, -1);
+        if (active) stockham_stage<false>(x, y, lg, ls, t, twr, twi, -1);
         __syncthreads();
         Cx<float> *tmp = x; x = y; y = tmp;
     }
@@ -115,7 +119,7 @@ __global__ void k_xinv_t(const float2 *__restrict__ S, Out out, int nx, int nrow
     __syncthreads();
     const int lg = ilog2_pow2(nx);
     for (int ls = 0; ls < lg; ++ls) {
-        if (active) stockham_stage(x, y, lg, ls, t, twr, twi, +1);
+        if (active) stockham_stage<true>(x, y, lg, ls, t, twr, twi, +1);
         __syncthreads();
         Cx<float> *tmp = x; x = y; y = tmp;
     }
@@ -176,53 +180,19 @@ __device__ inline void dif_lines(float2 *P, int n, int nlines, int lstride, int 
     }
 }
 
-// Periodic y and z: forward 2-D transform, divide by ntot * LHS (LHS = lhs0 +
-// lhs1 (kx2 + ky2 + kz2); zero where |LHS| < 1e-16), inverse transform.
-struct PlaneSpec {
-    const float *kx2, *ky2, *kz2;   // modified wavenumbers (FP32 copies)
-    float lhs0, lhs1, inv_ntot;
-    // walls: row coefficients of the y systems (see k_plane_walls)
+// Walls in y, general NZ: coefficients of the y systems
+struct WallPlane {
+    const float *kx2, *kz2;   // modified wavenumbers
     float ai_base, bc;        // interior a = ai_base + kap * lam; b = c = bc
     float kap;                // dt beta / (2 Re) (Helmholtz) or -1 (Poisson: a = -(lam + 2/dy^2))
     int sys;                  // WallSys
     float nxz_inv;            // 1 / (NX NZ)
 };
 
-__global__ void k_plane_periodic(float2 *S, int ny, int nz, int lgy, int lgz, const float *twyr, const float *twyi,
-                                 const float *twzr, const float *twzi, PlaneSpec ps) {
-    extern __shared__ unsigned char smem_raw[];
-    const int nys = ny + 1;                              // odd shared-memory row stride
-    float2 *P = reinterpret_cast<float2 *>(smem_raw);    // [k][j], bit-reversed in both on load
-    const int kx = blockIdx.x;
-    float2 *Sp = S + (size_t)kx * nz * ny;
-    for (int q = threadIdx.x; q < ny * nz; q += blockDim.x) {
-        const int k = q / ny, j = q % ny;
-        P[(size_t)bitrev(k, lgz) * nys + bitrev(j, lgy)] = Sp[q];
-    }
-    __syncthreads();
-    dit_lines(P, ny, lgy, nz, nys, 1, twyr, twyi, 1.0f);     // along y (lines k)
-    dit_lines(P, nz, lgz, ny, 1, nys, twzr, twzi, 1.0f);     // along z (lines j)
-    const float k2x = ps.kx2[kx];
-    for (int q = threadIdx.x; q < ny * nz; q += blockDim.x) {
-        const int k = q / ny, j = q % ny;
-        const float lhs = ps.lhs0 + ps.lhs1 * (k2x + ps.ky2[j] + ps.kz2[k]);
-        const float sc = fabsf(lhs) < 1.0e-16f ? 0.0f : ps.inv_ntot / lhs;
-        const float2 v = P[(size_t)k * nys + j];
-        P[(size_t)k * nys + j] = make_float2(v.x * sc, v.y * sc);
-    }
-    __syncthreads();
-    dif_lines(P, nz, ny, 1, nys, twzr, twzi, -1.0f);
-    dif_lines(P, ny, nz, nys, 1, twyr, twyi, -1.0f);
-    for (int q = threadIdx.x; q < ny * nz; q += blockDim.x) {
-        const int k = q / ny, j = q % ny;
-        Sp[q] = P[(size_t)bitrev(k, lgz) * nys + bitrev(j, lgy)];
-    }
-}
-
 // Walls in y: forward z transform of rows 1..NY, Thomas solve along y of each
 // kz over rows 0..NY+1 with the boundary rows of the system (homogeneous:
 // the mixed path solves for increments), inverse z transform of all rows.
-__global__ void k_plane_walls(float2 *S, int ny, int nz, int lgz, const float *twzr, const float *twzi, PlaneSpec ps) {
+__global__ void k_plane_walls(float2 *S, int ny, int nz, int lgz, const float *twzr, const float *twzi, WallPlane ps) {
     extern __shared__ unsigned char smem_raw[];
     const int lj = ny + 2;
     const int ljs = lj | 1;                                            // odd shared-memory row stride
@@ -295,10 +265,6 @@ __global__ void k_plane_walls(float2 *S, int ny, int nz, int lgz, const float *t
     }
 }
 
-}  // namespace f8
-
-namespace f8 {
-
 // ---------------------------------------------------------------------------
 // Warp-level radix-2 transform of one line of N = 32*V points: lane t holds
 // elements t + 32 s (s < V).  Spans >= 32 are butterflies inside the lane,
@@ -309,10 +275,6 @@ namespace f8 {
 // has lane stride N/(2m)).  The complex arithmetic uses packed FP32x2
 // operations; the cross-lane butterflies are branch-free (the lanes holding
 // the first element of a pair multiply by 1).
-__device__ __forceinline__ float2 cmul_p(float2 a, float2 w) {
-    return __ffma2_rn(make_float2(a.x, a.x), w, __fmul2_rn(make_float2(a.y, a.y), make_float2(-w.y, w.x)));
-}
-
 template <int V>
 __device__ inline void warp_dif_fwd(float2 (&v)[V], const float2 *tw, int lane) {
     constexpr int N = 32 * V;
@@ -384,6 +346,222 @@ __device__ inline void warp_dit_inv(float2 (&v)[V], const float2 *tw, int lane) 
                 v[s] = __ffma2_rn(make_float2(sg, sg), p, o);
             }
         }
+    }
+}
+
+// Periodic y and z: the (z, y) plane of one kx is transformed, divided by
+// ntot * LHS (LHS = lhs0 + lhs1 (kx2 + ky2 + kz2); zero where |LHS| < 1e-16) and
+// transformed back.
+struct PlaneSpec {
+    const float *kx2, *ky2, *kz2;   // modified wavenumbers (FP32 copies)
+    const float2 *twy, *twz;        // stage-major twiddles
+    float lhs0, lhs1, inv_ntot;
+};
+
+// lanes per line, lines per warp and elements per lane of an N-point line (with
+// N < 32 a warp holds 32 / N lines of N consecutive lanes)
+template <int N>
+struct LineOf {
+    static constexpr int V = N >= 32 ? N / 32 : 1, L = N >= 32 ? 32 : N, W = 32 / L;
+};
+template <int N>
+__device__ __forceinline__ int line_brev(int e) {
+    constexpr int LG = N == 4 ? 2 : N == 8 ? 3 : N == 16 ? 4 : N == 32 ? 5 : N == 64 ? 6 : N == 128 ? 7 : N == 256 ? 8 : 9;
+    return (int)(__brev((unsigned)e) >> (32 - LG));
+}
+
+// Forward transform, decimation in time: the value at position p of the line
+// (lane p % 32, element p / 32) is that of index brev(p); out in natural order.
+// In the butterflies a + b w, a - b w the lanes holding b multiply before the
+// exchange.
+template <int N>
+__device__ __forceinline__ void line_dit_fwd(float2 (&v)[LineOf<N>::V], const float2 *tw, int lane) {
+    constexpr int V = LineOf<N>::V;
+#pragma unroll
+    for (int m = 1; m < N; m <<= 1) {
+        const float2 *tm = tw + (m - 1);
+        if (m >= 32) {
+            const int sm = m / 32;
+#pragma unroll
+            for (int s = 0; s < V; ++s) {
+                if ((s / sm) % 2) continue;
+                const float2 t = cmul_p(v[s + sm], tm[(lane + 32 * s) % (2 * m)]), a = v[s];
+                v[s] = __fadd2_rn(a, t);
+                v[s + sm] = make_float2(a.x - t.x, a.y - t.y);
+            }
+        } else {
+            const bool second = lane & m;
+            const float2 w = tm[lane & (m - 1)];
+#pragma unroll
+            for (int s = 0; s < V; ++s) {
+                const float2 t = cmul_p(v[s], w);
+                const float2 p = second ? t : v[s];
+                const float ox = __shfl_xor_sync(0xffffffffu, p.x, m), oy = __shfl_xor_sync(0xffffffffu, p.y, m);
+                v[s] = second ? make_float2(ox - p.x, oy - p.y) : make_float2(p.x + ox, p.y + oy);
+            }
+        }
+    }
+}
+
+// d * conj(w) with the sum's fused product as twiddle_mul<true> has it
+__device__ __forceinline__ float2 cmul_conj(float2 d, float2 w) {
+    return __ffma2_rn(d, make_float2(w.x, w.x), __fmul2_rn(make_float2(d.y, d.x), make_float2(w.y, -w.y)));
+}
+
+// Inverse transform, decimation in frequency: natural order in, the value at
+// position p is that of index brev(p)
+template <int N>
+__device__ __forceinline__ void line_dif_inv(float2 (&v)[LineOf<N>::V], const float2 *tw, int lane) {
+    constexpr int V = LineOf<N>::V;
+#pragma unroll
+    for (int m = N / 2; m >= 1; m >>= 1) {
+        const float2 *tm = tw + (m - 1);
+        if (m >= 32) {
+            const int sm = m / 32;
+#pragma unroll
+            for (int s = 0; s < V; ++s) {
+                if ((s / sm) % 2) continue;
+                const float2 a = v[s], b = v[s + sm];
+                v[s] = __fadd2_rn(a, b);
+                v[s + sm] = cmul_conj(make_float2(a.x - b.x, a.y - b.y), tm[(lane + 32 * s) % (2 * m)]);
+            }
+        } else {
+            const bool second = lane & m;
+            const float2 w = tm[lane & (m - 1)];
+#pragma unroll
+            for (int s = 0; s < V; ++s) {
+                const float ox = __shfl_xor_sync(0xffffffffu, v[s].x, m), oy = __shfl_xor_sync(0xffffffffu, v[s].y, m);
+                const float2 t = cmul_conj(make_float2(ox - v[s].x, oy - v[s].y), w);
+                v[s] = second ? t : make_float2(v[s].x + ox, v[s].y + oy);
+            }
+        }
+    }
+}
+
+// rows: global -> transform along y -> shared memory, row k at brev(k) for the
+// z transform
+template <int N>
+__device__ __forceinline__ void plane_y_fwd(const float2 *Sp, float2 *P, int nz, int lgz, int nys, const float2 *tw) {
+    using T = LineOf<N>;
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, e = lane & (T::L - 1);
+    for (int k0 = (threadIdx.x >> 5) * T::W; k0 < nz; k0 += nw * T::W) {
+        const int k = k0 + lane / T::L;
+        float2 v[T::V];
+#pragma unroll
+        for (int s = 0; s < T::V; ++s) v[s] = k < nz ? Sp[k * N + line_brev<N>(e + 32 * s)] : make_float2(0.0f, 0.0f);
+        line_dit_fwd<N>(v, tw, lane);
+        if (k < nz) {
+            float2 *row = P + bitrev(k, lgz) * nys;
+#pragma unroll
+            for (int s = 0; s < T::V; ++s) row[e + 32 * s] = v[s];
+        }
+    }
+}
+
+// columns: transform along z, divide, transform back, in registers
+template <int N>
+__device__ __forceinline__ void plane_z(float2 *P, int ny, int nys, const float2 *tw, const float *kxy, const float *kz2,
+                                        float lhs0, float lhs1, float inv_ntot) {
+    using T = LineOf<N>;
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, e = lane & (T::L - 1);
+    for (int j0 = (threadIdx.x >> 5) * T::W; j0 < ny; j0 += nw * T::W) {
+        const int j = j0 + lane / T::L;
+        float2 v[T::V];
+#pragma unroll
+        for (int s = 0; s < T::V; ++s) v[s] = j < ny ? P[(e + 32 * s) * nys + j] : make_float2(0.0f, 0.0f);
+        line_dit_fwd<N>(v, tw, lane);
+        const float ky = j < ny ? kxy[j] : 0.0f;
+#pragma unroll
+        for (int s = 0; s < T::V; ++s) {
+            const float lhs = __fmaf_rn(lhs1, __fadd_rn(ky, kz2[e + 32 * s]), lhs0);
+            const float sc = fabsf(lhs) < 1.0e-16f ? 0.0f : inv_ntot / lhs;
+            v[s] = make_float2(v[s].x * sc, v[s].y * sc);
+        }
+        line_dif_inv<N>(v, tw, lane);
+        if (j < ny)
+#pragma unroll
+            for (int s = 0; s < T::V; ++s) P[(e + 32 * s) * nys + j] = v[s];
+    }
+}
+
+// rows: shared memory -> inverse transform along y -> global (row r holds
+// plane brev(r))
+template <int N>
+__device__ __forceinline__ void plane_y_inv(float2 *Sp, const float2 *P, int nz, int lgz, int nys, const float2 *tw) {
+    using T = LineOf<N>;
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, e = lane & (T::L - 1);
+    for (int r0 = (threadIdx.x >> 5) * T::W; r0 < nz; r0 += nw * T::W) {
+        const int r = r0 + lane / T::L;
+        float2 v[T::V];
+#pragma unroll
+        for (int s = 0; s < T::V; ++s) v[s] = r < nz ? P[r * nys + e + 32 * s] : make_float2(0.0f, 0.0f);
+        line_dif_inv<N>(v, tw, lane);
+        if (r < nz) {
+            float2 *row = Sp + bitrev(r, lgz) * N;
+#pragma unroll
+            for (int s = 0; s < T::V; ++s) row[line_brev<N>(e + 32 * s)] = v[s];
+        }
+    }
+}
+
+// shared memory: the plane (rows of ny + 1, an odd stride), both twiddle tables
+// and both wavenumber tables
+inline size_t plane_periodic_smem(int ny, int nz) { return (size_t)8 * (ny + 1) * nz + (size_t)12 * (ny + nz); }
+
+// Warp transforms of whole lines: the plane passes shared memory twice (after
+// the y transform and after the z round trip) where radix-2 stages in shared
+// memory passed it once per stage; the butterflies and their order are the
+// same, and so are the bits.  One CTA per kx (nx/2 + 1 of 152 SMs).  Step of a
+// 64^3 box: 199 us with the stages in shared memory (33.8 us a launch), 126 now.
+__global__ void __launch_bounds__(1024, 1) k_plane_periodic(float2 *S, int ny, int nz, int lgy, int lgz, PlaneSpec ps) {
+    extern __shared__ unsigned char smem_raw[];
+    const int nys = ny + 1;
+    float2 *P = reinterpret_cast<float2 *>(smem_raw);    // [k][j]
+    float2 *twy = P + (size_t)nys * nz, *twz = twy + ny;
+    float *kxy = reinterpret_cast<float *>(twz + nz), *kz2 = kxy + ny;
+    const int kx = blockIdx.x;
+    float2 *Sp = S + (size_t)kx * nz * ny;
+    const float k2x = ps.kx2[kx];
+    for (int q = threadIdx.x; q < ny; q += blockDim.x) {
+        twy[q] = ps.twy[q];
+        kxy[q] = k2x + ps.ky2[q];
+    }
+    for (int q = threadIdx.x; q < nz; q += blockDim.x) {
+        twz[q] = ps.twz[q];
+        kz2[q] = ps.kz2[q];
+    }
+    __syncthreads();
+    switch (lgy) {
+    case 2: plane_y_fwd<4>(Sp, P, nz, lgz, nys, twy); break;
+    case 3: plane_y_fwd<8>(Sp, P, nz, lgz, nys, twy); break;
+    case 4: plane_y_fwd<16>(Sp, P, nz, lgz, nys, twy); break;
+    case 5: plane_y_fwd<32>(Sp, P, nz, lgz, nys, twy); break;
+    case 6: plane_y_fwd<64>(Sp, P, nz, lgz, nys, twy); break;
+    case 7: plane_y_fwd<128>(Sp, P, nz, lgz, nys, twy); break;
+    case 8: plane_y_fwd<256>(Sp, P, nz, lgz, nys, twy); break;
+    default: plane_y_fwd<512>(Sp, P, nz, lgz, nys, twy); break;
+    }
+    __syncthreads();
+    switch (lgz) {
+    case 2: plane_z<4>(P, ny, nys, twz, kxy, kz2, ps.lhs0, ps.lhs1, ps.inv_ntot); break;
+    case 3: plane_z<8>(P, ny, nys, twz, kxy, kz2, ps.lhs0, ps.lhs1, ps.inv_ntot); break;
+    case 4: plane_z<16>(P, ny, nys, twz, kxy, kz2, ps.lhs0, ps.lhs1, ps.inv_ntot); break;
+    case 5: plane_z<32>(P, ny, nys, twz, kxy, kz2, ps.lhs0, ps.lhs1, ps.inv_ntot); break;
+    case 6: plane_z<64>(P, ny, nys, twz, kxy, kz2, ps.lhs0, ps.lhs1, ps.inv_ntot); break;
+    case 7: plane_z<128>(P, ny, nys, twz, kxy, kz2, ps.lhs0, ps.lhs1, ps.inv_ntot); break;
+    case 8: plane_z<256>(P, ny, nys, twz, kxy, kz2, ps.lhs0, ps.lhs1, ps.inv_ntot); break;
+    default: plane_z<512>(P, ny, nys, twz, kxy, kz2, ps.lhs0, ps.lhs1, ps.inv_ntot); break;
+    }
+    __syncthreads();
+    switch (lgy) {
+    case 2: plane_y_inv<4>(Sp, P, nz, lgz, nys, twy); break;
+    case 3: plane_y_inv<8>(Sp, P, nz, lgz, nys, twy); break;
+    case 4: plane_y_inv<16>(Sp, P, nz, lgz, nys, twy); break;
+    case 5: plane_y_inv<32>(Sp, P, nz, lgz, nys, twy); break;
+    case 6: plane_y_inv<64>(Sp, P, nz, lgz, nys, twy); break;
+    case 7: plane_y_inv<128>(Sp, P, nz, lgz, nys, twy); break;
+    case 8: plane_y_inv<256>(Sp, P, nz, lgz, nys, twy); break;
+    default: plane_y_inv<512>(Sp, P, nz, lgz, nys, twy); break;
     }
 }
 
@@ -537,7 +715,7 @@ __global__ void __launch_bounds__(32 * XW_WARPS) k_xinv_w(const float2 *__restri
 // system scan the composed maps with shuffles, the CTAs of the cluster
 // exchange their composed maps through distributed shared memory, and each
 // thread then replays its chunk from its incoming value.  The coefficients
-// are those of the sequential Thomas solve of k_plane_walls (tdma,
+// are those of the sequential Thomas solve (tdma,
 // fenep_2d.f90:1145-1177); the 1/den table of the CTA's rows is staged in
 // shared memory, its rows in the bit-reversed kz order of the spectrum rows.
 // The cluster barriers are hardware barriers; no thread waits on a flag.

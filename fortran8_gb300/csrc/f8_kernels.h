@@ -39,6 +39,7 @@ struct Dev {
     int *csr_off[3], *csr_idx[3];          // per component over (SX*SY) columns
     int *mperm, *moff;                     // markers grouped by cylinder (drag reduction)
     double *dragpart;                      // ncyl * nz * 3 partial sums
+    unsigned *dragcnt;                     // per cylinder: blocks of k_drag that are done (back to 0 by itself)
     double *mvol;                          // per marker: the volume its force is spread with
     double *cylvol;                        // per cylinder: the marker volume of its drag
     int ibm_repeats;                       // direct-forcing iterations per step (NS)
@@ -64,15 +65,16 @@ struct Dev {
                                            // beside the U solve (fused spectral path)
     cudaStream_t aux[2];                   // the side streams of those two solves (0: none)
     cudaEvent_t ev_fork, ev_join[2];
-    cudaEvent_t ev_g[4];                   // wall ghost-row branch: start, codes ready, update done, momentum done
+    cudaEvent_t ev_g[6];                   // wall ghost-row branch: start, codes ready, update done, momentum done;
+                                           // drag branch: forces ready, drag done
     float *twxf_r, *twxf_i, *twyf_r, *twyf_i, *twzf_r, *twzf_i;
     float *kx2f, *ky2f, *kz2f;             // FP32 copies of the modified wavenumbers
-    int fused_planes;                      // 1: (z, y) plane of one kx fits in shared memory
+    int fused_planes;                      // 1: (z, y) plane of one kx fits in shared memory and has a kernel
     int plane_cl;                          // walls: CTAs per cluster holding one (z, y) plane (0: none)
     WallLayout plane_wl;                   // its shared-memory layout (wall_layout)
     int march_runs, march_ctas;            // staged projection: z runs per y tile, persistent CTAs (0: direct loads)
     int march_depth;                       // its steps of copies in flight
-    float2 *twz2;                          // stage-major twiddles of the warp z transforms (NZ entries)
+    float2 *twz2, *twy2;                   // stage-major twiddles of the warp z and y transforms (NZ, NY entries)
     float2 *twx2;                          // and of the warp x transforms (NX entries)
     float *wtR[3];                         // Thomas 1/den tables of the U, V, P wall systems
     float *mwx[3], *mwy[3];                // per-marker 1D kernel weights (3 each)
@@ -257,6 +259,7 @@ cudaError_t take_interior_f(const float *src, float *dst, const Geo &g, int n, c
 cudaError_t init_kernels_mixed();
 cudaError_t wall_tables_mixed(Dev &d, cudaStream_t s);
 cudaError_t setup_sor_mixed(Dev &d);
+bool periodic_plane_fits(int ny, int nz, size_t limit);   // k_plane_periodic takes such a plane
 cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_iters, cudaStream_t s);
 cudaError_t bc_all_state_mixed(Dev &d, cudaStream_t s);
 cudaError_t mixed_state_to_fp64(Dev &d, cudaStream_t s);

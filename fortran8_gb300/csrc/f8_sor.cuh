@@ -84,7 +84,24 @@ struct SorArgs {
     int itrmax, lgx, lgy;   // log2 of nx / 2 and ny
 };
 
-__device__ __forceinline__ float sor_update(float phi, float e, const SorArgs<float> &a) { return phi + a.om * e / a.b0; }
+// the residual, summed in the reference's order (fenep.f90:885-893); FP32: with
+// the products fused into the sum, the same in both forms of the kernel
+__device__ __forceinline__ double sor_residual(const SorArgs<double> &a, double zm, double ym, double xm, double p0,
+                                               double xp, double yp, double zp, double f) {
+    return a.bz * zm + a.by * ym + a.bx * xm - a.b0 * p0 + a.bx * xp + a.by * yp + a.bz * zp - f;
+}
+__device__ __forceinline__ float sor_residual(const SorArgs<float> &a, float zm, float ym, float xm, float p0, float xp,
+                                              float yp, float zp, float f) {
+    float e = __fmaf_rn(a.bz, zm, __fmul_rn(a.by, ym));
+    e = __fmaf_rn(a.bx, xm, e);
+    e = __fmaf_rn(-a.b0, p0, e);
+    e = __fmaf_rn(a.bx, xp, e);
+    e = __fmaf_rn(a.by, yp, e);
+    return __fsub_rn(__fmaf_rn(a.bz, zp, e), f);
+}
+__device__ __forceinline__ float sor_update(float phi, float e, const SorArgs<float> &a) {
+    return __fadd_rn(phi, __fmul_rn(a.om, e) / a.b0);
+}
 // the division by the known divisor b0 from its two-part reciprocal (2 FP64
 // slots; Brisebarre, Muller and Raina, IEEE Trans. Comput. 53 (2004) 1069)
 __device__ __forceinline__ double sor_update(double phi, double e, const SorArgs<double> &a) {
@@ -158,8 +175,8 @@ __global__ void __launch_bounds__(SOR_THREADS, 1) k_sor_grid(SorArgs<T> a, Geo g
                 const int ym = j > 1 ? -oy : (g.walls ? 0 : (g.ny - 1) * oy), yp = j < g.ny ? oy : (g.walls ? 0 : (1 - g.ny) * oy);
                 const int zm = k > 1 ? -oz : (g.nz - 1) * oz, zp = k < g.nz ? oz : (1 - g.nz) * oz;
                 const T p0 = __ldcg(P);
-                const T e = a.bz * __ldcg(P + zm) + a.by * __ldcg(P + ym) + a.bx * __ldcg(P + xm) - a.b0 * p0
-                            + a.bx * __ldcg(P + xp) + a.by * __ldcg(P + yp) + a.bz * __ldcg(P + zp) - a.R[q];
+                const T e = sor_residual(a, __ldcg(P + zm), __ldcg(P + ym), __ldcg(P + xm), p0, __ldcg(P + xp),
+                                         __ldcg(P + yp), __ldcg(P + zp), a.R[q]);
                 s.add_sq(e);
                 __stcg(a.Phi + h, sor_update(p0, e, a));
             }
@@ -287,8 +304,7 @@ __global__ void __launch_bounds__(SOR_CLUSTER_THREADS, 1) k_sor_cluster(SorArgs<
                 const float xm = o ? xi : xo, xp = o ? xo : xi;
                 const float p0 = pv[t][color];
                 const float ym = dn[t] ? at[dn[t]] : p0, yp = up[t] ? at[up[t]] : p0;
-                const float e = a.bz * at[-plane] + a.by * ym + a.bx * xm - a.b0 * p0 + a.bx * xp + a.by * yp
-                                + a.bz * at[plane] - rv[t][color];
+                const float e = sor_residual(a, at[-plane], ym, xm, p0, xp, yp, at[plane], rv[t][color]);
                 s.add_sq(e);
                 const float v = sor_update(p0, e, a);
                 pv[t][color] = v;

@@ -1259,44 +1259,45 @@ __global__ void k_ibm_spread_q(IbmArgs a, Geo g) {
     a.Q[comp][o] = a.Ua[comp][h] + dt * fz - dt * a.B[comp][o] / 2;
 }
 
-// drag of each cylinder: -sum(Fc) * dv per component.  Stage 1: block
-// (l, n) sums the forces of cylinder l's markers on plane n (markers listed
-// per cylinder in mperm, ranges moff); stage 2 sums the planes.  Fixed tree
-// orders make the result deterministic.
-__global__ void k_drag_part(const double *Fx, const double *Fy, const double *Fz, const int *mperm, const int *moff,
-                            int nm, int ncomp, double *part) {
+// drag of each cylinder: -sum(Fc) * dv per component.  Block (l, n) sums the
+// forces of cylinder l's markers on plane n (markers listed per cylinder in
+// mperm, ranges moff); the cylinder's last block to finish sums the planes.
+// Fixed tree orders make the result deterministic.
+__device__ inline void drag_tree(double (&sh)[3][256], const double (&s)[3]) {
+    for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = s[c];
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w)
+            for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + w];
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(256) k_drag(const double *Fx, const double *Fy, const double *Fz, const int *mperm,
+                                              const int *moff, int nm, int ncomp, double *part, unsigned *done,
+                                              const double *cylvol, double *out) {
     const int l = blockIdx.x, n = blockIdx.y, nz = gridDim.y;
     __shared__ double sh[3][256];
+    __shared__ bool last;
     double s[3] = {0.0, 0.0, 0.0};
     const double *F[3] = {Fx, Fy, Fz};
     for (int q = moff[l] + threadIdx.x; q < moff[l + 1]; q += blockDim.x) {
         const size_t o = (size_t)mperm[q] + (size_t)nm * n;
         for (int c = 0; c < ncomp; ++c) s[c] += F[c][o];
     }
-    for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = s[c];
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
+    drag_tree(sh, s);
+    if (threadIdx.x == 0) {
         for (int c = 0; c < 3; ++c) part[((size_t)l * nz + n) * 3 + c] = sh[c][0];
-}
-
-__global__ void k_drag_final(const double *part, int nz, int ncomp, const double *cylvol, double *out) {
-    const int l = blockIdx.x;
-    __shared__ double sh[3][256];
-    double s[3] = {0.0, 0.0, 0.0};
-    for (int n = threadIdx.x; n < nz; n += blockDim.x)
-        for (int c = 0; c < 3; ++c) s[c] += part[((size_t)l * nz + n) * 3 + c];
-    for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = s[c];
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + w];
-        __syncthreads();
+        __threadfence();
+        last = atomicInc(&done[l], nz - 1) == (unsigned)(nz - 1);   // wraps to 0 for the next launch
+        __threadfence();
     }
+    __syncthreads();
+    if (!last) return;
+    for (int c = 0; c < 3; ++c) s[c] = 0.0;
+    for (int p = threadIdx.x; p < nz; p += blockDim.x)
+        for (int c = 0; c < 3; ++c) s[c] += __ldcg(&part[((size_t)l * nz + p) * 3 + c]);
+    drag_tree(sh, s);
     if (threadIdx.x == 0)
         for (int c = 0; c < 3; ++c) out[3 * l + c] = c < ncomp ? -sh[c][0] * cylvol[l] : 0.0;
 }
@@ -1579,8 +1580,8 @@ cudaError_t marker_weights_fp64(Dev &d, cudaStream_t s) {
 cudaError_t launch_drag(Dev &d, double *out, cudaStream_t s) {
     const Geo &g = d.g;
     const bool d3 = g.dim == 3;
-    k_drag_part<<<dim3(d.ncyl, g.nz), 256, 0, s>>>(d.Fc[0], d.Fc[1], d.Fc[2], d.mperm, d.moff, d.nm, d3 ? 3 : 2, d.dragpart); count_launch();
-    k_drag_final<<<d.ncyl, 256, 0, s>>>(d.dragpart, g.nz, d3 ? 3 : 2, d.cylvol, out); count_launch();
+    k_drag<<<dim3(d.ncyl, g.nz), 256, 0, s>>>(d.Fc[0], d.Fc[1], d.Fc[2], d.mperm, d.moff, d.nm, d3 ? 3 : 2, d.dragpart,
+                                              d.dragcnt, d.cylvol, out); count_launch();
     return cudaGetLastError();
 }
 

@@ -1914,19 +1914,21 @@ cudaError_t solve_periodic_fused(Dev &d, const TS *src, XOutF out, float lhs0, f
     const int nx = g.nx, ny = g.ny, nz = g.nz, nxh = nx / 2 + 1;
     float2 *S = reinterpret_cast<float2 *>(spec ? spec : d.Hf);
     const int rb = x_rows_per_block(nx);
-    const int thr = (rb / 2) * (nx / 2);
+    const int thrx = (rb / 2) * (nx / 2);
     const size_t smx = x_smem(nx, rb);
     const int bpp = (ny + rb - 1) / rb;
     if (!xfwd_warp<TS>(d, src, S, ny, ny, -1, s)) {
-        k_xfwd_t<TS><<<bpp * nz, thr, smx, s>>>(src, S, nx, ny, nz, rb, ny, -1, d.twxf_r, d.twxf_i); count_launch();
+        k_xfwd_t<TS><<<bpp * nz, thrx, smx, s>>>(src, S, nx, ny, nz, rb, ny, -1, d.twxf_r, d.twxf_i); count_launch();
     }
     PlaneSpec ps{};
     ps.kx2 = d.kx2f; ps.ky2 = d.ky2f; ps.kz2 = d.kz2f;
     ps.lhs0 = lhs0; ps.lhs1 = lhs1; ps.inv_ntot = (float)(1.0 / ((double)nx * ny * nz));
-    k_plane_periodic<<<nxh, 1024, (size_t)8 * (ny + 1) * nz, s>>>(S, ny, nz, ilog2(ny), ilog2(nz), d.twyf_r, d.twyf_i,
-                                                                 d.twzf_r, d.twzf_i, ps); count_launch();
+    ps.twy = d.twy2; ps.twz = d.twz2;
+    // a warp per line (32 / N short ones) of the longer phase
+    const int thr = std::max(128, std::min(1024, 32 * std::max(nz / std::max(1, 32 / ny), ny / std::max(1, 32 / nz))));
+    k_plane_periodic<<<nxh, thr, plane_periodic_smem(ny, nz), s>>>(S, ny, nz, ilog2(ny), ilog2(nz), ps); count_launch();
     if (!xinv_warp(d, S, out, ny, 1, ny, -1, s)) {
-        k_xinv_t<XOutF><<<bpp * nz, thr, smx, s>>>(S, out, nx, ny, 1, nz, rb, ny, -1, g.sx, g.sy, d.twxf_r, d.twxf_i); count_launch();
+        k_xinv_t<XOutF><<<bpp * nz, thrx, smx, s>>>(S, out, nx, ny, 1, nz, rb, ny, -1, g.sx, g.sy, d.twxf_r, d.twxf_i); count_launch();
     }
     return cudaGetLastError();
 }
@@ -1942,18 +1944,12 @@ cudaError_t solve_walls_fused(Dev &d, const TS *src, XOutF out, int sys, cudaStr
     if (!xfwd_warp<TS>(d, src, S, ny, lj, 0, s)) {
         k_xfwd_t<TS><<<((ny + rb - 1) / rb) * nz, thr, smx, s>>>(src, S, nx, ny, nz, rb, lj, 0, d.twxf_r, d.twxf_i); count_launch();
     }
-    PlaneSpec ps{};
-    ps.kx2 = d.kx2f; ps.ky2 = d.ky2f; ps.kz2 = d.kz2f;
     const double kap = d.ph.dt * d.ph.beta / d.ph.re / 2.0, idy2 = 1.0 / (g.dy * g.dy);
-    ps.sys = sys;
-    ps.nxz_inv = (float)(1.0 / ((double)nx * nz));
-    if (sys == SYS_P) { ps.ai_base = (float)(2.0 * idy2); ps.bc = (float)idy2; ps.kap = -1.0f; }
-    else { ps.ai_base = (float)(1.0 + kap * 2.0 * idy2); ps.bc = (float)(-kap * idy2); ps.kap = (float)kap; }
-    const size_t smp = (size_t)12 * (lj | 1) * nz;
-    if (d.plane_cl > 0 && d.wtR[0]) {
+    if (d.plane_cl > 0) {
         const int t = sys == SYS_P ? 2 : (sys == SYS_V ? 1 : 0);
         const float b_first = sys == SYS_P ? -1.0f : (sys == SYS_V ? 0.0f : 1.0f);
-        WallTables wt{d.wtR[t], ps.bc, sys == SYS_P ? -1.0f : 1.0f, b_first, ps.nxz_inv, sys, d.plane_wl};
+        const WallTables wt{d.wtR[t], (float)(sys == SYS_P ? idy2 : -kap * idy2), sys == SYS_P ? -1.0f : 1.0f, b_first,
+                            (float)(1.0 / ((double)nx * nz)), sys, d.plane_wl};
         const int cl = d.plane_cl;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(nxh * cl));
@@ -1975,7 +1971,13 @@ cudaError_t solve_walls_fused(Dev &d, const TS *src, XOutF out, int sys, cudaStr
         count_launch();
         if (e) return e;
     } else {
-        k_plane_walls<<<nxh, 1024, smp, s>>>(S, ny, nz, ilog2(nz), d.twzf_r, d.twzf_i, ps); count_launch();
+        WallPlane ps{};
+        ps.kx2 = d.kx2f; ps.kz2 = d.kz2f;
+        ps.sys = sys;
+        ps.nxz_inv = (float)(1.0 / ((double)nx * nz));
+        if (sys == SYS_P) { ps.ai_base = (float)(2.0 * idy2); ps.bc = (float)idy2; ps.kap = -1.0f; }
+        else { ps.ai_base = (float)(1.0 + kap * 2.0 * idy2); ps.bc = (float)(-kap * idy2); ps.kap = (float)kap; }
+        k_plane_walls<<<nxh, 1024, (size_t)12 * (lj | 1) * nz, s>>>(S, ny, nz, ilog2(nz), d.twzf_r, d.twzf_i, ps); count_launch();
     }
     if (!xinv_warp(d, S, out, lj, 0, lj, 0, s)) {
         k_xinv_t<XOutF><<<((lj + rb - 1) / rb) * nz, thr, smx, s>>>(S, out, nx, lj, 0, nz, rb, lj, 0, g.sx, g.sy,
@@ -2127,6 +2129,10 @@ cudaError_t setup_staged_projection(Dev &d) {
     d.march_ctas = std::min(nsm, ntiles * best);
     d.march_depth = depth;
     return cudaSuccess;
+}
+
+bool periodic_plane_fits(int ny, int nz, size_t limit) {
+    return ny <= 512 && nz >= 4 && nz <= 512 && plane_periodic_smem(ny, nz) <= limit;
 }
 
 cudaError_t setup_sor_mixed(Dev &d) { return sor_cluster_size(&d.sor_cluster); }
@@ -2481,10 +2487,19 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
                     F8_CUDA_RET(cudaMemcpyAsync(d.Qpre[c], d.Qf[c], (size_t)d.ni * sizeof(float), cudaMemcpyDeviceToDevice, s));
             dim3 gi((d.nm + 31) / 32, g.nz, nvc);
             k_ibm_interp_f<<<gi, dim3(32, 3), 0, s>>>(a, g); count_launch();
+            // the drag needs only the marker forces: beside the spreading and
+            // the solves (joined after the solves)
+            const bool want_drag = last && drag_out_dev;
+            if (want_drag && d.aux[1]) {
+                F8_CUDA_RET(cudaEventRecord(d.ev_g[4], s));
+                F8_CUDA_RET(cudaStreamWaitEvent(d.aux[1], d.ev_g[4], 0));
+                F8_CUDA_RET(launch_drag(d, drag_out_dev, d.aux[1]));
+                F8_CUDA_RET(cudaEventRecord(d.ev_g[5], d.aux[1]));
+            }
             int maxact = 0;
             for (int c = 0; c < nvc; ++c) maxact = std::max(maxact, d.nact[c]);
             if (maxact > 0) { k_ibm_spread_f<<<dim3((maxact + 127) / 128, g.nz, nvc), 128, 0, s>>>(a, g); count_launch(); }
-            if (last && drag_out_dev) F8_CUDA_RET(launch_drag(d, drag_out_dev, s));
+            if (want_drag && !d.aux[1]) F8_CUDA_RET(launch_drag(d, drag_out_dev, s));
             if ((e = cudaGetLastError())) return e;
             if (tp && last)
                 for (int c = 0; c < 3; ++c)
@@ -2494,6 +2509,7 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
         if (r == 0) mark(4);
         // Helmholtz solves for the FP32 increments dU (U* = U^n + dU)
         if ((e = mixed_helmholtz(d, nvc, d.Qf, d.dUf, s))) return e;
+        if (o.ibm && r == repeats - 1 && drag_out_dev && d.aux[1]) F8_CUDA_RET(cudaStreamWaitEvent(s, d.ev_g[5], 0));
         if (tp) {
             const TapeUp a{{d.Uf, d.Vf, d.Wf}, {d.dUf[0], d.dUf[1], d.dUf[2]}, {tp->Up[0], tp->Up[1], tp->Up[2]}};
             k_tape_up<<<dim3(tnb, 3), 256, 0, s>>>(a, g); count_launch();

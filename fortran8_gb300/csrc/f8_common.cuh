@@ -108,13 +108,14 @@ __device__ inline bool halo_cell(const Geo &g, long tl, int &i, int &j, int &k) 
 // Shared-memory layout of the wall-plane kernel for R rows per CTA and T
 // threads per (kx, kz) system: the row stride ps (float2) of the spectrum
 // tile, the row stride rs (float) of the pivot table and the rows L per
-// thread of the scan-parallel Thomas solve (L >= ceil(R / T)).  The thread
-// (row, t) = (lane / T, lane % T) of the solve touches row * stride + t * L +
-// it at step it; the layout minimises the wavefronts of those accesses: a
-// 64-bit access takes one wavefront per half-warp whose 16 lanes hit distinct
-// 8-byte bank pairs, a 32-bit access one per warp on 32 distinct banks.  ps
-// stays odd, which keeps the z transforms' accesses (lane stride ps) free of
-// conflicts.  Evaluated once per context on the host.
+// thread of the scan-parallel Thomas solve (L >= ceil(R / T)).  The search
+// minimises the wavefronts of a solve whose thread (row, t) = (lane / T,
+// lane % T) touches row * stride + t * L + it at step it: a 64-bit access takes
+// one wavefront per half-warp whose 16 lanes hit distinct 8-byte bank pairs, a
+// 32-bit access one per warp on 32 distinct banks.  The kernel's lanes are the
+// rows of one chunk now, free of conflicts with any odd stride (ps is odd for
+// the z transforms, too), and the search stays for L: the chunks fix the
+// rounding of the solve.  Evaluated once per context on the host.
 struct WallLayout {
     int ps, rs, L;
 };
@@ -161,13 +162,25 @@ inline size_t wall_plane_smem(const WallLayout &wl, int nz) {
     return (size_t)8 * wl.ps * nz + (size_t)4 * wl.rs * nz + (size_t)nz * 8 + (size_t)24 * nz;
 }
 
+// The scan of the composed maps of a system's chunks (3 floats per thread, the
+// rows of a chunk NZ / 32 apart) lies in the spectrum tile, whose values are in
+// registers then, or behind the maps where the tile is smaller.
+constexpr int WALL_SCAN = 3 * (1024 + 32);
+// rows of a chunk held in registers: wall_layout's L is at most 21 where a
+// plane fits (R NZ <= 19370 and 1024 threads)
+constexpr int WALL_CHUNK = 21;
+__host__ __device__ inline bool wall_scan_in_plane(int ps, int nz) { return 2 * ps * nz >= WALL_SCAN; }
+inline size_t wall_kernel_smem(const WallLayout &wl, int nz) {
+    return wall_plane_smem(wl, nz) + (wall_scan_in_plane(wl.ps, nz) ? 0 : 4 * (size_t)WALL_SCAN);
+}
+
 // the layout of least cost whose shared memory fits in `limit` bytes (ps = 0:
 // none fits)
 inline WallLayout wall_layout(int R, int T, int nz, size_t limit) {
     const int L0 = (R + T - 1) / T;
     WallLayout best{0, 0, 0};
     long bc = -1;
-    for (int L = L0; L < L0 + 12; ++L)
+    for (int L = L0; L < L0 + 12 && L <= WALL_CHUNK; ++L)
         for (int ps = R | 1; ps < (R | 1) + 16; ps += 2)      // ps matters modulo 16 (8-byte pairs)
             for (int rs = R; rs < R + 32; ++rs) {             // rs modulo 32
                 if (wall_plane_smem(WallLayout{ps, rs, L}, nz) > limit) continue;

@@ -8,7 +8,8 @@
 //   k_xfwd_t   real rows -> S: two rows per complex FFT of length NX (the
 //              same pairing as the FP64 kernels), transposed through shared
 //              memory so that each kx receives RB consecutive rows.
-//   k_plane_*  one CTA (or a cluster) per kx: warp transforms along z (and y
+//   k_xfwd_w, k_xinv_w   the x passes of NX = 32 .. 512 in registers
+//   k_plane_*  one CTA (or a cluster) per kx: transforms along z (and y
 //              when periodic), the spectral divide (fft_solve, fenep.f90:1400-
 //              1428) or the Thomas solve along y (tdma, fenep_2d.f90:1145-1177),
 //              and the inverse transforms.  Forward transforms leave their
@@ -23,9 +24,11 @@ namespace f8 {
 
 __device__ inline int bitrev(int v, int lg) { return lg ? (int)(__brev((unsigned)v) >> (32 - lg)) : 0; }
 
-// a * w in packed FP32x2: (fma(ax, wx, -(ay wy)), fma(ax, wy, ay wx))
+// a * w: (fma(ax, wx, -(ay wy)), fma(ax, wy, ay wx)).  Four scalar operations:
+// the packed FP32x2 form of the same bits is two, but needs (ax, ax), (ay, ay)
+// and (-wy, wx) in register pairs, four moves on the same issue slots.
 __device__ __forceinline__ float2 cmul_p(float2 a, float2 w) {
-    return __ffma2_rn(make_float2(a.x, a.x), w, __fmul2_rn(make_float2(a.y, a.y), make_float2(-w.y, w.x)));
+    return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)), __fmaf_rn(a.x, w.y, __fmul_rn(a.y, w.x)));
 }
 
 // ---------------------------------------------------------------------------
@@ -266,84 +269,47 @@ __global__ void k_plane_walls(float2 *S, int ny, int nz, int lgz, const float *t
 }
 
 // ---------------------------------------------------------------------------
-// Warp-level radix-2 transform of one line of N = 32*V points: lane t holds
-// elements t + 32 s (s < V).  Spans >= 32 are butterflies inside the lane,
-// spans < 32 exchange with lane t ^ span.  tw: forward twiddles in shared
-// memory, stage-major: the stage of span m reads w^(p N / (2m)), p < m, at
-// tw[m - 1 + p], w = (cos, -sin)(2 pi / N), so the lanes of a stage read
-// consecutive entries (no bank conflicts, where a table indexed by p N/(2m)
-// has lane stride N/(2m)).  The complex arithmetic uses packed FP32x2
-// operations; the cross-lane butterflies are branch-free (the lanes holding
-// the first element of a pair multiply by 1).
-template <int V>
-__device__ inline void warp_dif_fwd(float2 (&v)[V], const float2 *tw, int lane) {
-    constexpr int N = 32 * V;
+// Radix-2 passes in registers over the V elements t + S s (s < V) of a line.
+// tw: forward twiddles in shared memory, stage-major: the stage of span m
+// reads w^(p N / (2m)), p < m, at tw[m - 1 + p], w = (cos, -sin)(2 pi / N), so
+// that neighbouring t read consecutive entries.  With S = 1 the first twiddle
+// of a stage is one.
+//
+// Forward, decimation in frequency, spans S V / 2 .. S (natural in, bit-reversed out)
+template <int V, int S>
+__device__ __forceinline__ void reg_dif(float2 (&v)[V], const float2 *tw, int t) {
 #pragma unroll
-    for (int m = N / 2; m >= 1; m >>= 1) {
-        const float2 *tm = tw + (m - 1);
-        if (m >= 32) {
-            const int sm = m / 32;
+    for (int m = V / 2; m >= 1; m >>= 1) {
+        const float2 *tm = tw + (m * S - 1) + t;
 #pragma unroll
-            for (int s = 0; s < V; ++s) {
-                if ((s / sm) % 2) continue;          // upper element of the pair
-                const int pos = (lane + 32 * s) % (2 * m);
-                const float2 w = tm[pos];
-                const float2 a = v[s], b = v[s + sm];
+        for (int p = 0; p < m; ++p) {
+            const float2 w = S == 1 && p == 0 ? make_float2(1.0f, 0.0f) : tm[S * p];
+#pragma unroll
+            for (int s = p; s < V; s += 2 * m) {
+                const float2 a = v[s], b = v[s + m];
                 v[s] = __fadd2_rn(a, b);
-                v[s + sm] = cmul_p(__ffma2_rn(b, make_float2(-1.0f, -1.0f), a), w);
-            }
-        } else {
-            const bool second = lane & m;            // this lane holds the second element
-            const float2 w = second ? tm[(lane % (2 * m)) - m] : make_float2(1.0f, 0.0f);
-            const float sg = second ? -1.0f : 1.0f;
-#pragma unroll
-            for (int s = 0; s < V; ++s) {
-                float2 o;
-                o.x = __shfl_xor_sync(0xffffffffu, v[s].x, m);
-                o.y = __shfl_xor_sync(0xffffffffu, v[s].y, m);
-                // first: a + b; second: (a - b) w, with a the first element
-                v[s] = cmul_p(__ffma2_rn(make_float2(sg, sg), v[s], o), w);
+                const float2 c = __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
+                v[s + m] = S == 1 && p == 0 ? c : cmul_p(c, w);
             }
         }
     }
 }
 
-// inverse (conjugate twiddles), decimation in time: bit-reversed in, natural out
-template <int V>
-__device__ inline void warp_dit_inv(float2 (&v)[V], const float2 *tw, int lane) {
-    constexpr int N = 32 * V;
+// Inverse (conjugate twiddles), decimation in time, spans S .. S V / 2
+template <int V, int S>
+__device__ __forceinline__ void reg_dit(float2 (&v)[V], const float2 *tw, int t) {
 #pragma unroll
-    for (int m = 1; m < N; m <<= 1) {
-        const float2 *tm = tw + (m - 1);
-        if (m >= 32) {
-            const int sm = m / 32;
+    for (int m = 1; m < V; m <<= 1) {
+        const float2 *tm = tw + (m * S - 1) + t;
 #pragma unroll
-            for (int s = 0; s < V; ++s) {
-                if ((s / sm) % 2) continue;
-                const int pos = (lane + 32 * s) % (2 * m);
-                const float2 w = tm[pos];
-                const float2 t = cmul_p(v[s + sm], make_float2(w.x, -w.y));
-                const float2 a = v[s];
-                v[s] = __fadd2_rn(a, t);
-                v[s + sm] = __ffma2_rn(t, make_float2(-1.0f, -1.0f), a);
-            }
-        } else {
-            const bool second = lane & m;
-            float2 w = make_float2(1.0f, 0.0f);
-            if (second) {
-                const float2 tv = tm[(lane % (2 * m)) - m];
-                w = make_float2(tv.x, -tv.y);
-            }
-            const float sg = second ? -1.0f : 1.0f;
+        for (int p = 0; p < m; ++p) {
+            float2 w = S == 1 && p == 0 ? make_float2(1.0f, 0.0f) : tm[S * p];
+            w.y = -w.y;
 #pragma unroll
-            for (int s = 0; s < V; ++s) {
-                // the second element is multiplied by the twiddle before the
-                // exchange: first: a + b w; second: a - b w
-                const float2 p = cmul_p(v[s], w);
-                float2 o;
-                o.x = __shfl_xor_sync(0xffffffffu, p.x, m);
-                o.y = __shfl_xor_sync(0xffffffffu, p.y, m);
-                v[s] = __ffma2_rn(make_float2(sg, sg), p, o);
+            for (int s = p; s < V; s += 2 * m) {
+                const float2 a = v[s], c = S == 1 && p == 0 ? v[s + m] : cmul_p(v[s + m], w);
+                v[s] = __fadd2_rn(a, c);
+                v[s + m] = __ffma2_rn(c, make_float2(-1.0f, -1.0f), a);
             }
         }
     }
@@ -580,127 +546,162 @@ struct WallTables {
 };
 
 // ---------------------------------------------------------------------------
-// Warp-per-row-pair x passes (NX = 32 E).  Each warp transforms two real rows
-// packed as one complex line with warp_dif_fwd / warp_dit_inv (lane t holds
-// x = t + 32 s), unpacks / packs the two half spectra through a per-warp
-// buffer, and the block exchanges RB rows with the [kx][row] tile as the
-// radix-2 passes above do.  Per-warp buffer index of X[k]: k + (k >> lg E),
-// which makes both the bit-reversed (lane stride E + 1) and the natural
-// accesses free of bank conflicts.
-template <int E> struct LgE { static constexpr int v = E == 1 ? 0 : E == 2 ? 1 : E == 4 ? 2 : E == 8 ? 3 : 4; };
-
-__device__ __forceinline__ int zb_ix(int k, int lge) { return k + (k >> lge); }
-
-// natural index of element s of lane t after a DIF transform (bit-reversed)
-template <int E>
-__device__ __forceinline__ int brev_elem(int lane, int s) {
-    constexpr int LG = LgE<E>::v;
-    const int bl = (int)(__brev((unsigned)lane) >> 27);
-    const int bs = LG ? (int)(__brev((unsigned)s) >> (32 - LG)) : 0;
-    return (bl << LG) | bs;
-}
-
-constexpr int XW_WARPS = 4;   // warps per block of the x passes
+// x passes of XW_RB rows per block (NX = 32 .. 512).  Two real rows are one
+// complex line, held by G threads with E elements each: the spans of G and more
+// run in registers on the elements t + G s, the rest after one exchange through
+// shared memory on the groups of G consecutive elements (NX = 512: on 16
+// elements of a group of 32, with the last span between lanes).  The block then
+// unpacks the half spectra of its rows from (packs them into) the lines while
+// it writes (reads) the [kx][row] lines of 16 consecutive rows, the two rows of
+// a pair on neighbouring lanes.  Bound by instruction issue and shared memory:
+// with a warp per line, lane exchanges in the spans below 32 and a second
+// shared tile between the lines and the rows, 256x128x128 took 12.8 us forward and
+// 15.0 us inverse, this form 9.0 and 10.7 us.
 constexpr int XW_RB = 16;     // rows per block of the x passes (a constant: the tile indexing divides by it)
 
-inline size_t xw_smem(int nx, int rb) {
-    const int nh = nx / 2;
-    return ((size_t)nx + (size_t)(nh + 1) * (rb + 1) + (size_t)XW_WARPS * (nx + 32)) * sizeof(float2);
+template <int N> struct XLine {
+    static constexpr int E = N >= 128 ? 16 : 8, G = N / E, THREADS = XW_RB / 2 * G;
+    static constexpr int LG = N == 32 ? 5 : N == 64 ? 6 : N == 128 ? 7 : N == 256 ? 8 : 9;
+    // element e of a line at e + PAD (e / G), lines PITCH apart (odd): strided
+    // and consecutive elements, and one element of the lines, in distinct banks
+    static constexpr int PAD = N == 512 ? 2 : 1, PITCH = N + PAD * E + 1;
+    static constexpr size_t smem = (size_t)(N + XW_RB / 2 * PITCH) * sizeof(float2);
+    static __device__ __forceinline__ int ix(int e) { return e + e / G * PAD; }
+    static __device__ __forceinline__ int at(int k) { return ix((int)(__brev((unsigned)k) >> (32 - LG))); }   // X[k]
+};
+
+// spans below G of a line in shared memory (in place), forward or inverse
+template <int N, bool FWD>
+__device__ __forceinline__ void x_inner(float2 *z, const float2 *tws, int t) {
+    using X = XLine<N>;
+    if constexpr (N == 512) {
+        float2 *x = z + X::ix(t / 2 * 32) + (t & 1);
+        float2 v[16];
+        const float sg = t & 1 ? -1.0f : 1.0f;
+        auto last = [&] {                 // first: a + b, second: a - b
+#pragma unroll
+            for (int s = 0; s < 16; ++s) {
+                const float ox = __shfl_xor_sync(0xffffffffu, v[s].x, 1), oy = __shfl_xor_sync(0xffffffffu, v[s].y, 1);
+                v[s] = __ffma2_rn(make_float2(sg, sg), v[s], make_float2(ox, oy));
+            }
+        };
+#pragma unroll
+        for (int s = 0; s < 16; ++s) v[s] = x[2 * s];
+        if (FWD) { reg_dif<16, 2>(v, tws, t & 1); last(); }
+        else { last(); reg_dit<16, 2>(v, tws, t & 1); }
+#pragma unroll
+        for (int s = 0; s < 16; ++s) x[2 * s] = v[s];
+    } else {
+#pragma unroll
+        for (int u = 0; u < X::E / X::G; ++u) {
+            float2 *x = z + X::ix((t + X::G * u) * X::G);
+            float2 v[X::G];
+#pragma unroll
+            for (int s = 0; s < X::G; ++s) v[s] = x[s];
+            if (FWD) reg_dif<X::G, 1>(v, tws, 0);
+            else reg_dit<X::G, 1>(v, tws, 0);
+#pragma unroll
+            for (int s = 0; s < X::G; ++s) x[s] = v[s];
+        }
+    }
 }
 
-template <int E, typename TS>
-__global__ void __launch_bounds__(32 * XW_WARPS) k_xfwd_w(const TS *__restrict__ src, float2 *__restrict__ S, int ny,
-                                                         int nz, int lj, int joff, const float2 *__restrict__ twx) {
-    constexpr int N = 32 * E, NH = N / 2, LG = LgE<E>::v, rb = XW_RB;
+template <int N, typename TS>
+__global__ void __launch_bounds__(XLine<N>::THREADS) k_xfwd_w(const TS *__restrict__ src, float2 *__restrict__ S, int ny,
+                                                             int nz, int lj, int joff, const float2 *__restrict__ twx) {
+    using X = XLine<N>;
+    constexpr int E = X::E, G = X::G, NH = N / 2;
     extern __shared__ unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float2 *tws = reinterpret_cast<float2 *>(smem_raw);
-    float2 *tile = tws + N;
-    float2 *zb = tile + (size_t)(NH + 1) * (rb + 1) + (size_t)warp * (N + 32);
-    for (int q = threadIdx.x; q < N; q += blockDim.x) tws[q] = twx[q];
-    const int bpp = (ny + rb - 1) / rb;
+    float2 *zb = tws + N;
+    const int p = threadIdx.x / G, t = threadIdx.x % G;
+    float2 *z = zb + p * X::PITCH;
+    const int bpp = (ny + XW_RB - 1) / XW_RB;
     const int k = blockIdx.x / bpp;
-    const int r0 = (blockIdx.x % bpp) * rb;
-    const int nrows = min(rb, ny - r0);
+    const int r0 = (blockIdx.x % bpp) * XW_RB;
+    const int nrows = min(XW_RB, ny - r0);
+    const bool has_a = 2 * p < nrows, has_b = 2 * p + 1 < nrows;
+    const TS *ra = src + (size_t)N * ((size_t)(r0 + 2 * p) + (size_t)ny * k) + t;
+    float2 v[E];
+#pragma unroll
+    for (int s = 0; s < E; ++s)
+        v[s] = make_float2(has_a ? (float)ra[G * s] : 0.0f, has_b ? (float)ra[N + G * s] : 0.0f);
+    for (int q = threadIdx.x; q < N; q += X::THREADS) tws[q] = twx[q];
     __syncthreads();
-    for (int p = warp; 2 * p < nrows; p += XW_WARPS) {
-        const bool has_b = 2 * p + 1 < nrows;
-        const TS *ra = src + (size_t)N * ((size_t)(r0 + 2 * p) + (size_t)ny * k);
-        float2 v[E];
+    reg_dif<E, G>(v, tws, t);
 #pragma unroll
-        for (int s = 0; s < E; ++s)
-            v[s] = make_float2((float)ra[lane + 32 * s], has_b ? (float)ra[N + lane + 32 * s] : 0.0f);
-        warp_dif_fwd<E>(v, tws, lane);
-#pragma unroll
-        for (int s = 0; s < E; ++s) zb[zb_ix(brev_elem<E>(lane, s), LG)] = v[s];
-        __syncwarp();
-        for (int kx = lane; kx <= NH; kx += 32) {
-            const float2 zk = zb[zb_ix(kx, LG)], zm = zb[zb_ix((N - kx) & (N - 1), LG)];
-            tile[(size_t)kx * (rb + 1) + 2 * p] = make_float2((zk.x + zm.x) * 0.5f, (zk.y - zm.y) * 0.5f);
-            tile[(size_t)kx * (rb + 1) + 2 * p + 1] = make_float2((zk.y + zm.y) * 0.5f, (zm.x - zk.x) * 0.5f);
+    for (int s = 0; s < E; ++s) z[X::ix(G * s) + t] = v[s];
+    __syncwarp();
+    x_inner<N, true>(z, tws, t);
+    __syncthreads();
+    const int r = threadIdx.x % XW_RB, b = r & 1;
+    const float2 *zr = zb + (r >> 1) * X::PITCH;
+    float2 *Sr = S + (size_t)k * lj + (r0 + r + 1 + joff);
+    const int skx = nz * lj;
+    if (r < nrows) {
+#pragma unroll 4
+        for (int kx = threadIdx.x / XW_RB; kx <= NH; kx += X::THREADS / XW_RB) {
+            const float2 zk = zr[X::at(kx)], zm = zr[X::at((N - kx) & (N - 1))];
+            // A = (zk + conj zm) / 2, B = (zk - conj zm) / 2i
+            const float ax = b ? zk.y : zk.x, bx = b ? zm.y : zm.x, ay = b ? zm.x : zk.y, by = b ? zk.x : zm.y;
+            Sr[(size_t)kx * skx] = make_float2((ax + bx) * 0.5f, (ay - by) * 0.5f);
         }
-        __syncwarp();
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < (NH + 1) * rb; q += blockDim.x) {
-        const int kx = q / rb, r = q % rb;
-        if (r < nrows) S[((size_t)kx * nz + k) * lj + (r0 + r + 1 + joff)] = tile[(size_t)kx * (rb + 1) + r];
     }
 }
 
-template <int E, typename Out>
-__global__ void __launch_bounds__(32 * XW_WARPS) k_xinv_w(const float2 *__restrict__ S, Out out,
-                                                         int nrow, int jlo, int nz, int lj, int joff2, int sx,
-                                                         int sy, const float2 *__restrict__ twx) {
-    constexpr int N = 32 * E, NH = N / 2, LG = LgE<E>::v, rb = XW_RB;
+template <int N, typename Out>
+__global__ void __launch_bounds__(XLine<N>::THREADS) k_xinv_w(const float2 *__restrict__ S, Out out, int nrow, int jlo,
+                                                             int nz, int lj, int joff2, int sx, int sy,
+                                                             const float2 *__restrict__ twx) {
+    using X = XLine<N>;
+    constexpr int E = X::E, G = X::G, NH = N / 2, STEP = X::THREADS / XW_RB, BATCH = 8;
     extern __shared__ unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float2 *tws = reinterpret_cast<float2 *>(smem_raw);
-    float2 *tile = tws + N;
-    float2 *zb = tile + (size_t)(NH + 1) * (rb + 1) + (size_t)warp * (N + 32);
-    for (int q = threadIdx.x; q < N; q += blockDim.x) tws[q] = twx[q];
-    const int bpp = (nrow + rb - 1) / rb;
+    float2 *zb = tws + N;
+    const int bpp = (nrow + XW_RB - 1) / XW_RB;
     const int k = blockIdx.x / bpp;
-    const int r0 = (blockIdx.x % bpp) * rb;
-    const int nrows = min(rb, nrow - r0);
-    // gather the tile: four loads in flight per thread before their stores
-    for (int q0 = threadIdx.x; q0 < (NH + 1) * rb; q0 += 4 * blockDim.x) {
-        float2 v[4];
+    const int r0 = (blockIdx.x % bpp) * XW_RB;
+    const int nrows = min(XW_RB, nrow - r0);
+    for (int q = threadIdx.x; q < N; q += X::THREADS) tws[q] = twx[q];
+    {
+        // Z = A + i B over the full line from the two half spectra: the lane of
+        // row a writes Z[kx], that of row b Z[N - kx]
+        const int r = threadIdx.x % XW_RB, b = r & 1;
+        float2 *zr = zb + (r >> 1) * X::PITCH;
+        const float2 *Sr = S + (size_t)k * lj + (jlo + r0 + r + joff2);
+        const int skx = nz * lj;
+        auto put = [&](int kx, float2 v, bool keep) {
+            const float ox = __shfl_xor_sync(0xffffffffu, v.x, 1), oy = __shfl_xor_sync(0xffffffffu, v.y, 1);
+            const float2 zv = make_float2((b ? v.y : v.x) + (b ? ox : -oy), (b ? v.x : v.y) + (b ? -oy : ox));
+            if (keep && !(b && (kx == 0 || kx == NH))) zr[X::at(b ? N - kx : kx)] = zv;
+        };
+        const bool first = threadIdx.x < XW_RB;      // kx = NH, by the first lanes of the first warp
+        const float2 vl = first && r < nrows ? Sr[(size_t)NH * skx] : make_float2(0.f, 0.f);
+        for (int k0 = threadIdx.x / XW_RB; k0 < NH; k0 += BATCH * STEP) {   // NH is a multiple of BATCH STEP
+            float2 v[BATCH];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int q = q0 + u * blockDim.x;
-            const int kx = q / rb, r = q % rb;
-            v[u] = (q < (NH + 1) * rb && r < nrows) ? S[((size_t)kx * nz + k) * lj + (jlo + r0 + r + joff2)]
-                                                   : make_float2(0.f, 0.f);
-        }
+            for (int u = 0; u < BATCH; ++u)
+                v[u] = r < nrows ? Sr[(size_t)(k0 + u * STEP) * skx] : make_float2(0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int q = q0 + u * blockDim.x;
-            if (q < (NH + 1) * rb) tile[(size_t)(q / rb) * (rb + 1) + q % rb] = v[u];
+            for (int u = 0; u < BATCH; ++u) put(k0 + u * STEP, v[u], true);
         }
+        if (threadIdx.x < 32) put(NH, vl, first);
     }
     __syncthreads();
-    for (int p = warp; 2 * p < nrows; p += XW_WARPS) {
-        const bool has_b = 2 * p + 1 < nrows;
-        // Z = A + i B over the full line from the two half spectra
-        for (int e = lane; e < N; e += 32) {
-            const int m = e <= NH ? e : N - e;
-            const float2 A = tile[(size_t)m * (rb + 1) + 2 * p], B = tile[(size_t)m * (rb + 1) + 2 * p + 1];
-            zb[zb_ix(e, LG)] = e <= NH ? make_float2(A.x - B.y, A.y + B.x) : make_float2(A.x + B.y, B.x - A.y);
-        }
-        __syncwarp();
-        float2 v[E];
+    const int p = threadIdx.x / G, t = threadIdx.x % G;
+    float2 *z = zb + p * X::PITCH;
+    x_inner<N, false>(z, tws, t);
+    __syncwarp();
+    float2 v[E];
 #pragma unroll
-        for (int s = 0; s < E; ++s) v[s] = zb[zb_ix(brev_elem<E>(lane, s), LG)];
-        __syncwarp();
-        warp_dit_inv<E>(v, tws, lane);
-        const size_t oa = 1 + (size_t)sx * ((size_t)(jlo + r0 + 2 * p) + (size_t)sy * (k + 1));
+    for (int s = 0; s < E; ++s) v[s] = z[X::ix(G * s) + t];
+    reg_dit<E, G>(v, tws, t);
+    const bool has_a = 2 * p < nrows, has_b = 2 * p + 1 < nrows;
+    const size_t oa = 1 + (size_t)sx * ((size_t)(jlo + r0 + 2 * p) + (size_t)sy * (k + 1)) + t;
 #pragma unroll
-        for (int s = 0; s < E; ++s) {
-            const int e = lane + 32 * s;
-            out.put(oa + e, v[s].x);
-            if (has_b) out.put(oa + sx + e, v[s].y);
-        }
+    for (int s = 0; s < E; ++s) {
+        if (has_a) out.put(oa + G * s, v[s].x);
+        if (has_b) out.put(oa + sx + G * s, v[s].y);
     }
 }
 
@@ -719,12 +720,63 @@ __global__ void __launch_bounds__(32 * XW_WARPS) k_xinv_w(const float2 *__restri
 // fenep_2d.f90:1145-1177); the 1/den table of the CTA's rows is staged in
 // shared memory, its rows in the bit-reversed kz order of the spectrum rows.
 // The cluster barriers are hardware barriers; no thread waits on a flag.
+//
+// The z transforms of the rows are radix-2 passes over registers, V1 and then
+// S = NZ / V1 elements of a line per thread, with the lanes of a warp on
+// neighbouring rows: global and shared accesses are contiguous, the twiddles
+// of a warp are broadcasts, and no lane multiplies for the other half of a
+// pair.  The first pass of the forward transform reads the plane from global
+// memory and the last of the inverse writes it there (16 loads in flight per
+// thread), and the pivot table arrives by asynchronous copies meanwhile.  The
+// kernel is bound by instruction issue: a warp per line with lane exchanges
+// executed 275 instructions per value of the plane and took 30.0 us at
+// 256x128x128 (one CTA per kx), this form takes 20.2 us.
+__device__ __forceinline__ void copy_async4(float *smem, const float *gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+template <int N> struct ZSplit {
+    static constexpr int V1 = N >= 128 ? 16 : 8, S = N / V1;
+};
+
+// Exclusive scan of the composed maps (A, B) of the T chunks of each system, in
+// order (UP) or from the end, and the map of all chunks to tot[3][NZ].  The
+// thread t NZ + row holds the map of chunk t; the threads row T + t scan them
+// with shuffles.  sc: WALL_SCAN floats, pitch NZ + NZ / 32 against conflicts.
+template <int NZ, bool UP>
+__device__ __forceinline__ void wall_scan(float *sc, float *tot, float &A, float2 &B) {
+    constexpr int T = 1024 / NZ, W = NZ + NZ / 32, F = T * W;
+    const int own = threadIdx.x / NZ * W + threadIdx.x % NZ;
+    const int row = threadIdx.x / T, t = threadIdx.x % T, at = t * W + row;
+    __syncthreads();   // earlier reads of what lies under sc
+    sc[own] = A; sc[F + own] = B.x; sc[2 * F + own] = B.y;
+    __syncthreads();
+    A = sc[at]; B = make_float2(sc[F + at], sc[2 * F + at]);
+#pragma unroll
+    for (int o = 1; o < T; o <<= 1) {
+        const float Ap = UP ? __shfl_up_sync(0xffffffffu, A, o, T) : __shfl_down_sync(0xffffffffu, A, o, T);
+        const float Bx = UP ? __shfl_up_sync(0xffffffffu, B.x, o, T) : __shfl_down_sync(0xffffffffu, B.x, o, T);
+        const float By = UP ? __shfl_up_sync(0xffffffffu, B.y, o, T) : __shfl_down_sync(0xffffffffu, B.y, o, T);
+        if (UP ? t >= o : t + o < T) { B = make_float2(fmaf(A, Bx, B.x), fmaf(A, By, B.y)); A *= Ap; }
+    }
+    // the inclusive map of chunk t is the exclusive one of the next
+    if (t == (UP ? T - 1 : 0)) { tot[row] = A; tot[NZ + row] = B.x; tot[2 * NZ + row] = B.y; }
+    const int nx = (UP ? (t == T - 1 ? 0 : t + 1) : (t == 0 ? T - 1 : t - 1)) * W + row;
+    const bool end = t == (UP ? T - 1 : 0);
+    __syncwarp();      // the threads of a system lie in one warp
+    sc[nx] = end ? 1.0f : A; sc[F + nx] = end ? 0.0f : B.x; sc[2 * F + nx] = end ? 0.0f : B.y;
+    __syncthreads();
+    A = sc[own]; B = make_float2(sc[F + own], sc[2 * F + own]);
+}
+
 template <int V>
 __global__ void __launch_bounds__(1024, 1) k_plane_walls_c(float2 *S, int ny, int cl, const float2 *twz,
                                                            WallTables wt) {
     constexpr int NZ = 32 * V;
     constexpr int LG = V == 1 ? 5 : (V == 2 ? 6 : (V == 4 ? 7 : 8));
-    constexpr int T = 1024 / NZ;
     namespace cg = cooperative_groups;
     extern __shared__ unsigned char smem_raw[];
     const int lj = ny + 2;
@@ -740,154 +792,142 @@ __global__ void __launch_bounds__(1024, 1) k_plane_walls_c(float2 *S, int ny, in
     float2 *tws = reinterpret_cast<float2 *>(Rs + (size_t)rs * NZ);   // NZ stage-major twiddles
     float *mapF = reinterpret_cast<float *>(tws + NZ);                // [3][NZ]: A, Bx, By
     float *mapB = mapF + 3 * NZ;
+    constexpr int V1 = ZSplit<NZ>::V1, S1 = ZSplit<NZ>::S;
+    float *sc = wall_scan_in_plane(ps, NZ) ? reinterpret_cast<float *>(P) : mapB + 3 * NZ;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    float2 *Sp = S + (size_t)kx * NZ * lj;
-    const float *Rg = wt.rden + (size_t)kx * NZ * lj;
+    float2 *Sp = S + (size_t)kx * NZ * lj + jlo;
+    const float *Rg = wt.rden + (size_t)kx * NZ * lj + jlo;
+    const bool sysv = wt.sys == SYS_V;
     for (int q = threadIdx.x; q < NZ; q += blockDim.x) tws[q] = twz[q];
     for (int k = warp; k < NZ; k += nwarp) {
         float *rrow = Rs + (size_t)(__brev((unsigned)k) >> (32 - LG)) * rs;
-        for (int jl0 = lane; jl0 < nr; jl0 += 128) {   // four loads of each array in flight per lane
-            float2 pv[4];
-            float rv[4];
+        for (int jl = lane; jl < nr; jl += 32) copy_async4(rrow + jl, Rg + k * lj + jl);
+    }
+    copy_async_commit();
+    // ghost rows, and the row of V on the upper wall, carry no right-hand side
+    for (int q = threadIdx.x; q < 3 * NZ; q += blockDim.x) {
+        const int j = q < NZ ? 0 : (q < 2 * NZ ? ny : ny + 1), jl = j - jlo;
+        if (jl >= 0 && jl < nr && (j != ny || sysv)) P[(q & (NZ - 1)) * ps + jl] = make_float2(0.f, 0.f);
+    }
+    const int f0 = max(0, 1 - jlo), nf = max(0, min(nr, ny + (sysv ? 0 : 1) - jlo) - f0);   // rows to transform
+    __syncthreads();   // twiddles
+    for (int q = threadIdx.x; q < nf * S1; q += blockDim.x) {
+        const int t = q / nf, jl = f0 + q - t * nf;
+        float2 v[V1];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int jl = jl0 + 32 * u, j = jlo + jl;
-                const size_t q = (size_t)k * lj + j;
-                pv[u] = (jl < nr && j >= 1 && j <= ny) ? Sp[q] : make_float2(0.f, 0.f);
-                rv[u] = jl < nr ? Rg[q] : 0.0f;
-            }
+        for (int s = 0; s < V1; ++s) v[s] = Sp[(t + S1 * s) * lj + jl];
+        reg_dif<V1, S1>(v, tws, t);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int jl = jl0 + 32 * u;
-                if (jl < nr) { P[(size_t)k * ps + jl] = pv[u]; rrow[jl] = rv[u]; }
-            }
-        }
+        for (int s = 0; s < V1; ++s) P[(t + S1 * s) * ps + jl] = v[s];
     }
     __syncthreads();
-    for (int jl = warp; jl < nr; jl += nwarp) {
-        const int j = jlo + jl;
-        if (j < 1 || j > ny) continue;   // ghost rows are zero
-        float2 v[V];
+    for (int q = threadIdx.x; q < nf * V1; q += blockDim.x) {
+        const int u = q / nf, jl = f0 + q - u * nf;
+        float2 *x = P + u * S1 * ps + jl;
+        float2 v[S1];
 #pragma unroll
-        for (int s = 0; s < V; ++s) v[s] = P[(size_t)(lane + 32 * s) * ps + jl];
-        warp_dif_fwd<V>(v, tws, lane);
+        for (int s = 0; s < S1; ++s) v[s] = x[s * ps];
+        reg_dif<S1, 1>(v, tws, 0);
 #pragma unroll
-        for (int s = 0; s < V; ++s) P[(size_t)(lane + 32 * s) * ps + jl] = v[s];
+        for (int s = 0; s < S1; ++s) x[s * ps] = v[s];
     }
+    copy_async_wait();
     __syncthreads();
     {
-        const int row = threadIdx.x / T, t = threadIdx.x % T;
-        float2 *x = P + (size_t)row * ps;
-        const float *rd = Rs + (size_t)row * rs;
+        const int row = threadIdx.x % NZ, t = threadIdx.x / NZ;   // one chunk number per warp
         const int L = wt.wl.L;
-        const int c0 = min(nr, t * L), c1 = min(nr, c0 + L);
-        const bool sysv = wt.sys == SYS_V;
-        auto fwd_coef = [&](int jl, float &al, float2 &be) {
-            const int j = jlo + jl;
-            const bool ident = sysv ? (j >= ny) : (j == lj - 1);
-            const float c = ident ? (sysv ? 0.f : wt.c_last) : wt.bc;
-            const float r = j == 0 ? 0.0f : rd[jl];
-            const float2 d = ident ? make_float2(0.f, 0.f) : x[jl];
-            al = -c * r;
-            const float dr = wt.nxz_inv * r;
-            be = make_float2(d.x * dr, d.y * dr);
-        };
-        auto pmul = [&](int jl) {
-            const int j = jlo + jl;
-            const bool zero_b = (j == lj - 1) || (sysv && j >= ny);
-            const float b = j == 0 ? wt.b_first : (zero_b ? 0.0f : wt.bc);
-            return -b * rd[jl];
-        };
-        // forward: compose the chunk's maps (row 0: q_0 = 0)
+        const int c0 = min(nr, t * L), n = min(nr, c0 + L) - c0;
+        float2 *x = P + row * ps + c0;
+        const float *rd = Rs + row * rs + c0;
+        // rows of the chunk with the interior's coefficients; behind them the
+        // last row (V: also the row on the wall), where d = 0 and b = 0
+        const int nin = min(n, (sysv ? ny : ny + 1) - jlo - c0);
+        const float nbc = -wt.bc, nlast = sysv ? -0.0f : -wt.c_last;
+        const float nb0 = jlo + c0 == 0 ? -wt.b_first : nbc;
+        float2 v[WALL_CHUNK];
+        // forward: compose the chunk's maps (row 0 has no predecessor: q = 0)
         float A = 1.0f;
         float2 B = make_float2(0.f, 0.f);
-        for (int jl = c0; jl < c1; ++jl) {
-            float al;
-            float2 be;
-            fwd_coef(jl, al, be);
-            B = make_float2(fmaf(al, B.x, be.x), fmaf(al, B.y, be.y));
+#pragma unroll
+        for (int i = 0; i < WALL_CHUNK; ++i) {
+            if (i >= n) break;
+            v[i] = x[i];
+            const float r = rd[i], al = (i < nin ? nbc : nlast) * r, dr = wt.nxz_inv * r;
+            B = make_float2(fmaf(al, B.x, v[i].x * dr), fmaf(al, B.y, v[i].y * dr));
             A *= al;
         }
-#pragma unroll
-        for (int o = 1; o < T; o <<= 1) {
-            const float Ap = __shfl_up_sync(0xffffffffu, A, o, T);
-            const float Bx = __shfl_up_sync(0xffffffffu, B.x, o, T), By = __shfl_up_sync(0xffffffffu, B.y, o, T);
-            if (t >= o) { B = make_float2(fmaf(A, Bx, B.x), fmaf(A, By, B.y)); A *= Ap; }
-        }
-        if (t == T - 1) { mapF[row] = A; mapF[NZ + row] = B.x; mapF[2 * NZ + row] = B.y; }
-        float Ae = __shfl_up_sync(0xffffffffu, A, 1, T);
-        float2 Be;
-        Be.x = __shfl_up_sync(0xffffffffu, B.x, 1, T);
-        Be.y = __shfl_up_sync(0xffffffffu, B.y, 1, T);
-        if (t == 0) { Ae = 1.0f; Be = make_float2(0.f, 0.f); }
-        float2 qin = make_float2(0.f, 0.f);
+        wall_scan<NZ, true>(sc, mapF, A, B);
+        float2 q = make_float2(0.f, 0.f);
         if (cl > 1) {
             cg::this_cluster().sync();
             for (int rr = 0; rr < rank; ++rr) {
                 const float *m = cg::this_cluster().map_shared_rank(mapF, rr);
                 const float a = m[row];
-                qin = make_float2(fmaf(a, qin.x, m[NZ + row]), fmaf(a, qin.y, m[2 * NZ + row]));
+                q = make_float2(fmaf(a, q.x, m[NZ + row]), fmaf(a, q.y, m[2 * NZ + row]));
             }
         }
-        float2 q = make_float2(fmaf(Ae, qin.x, Be.x), fmaf(Ae, qin.y, Be.y));
-        for (int jl = c0; jl < c1; ++jl) {
-            float al;
-            float2 be;
-            fwd_coef(jl, al, be);
-            q = make_float2(fmaf(al, q.x, be.x), fmaf(al, q.y, be.y));
-            x[jl] = q;
+        q = make_float2(fmaf(A, q.x, B.x), fmaf(A, q.y, B.y));
+#pragma unroll
+        for (int i = 0; i < WALL_CHUNK; ++i) {
+            if (i >= n) break;
+            const float r = rd[i], al = (i < nin ? nbc : nlast) * r, dr = wt.nxz_inv * r;
+            q = make_float2(fmaf(al, q.x, v[i].x * dr), fmaf(al, q.y, v[i].y * dr));
+            v[i] = q;
         }
-        // backward: x_j = P_j x_{j+1} + q_j (b and so P of the last row are 0)
+        // backward: x_j = P_j x_{j+1} + q_j (b and so P of the rows behind the
+        // interior are 0; row 0 has its own b)
         A = 1.0f;
         B = make_float2(0.f, 0.f);
-        for (int jl = c1 - 1; jl >= c0; --jl) {
-            const float pj = pmul(jl);
-            const float2 qj = x[jl];
-            B = make_float2(fmaf(pj, B.x, qj.x), fmaf(pj, B.y, qj.y));
+#pragma unroll
+        for (int i = WALL_CHUNK - 1; i >= 0; --i) {
+            if (i >= n) continue;
+            const float pj = (i >= nin ? -0.0f : (i == 0 ? nb0 : nbc)) * rd[i];
+            B = make_float2(fmaf(pj, B.x, v[i].x), fmaf(pj, B.y, v[i].y));
             A *= pj;
         }
-#pragma unroll
-        for (int o = 1; o < T; o <<= 1) {
-            const float An = __shfl_down_sync(0xffffffffu, A, o, T);
-            const float Bx = __shfl_down_sync(0xffffffffu, B.x, o, T), By = __shfl_down_sync(0xffffffffu, B.y, o, T);
-            if (t + o < T) { B = make_float2(fmaf(A, Bx, B.x), fmaf(A, By, B.y)); A *= An; }
-        }
-        if (t == 0) { mapB[row] = A; mapB[NZ + row] = B.x; mapB[2 * NZ + row] = B.y; }
-        Ae = __shfl_down_sync(0xffffffffu, A, 1, T);
-        Be.x = __shfl_down_sync(0xffffffffu, B.x, 1, T);
-        Be.y = __shfl_down_sync(0xffffffffu, B.y, 1, T);
-        if (t == T - 1) { Ae = 1.0f; Be = make_float2(0.f, 0.f); }
-        float2 xin = make_float2(0.f, 0.f);
+        wall_scan<NZ, false>(sc, mapB, A, B);
+        q = make_float2(0.f, 0.f);
         if (cl > 1) {
             cg::this_cluster().sync();
             for (int rr = cl - 1; rr > rank; --rr) {
                 const float *m = cg::this_cluster().map_shared_rank(mapB, rr);
                 const float a = m[row];
-                xin = make_float2(fmaf(a, xin.x, m[NZ + row]), fmaf(a, xin.y, m[2 * NZ + row]));
+                q = make_float2(fmaf(a, q.x, m[NZ + row]), fmaf(a, q.y, m[2 * NZ + row]));
             }
         }
-        float2 xv = make_float2(fmaf(Ae, xin.x, Be.x), fmaf(Ae, xin.y, Be.y));
-        for (int jl = c1 - 1; jl >= c0; --jl) {
-            const float pj = pmul(jl);
-            const float2 qj = x[jl];
-            xv = make_float2(fmaf(pj, xv.x, qj.x), fmaf(pj, xv.y, qj.y));
-            x[jl] = xv;
+        q = make_float2(fmaf(A, q.x, B.x), fmaf(A, q.y, B.y));
+        __syncthreads();   // every thread has read its map: the scan buffer lies in the plane
+#pragma unroll
+        for (int i = WALL_CHUNK - 1; i >= 0; --i) {
+            if (i >= n) continue;
+            const float pj = (i >= nin ? -0.0f : (i == 0 ? nb0 : nbc)) * rd[i];
+            q = make_float2(fmaf(pj, q.x, v[i].x), fmaf(pj, q.y, v[i].y));
+            x[i] = q;
         }
     }
     // the other CTAs' reads of this CTA's maps are complete past this barrier
     if (cl > 1) cg::this_cluster().sync();
     else __syncthreads();
-    for (int jl = warp; jl < nr; jl += nwarp) {
-        float2 v[V];
+    for (int q = threadIdx.x; q < nr * V1; q += blockDim.x) {
+        const int u = q / nr, jl = q - u * nr;
+        float2 *x = P + u * S1 * ps + jl;
+        float2 v[S1];
 #pragma unroll
-        for (int s = 0; s < V; ++s) v[s] = P[(size_t)(lane + 32 * s) * ps + jl];
-        warp_dit_inv<V>(v, tws, lane);
+        for (int s = 0; s < S1; ++s) v[s] = x[s * ps];
+        reg_dit<S1, 1>(v, tws, 0);
 #pragma unroll
-        for (int s = 0; s < V; ++s) P[(size_t)(lane + 32 * s) * ps + jl] = v[s];
+        for (int s = 0; s < S1; ++s) x[s * ps] = v[s];
     }
     __syncthreads();
-    for (int k = warp; k < NZ; k += nwarp)
-        for (int jl = lane; jl < nr; jl += 32) Sp[(size_t)k * lj + jlo + jl] = P[(size_t)k * ps + jl];
+    for (int q = threadIdx.x; q < nr * S1; q += blockDim.x) {
+        const int t = q / nr, jl = q - t * nr;
+        float2 v[V1];
+#pragma unroll
+        for (int s = 0; s < V1; ++s) v[s] = P[(t + S1 * s) * ps + jl];
+        reg_dit<V1, S1>(v, tws, t);
+#pragma unroll
+        for (int s = 0; s < V1; ++s) Sp[(t + S1 * s) * lj + jl] = v[s];
+    }
 }
 
 }  // namespace f8

@@ -1876,14 +1876,16 @@ template <typename TS>
 bool xfwd_warp(const Dev &d, const TS *src, float2 *S, int ny, int lj, int joff, cudaStream_t s) {
     const Geo &g = d.g;
     const unsigned grid = (unsigned)(((ny + XW_RB - 1) / XW_RB) * g.nz);
-    const size_t sm = xw_smem(g.nx, XW_RB);
-    const int thr = 32 * XW_WARPS;
+    auto go = [&](auto n) {
+        using X = XLine<decltype(n)::value>;
+        k_xfwd_w<decltype(n)::value, TS><<<grid, X::THREADS, X::smem, s>>>(src, S, ny, g.nz, lj, joff, d.twx2);
+    };
     switch (g.nx) {
-    case 32: k_xfwd_w<1, TS><<<grid, thr, sm, s>>>(src, S, ny, g.nz, lj, joff, d.twx2); break;
-    case 64: k_xfwd_w<2, TS><<<grid, thr, sm, s>>>(src, S, ny, g.nz, lj, joff, d.twx2); break;
-    case 128: k_xfwd_w<4, TS><<<grid, thr, sm, s>>>(src, S, ny, g.nz, lj, joff, d.twx2); break;
-    case 256: k_xfwd_w<8, TS><<<grid, thr, sm, s>>>(src, S, ny, g.nz, lj, joff, d.twx2); break;
-    case 512: k_xfwd_w<16, TS><<<grid, thr, sm, s>>>(src, S, ny, g.nz, lj, joff, d.twx2); break;
+    case 32: go(std::integral_constant<int, 32>{}); break;
+    case 64: go(std::integral_constant<int, 64>{}); break;
+    case 128: go(std::integral_constant<int, 128>{}); break;
+    case 256: go(std::integral_constant<int, 256>{}); break;
+    case 512: go(std::integral_constant<int, 512>{}); break;
     default: return false;
     }
     count_launch();
@@ -1893,14 +1895,17 @@ bool xfwd_warp(const Dev &d, const TS *src, float2 *S, int ny, int lj, int joff,
 bool xinv_warp(const Dev &d, const float2 *S, XOutF out, int nrow, int jlo, int lj, int joff2, cudaStream_t s) {
     const Geo &g = d.g;
     const unsigned grid = (unsigned)(((nrow + XW_RB - 1) / XW_RB) * g.nz);
-    const size_t sm = xw_smem(g.nx, XW_RB);
-    const int thr = 32 * XW_WARPS;
+    auto go = [&](auto n) {
+        using X = XLine<decltype(n)::value>;
+        k_xinv_w<decltype(n)::value, XOutF><<<grid, X::THREADS, X::smem, s>>>(S, out, nrow, jlo, g.nz, lj, joff2, g.sx,
+                                                                             g.sy, d.twx2);
+    };
     switch (g.nx) {
-    case 32: k_xinv_w<1, XOutF><<<grid, thr, sm, s>>>(S, out, nrow, jlo, g.nz, lj, joff2, g.sx, g.sy, d.twx2); break;
-    case 64: k_xinv_w<2, XOutF><<<grid, thr, sm, s>>>(S, out, nrow, jlo, g.nz, lj, joff2, g.sx, g.sy, d.twx2); break;
-    case 128: k_xinv_w<4, XOutF><<<grid, thr, sm, s>>>(S, out, nrow, jlo, g.nz, lj, joff2, g.sx, g.sy, d.twx2); break;
-    case 256: k_xinv_w<8, XOutF><<<grid, thr, sm, s>>>(S, out, nrow, jlo, g.nz, lj, joff2, g.sx, g.sy, d.twx2); break;
-    case 512: k_xinv_w<16, XOutF><<<grid, thr, sm, s>>>(S, out, nrow, jlo, g.nz, lj, joff2, g.sx, g.sy, d.twx2); break;
+    case 32: go(std::integral_constant<int, 32>{}); break;
+    case 64: go(std::integral_constant<int, 64>{}); break;
+    case 128: go(std::integral_constant<int, 128>{}); break;
+    case 256: go(std::integral_constant<int, 256>{}); break;
+    case 512: go(std::integral_constant<int, 512>{}); break;
     default: return false;
     }
     count_launch();
@@ -1948,13 +1953,16 @@ cudaError_t solve_walls_fused(Dev &d, const TS *src, XOutF out, int sys, cudaStr
     if (d.plane_cl > 0) {
         const int t = sys == SYS_P ? 2 : (sys == SYS_V ? 1 : 0);
         const float b_first = sys == SYS_P ? -1.0f : (sys == SYS_V ? 0.0f : 1.0f);
+        // an odd stride of the pivot table where the layout leaves room for one
+        WallLayout wl = d.plane_wl;
+        if (!(wl.rs & 1) && wl.rs > wall_rows_per_cta(lj, d.plane_cl)) --wl.rs;
         const WallTables wt{d.wtR[t], (float)(sys == SYS_P ? idy2 : -kap * idy2), sys == SYS_P ? -1.0f : 1.0f, b_first,
-                            (float)(1.0 / ((double)nx * nz)), sys, d.plane_wl};
+                            (float)(1.0 / ((double)nx * nz)), sys, wl};
         const int cl = d.plane_cl;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(nxh * cl));
         cfg.blockDim = dim3(1024);
-        cfg.dynamicSmemBytes = wall_plane_smem(d.plane_wl, nz);
+        cfg.dynamicSmemBytes = wall_kernel_smem(d.plane_wl, nz);
         cfg.stream = s;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2158,11 +2166,6 @@ cudaError_t init_kernels_mixed() {
     F8_CUDA_RET(cudaFuncSetAttribute(k_plane_walls_c<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     F8_CUDA_RET(cudaFuncSetAttribute(k_plane_walls_c<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     F8_CUDA_RET(cudaFuncSetAttribute(k_plane_walls_c<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-#define F8_XW_ATTR(E)                                                                                           \
-    F8_CUDA_RET(cudaFuncSetAttribute(k_xfwd_w<E, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));   \
-    F8_CUDA_RET(cudaFuncSetAttribute(k_xinv_w<E, XOutF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    F8_XW_ATTR(1) F8_XW_ATTR(2) F8_XW_ATTR(4) F8_XW_ATTR(8) F8_XW_ATTR(16)
-#undef F8_XW_ATTR
     F8_CUDA_RET(cudaFuncSetAttribute(k_xfwd_t<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     F8_CUDA_RET(cudaFuncSetAttribute(k_xinv_t<XOutF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     return cudaSuccess;

@@ -479,15 +479,13 @@ int setup(f8_ctx *c) {
         }
         // side streams (the V and W Helmholtz solves, the wall ghost rows, the drag)
         // and the spectra of those solves
-        if (g.dim == 3) {
-            for (int b = 0; b < 2; ++b) {
-                if (d.fused_planes) API_CUDA(c, c->alloc(&d.HfB[b], nspec));
-                API_CUDA(c, cudaStreamCreateWithFlags(&d.aux[b], cudaStreamNonBlocking));
-                API_CUDA(c, cudaEventCreateWithFlags(&d.ev_join[b], cudaEventDisableTiming));
-            }
-            API_CUDA(c, cudaEventCreateWithFlags(&d.ev_fork, cudaEventDisableTiming));
-            for (int q = 0; q < 6; ++q) API_CUDA(c, cudaEventCreateWithFlags(&d.ev_g[q], cudaEventDisableTiming));
+        for (int b = 0; b < 2; ++b) {
+            if (d.fused_planes) API_CUDA(c, c->alloc(&d.HfB[b], nspec));
+            API_CUDA(c, cudaStreamCreateWithFlags(&d.aux[b], cudaStreamNonBlocking));
+            API_CUDA(c, cudaEventCreateWithFlags(&d.ev_join[b], cudaEventDisableTiming));
         }
+        API_CUDA(c, cudaEventCreateWithFlags(&d.ev_fork, cudaEventDisableTiming));
+        for (int q = 0; q < 6; ++q) API_CUDA(c, cudaEventCreateWithFlags(&d.ev_g[q], cudaEventDisableTiming));
         {
             // stage-major twiddles of the warp transforms: stage span m holds
             // w^(p N / (2m)), p < m, at m - 1 + p (N entries, the last unused)

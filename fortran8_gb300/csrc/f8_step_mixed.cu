@@ -1250,71 +1250,78 @@ struct IbmArgsF {
     float dtf;                       // dt
 };
 
-// One marker per threadIdx.x and one z plane of its 3 x 3 x 3 stencil per
-// threadIdx.y (blocks of 32 x 3): each thread sums 9 points in df64, and the
-// three plane sums are added in plane order.
-__global__ void __launch_bounds__(96) k_ibm_interp_f(IbmArgsF a, Geo g) {
-    __shared__ df part[3][32];
+// One marker per lane and NB consecutive marker planes n per thread.  A plane k
+// of the field enters the sums of n = k + 1, k, k - 1 with the z weights 0, 1, 2,
+// so the thread reads the 9 points of each of its NB + 2 planes once and adds
+// the plane's sum to the up to three planes n that use it, in the order k =
+// n - 1, n, n + 1.  Bound by the L1 wavefronts of the gathered loads (the
+// markers of a warp lie on a circle): a thread per plane of one n read each
+// point three times, 28.5 us for 4 cylinders in 256x128x128, XXX us with NB = 4.
+// In 2D the one plane has weight 1.
+template <int NB, bool D3>
+__global__ void __launch_bounds__(128) k_ibm_interp_f(IbmArgsF a, Geo g) {
     const int m = blockIdx.x * 32 + threadIdx.x;
-    const int dk = threadIdx.y;
-    const int n = blockIdx.y + 1;
+    const int n0 = (blockIdx.y * blockDim.y + threadIdx.y) * NB + 1;
     const int comp = blockIdx.z;
-    df ub{0.0f, 0.0f};
-    if (m < a.nm) {
-        const int i0 = a.i0[comp][m], j0 = a.j0[comp][m];
-        const float *wx = a.wx[comp] + 3 * m, *wy = a.wy[comp] + 3 * m;
-        const int k = n - 1 + dk;
-        const float wz = a.wz[comp][dk];
-        // a stencil inside the interior columns and rows (no x wrap, no wall
-        // rule) reads its 9 points at fixed offsets from one base index; the
-        // values and their order of summation are those of ua_at / ustar_at
-        const bool inner = i0 >= 1 && i0 + 2 <= g.nx && j0 >= 1 && j0 + 2 <= g.ny &&
-                           !(g.walls && comp == 1 && j0 + 2 == g.ny);
+    if (m >= a.nm || n0 > g.nz) return;
+    const int i0 = a.i0[comp][m], j0 = a.j0[comp][m];
+    float wxy[9];
+#pragma unroll
+    for (int dj = 0; dj < 3; ++dj)
+#pragma unroll
+        for (int di = 0; di < 3; ++di) wxy[3 * dj + di] = a.wx[comp][3 * m + di] * a.wy[comp][3 * m + dj];
+    const float *Uh = a.Uh[comp], *Ul = a.Ul[comp];
+    const float *X = a.mode ? a.D[comp] : a.Qc[comp];
+    const int xs = a.mode ? g.sx : g.nx;
+    // a stencil inside the interior columns and rows (no x wrap, no wall
+    // rule) reads its 9 points at fixed offsets from one base index; the
+    // values and their order of summation are those of ua_at / ustar_at
+    const bool inner = i0 >= 1 && i0 + 2 <= g.nx && j0 >= 1 && j0 + 2 <= g.ny &&
+                       !(g.walls && comp == 1 && j0 + 2 == g.ny);
+    df sum[NB];
+#pragma unroll
+    for (int p = D3 ? 0 : 1; p < (D3 ? NB + 2 : 2); ++p) {
+        const int k = n0 - 1 + p;
+        if (k > g.nz + 1) break;
+        df u[9];
         if (inner) {
             const int kk = wrapz(g, k);
             const int hb = hix(g, i0, j0, k);
-            const float *Uh = a.Uh[comp], *Ul = a.Ul[comp];
-            const float *X = a.mode ? a.D[comp] : a.Qc[comp];
             const int xb = a.mode ? hix(g, i0, j0, kk) : qix(g, i0, j0, kk);
-            const int xs = a.mode ? g.sx : g.nx;
             float uh[9], ul[9], xv[9];
 #pragma unroll
-            for (int dj = 0; dj < 3; ++dj)
+            for (int q = 0; q < 9; ++q) {
+                const int h = hb + q % 3 + g.sx * (q / 3);
+                uh[q] = Uh[h];
+                ul[q] = Ul[h];
+                xv[q] = X[xb + q % 3 + xs * (q / 3)];
+            }
 #pragma unroll
-                for (int di = 0; di < 3; ++di) {
-                    const int h = hb + di + g.sx * dj;
-                    uh[3 * dj + di] = Uh[h];
-                    ul[3 * dj + di] = Ul[h];
-                    xv[3 * dj + di] = X[xb + di + xs * dj];
-                }
-#pragma unroll
-            for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-                for (int di = 0; di < 3; ++di) {
-                    const float w = wx[di] * wy[dj] * wz;
-                    const int q = 3 * dj + di;
-                    ub = df_add(ub, df_mul_f(df_add_f(df{uh[q], ul[q]}, xv[q]), w));
-                }
+            for (int q = 0; q < 9; ++q) u[q] = df_add_f(df{uh[q], ul[q]}, xv[q]);
         } else {
 #pragma unroll
-            for (int dj = 0; dj < 3; ++dj)
+            for (int q = 0; q < 9; ++q)
+                u[q] = a.mode ? ustar_at(g, Uh, Ul, X, comp, i0 + q % 3, j0 + q / 3, k, a.uw2)
+                              : ua_at(g, Uh, Ul, X, comp, i0 + q % 3, j0 + q / 3, k, a.uw2);
+        }
 #pragma unroll
-                for (int di = 0; di < 3; ++di) {
-                    const float w = wx[di] * wy[dj] * wz;
-                    const df uv = a.mode ? ustar_at(g, a.Uh[comp], a.Ul[comp], a.D[comp], comp, i0 + di, j0 + dj, k, a.uw2)
-                                         : ua_at(g, a.Uh[comp], a.Ul[comp], a.Qc[comp], comp, i0 + di, j0 + dj, k, a.uw2);
-                    ub = df_add(ub, df_mul_f(uv, w));
-                }
+        for (int dk = 0; dk < 3; ++dk) {
+            const int r = p - dk;            // plane n0 + r has this plane at its offset dk - 1
+            if (r < 0 || r >= NB || (!D3 && dk != 1)) continue;
+            const float wz = a.wz[comp][dk];
+            df ub{0.0f, 0.0f};
+#pragma unroll
+            for (int q = 0; q < 9; ++q) ub = df_add(ub, df_mul_f(u[q], wxy[q] * wz));
+            sum[r] = dk == 0 || !D3 ? ub : df_add(sum[r], ub);
         }
     }
-    part[dk][threadIdx.x] = ub;
-    __syncthreads();
-    if (dk == 0 && m < a.nm) {
-        const df s3 = df_add(df_add(part[0][threadIdx.x], part[1][threadIdx.x]), part[2][threadIdx.x]);
-        const double uc = comp == 0 ? a.mu[m] : (comp == 1 ? a.mv[m] : 0.0);
-        const size_t q = m + (size_t)a.nm * (n - 1);
+    const double uc = comp == 0 ? a.mu[m] : (comp == 1 ? a.mv[m] : 0.0);
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+        if (n0 + r > g.nz) break;
+        const size_t q = m + (size_t)a.nm * (n0 + r - 1);
         double *fc = &a.Fc[comp][q];
-        const double v = (a.accumulate ? *fc : 0.0) + (uc - ((double)s3.hi + (double)s3.lo)) * a.idt;
+        const double v = (a.accumulate ? *fc : 0.0) + (uc - ((double)sum[r].hi + (double)sum[r].lo)) * a.idt;
         *fc = v;
         // one conversion per marker and plane: the spreading reads each
         // force once per list entry and plane, and a double-to-float
@@ -2488,8 +2495,16 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
             if (r == 0 && repeats > 1)
                 for (int c = 0; c < nvc; ++c)
                     F8_CUDA_RET(cudaMemcpyAsync(d.Qpre[c], d.Qf[c], (size_t)d.ni * sizeof(float), cudaMemcpyDeviceToDevice, s));
-            dim3 gi((d.nm + 31) / 32, g.nz, nvc);
-            k_ibm_interp_f<<<gi, dim3(32, 3), 0, s>>>(a, g); count_launch();
+            // planes per thread: as many as leave the chip 12 warps an SM or more
+            // (us of the IBM stage with 1, 2, 4: 548 markers x 128 planes 54.6,
+            // 43.9, 48.4; 2864 x 256 planes -, 324, 278; 66 x 64 planes 18.6, 20.9, 25.9)
+            const unsigned mb = (unsigned)((d.nm + 31) / 32);
+            const long mw = 3l * mb * g.nz, fill = 12l * device_sm_count();
+            if (!d3) k_ibm_interp_f<1, false><<<dim3(mb, 1, 2), 32, 0, s>>>(a, g);
+            else if (mw >= 8 * fill) k_ibm_interp_f<4, true><<<dim3(mb, (g.nz + 15) / 16, 3), dim3(32, 4), 0, s>>>(a, g);
+            else if (mw >= 2 * fill) k_ibm_interp_f<2, true><<<dim3(mb, (g.nz + 7) / 8, 3), dim3(32, 4), 0, s>>>(a, g);
+            else k_ibm_interp_f<1, true><<<dim3(mb, (g.nz + 3) / 4, 3), dim3(32, 4), 0, s>>>(a, g);
+            count_launch();
             // the drag needs only the marker forces: beside the spreading and
             // the solves (joined after the solves)
             const bool want_drag = last && drag_out_dev;

@@ -10,6 +10,7 @@
 // kx = 0..NX/2 (NXH = NX/2+1 values per row).
 #pragma once
 #include <algorithm>
+#include <type_traits>
 #include "f8_common.cuh"
 #include "f8_df64.cuh"
 
@@ -64,6 +65,7 @@ __device__ __forceinline__ void stockham_stage(const Cx<T> *x, Cx<T> *y, int lg,
 // there are two blocks per SM (304).  2D 128^2, FP64: 19 us a pass with 16
 // columns in each of 5 blocks, 4 us with one in each of 65.
 constexpr long FFT_MIN_BLOCKS = 304;
+constexpr long FFT_REG_WARPS = 150;
 
 // lines (row pairs) per block of an x pass over `pairs` row pairs
 inline int fft_pairs_per_block(int n, long pairs) {
@@ -83,6 +85,107 @@ inline int fft_cols_per_block(int n, int ncols, long sets) {
 template <typename T>
 inline int fft_line_threads(int n, int tx) {
     return std::min(256, std::max(32, n / 2 * tx));
+}
+
+// ---------------------------------------------------------------------------
+// A line of n = 2^LG values (32 .. 1024) held by G = n / 8 threads: the stages of
+// the Stockham kernels below (the same butterflies, twiddles and order, so the
+// same bits) as decimation in time, up to three of them at a time on eight
+// values in registers, with one exchange through shared memory between the
+// passes instead of one per stage.  The value of element e lies at ix(e); lanes
+// of one line and neighbouring lines fall into distinct banks.
+template <int LG>
+struct LineFft {
+    static constexpr int N = 1 << LG, G = N / 8, PITCH = N + N / 8 + 1;
+    static __device__ __forceinline__ int ix(int e) { return e + (e >> 3); }
+    static __device__ __forceinline__ int brev(int e) { return (int)(__brev((unsigned)e) >> (32 - LG)); }
+};
+
+// stages L0 .. L0 + R - 1 on the groups base + (s << L0), s < 2^R, of thread t
+template <bool INV, int LG, int L0, int R, typename T, typename Load, typename Store>
+__device__ __forceinline__ void fft_pass(int t, const T *twr, const T *twi, Load load, Store store) {
+    constexpr int W = 1 << R, U = 8 / W;
+    Cx<T> v[8];
+    int lo[U], base[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int g = t + u * LineFft<LG>::G;
+        lo[u] = g & ((1 << L0) - 1);
+        base[u] = ((g >> L0) << (L0 + R)) | lo[u];
+#pragma unroll
+        for (int s = 0; s < W; ++s) v[u * W + s] = load(base[u] + (s << L0));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int a = 0; a < R; ++a) {
+            const int m = 1 << a;
+#pragma unroll
+            for (int s = 0; s < W; ++s) {
+                if (s & m) continue;
+                const Cx<T> x = v[u * W + s], b = v[u * W + s + m];
+                Cx<T> c = b;
+                if (L0 > 0 || (s & (m - 1))) {       // the others' twiddle is 1
+                    const int q = (lo[u] + ((s & (m - 1)) << L0)) << (LG - 1 - L0 - a);
+                    c = twiddle_mul<INV>(b, twr[q], INV ? -twi[q] : twi[q]);
+                }
+                v[u * W + s] = Cx<T>{x.r + c.r, x.i + c.i};
+                v[u * W + s + m] = Cx<T>{x.r - c.r, x.i - c.i};
+            }
+        }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int s = 0; s < W; ++s) store(base[u] + (s << L0), v[u * W + s]);
+}
+
+// natural order in (load(e)) and out (store(e, value)); z: the line's PITCH
+// values of shared memory, free on entry.  Every thread of the block takes part.
+template <bool INV, int LG, typename T, typename Load, typename Store>
+__device__ __forceinline__ void fft_line(Cx<T> *z, int t, const T *twr, const T *twi, Load load, Store store) {
+    using L = LineFft<LG>;
+    auto get = [&](int e) { return z[L::ix(e)]; };
+    auto put = [&](int e, Cx<T> v) { z[L::ix(e)] = v; };
+    fft_pass<INV, LG, 0, 3, T>(t, twr, twi, [&](int e) { return load(L::brev(e)); }, put);
+    __syncthreads();
+    if constexpr (LG == 5) fft_pass<INV, LG, 3, 2, T>(t, twr, twi, get, store);
+    else if constexpr (LG == 6) fft_pass<INV, LG, 3, 3, T>(t, twr, twi, get, store);
+    else {
+        constexpr int R1 = LG == 7 ? 2 : 3, L2 = 3 + R1;
+        fft_pass<INV, LG, 3, R1, T>(t, twr, twi, get, put);
+        __syncthreads();
+        if constexpr (LG == 10) {
+            fft_pass<INV, LG, 6, 2, T>(t, twr, twi, get, put);
+            __syncthreads();
+            fft_pass<INV, LG, 8, 2, T>(t, twr, twi, get, store);
+        } else fft_pass<INV, LG, L2, LG - L2, T>(t, twr, twi, get, store);
+    }
+}
+
+// Lines of 32 to 1024 values go through registers in FP32, and in FP64 where
+// they make 150 warps or more: a smaller FP64 problem is a chain of stages,
+// shortest with one butterfly per thread (f8_fft_solve, us, stages in shared
+// memory / in registers: 128^2 46.5 / 68.8, 256^2 (128 warps) 55 / 78, 512^2 104 / 99,
+// 64^3 119 / 115, 128x64x64 298 / 266, 256x128x128 1179 / 1100; batches of three
+// 64^3 solves 79 / 76 each).  FP32 lines of 512: x pass 6.3 / 4.3, y lines with
+// the division 11.4 / 9.8.
+template <typename T>
+inline bool fft_in_registers(int n, long lines) {
+    if (n < 32 || n > 1024) return false;
+    return sizeof(T) == 4 || lines * (n / 8) >= 32 * FFT_REG_WARPS;
+}
+
+// go(integral_constant LG) for a line of n = 2^LG values, 32 .. 1024
+template <typename F>
+inline void fft_by_length(int n, F go) {
+    switch (n) {
+    case 32: go(std::integral_constant<int, 5>{}); break;
+    case 64: go(std::integral_constant<int, 6>{}); break;
+    case 128: go(std::integral_constant<int, 7>{}); break;
+    case 256: go(std::integral_constant<int, 8>{}); break;
+    case 512: go(std::integral_constant<int, 9>{}); break;
+    default: go(std::integral_constant<int, 10>{}); break;
+    }
 }
 
 // Up to three transforms of the same shape in one launch (blockIdx.z; their
@@ -139,9 +242,55 @@ __global__ void k_fft_x_fwd(Batch<const TS *> srcs, T *__restrict__ H, size_t hs
     }
 }
 
+template <int LG, typename T, typename TS>
+__global__ void __launch_bounds__(256) k_fft_x_fwd_r(Batch<const TS *> srcs, T *__restrict__ H, size_t hstride,
+                                                     int nrow_src, int j0, int nrow_h, int npairs_per_plane, int nplanes,
+                                                     const T *__restrict__ twr, const T *__restrict__ twi) {
+    using L = LineFft<LG>;
+    extern __shared__ unsigned char smem_raw[];
+    const TS *__restrict__ src = srcs.p[blockIdx.z];
+    H += (size_t)blockIdx.z * hstride;
+    const int p = threadIdx.x / L::G, t = threadIdx.x % L::G;
+    const long pair = (long)blockIdx.x * (blockDim.x / L::G) + p;
+    const bool active = pair < (long)npairs_per_plane * nplanes;
+    Cx<T> *z = reinterpret_cast<Cx<T> *>(smem_raw) + p * L::PITCH;
+    const int k = active ? (int)(pair / npairs_per_plane) : 0, jj = active ? 2 * (int)(pair % npairs_per_plane) : 0;
+    const TS *ra = src + (size_t)L::N * ((size_t)(j0 + jj - 1) + (size_t)nrow_src * k), *rb = ra + L::N;
+    fft_line<false, LG, T>(z, t, twr, twi, [&](int e) { return active ? Cx<T>{T(ra[e]), T(rb[e])} : Cx<T>{T(0), T(0)}; },
+                           [&](int e, Cx<T> v) { z[L::ix(e)] = v; });
+    __syncthreads();
+    if (!active) return;
+    constexpr int nxh = L::N / 2 + 1;
+    Cx<T> *ha = reinterpret_cast<Cx<T> *>(H) + (size_t)nxh * ((size_t)jj + (size_t)nrow_h * k), *hb = ha + nxh;
+    for (int kx = t; kx < nxh; kx += L::G) {
+        const Cx<T> zk = z[L::ix(kx)], zm = z[L::ix((L::N - kx) & (L::N - 1))];
+        ha[kx] = Cx<T>{(zk.r + zm.r) * T(0.5), (zk.i - zm.i) * T(0.5)};
+        hb[kx] = Cx<T>{(zk.i + zm.i) * T(0.5), (zm.r - zk.r) * T(0.5)};
+    }
+}
+
+// row pairs per block of the register passes
+inline int fft_reg_lines(int n, long lines) {
+    int p = std::max(1, 2048 / n);
+    while (p > 1 && p * n > 256 && (lines + p - 1) / p < FFT_MIN_BLOCKS) p >>= 1;
+    return p;
+}
+
 template <typename T, typename TS>
 inline void fft_x_fwd(int nb, Batch<const TS *> src, T *H, size_t hstride, int n, int nrow_src, int j0, int nrow_h,
                       int npairs, int nplanes, const T *twr, const T *twi, cudaStream_t s) {
+    const long lines = (long)npairs * nplanes;
+    if (fft_in_registers<T>(n, lines * nb)) {
+        const int pl = fft_reg_lines(n, lines * nb);
+        fft_by_length(n, [&](auto lg) {
+            using L = LineFft<decltype(lg)::value>;
+            k_fft_x_fwd_r<decltype(lg)::value, T, TS>
+                <<<dim3((unsigned)((lines + pl - 1) / pl), 1, nb), pl * L::G, pl * L::PITCH * sizeof(Cx<T>), s>>>(
+                    src, H, hstride, nrow_src, j0, nrow_h, npairs, nplanes, twr, twi);
+        });
+        count_launch();
+        return;
+    }
     const int ppc = fft_pairs_per_block(n, (long)npairs * nplanes * nb);
     const size_t smem = (size_t)ppc * 2 * n * sizeof(Cx<T>);
     const dim3 grid((unsigned)(((long)npairs * nplanes + ppc - 1) / ppc), 1, nb);
@@ -224,9 +373,54 @@ __global__ void k_fft_x_inv(const T *__restrict__ H, size_t hstride, Batch<Out> 
     for (int e = t; e < n; e += tpp) { out.put(oa + e, x[e].r); out.put(ob + e, x[e].i); }
 }
 
+template <int LG, typename T, typename Out>
+__global__ void __launch_bounds__(256) k_fft_x_inv_r(const T *__restrict__ H, size_t hstride, Batch<Out> outs, int nrow_h,
+                                                     int npairs_per_plane, int nplanes, int jdst0, int sx, int sy,
+                                                     const T *__restrict__ twr, const T *__restrict__ twi, int plain) {
+    using L = LineFft<LG>;
+    extern __shared__ unsigned char smem_raw[];
+    const Out out = outs.p[blockIdx.z];
+    H += (size_t)blockIdx.z * hstride;
+    const int p = threadIdx.x / L::G, t = threadIdx.x % L::G;
+    const long pair = (long)blockIdx.x * (blockDim.x / L::G) + p;
+    const bool active = pair < (long)npairs_per_plane * nplanes;
+    Cx<T> *z = reinterpret_cast<Cx<T> *>(smem_raw) + p * L::PITCH;
+    const int k = active ? (int)(pair / npairs_per_plane) : 0, jj = active ? 2 * (int)(pair % npairs_per_plane) : 0;
+    constexpr int half = L::N / 2, nxh = half + 1;
+    const Cx<T> *ha = reinterpret_cast<const Cx<T> *>(H) + (size_t)nxh * ((size_t)jj + (size_t)nrow_h * k), *hb = ha + nxh;
+    const size_t oa = plain ? (size_t)L::N * ((size_t)(jdst0 + jj) + (size_t)sy * k)
+                            : 1 + (size_t)sx * ((size_t)(jdst0 + jj) + (size_t)sy * (k + 1));
+    const size_t ob = oa + (plain ? L::N : sx);
+    fft_line<true, LG, T>(
+        z, t, twr, twi,
+        [&](int e) {
+            if (!active) return Cx<T>{T(0), T(0)};
+            const int m = e <= half ? e : L::N - e;
+            const Cx<T> a = ha[m], b = hb[m];
+            return e <= half ? Cx<T>{a.r - b.i, a.i + b.r} : Cx<T>{a.r + b.i, b.r - a.i};
+        },
+        [&](int e, Cx<T> v) {
+            if (!active) return;
+            out.put(oa + e, v.r);
+            out.put(ob + e, v.i);
+        });
+}
+
 template <typename T, typename Out>
 inline void fft_x_inv(int nb, const T *H, size_t hstride, Batch<Out> out, int n, int nrow_h, int npairs, int nplanes,
                       int jdst0, int sx, int sy, const T *twr, const T *twi, int plain, cudaStream_t s) {
+    const long lines = (long)npairs * nplanes;
+    if (fft_in_registers<T>(n, lines * nb)) {
+        const int pl = fft_reg_lines(n, lines * nb);
+        fft_by_length(n, [&](auto lg) {
+            using L = LineFft<decltype(lg)::value>;
+            k_fft_x_inv_r<decltype(lg)::value, T, Out>
+                <<<dim3((unsigned)((lines + pl - 1) / pl), 1, nb), pl * L::G, pl * L::PITCH * sizeof(Cx<T>), s>>>(
+                    H, hstride, out, nrow_h, npairs, nplanes, jdst0, sx, sy, twr, twi, plain);
+        });
+        count_launch();
+        return;
+    }
     const int ppc = fft_pairs_per_block(n, (long)npairs * nplanes * nb);
     const size_t smem = (size_t)ppc * 2 * n * sizeof(Cx<T>);
     const dim3 grid((unsigned)(((long)npairs * nplanes + ppc - 1) / ppc), 1, nb);
@@ -307,10 +501,70 @@ __global__ void __launch_bounds__(256) k_fft_lines(T *__restrict__ H, size_t hst
     }
 }
 
+// mode 0 (INV: the sign) and 1 of k_fft_lines on register lines; neighbouring
+// threads take neighbouring columns
+template <int LG, bool SOLVE, bool INV, typename T>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256) k_fft_lines_r(T *__restrict__ H, size_t hstride, int lstride, int ncols,
+                                                     int sstride, int tx, const T *__restrict__ twr,
+                                                     const T *__restrict__ twi, DivideSpec dv) {
+    using L = LineFft<LG>;
+    extern __shared__ unsigned char smem_raw[];
+    const int c = threadIdx.x & (tx - 1), t = threadIdx.x >> (31 - __clz(tx)), kx = blockIdx.x * tx + c, set = blockIdx.y;
+    const bool active = kx < ncols;
+    Cx<T> *z = reinterpret_cast<Cx<T> *>(smem_raw) + c * L::PITCH;
+    Cx<T> *Hc = reinterpret_cast<Cx<T> *>(H + (size_t)blockIdx.z * hstride) + (size_t)set * sstride + kx;
+    auto load = [&](int e) { return active ? Hc[(size_t)e * lstride] : Cx<T>{T(0), T(0)}; };
+    auto store = [&](int e, Cx<T> v) {
+        if (active) Hc[(size_t)e * lstride] = v;
+    };
+    if constexpr (!SOLVE) {
+        fft_line<INV, LG, T>(z, t, twr, twi, load, store);
+    } else {
+        Cx<T> keep[8];
+        int at = 0;
+        fft_line<false, LG, T>(z, t, twr, twi, load, [&](int e, Cx<T> v) {
+            // element e of the line: along z -> kz = e, ky = set; along y -> ky = e, kz = set
+            const int jy = dv.line_is_z ? set : e, kz = dv.line_is_z ? e : set;
+            const double lhs = dv.lhs0 + dv.lhs1 * (dv.kx2[active ? kx : 0] + dv.ky2[jy] + dv.kz2[kz]);
+            const T qr = v.r * T(dv.inv_ntot), qi = v.i * T(dv.inv_ntot);
+            keep[at++] = fabs(lhs) < 1.0e-16 ? Cx<T>{T(0), T(0)} : Cx<T>{qr / T(lhs), qi / T(lhs)};
+        });
+        __syncthreads();      // the last pass has read the line
+        constexpr int RL = LG == 5 || LG == 7 || LG == 8 || LG == 10 ? 2 : 3, L0 = LG - RL, W = 1 << RL;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int g = t + q / W * L::G, e = ((g >> L0) << LG) | (g & ((1 << L0) - 1)) | (q % W << L0);
+            z[L::ix(e)] = keep[q];
+        }
+        __syncthreads();
+        Cx<T> in[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) in[s] = z[L::ix(L::brev(8 * t + s))];
+        __syncthreads();
+        at = 0;
+        fft_line<true, LG, T>(z, t, twr, twi, [&](int) { return in[at++]; }, store);
+    }
+}
+
 template <typename T>
 inline void fft_lines(int nb, T *H, size_t hstride, int n, int lstride, int ncols, int sets, int sstride, const T *twr,
                       const T *twi, int sign, int mode, const DivideSpec &dv, cudaStream_t s) {
     const int tx = fft_cols_per_block<T>(n, ncols, (long)sets * nb);
+    if (fft_in_registers<T>(n, (long)ncols * sets * nb)) {
+        fft_by_length(n, [&](auto lg) {
+            constexpr int LG = decltype(lg)::value;
+            using L = LineFft<LG>;
+            auto go = [&](auto kernel) {
+                kernel<<<dim3((ncols + tx - 1) / tx, sets, nb), tx * L::G, tx * L::PITCH * sizeof(Cx<T>), s>>>(
+                    H, hstride, lstride, ncols, sstride, tx, twr, twi, dv);
+            };
+            if (mode == 1) go(k_fft_lines_r<LG, true, false, T>);
+            else if (sign < 0) go(k_fft_lines_r<LG, false, false, T>);
+            else go(k_fft_lines_r<LG, false, true, T>);
+        });
+        count_launch();
+        return;
+    }
     const size_t smem = (size_t)2 * n * tx * sizeof(Cx<T>);
     k_fft_lines<T><<<dim3((ncols + tx - 1) / tx, sets, nb), fft_line_threads<T>(n, tx), smem, s>>>(
         H, hstride, ilog2_pow2(n), lstride, ncols, sstride, tx, twr, twi, sign, mode, dv);

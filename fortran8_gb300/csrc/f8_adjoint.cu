@@ -16,7 +16,7 @@ namespace f8 {
 
 cudaError_t adjoint_fold_state(AdjState &A, const Dev &d, cudaStream_t s) {
     const Geo &g = d.g;
-    return fold(fold_with_c(fold_set<double>({{A.lU, BC_U}, {A.lV, BC_V}, {A.lW, BC_W}, {A.lP, BC_P}}), A.lC, d.cs, 6), g, s);
+    return fold_walls(fold_with_c(fold_set<double>({{A.lU, BC_U}, {A.lV, BC_V}, {A.lW, BC_W}, {A.lP, BC_P}}), A.lC, d.cs, 6), g, s);
 }
 
 cudaError_t take_interior(const double *src, double *dst, const Geo &g, int n, cudaStream_t s) {
@@ -31,18 +31,16 @@ cudaError_t step_fp64_adjoint(Dev &d, AdjState &A, const TapeStep &t, const doub
     const size_t hb = (size_t)cs * sizeof(double);
     const double dt = d.ph.dt, re = d.ph.re, beta = d.ph.beta, wi = d.ph.wi;
     const double kap = dt * beta / re / 2.0;
-    const unsigned nb = (unsigned)((cs + 255) / 256);
     dim3 blk(32, 8);
     const AdjCoef<double> kc = adj_coef<double>(g);
     // 6. projection / pressure update
-    k_march_adj<double><<<nb, 256, 0, s>>>(A.lU, A.lV, A.lW, A.lP, A.lPhi, t.Phi, g, kap, dt / (2.0 * re), kc, A.grad); count_launch();
-    F8_CUDA_RET(fold(fold_set<double>({{A.lPhi, BC_P}}), g, s));
+    k_march_adj<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lU, A.lV, A.lW, A.lP, A.pack, t.Phi, g, kap, dt / (2.0 * re), kc,
+                                                          A.grad); count_launch();
     // 5. Poisson.  The solve maps the right-hand side to the zero-mean Phi
     // through the pseudo-inverse of the symmetric Laplacian, so its transpose
     // is the same map applied to the zero-mean part of the adjoint: the FFT
     // solve (which drops the mean mode), or, for the SOR variant, the same
     // red-black SOR to the same tolerance (then shifted to zero mean)
-    k_pack<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lPhi, A.pack, g); count_launch();
     double *lq = A.lQ[0];
     if (A.sor) {
         F8_CUDA_RET(remove_mean_fp64(d, A.pack, d.ni, s));
@@ -53,32 +51,25 @@ cudaError_t step_fp64_adjoint(Dev &d, AdjState &A, const TapeStep &t, const doub
     } else {
         F8_CUDA_RET(poisson_solve_fp64(d, A.pack, A.lQ[0], s));
     }
-    k_div_adj<double><<<nb, 256, 0, s>>>(A.lU, A.lV, A.lW, lq, A.lUp[0], A.lUp[1], A.lUp[2], g); count_launch();
-    F8_CUDA_RET(fold(fold_set<double>({{A.lUp[0], BC_U}, {A.lUp[1], BC_V}, {A.lUp[2], BC_W}}), g, s));
+    DivAdjOut<double> dout{};
+    for (int c = 0; c < 3; ++c) { dout.pk[c] = A.pack + (size_t)c * d.ni; dout.lUa[c] = A.lUa[c]; }
+    k_div_adj<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lU, A.lV, A.lW, lq, dout, g); count_launch();
     // 4. Helmholtz
-    {
-        double *pk[3];
-        for (int c = 0; c < 3; ++c) pk[c] = A.pack + (size_t)c * d.ni;
-        k_pack3<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lUp[0], A.lUp[1], A.lUp[2], pk[0], pk[1], pk[2], g);
-        count_launch();
-        F8_CUDA_RET(helmholtz_solves_fp64(d, 3, pk, A.lQ, s));
-    }
+    F8_CUDA_RET(helmholtz_solves_fp64(d, 3, dout.pk, A.lQ, s));
     // 3. IBM
-    for (int c = 0; c < 3; ++c) F8_CUDA_RET(cudaMemsetAsync(A.lUa[c], 0, hb, s));
     if (d.nm > 0) {
         IbmAdjArgs<double> ia{};
         ia.mx = d.mx; ia.my = d.my; ia.mcyl = d.mcyl; ia.nm = d.nm; ia.ncyl = d.ncyl;
-        ia.dvol = (g.dx * g.dy) * g.dz; ia.dxn = g.dx * g.dx * g.dx; ia.mvol = d.mvol; ia.cylvol = d.cylvol;
+        ia.idx = 1.0 / g.dx; ia.idy = 1.0 / g.dy; ia.mvol = d.mvol;
+        ia.idvol = 1.0 / ((g.dx * g.dy) * g.dz); ia.dvn = (g.dx * g.dx * g.dx) / ((g.dx * g.dy) * g.dz); ia.cylvol = d.cylvol;
         for (int c = 0; c < 3; ++c) {
+            ia.i0[c] = d.mi0d[c]; ia.j0[c] = d.mj0d[c];
             ia.Ua[c] = t.Ua[c]; ia.Fc[c] = t.Fc[c]; ia.lQ[c] = A.lQ[c]; ia.lUa[c] = A.lUa[c];
         }
         ia.w = drag_w;
         ia.grad = A.grad;
         ia.d3 = 1;
-        k_ibm_adj<double><<<dim3((d.nm + 127) / 128, g.nz, 3), 128, 0, s>>>(ia, g); count_launch();
-        // the y and x passes only where a stencil reaches a ghost column or row
-        const FoldSet<double> fa = fold_set<double>({{A.lUa[0], BC_U}, {A.lUa[1], BC_V}, {A.lUa[2], BC_W}});
-        F8_CUDA_RET(d.ibm_edge ? fold(fa, g, s) : fold_z_only(fa, g, s));
+        k_ibm_adj<double><<<dim3(g.nz, 3), ibm_adj_block(d.nm), 0, s>>>(ia, g); count_launch();
     }
     // 2. momentum right-hand side: per-cell sources, then the gather of the
     // velocity, pressure and (with the polymer) C0 / C adjoints
@@ -102,28 +93,22 @@ cudaError_t step_fp64_adjoint(Dev &d, AdjState &A, const TapeStep &t, const doub
         mg.lp2 = d.ph.lp2; mg.inv_1mb = 1.0 / (1.0 - beta); mg.inv_wi = 1.0 / wi;
         mg.grad = A.grad;
         mg.kc = kc;
-        k_momadj_gather<double><<<nb, 256, 0, s>>>(mg, g); count_launch();
+        k_momadj_gather<double><<<adj_rows(g, blk), blk, 0, s>>>(mg, g); count_launch();
     }
     // 1. polymer: per-cell implicit-function adjoint and Cstar weights, then
     // the gather of the adjoint of C^n and of the velocity
     if (polymer) {
-        // with walls the stress read the updated ghost rows and their x/z
-        // copies; the state's C (wall-extrapolated) adjoint is interior already
-        if (g.walls) F8_CUDA_RET(fold_xz(fold_c(A.lC, cs), g, s));
-        else F8_CUDA_RET(fold(fold_c(A.lC, cs), g, s));
         PolyAdjArgs<double> pa{};
         pa.C = t.C; pa.Cn = t.Cn; pa.codes = t.codes; pa.codes_g = t.codes_g; pa.U = t.U; pa.V = t.V; pa.W = t.W;
         pa.lX = A.lC;
         pa.cs = cs; pa.dt = dt; pa.wi = wi; pa.lp2 = d.ph.lp2; pa.grad = A.grad;
         pa.kc = kc; pa.dtwi = dt / wi; pa.dtwi2 = dt / (wi * wi);
-        dim3 pb(32, 4);
-        const dim3 pg((g.nx + pb.x - 1) / pb.x, (prows(g) + pb.y - 1) / pb.y, g.nz);
-        k_polyadj_mu<double><<<pg, pb, 0, s>>>(pa, A.work, g); count_launch();
-        const dim3 pb2(32, 8), pg2((g.nx + pb2.x - 1) / pb2.x, (prows(g) + pb2.y - 1) / pb2.y, g.nz);
-        k_polyadj_cstar<double><<<pg2, pb2, 0, s>>>(pa, A.work, g); count_launch();
+        const dim3 pb(32, 4);
+        k_polyadj_mu<double><<<adj_rows(g, pb), pb, 0, s>>>(pa, A.work, g); count_launch();
+        k_polyadj_cstar<double><<<adj_rows(g, blk), blk, 0, s>>>(pa, A.work, g); count_launch();
         PolyGatherArgs<double> pga{};
         pga.src = A.work; pga.lC = A.lC2; pga.lU = A.lU; pga.lV = A.lV; pga.lW = A.lW; pga.cs = cs;
-        k_polyadj_gather<double><<<nb, 256, 0, s>>>(pga, g); count_launch();
+        k_polyadj_gather<double><<<adj_rows(g, blk), blk, 0, s>>>(pga, g); count_launch();
         std::swap(A.lC, A.lC2);
     } else {
         F8_CUDA_RET(cudaMemsetAsync(A.lC, 0, 6 * hb, s));
@@ -500,10 +485,9 @@ cudaError_t step_fp64_adjoint2(Dev &d, AdjState &A, const TapeStep &t, const dou
     kc.id[2] = kc.id2[2] = kc.i4[2] = kc.dtd[2] = kc.dt2d[2] = kc.dt4d[2] = 0.0;   // no z terms
     F8_CUDA_RET(cudaMemsetAsync(A.lW, 0, hb, s));
     // 6. projection / pressure update
-    k_march_adj<double><<<nb, 256, 0, s>>>(A.lU, A.lV, A.lW, A.lP, A.lPhi, t.Phi, g, kap, dt / (2.0 * re), kc, A.grad); count_launch();
-    F8_CUDA_RET(fold(fold_set<double>({{A.lPhi, BC_P}}), g, s));
+    k_march_adj<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lU, A.lV, A.lW, A.lP, A.pack, t.Phi, g, kap, dt / (2.0 * re), kc,
+                                                          A.grad); count_launch();
     // 5. Poisson
-    k_pack<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lPhi, A.pack, g); count_launch();
     double *lq = A.lQ[0];
     if (A.sor) {
         F8_CUDA_RET(remove_mean_fp64(d, A.pack, d.ni, s));
@@ -514,31 +498,25 @@ cudaError_t step_fp64_adjoint2(Dev &d, AdjState &A, const TapeStep &t, const dou
     } else {
         F8_CUDA_RET(poisson_solve_fp64(d, A.pack, A.lQ[0], s));
     }
-    k_div_adj<double><<<nb, 256, 0, s>>>(A.lU, A.lV, A.lW, lq, A.lUp[0], A.lUp[1], A.lUp[2], g); count_launch();
-    F8_CUDA_RET(fold(fold_set<double>({{A.lUp[0], BC_U}, {A.lUp[1], BC_V}}), g, s));
+    DivAdjOut<double> dout{};
+    for (int c = 0; c < 2; ++c) { dout.pk[c] = A.pack + (size_t)c * d.ni; dout.lUa[c] = A.lUa[c]; }
+    k_div_adj<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lU, A.lV, A.lW, lq, dout, g); count_launch();
     // 4. Helmholtz
-    {
-        double *pk[2];
-        for (int c = 0; c < 2; ++c) {
-            pk[c] = A.pack + (size_t)c * d.ni;
-            k_pack<double><<<adj_cells(g, blk), blk, 0, s>>>(A.lUp[c], pk[c], g); count_launch();
-        }
-        F8_CUDA_RET(helmholtz_solves_fp64(d, 2, pk, A.lQ, s));
-    }
+    F8_CUDA_RET(helmholtz_solves_fp64(d, 2, dout.pk, A.lQ, s));
     // 3. IBM
-    for (int c = 0; c < 2; ++c) F8_CUDA_RET(cudaMemsetAsync(A.lUa[c], 0, hb, s));
     if (d.nm > 0) {
         IbmAdjArgs<double> ia{};
         ia.mx = d.mx; ia.my = d.my; ia.mcyl = d.mcyl; ia.nm = d.nm; ia.ncyl = d.ncyl;
-        ia.dvol = g.dx * g.dy; ia.dxn = g.dx * g.dx; ia.mvol = d.mvol; ia.cylvol = d.cylvol;
+        ia.idx = 1.0 / g.dx; ia.idy = 1.0 / g.dy; ia.mvol = d.mvol;
+        ia.idvol = 1.0 / (g.dx * g.dy); ia.dvn = (g.dx * g.dx) / (g.dx * g.dy); ia.cylvol = d.cylvol;
         for (int c = 0; c < 2; ++c) {
+            ia.i0[c] = d.mi0d[c]; ia.j0[c] = d.mj0d[c];
             ia.Ua[c] = t.Ua[c]; ia.Fc[c] = t.Fc[c]; ia.lQ[c] = A.lQ[c]; ia.lUa[c] = A.lUa[c];
         }
         ia.w = drag_w;
         ia.grad = A.grad;
         ia.d3 = 0;
-        k_ibm_adj<double><<<dim3((d.nm + 127) / 128, 1, 2), 128, 0, s>>>(ia, g); count_launch();
-        F8_CUDA_RET(fold(fold_set<double>({{A.lUa[0], BC_U}, {A.lUa[1], BC_V}}), g, s));
+        k_ibm_adj<double><<<dim3(1, 2), ibm_adj_block(d.nm), 0, s>>>(ia, g); count_launch();
     }
     // 2. momentum right-hand side (the adjoint of U^n starts here; P^n keeps
     // the identity part from P^{n+1})

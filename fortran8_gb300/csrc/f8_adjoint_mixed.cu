@@ -23,7 +23,7 @@ namespace f8 {
 
 cudaError_t adjoint_fold_state_f(AdjStateF &A, const Dev &d, cudaStream_t s) {
     const Geo &g = d.g;
-    return fold(fold_with_c(fold_set<float>({{A.lU, BC_U}, {A.lV, BC_V}, {A.lW, BC_W}, {A.lP, BC_P}}), A.lC, d.cs, 6), g, s);
+    return fold_walls(fold_with_c(fold_set<float>({{A.lU, BC_U}, {A.lV, BC_V}, {A.lW, BC_W}, {A.lP, BC_P}}), A.lC, d.cs, 6), g, s);
 }
 
 cudaError_t take_interior_f(const float *src, float *dst, const Geo &g, int n, cudaStream_t s) {
@@ -39,25 +39,19 @@ cudaError_t poisson_solve_f(Dev &d, const float *src, float *dst, float *lo, int
 }
 
 // k_div_adj with the pressure adjoint q as a double-float pair (qh, ql): the
-// adjoint projection lUp = lU + (q - q(+e))/(d dt) cancels the gradient part of
+// adjoint projection lU + (q - q(+e))/(d dt) cancels the gradient part of
 // lU, so the difference and its scaling are formed in df64 and only the
 // result is rounded to FP32
 __global__ void k_div_adj_df(const float *__restrict__ lU, const float *__restrict__ lV, const float *__restrict__ lW,
-                             const float *__restrict__ qh, const float *__restrict__ ql, float *__restrict__ lUp,
-                             float *__restrict__ lVp, float *__restrict__ lWp, Geo g, df cx, df cy, df cz) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int cs = g.sx * g.sy * g.sz;
-    if (t >= cs) return;
-    const int i = t % g.sx, j = (t / g.sx) % g.sy, k = t / (g.sx * g.sy);
-    auto q = [&](int ii, int jj, int kk) {
-        if (!adj_inner(g, ii, jj, kk)) return df{0.0f, 0.0f};
-        const int h = hix(g, ii, jj, kk);
-        return df{qh[h], ql[h]};
-    };
-    const df q0 = q(i, j, k);
-    lUp[t] = df_to_f(df_add_f(df_mul(df_sub(q0, q(i + 1, j, k)), cx), lin(lU, g, i, j, k)));
-    lVp[t] = df_to_f(df_add_f(df_mul(df_sub(q0, q(i, j + 1, k)), cy), lin(lV, g, i, j, k)));
-    lWp[t] = df_to_f(df_add_f(df_mul(df_sub(q0, q(i, j, k + 1)), cz), lin(lW, g, i, j, k)));
+                             const float *__restrict__ qh, const float *__restrict__ ql, DivAdjOut<float> o, Geo g, df cx,
+                             df cy, df cz) {
+    div_adj_cell<float>(o, g, [&](int h, int xp, int yp, int zp, float &x, float &y, float &z) {
+        auto q = [&](int p) { return df{qh[p], ql[p]}; };
+        const df q0 = q(h);
+        x = df_to_f(df_add_f(df_mul(df_sub(q0, q(xp)), cx), lU[h]));
+        y = df_to_f(df_add_f(df_mul(df_sub(q0, q(yp)), cy), lV[h]));
+        z = df_to_f(df_add_f(df_mul(df_sub(q0, q(zp)), cz), lW[h]));
+    });
 }
 
 }  // namespace
@@ -69,50 +63,40 @@ cudaError_t step_mixed_adjoint(Dev &d, AdjStateF &A, const MixTape &t, const dou
     const size_t hb = (size_t)cs * sizeof(float);
     const double dt = d.ph.dt, re = d.ph.re, beta = d.ph.beta, wi = d.ph.wi;
     const double kap = dt * beta / re / 2.0;
-    const unsigned nb = (unsigned)((cs + 255) / 256);
     dim3 blk(32, 8);
     const AdjCoef<float> kc = adj_coef<float>(g);
     // 6. projection / pressure update
-    k_march_adj<float><<<nb, 256, 0, s>>>(A.lU, A.lV, A.lW, A.lP, A.lPhi, t.Phi, g, (float)kap, (float)(dt / (2.0 * re)),
-                                          kc, A.grad); count_launch();
-    F8_CUDA_RET(fold(fold_set<float>({{A.lPhi, BC_P}}), g, s));
+    k_march_adj<float><<<adj_cells(g, blk), blk, 0, s>>>(A.lU, A.lV, A.lW, A.lP, A.pack, t.Phi, g, (float)kap,
+                                                         (float)(dt / (2.0 * re)), kc, A.grad); count_launch();
     // 5. Poisson, refined as the forward's pressure solve: q0 = L^-1 r in FP32,
     // the defect r - L_h q0 in df64, q = q0 + L^-1 (defect) as a df64 pair
-    k_pack<float><<<adj_cells(g, blk), blk, 0, s>>>(A.lPhi, A.pack, g); count_launch();
     F8_CUDA_RET(poisson_solve_f(d, A.pack, A.lQ[0], nullptr, 0, s));
     F8_CUDA_RET(mixed_defect(d, A.lQ[0], A.pack, A.zero, A.rdef, s));
     F8_CUDA_RET(poisson_solve_f(d, A.rdef, A.lQ[0], A.qlo, 2, s));
-    k_div_adj_df<<<nb, 256, 0, s>>>(A.lU, A.lV, A.lW, A.lQ[0], A.qlo, A.lUp[0], A.lUp[1], A.lUp[2], g,
-                                    df_from_d(1.0 / (g.dx * dt)), df_from_d(1.0 / (g.dy * dt)),
-                                    df_from_d(1.0 / (g.dz * dt))); count_launch();
-    F8_CUDA_RET(fold(fold_set<float>({{A.lUp[0], BC_U}, {A.lUp[1], BC_V}, {A.lUp[2], BC_W}}), g, s));
+    DivAdjOut<float> dout{};
+    for (int c = 0; c < 3; ++c) { dout.pk[c] = A.pack + (size_t)c * d.ni; dout.lUa[c] = A.lUa[c]; }
+    k_div_adj_df<<<adj_cells(g, blk), blk, 0, s>>>(A.lU, A.lV, A.lW, A.lQ[0], A.qlo, dout, g, df_from_d(1.0 / (g.dx * dt)),
+                                                   df_from_d(1.0 / (g.dy * dt)), df_from_d(1.0 / (g.dz * dt)));
+    count_launch();
     // 4. Helmholtz: the three solves as the forward's parallel branches
     {
-        float *pk[3];
-        for (int c = 0; c < 3; ++c) pk[c] = A.pack + (size_t)c * d.ni;
-        k_pack3<float><<<adj_cells(g, blk), blk, 0, s>>>(A.lUp[0], A.lUp[1], A.lUp[2], pk[0], pk[1], pk[2], g);
-        count_launch();
-        const float *src[3] = {pk[0], pk[1], pk[2]};
+        const float *src[3] = {dout.pk[0], dout.pk[1], dout.pk[2]};
         F8_CUDA_RET(mixed_helmholtz(d, 3, src, A.lQ, s));
     }
     // 3. IBM
-    for (int c = 0; c < 3; ++c) F8_CUDA_RET(cudaMemsetAsync(A.lUa[c], 0, hb, s));
     if (d.nm > 0) {
         IbmAdjArgs<float> ia{};
         ia.mx = d.mx; ia.my = d.my; ia.mcyl = d.mcyl; ia.nm = d.nm; ia.ncyl = d.ncyl;
-        ia.dvol = (g.dx * g.dy) * g.dz; ia.dxn = g.dx * g.dx * g.dx; ia.mvol = d.mvol; ia.cylvol = d.cylvol;
+        ia.idx = 1.0 / g.dx; ia.idy = 1.0 / g.dy; ia.mvol = d.mvol;
+        ia.idvol = 1.0 / ((g.dx * g.dy) * g.dz); ia.dvn = (g.dx * g.dx * g.dx) / ((g.dx * g.dy) * g.dz); ia.cylvol = d.cylvol;
         for (int c = 0; c < 3; ++c) {
+            ia.i0[c] = d.mi0[c]; ia.j0[c] = d.mj0[c];
             ia.Ua[c] = t.Ua[c]; ia.Fc[c] = t.Fc[c]; ia.lQ[c] = A.lQ[c]; ia.lUa[c] = A.lUa[c];
         }
         ia.w = drag_w;
         ia.grad = A.grad;
         ia.d3 = 1;
-        k_ibm_adj<float><<<dim3((d.nm + 127) / 128, g.nz, 3), 128, 0, s>>>(ia, g); count_launch();
-        // the markers' stencils reach the ghost planes in z; where they reach
-        // no ghost column or row (nor row NY, which the V wall rule zeroes)
-        // the y and x passes have nothing to do
-        const FoldSet<float> fa = fold_set<float>({{A.lUa[0], BC_U}, {A.lUa[1], BC_V}, {A.lUa[2], BC_W}});
-        F8_CUDA_RET(d.ibm_edge ? fold(fa, g, s) : fold_z_only(fa, g, s));
+        k_ibm_adj<float><<<dim3(g.nz, 3), ibm_adj_block(d.nm), 0, s>>>(ia, g); count_launch();
     }
     // 2. momentum right-hand side: per-cell sources, then the gather of the
     // velocity, pressure and (with the polymer) C0 / C adjoints
@@ -136,28 +120,22 @@ cudaError_t step_mixed_adjoint(Dev &d, AdjStateF &A, const MixTape &t, const dou
         mg.lp2 = (float)(d.ph.lp2); mg.inv_1mb = (float)(1.0 / (1.0 - beta)); mg.inv_wi = (float)(1.0 / wi);
         mg.grad = A.grad;
         mg.kc = kc;
-        k_momadj_gather<float><<<nb, 256, 0, s>>>(mg, g); count_launch();
+        k_momadj_gather<float><<<adj_rows(g, blk), blk, 0, s>>>(mg, g); count_launch();
     }
     // 1. polymer: per-cell implicit-function adjoint and Cstar weights, then
     // the gather of the adjoint of C^n and of the velocity
     if (polymer) {
-        // with walls the stress read the updated ghost rows and their x/z
-        // copies; the state's C (wall-extrapolated) adjoint is interior already
-        if (g.walls) F8_CUDA_RET(fold_xz(fold_c(A.lC, cs), g, s));
-        else F8_CUDA_RET(fold(fold_c(A.lC, cs), g, s));
         PolyAdjArgs<float> pa{};
         pa.C = t.C; pa.Cn = t.Cn; pa.codes = t.codes; pa.codes_g = t.codes_g; pa.U = t.U; pa.V = t.V; pa.W = t.W;
         pa.lX = A.lC;
         pa.cs = cs; pa.dt = (float)(dt); pa.wi = (float)(wi); pa.lp2 = (float)(d.ph.lp2); pa.grad = A.grad;
         pa.kc = kc; pa.dtwi = (float)(dt / wi); pa.dtwi2 = (float)(dt / (wi * wi));
-        dim3 pb(32, 4);
-        const dim3 pg((g.nx + pb.x - 1) / pb.x, (prows(g) + pb.y - 1) / pb.y, g.nz);
-        k_polyadj_mu<float><<<pg, pb, 0, s>>>(pa, A.work, g); count_launch();
-        const dim3 pb2(32, 8), pg2((g.nx + pb2.x - 1) / pb2.x, (prows(g) + pb2.y - 1) / pb2.y, g.nz);
-        k_polyadj_cstar<float><<<pg2, pb2, 0, s>>>(pa, A.work, g); count_launch();
+        const dim3 pb(32, 4);
+        k_polyadj_mu<float><<<adj_rows(g, pb), pb, 0, s>>>(pa, A.work, g); count_launch();
+        k_polyadj_cstar<float><<<adj_rows(g, blk), blk, 0, s>>>(pa, A.work, g); count_launch();
         PolyGatherArgs<float> pga{};
         pga.src = A.work; pga.lC = A.lC2; pga.lU = A.lU; pga.lV = A.lV; pga.lW = A.lW; pga.cs = cs;
-        k_polyadj_gather<float><<<nb, 256, 0, s>>>(pga, g); count_launch();
+        k_polyadj_gather<float><<<adj_rows(g, blk), blk, 0, s>>>(pga, g); count_launch();
         std::swap(A.lC, A.lC2);
     } else {
         F8_CUDA_RET(cudaMemsetAsync(A.lC, 0, 6 * hb, s));

@@ -613,7 +613,6 @@ int setup(f8_ctx *c) {
                         for (int ii = i0; ii <= i0 + 2; ++ii) {
                             if (ii < 0 || ii >= g.sx || jj < 0 || jj >= g.sy) return F8_ERR_ARG;  // marker too close to the edge
                             lists[ii + g.sx * jj].push_back(m);
-                            if (ii == 0 || ii == g.sx - 1 || jj == 0 || jj >= g.ny) d.ibm_edge = 1;
                         }
                 }
             for (int q = 0; q < ncol; ++q) off[q + 1] = off[q] + (int)lists[q].size();
@@ -1129,13 +1128,12 @@ int grad_alloc(f8_ctx *c, int K, int nck, int nsteps) {
     const size_t cs = d.cs, ni = d.ni, ncyl = c->cyl.size(), nfc = (size_t)d.nm * d.g.nz;
     if (!G.A.grad) {
         AdjState &A = G.A;
-        for (double **p : {&A.lU, &A.lV, &A.lW, &A.lP, &A.lPhi}) API_CUDA(c, G.get(0, p, cs));
+        for (double **p : {&A.lU, &A.lV, &A.lW, &A.lP}) API_CUDA(c, G.get(0, p, cs));
         for (double **p : {&A.lC, &A.lC2}) API_CUDA(c, G.get(0, p, 6 * cs));
         for (int q = 0; q < 3; ++q) {
             API_CUDA(c, G.get(0, &A.lA0[q], ni));
             API_CUDA(c, G.get(0, &A.lT0[q], ni));
             API_CUDA(c, G.get(0, &A.lUa[q], cs));
-            API_CUDA(c, G.get(0, &A.lUp[q], cs));
             API_CUDA(c, G.get(0, &A.lQ[q], cs));
         }
         API_CUDA(c, G.get(0, &A.pack, 3 * ni));   // one interior array per Helmholtz solve
@@ -1248,13 +1246,12 @@ int grad_alloc_mixed(f8_ctx *c, int K, int nck, int nsteps) {
     const size_t cs = d.cs, ni = d.ni, ncyl = c->cyl.size(), nfc = (size_t)d.nm * d.g.nz;
     if (!G.AF.grad) {
         AdjStateF &A = G.AF;
-        for (float **p : {&A.lU, &A.lV, &A.lW, &A.lP, &A.lPhi}) API_CUDA(c, G.get(0, p, cs));
+        for (float **p : {&A.lU, &A.lV, &A.lW, &A.lP}) API_CUDA(c, G.get(0, p, cs));
         for (float **p : {&A.lC, &A.lC2}) API_CUDA(c, G.get(0, p, 6 * cs));
         for (int q = 0; q < 3; ++q) {
             API_CUDA(c, G.get(0, &A.lA0[q], ni));
             API_CUDA(c, G.get(0, &A.lT0[q], ni));
             API_CUDA(c, G.get(0, &A.lUa[q], cs));
-            API_CUDA(c, G.get(0, &A.lUp[q], cs));
             API_CUDA(c, G.get(0, &A.lQ[q], cs));
         }
         API_CUDA(c, G.get(0, &A.pack, 3 * ni));   // one interior array per Helmholtz solve
@@ -1492,6 +1489,8 @@ int grad_mixed(f8_ctx *c, int nsteps, int checkpoint_every, const double *drag_w
         }
         API_CUDA(c, cudaStreamSynchronize(c->s));
     }
+    // the gathers of the reverse sweep write no ghost column or plane of C
+    API_CUDA(c, cudaMemsetAsync(A.lC2, 0, 6 * cs * sizeof(float), c->s));
     // reverse sweep over the segments
     const bool polymer = c->phys.beta != 1.0;
     for (int seg = nseg - 1; seg >= 0; --seg) {
@@ -1682,6 +1681,8 @@ static int grad_impl(f8_ctx *c, int nsteps, int checkpoint_every, const double *
         if (!A.lsor) API_CUDA(c, G.get(0, &A.lsor, cs));
         API_CUDA(c, cudaMemsetAsync(A.lsor, 0, cs * sizeof(double), c->s));
     }
+    // the gathers of the reverse sweep write no ghost column or plane of C
+    API_CUDA(c, cudaMemsetAsync(A.lC2, 0, 6 * cs * sizeof(double), c->s));
     // reverse sweep over the segments
     const bool polymer = c->phys.beta != 1.0;
     for (int seg = nseg - 1; seg >= 0; --seg) {

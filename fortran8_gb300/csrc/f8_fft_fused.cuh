@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(XLine<N>::THREADS) k_xinv_w(const float2 *__re
                                                              int nz, int lj, int joff2, int sx, int sy,
                                                              const float2 *__restrict__ twx) {
     using X = XLine<N>;
-    constexpr int E = X::E, G = X::G, NH = N / 2, STEP = X::THREADS / XW_RB, BATCH = 8;
+    constexpr int E = X::E, G = X::G, NH = N / 2, STEP = X::THREADS / XW_RB;
     extern __shared__ unsigned char smem_raw[];
     float2 *tws = reinterpret_cast<float2 *>(smem_raw);
     float2 *zb = tws + N;
@@ -677,14 +677,12 @@ __global__ void __launch_bounds__(XLine<N>::THREADS) k_xinv_w(const float2 *__re
         };
         const bool first = threadIdx.x < XW_RB;      // kx = NH, by the first lanes of the first warp
         const float2 vl = first && r < nrows ? Sr[(size_t)NH * skx] : make_float2(0.f, 0.f);
-        for (int k0 = threadIdx.x / XW_RB; k0 < NH; k0 += BATCH * STEP) {   // NH is a multiple of BATCH STEP
-            float2 v[BATCH];
+        const int k0 = threadIdx.x / XW_RB;          // NH = E STEP: all loads of the tile in flight at once
+        float2 v[E];
 #pragma unroll
-            for (int u = 0; u < BATCH; ++u)
-                v[u] = r < nrows ? Sr[(size_t)(k0 + u * STEP) * skx] : make_float2(0.f, 0.f);
+        for (int u = 0; u < E; ++u) v[u] = r < nrows ? Sr[(size_t)(k0 + u * STEP) * skx] : make_float2(0.f, 0.f);
 #pragma unroll
-            for (int u = 0; u < BATCH; ++u) put(k0 + u * STEP, v[u], true);
-        }
+        for (int u = 0; u < E; ++u) put(k0 + u * STEP, v[u], true);
         if (threadIdx.x < 32) put(NH, vl, first);
     }
     __syncthreads();

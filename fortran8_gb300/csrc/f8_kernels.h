@@ -43,7 +43,6 @@ struct Dev {
     double *mvol;                          // per marker: the volume its force is spread with
     double *cylvol;                        // per cylinder: the marker volume of its drag
     int ibm_repeats;                       // direct-forcing iterations per step (NS)
-    int ibm_edge;                          // some marker stencil reaches a ghost column, a ghost row or row NY
     float *Qpre[3];                        // mixed, NS > 1: the right-hand sides before spreading
     float *Fcf[3];                         // mixed: FP32 copies of the marker forces (the spreading's)
     // mixed-precision state and work (F8_MIXED): the state as df64 pairs
@@ -199,10 +198,10 @@ cudaError_t device_diagnostics(Dev &d, bool mixed, double *part, double *out, Di
 // full halo arrays whose halo cells are zero between stages.
 constexpr int ADJ_WORK_FIELDS = 34;   // the largest per-cell source set of the gather kernels
 struct AdjState {
-    double *lU, *lV, *lW, *lP, *lPhi;      // state U, V, W, P and the pressure correction
+    double *lU, *lV, *lW, *lP;             // state U, V, W, P
     double *lC, *lC2;                      // C and a second C buffer (6 fields each)
     double *lA0[3], *lT0[3];               // AB2 histories (interior)
-    double *lUa[3], *lUp[3], *lQ[3];       // explicit velocity, Helmholtz solution, right-hand side
+    double *lUa[3], *lQ[3];                // explicit velocity, Helmholtz right-hand side
     double *pack;                          // packed interior fields (3 * ni)
     double *work;                          // per-cell sources of the gather kernels (ADJ_WORK_FIELDS halo fields)
     double *grad;                          // dJ/d(Wi, beta, L^2, (xc, yc) per cylinder), accumulated
@@ -233,10 +232,10 @@ cudaError_t take_interior(const double *src, double *dst, const Geo &g, int n, c
 // Discrete adjoint of the FP32-mixed 3D step (f8_adjoint_mixed.cu): the same
 // stage transposes as the FP64 adjoint in FP32, reading a MixTape.
 struct AdjStateF {
-    float *lU, *lV, *lW, *lP, *lPhi;
+    float *lU, *lV, *lW, *lP;
     float *lC, *lC2;
     float *lA0[3], *lT0[3];
-    float *lUa[3], *lUp[3], *lQ[3];
+    float *lUa[3], *lQ[3];
     float *pack;             // interior arrays of the solves' right-hand sides (3 * ni)
     float *qlo;              // low part of the refined pressure adjoint (halo, with lQ[0] its high part)
     float *zero, *rdef;      // interior: zeros (the right-hand side's low part), the defect

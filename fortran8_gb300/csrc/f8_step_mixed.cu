@@ -1256,7 +1256,7 @@ struct IbmArgsF {
 // the plane's sum to the up to three planes n that use it, in the order k =
 // n - 1, n, n + 1.  Bound by the L1 wavefronts of the gathered loads (the
 // markers of a warp lie on a circle): a thread per plane of one n read each
-// point three times, 28.5 us for 4 cylinders in 256x128x128, XXX us with NB = 4.
+// point three times, 28.5 us for 548 markers in 256x128x128, 23.0 us with NB = 2.
 // In 2D the one plane has weight 1.
 template <int NB, bool D3>
 __global__ void __launch_bounds__(128) k_ibm_interp_f(IbmArgsF a, Geo g) {
@@ -2285,10 +2285,9 @@ __global__ void k_tape_ua(const float *__restrict__ Uh, const float *__restrict_
                           const float *__restrict__ Qu, const float *__restrict__ Qv, const float *__restrict__ Qw,
                           float *__restrict__ ou, float *__restrict__ ov, float *__restrict__ ow,
                           float *__restrict__ tu, float *__restrict__ tv, float *__restrict__ tw, Geo g, df uw2) {
-    const int cs = g.sx * g.sy * g.sz;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= cs) return;
-    const int i = t % g.sx, j = (t / g.sx) % g.sy, k = t / (g.sx * g.sy);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+    if (i >= g.sx) return;
+    const int t = hix(g, i, j, k);
     const df a = ua_at(g, Uh, Ul, Qu, 0, i, j, k, uw2);
     const df b = ua_at(g, Vh, Vl, Qv, 1, i, j, k, uw2);
     const df c = ua_at(g, Wh, Wl, Qw, 2, i, j, k, uw2);
@@ -2310,28 +2309,27 @@ struct TapeUp {
 };
 // the three Helmholtz solutions U^n + dU (blockIdx.y: component)
 __global__ void k_tape_up(TapeUp a, Geo g) {
-    const int cs = g.sx * g.sy * g.sz;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= cs) return;
+    const int j = blockIdx.x * 8 + threadIdx.y, k = blockIdx.y, c = blockIdx.z;
+    if (j >= g.sy) return;
     // the component's pointers by selects (an index into the parameter
     // arrays would copy them to local memory)
-    const int c = blockIdx.y;
     const float *U = c == 0 ? a.U[0] : (c == 1 ? a.U[1] : a.U[2]);
     const float *D = c == 0 ? a.D[0] : (c == 1 ? a.D[1] : a.D[2]);
     float *out = c == 0 ? a.out[0] : (c == 1 ? a.out[1] : a.out[2]);
-    const int i = t % g.sx, j = (t / g.sx) % g.sy, k = t / (g.sx * g.sy);
     const int jj = g.walls ? j : wrapy(g, j);
-    out[t] = U[t] + D[hix(g, wrapx(g, i), jj, wrapz(g, k))];
+    const int h = hix(g, 0, j, k), hd = hix(g, 0, jj, wrapz(g, k));
+#pragma unroll 4
+    for (int i = threadIdx.x; i < g.sx; i += 32) out[h + i] = U[h + i] + D[hd + wrapx(g, i)];
 }
 
 // Phi (hi part) with the periodic wrap and the Neumann copy at the walls
 __global__ void k_tape_phi(const float *__restrict__ Phi, float *__restrict__ out, Geo g) {
-    const int cs = g.sx * g.sy * g.sz;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= cs) return;
-    const int i = t % g.sx, j = (t / g.sx) % g.sy, k = t / (g.sx * g.sy);
+    const int j = blockIdx.x * 8 + threadIdx.y, k = blockIdx.y;
+    if (j >= g.sy) return;
     const int jj = g.walls ? max(1, min(g.ny, j)) : wrapy(g, j);
-    out[t] = Phi[hix(g, wrapx(g, i), jj, wrapz(g, k))];
+    const int h = hix(g, 0, j, k), hp = hix(g, 0, jj, wrapz(g, k));
+#pragma unroll 4
+    for (int i = threadIdx.x; i < g.sx; i += 32) out[h + i] = Phi[hp + wrapx(g, i)];
 }
 
 cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_iters, cudaStream_t s) {
@@ -2344,7 +2342,7 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
     const DfF U{d.Uf, d.Ul}, V{d.Vf, d.Vl}, W{d.Wf, d.Wl}, P{d.Pf, d.Pl}, Phi{d.Phif, d.Phil};
     const MixTape *tp = o.tape;
     const size_t hbf = (size_t)d.cs * sizeof(float);
-    const unsigned tnb = (unsigned)((d.cs + 255) / 256);
+    const dim3 tthr(32, 8), trow((g.sy + 7) / 8, g.sz);   // tape kernels: eight rows of the halo box per block
     if (tp && o.polymer) F8_CUDA_RET(cudaMemcpyAsync(tp->C, d.Cf, 6 * hbf, cudaMemcpyDeviceToDevice, s));
     mark(0);
     // wall channel: the ghost rows' codes and update run on a side stream
@@ -2448,7 +2446,7 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
         else { k_extrap_ghost_f<3><<<(ng + 255) / 256, 256, 0, sg>>>(d.Cf, d.fpetf, g, d.cs, d.ph.lp2); count_launch(); }
     }
     if (tp) {
-        k_tape_ua<<<tnb, 256, 0, s>>>(d.Uf, d.Ul, d.Vf, d.Vl, d.Wf, d.Wl, d.Qf[0], d.Qf[1], d.Qf[2], tp->Ua[0],
+        k_tape_ua<<<dim3((g.sx + 127) / 128, g.sy, g.sz), std::min(128, (g.sx + 31) / 32 * 32), 0, s>>>(d.Uf, d.Ul, d.Vf, d.Vl, d.Wf, d.Wl, d.Qf[0], d.Qf[1], d.Qf[2], tp->Ua[0],
                                       tp->Ua[1], tp->Ua[2], tp->U, tp->V, tp->W, g, df_from_d(2.0 * g.uwall));
         count_launch();
     }
@@ -2530,7 +2528,7 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
         if (o.ibm && r == repeats - 1 && drag_out_dev && d.aux[1]) F8_CUDA_RET(cudaStreamWaitEvent(s, d.ev_g[5], 0));
         if (tp) {
             const TapeUp a{{d.Uf, d.Vf, d.Wf}, {d.dUf[0], d.dUf[1], d.dUf[2]}, {tp->Up[0], tp->Up[1], tp->Up[2]}};
-            k_tape_up<<<dim3(tnb, 3), 256, 0, s>>>(a, g); count_launch();
+            k_tape_up<<<dim3(trow.x, trow.y, 3), tthr, 0, s>>>(a, g); count_launch();
         }
     }
     mark(5);
@@ -2561,7 +2559,7 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
         else e = solve_walls_f(d, d.Rdf, out, SYS_P, s);
         if (e) return e;
     }
-    if (tp) { k_tape_phi<<<tnb, 256, 0, s>>>(d.Phif, tp->Phi, g); count_launch(); }
+    if (tp) { k_tape_phi<<<trow, tthr, 0, s>>>(d.Phif, tp->Phi, g); count_launch(); }
     mark(6);
     kmark(F8_KERNEL_MARCH, 0);
     if (d.march_runs > 0) {

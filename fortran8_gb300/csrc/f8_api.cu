@@ -238,6 +238,12 @@ struct f8_ctx {
             d.aux[b] = nullptr;
             d.ev_join[b] = nullptr;
         }
+        if (d.code_side) cudaStreamDestroy(d.code_side);
+        d.code_side = nullptr;
+        for (cudaEvent_t &ev : d.ev_code) {
+            if (ev) cudaEventDestroy(ev);
+            ev = nullptr;
+        }
         if (d.ev_fork) cudaEventDestroy(d.ev_fork);
         d.ev_fork = nullptr;
         for (cudaEvent_t &ev : d.ev_g) {
@@ -415,6 +421,16 @@ int setup(f8_ctx *c) {
     API_CUDA(c, c->alloc(&d.scal, 64));
     API_CUDA(c, c->alloc(&d.flag, 4));
     API_CUDA(c, c->alloc(&d.code_count, 4));
+    if (!mixed && g.dim == 3 && c->phys.beta != 1.0 && c->phys.eigen_test == 0) {
+        API_CUDA(c, c->alloc(&d.code_queue, 3 * (size_t)g.nx * (g.ny + 2) * g.nz));
+        // the SOR solve fills the chip with one cooperative grid: nothing beside it
+        if (c->poisson != F8_POISSON_SOR) {
+            int least = 0, greatest = 0;
+            API_CUDA(c, cudaDeviceGetStreamPriorityRange(&least, &greatest));
+            API_CUDA(c, cudaStreamCreateWithPriority(&d.code_side, cudaStreamNonBlocking, least));
+            for (cudaEvent_t &ev : d.ev_code) API_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        }
+    }
     c->res_bytes = sizeof(StepCounters) + c->cyl.size() * 3 * sizeof(double);
     static_assert(sizeof(StepCounters) % sizeof(double) == 0, "drag slot alignment");
     API_CUDA(c, c->alloc(&c->res_dev, c->res_bytes));
@@ -953,6 +969,11 @@ int f8_step(f8_ctx *c, int nsteps, double *drag) {
         o.ev = c->timing ? &c->evpool[per * s] : nullptr;
         o.kev = (c->timing && c->precision == F8_MIXED) ? &c->evpool[per * s + NSTAGE + 1] : nullptr;
         const bool mixed = c->precision == F8_MIXED;
+        // FP64: each step of this call but the last chooses the next one's
+        // face candidates beside its solves (not under stage timing)
+        const bool ahead = !mixed && o.polymer && d.code_side && !o.ev;
+        o.codes_ready = ahead && s > 0;
+        o.codes_next = ahead && s + 1 < nsteps;
         if (!o.polymer && s == 0) {
             // beta == 1: C and T vanish (fenep.f90:2479-2485)
             if (mixed) API_CUDA(c, cudaMemsetAsync(d.Cf, 0, (size_t)d.cs * d.ncomp * sizeof(float), c->s));

@@ -118,9 +118,8 @@ __global__ void __launch_bounds__(FILTER_THREADS) k_codes3_filter(const float2 *
 
 }  // namespace
 
-// C as double-float pairs goes to the C buffer of the next step (not yet
-// written there), the queues to the spectral scratch (one entry per cell and
-// direction at most: nx (ny+2) nz words each).
+// C as double-float pairs goes to the C buffer of the next update (not yet
+// written there), the queues hold one entry per cell and direction at most.
 cudaError_t codes3_filter(Dev &d, cudaStream_t s) {
     const Geo &g = d.g;
     const int n2 = d.cs / 2 * 6;   // cs is even (sx is)

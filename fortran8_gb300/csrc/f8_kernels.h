@@ -90,6 +90,9 @@ struct Dev {
     int *flag;                             // SOR: converged, iteration, barrier time-out, barrier arrivals
     int sor_cluster;                       // mixed SOR: CTAs of a cluster that the device can hold
     int *code_count;                       // FP64 3D: cells queued for the FP64 eigen test, per direction
+    unsigned *code_queue;                  // their queues: 3 x nx (ny + 2) nz words
+    cudaStream_t code_side;                // FP64 3D: side stream of the next step's face candidates (0: none)
+    cudaEvent_t ev_code[2];                // C of the step final, candidates chosen
     StepCounters *cnt;
 };
 
@@ -118,6 +121,8 @@ struct StepOpts {
     cudaEvent_t *kev;  // 2*NKERNEL events bracketing the single-launch kernels (f8_kernel), or null
     double *c_mid;     // FP64: receives C as the momentum stage read it (6 halo fields), or null
     const MixTape *tape;   // FP32-mixed: tape of this step, or null
+    bool codes_ready;  // FP64 3D: the previous step of the call chose this step's face candidates
+    bool codes_next;   // FP64 3D: choose the next step's beside the rest of this one (code_side)
 };
 constexpr int NSTAGE = 7;
 constexpr int NKERNEL = 6;   // enum f8_kernel
@@ -129,8 +134,7 @@ constexpr int NKERNEL = 6;   // enum f8_kernel
 // i - 1 + nx * (row + rows * (k - 1)), rows of the polymer update)
 cudaError_t codes3_filter(Dev &d, cudaStream_t s);
 inline unsigned *codes3_queue(const Dev &d, int dir) {
-    const size_t cap = (size_t)d.g.nx * (d.g.ny + 2) * d.g.nz;
-    return dir == 2 ? reinterpret_cast<unsigned *>(d.H2) : reinterpret_cast<unsigned *>(d.H) + (dir == 1 ? cap : 0);
+    return d.code_queue + (size_t)dir * d.g.nx * (d.g.ny + 2) * d.g.nz;
 }
 cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_iters, cudaStream_t s);
 cudaError_t bc_all_state_fp64(Dev &d, cudaStream_t s);

@@ -1620,6 +1620,18 @@ cudaError_t count_nonfinite(const double *a, int n, unsigned long long *out, cud
     return cudaGetLastError();
 }
 
+// the face candidates of d.C: the filter, then the FP64 test of its queue
+static cudaError_t choose_codes3(Dev &d, cudaStream_t s) {
+    const Geo &g = d.g;
+    F8_CUDA_RET(codes3_filter(d, s));
+    // at most two lanes for each (cell, direction); grid-stride beyond the chip
+    const long most = 2L * 3 * g.nx * prows(g) * g.nz;
+    const unsigned nb = (unsigned)std::min((most + 127) / 128, 16L * device_sm_count());
+    k_codes3_exact<<<nb, 128, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs, codes3_queue(d, 0), codes3_queue(d, 1),
+                                      codes3_queue(d, 2), d.code_count); count_launch();
+    return cudaGetLastError();
+}
+
 cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_iters, cudaStream_t s) {
     const Geo &g = d.g;
     const bool d3 = g.dim == 3;
@@ -1631,13 +1643,10 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
         dim3 blk(32, 4);
         // the rows of the polymer update (with walls the ghost rows too)
         dim3 grd((g.nx + blk.x - 1) / blk.x, (prows(g) + blk.y - 1) / blk.y, g.nz);
-        if (d3 && d.ph.eigen_test == 0) {
-            F8_CUDA_RET(codes3_filter(d, s));
-            // at most two lanes for each (cell, direction); grid-stride beyond the chip
-            const long most = 2L * 3 * g.nx * prows(g) * g.nz;
-            const unsigned nb = (unsigned)std::min((most + 127) / 128, 16L * device_sm_count());
-            k_codes3_exact<<<nb, 128, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs, codes3_queue(d, 0), codes3_queue(d, 1),
-                                              codes3_queue(d, 2), d.code_count); count_launch();
+        if (o.codes_ready) {
+            F8_CUDA_RET(cudaStreamWaitEvent(s, d.ev_code[1], 0));
+        } else if (d3 && d.ph.eigen_test == 0) {
+            F8_CUDA_RET(choose_codes3(d, s));
         } else if (d3) { k_polymer_codes3<<<grd, blk, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs, d.ph.eigen_test); count_launch(); }
         else { k_polymer_codes2<<<grd, blk, 0, s>>>(d.C, d.codes, d.codes_g, g, d.cs); count_launch(); }
         mark(1);
@@ -1672,6 +1681,23 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
         if (d3) { k_momentum<3><<<grd, blk, 0, s>>>(ma, g, grid_recip(g)); count_launch(); }
         else { k_momentum<2><<<grd, blk, 0, s>>>(ma, g, grid_recip(g)); count_launch(); }
         if ((e = cudaGetLastError())) return e;
+    }
+    // C is final but for the ghost rows that the momentum stage was the last to
+    // read: the next step's face candidates (FP32 but for their queue) beside
+    // the FP64 solves.  Six steps of a 64^3 box 12.82 ms with the candidates at the
+    // start of each, 12.49 beside; nine of 32x16x16 3.06 and 2.70.
+    auto extrapolate = [&](cudaStream_t q) {
+        // the wall extrapolation of the ghost rows (C_kabe at the end of the
+        // step, fenep_2d.f90:1374)
+        k_bc_c_pet<<<(unsigned)((halo_count(g) + 255) / 256), 256, 0, q>>>(d.C, d.fpet, g, d.ncomp, d.cs, d.ph.lp2);
+        count_launch();
+    };
+    if (o.codes_next) {
+        F8_CUDA_RET(cudaEventRecord(d.ev_code[0], s));
+        F8_CUDA_RET(cudaStreamWaitEvent(d.code_side, d.ev_code[0], 0));
+        if (g.walls) extrapolate(d.code_side);
+        F8_CUDA_RET(choose_codes3(d, d.code_side));
+        F8_CUDA_RET(cudaEventRecord(d.ev_code[1], d.code_side));
     }
     mark(3);
     // 3. IBM direct forcing and 4. Helmholtz (CN viscous) solves; with NS > 1
@@ -1744,12 +1770,7 @@ cudaError_t step_fp64(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor_
     if ((e = bc_state(d, s))) return e;
     if (o.c_mid) F8_CUDA_RET(cudaMemcpyAsync(o.c_mid, d.C, (size_t)d.ncomp * d.cs * sizeof(double),
                                              cudaMemcpyDeviceToDevice, s));
-    if (o.polymer && g.walls) {
-        // the wall extrapolation of the ghost rows (C_kabe at the end of the
-        // step, fenep_2d.f90:1374)
-        long n = halo_count(g);
-        k_bc_c_pet<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d.C, d.fpet, g, d.ncomp, d.cs, d.ph.lp2); count_launch();
-    }
+    if (o.polymer && g.walls && !o.codes_next) extrapolate(s);
     mark(7);
     return cudaGetLastError();
 }

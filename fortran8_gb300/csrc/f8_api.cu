@@ -970,8 +970,9 @@ int f8_step(f8_ctx *c, int nsteps, double *drag) {
         o.kev = (c->timing && c->precision == F8_MIXED) ? &c->evpool[per * s + NSTAGE + 1] : nullptr;
         const bool mixed = c->precision == F8_MIXED;
         // FP64: each step of this call but the last chooses the next one's
-        // face candidates beside its solves (not under stage timing)
-        const bool ahead = !mixed && o.polymer && d.code_side && !o.ev;
+        // face candidates beside its solves (not under stage timing, nor where
+        // the running statistics read the state between the steps)
+        const bool ahead = !mixed && o.polymer && d.code_side && !o.ev && !c->stats_mode;
         o.codes_ready = ahead && s > 0;
         o.codes_next = ahead && s + 1 < nsteps;
         if (!o.polymer && s == 0) {

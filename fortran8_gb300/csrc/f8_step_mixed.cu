@@ -245,6 +245,36 @@ __global__ void k_bc_set(BcSet b, Geo g) {
     }
 }
 
+// The conversions of the state's load and store without the FP64 pipe, on which
+// a conversion or an addition of a warp takes 64 cycles: the same values from
+// the bits, in the normal range.  Others by the conversion itself, out of line:
+// inlined, the compiler computes it for every value and selects.
+__device__ __noinline__ double double_by_conversion(float f) { return (double)f; }
+__device__ __noinline__ df df_by_conversion(double x) { return df_from_d(x); }
+
+// (double)f
+__device__ __forceinline__ double double_of_bits(float f) {
+    const unsigned b = __float_as_uint(f), e = (b >> 23) & 0xffu;
+    if ((b << 1) != 0 && e - 1u >= 254u) return double_by_conversion(f);   // not zero: denormal, infinite or NaN
+    const unsigned h = (b << 1) == 0 ? b : (b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u);
+    return __hiloint2double((int)h, (int)(b << 29));
+}
+
+// df_from_d(x): the rest of a number with exponent e after its upper 24 bits is
+// an integer of up to 29 bits times 2^(e - 52)
+__device__ __forceinline__ df df_of_bits(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const unsigned h = (unsigned)(b >> 32), e = (h >> 20) & 0x7ffu;
+    if ((b << 1) == 0) return df{__uint_as_float(h), 0.0f};
+    if (e - 953u >= 196u) return df_by_conversion(x);        // exponents -70 .. 125
+    const unsigned top = (h << 3) | ((unsigned)b >> 29);
+    const int rem = (int)((unsigned)b & 0x1fffffffu);
+    const int up = rem > 0x10000000 || (rem == 0x10000000 && (top & 1u)) ? 1 : 0;
+    const int r = rem - (up << 29);
+    const float hi = __uint_as_float((h & 0x80000000u) | (((e - 896u) << 23) + (top & 0x7fffffu) + (unsigned)up));
+    return df{hi, (float)(h & 0x80000000u ? -r : r) * __uint_as_float((e - 948u) << 23)};
+}
+
 // FP64 <-> df64 pairs (load / store) of the five state fields in one launch, two
 // values a thread (n is even).  256x128x128: 5 x 33.9 us split and 5 x 26.4 us
 // joined with conversions on the FP64 pipe, 57 and 59 us now (6 TB/s).

@@ -549,8 +549,8 @@ struct WallTables {
 // x passes of XW_RB rows per block (NX = 32 .. 512).  Two real rows are one
 // complex line, held by G threads with E elements each: the spans of G and more
 // run in registers on the elements t + G s, the rest after one exchange through
-// shared memory on the groups of G consecutive elements (NX = 512: on 16
-// elements of a group of 32, with the last span between lanes).  The block then
+// shared memory on the groups of G consecutive elements (NX = 128 and 512: on half
+// of a group, with the last span between lanes).  The block then
 // unpacks the half spectra of its rows from (packs them into) the lines while
 // it writes (reads) the [kx][row] lines of 16 consecutive rows, the two rows of
 // a pair on neighbouring lanes.  Bound by instruction issue and shared memory:
@@ -560,11 +560,12 @@ struct WallTables {
 constexpr int XW_RB = 16;     // rows per block of the x passes (a constant: the tile indexing divides by it)
 
 template <int N> struct XLine {
-    static constexpr int E = N >= 128 ? 16 : 8, G = N / E, THREADS = XW_RB / 2 * G;
+    static constexpr int E = N >= 256 ? 16 : 8, G = N / E, THREADS = XW_RB / 2 * G;
+    static constexpr bool PAIRS = G == 2 * E;      // NX = 128, 512
     static constexpr int LG = N == 32 ? 5 : N == 64 ? 6 : N == 128 ? 7 : N == 256 ? 8 : 9;
     // element e of a line at e + PAD (e / G), lines PITCH apart (odd): strided
     // and consecutive elements, and one element of the lines, in distinct banks
-    static constexpr int PAD = N == 512 ? 2 : 1, PITCH = N + PAD * E + 1;
+    static constexpr int PAD = PAIRS ? 2 : 1, PITCH = N + PAD * E + 1;
     static constexpr size_t smem = (size_t)(N + XW_RB / 2 * PITCH) * sizeof(float2);
     static __device__ __forceinline__ int ix(int e) { return e + e / G * PAD; }
     static __device__ __forceinline__ int at(int k) { return ix((int)(__brev((unsigned)k) >> (32 - LG))); }   // X[k]
@@ -574,23 +575,23 @@ template <int N> struct XLine {
 template <int N, bool FWD>
 __device__ __forceinline__ void x_inner(float2 *z, const float2 *tws, int t) {
     using X = XLine<N>;
-    if constexpr (N == 512) {
-        float2 *x = z + X::ix(t / 2 * 32) + (t & 1);
-        float2 v[16];
+    if constexpr (X::PAIRS) {
+        float2 *x = z + X::ix(t / 2 * X::G) + (t & 1);
+        float2 v[X::E];
         const float sg = t & 1 ? -1.0f : 1.0f;
         auto last = [&] {                 // first: a + b, second: a - b
 #pragma unroll
-            for (int s = 0; s < 16; ++s) {
+            for (int s = 0; s < X::E; ++s) {
                 const float ox = __shfl_xor_sync(0xffffffffu, v[s].x, 1), oy = __shfl_xor_sync(0xffffffffu, v[s].y, 1);
                 v[s] = __ffma2_rn(make_float2(sg, sg), v[s], make_float2(ox, oy));
             }
         };
 #pragma unroll
-        for (int s = 0; s < 16; ++s) v[s] = x[2 * s];
-        if (FWD) { reg_dif<16, 2>(v, tws, t & 1); last(); }
-        else { last(); reg_dit<16, 2>(v, tws, t & 1); }
+        for (int s = 0; s < X::E; ++s) v[s] = x[2 * s];
+        if (FWD) { reg_dif<X::E, 2>(v, tws, t & 1); last(); }
+        else { last(); reg_dit<X::E, 2>(v, tws, t & 1); }
 #pragma unroll
-        for (int s = 0; s < 16; ++s) x[2 * s] = v[s];
+        for (int s = 0; s < X::E; ++s) x[2 * s] = v[s];
     } else {
 #pragma unroll
         for (int u = 0; u < X::E / X::G; ++u) {

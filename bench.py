@@ -68,7 +68,7 @@ MIXED_STAGE_KERNELS = {
     "eigen": ["k_codes3_f", "k_codes_ghost3_f"],
     "newton": ["k_update3_f", "k_newton_fix_f", "k_update_ghost3_f", "k_bc_c_pet_xz_f"],
     "momentum": ["k_momentum3_f"],
-    "ibm": ["k_ibm_interp_f", "k_ibm_spread_f", "k_drag_part", "k_drag_final"],
+    "ibm": ["k_ibm_interp_f", "k_ibm_spread_f", "k_drag"],
     "helmholtz": ["3 x (k_xfwd_w, k_plane_walls_c, k_xinv_w)"],
     "poisson": ["k_poisson_rhs_df", "2 x (k_xfwd_w, k_plane_walls_c, k_xinv_w)", "k_defect_df"],
     "project": ["k_march_df", "k_bc_set"],
@@ -553,7 +553,7 @@ MIXED_STAGE_LAUNCHES = {
     "eigen": {"k_codes3_f": 1, "k_codes_ghost3_f": 1},
     "newton": {"k_update3_f": 1, "k_newton_fix_f": 1, "k_update_ghost3_f": 1, "k_bc_c_pet_xz_f": 1},
     "momentum": {"k_momentum3_f": 1, "k_extrap_ghost_f": 1},
-    "ibm": {"k_ibm_interp_f": 1, "k_ibm_spread_f": 1, "k_drag_part": 1, "k_drag_final": 1},
+    "ibm": {"k_ibm_interp_f": 1, "k_ibm_spread_f": 1, "k_drag": 1},
     "helmholtz": {"k_xfwd_w": 3, "k_plane_walls_c": 3, "k_xinv_w": 3},
     "poisson": {"k_poisson_rhs_df": 1, "k_xfwd_w": 2, "k_plane_walls_c": 2, "k_xinv_w": 2, "k_defect_df": 1},
     "project": {"k_march_df": 1, "k_bc_set": 1},

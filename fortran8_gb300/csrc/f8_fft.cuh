@@ -504,9 +504,9 @@ __global__ void __launch_bounds__(256) k_fft_lines(T *__restrict__ H, size_t hst
 // mode 0 (INV: the sign) and 1 of k_fft_lines on register lines; neighbouring
 // threads take neighbouring columns
 template <int LG, bool SOLVE, bool INV, typename T>
-__global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256) k_fft_lines_r(T *__restrict__ H, size_t hstride, int lstride, int ncols,
-                                                     int sstride, int tx, const T *__restrict__ twr,
-                                                     const T *__restrict__ twi, DivideSpec dv) {
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
+k_fft_lines_r(T *__restrict__ H, size_t hstride, int lstride, int ncols, int sstride, int tx, const T *__restrict__ twr,
+              const T *__restrict__ twi, DivideSpec dv) {
     using L = LineFft<LG>;
     extern __shared__ unsigned char smem_raw[];
     const int c = threadIdx.x & (tx - 1), t = threadIdx.x >> (31 - __clz(tx)), kx = blockIdx.x * tx + c, set = blockIdx.y;

@@ -37,7 +37,8 @@ constexpr int SOR_MAX_BLOCKS = 1024;    // partial sums per colour pair
 
 // sums of squared residuals: FP64 residuals in FP64; FP32 residuals (24 bits
 // each) as double-float, whose 48 bits are far below the residuals' own rounding
-// and keep the FP64 pipe out of the sweep
+// and keep the FP64 pipe out of the sweep.  A square has twice the exponent, so
+// FP32 residuals are scaled by a power of two first (sor_scale).
 template <typename T>
 struct SorSum;
 template <>
@@ -124,6 +125,21 @@ __device__ __forceinline__ SorSum<T> block_sum(SorSum<T> s, SorSum<T> *sh) {
     return s;
 }
 
+// The power of two that takes sqrt(er0) into [1, 2): FP32 residuals down to
+// 1e-19 of sqrt(er0) square without underflow, and one whose square overflows is
+// 1e19 above it, far from converged (the sum is not below any bound then).  The
+// scaling is exact, so the test is that of the plain squares wherever those are
+// in range.
+template <typename T>
+__device__ __forceinline__ T sor_scale(double er0) {
+    if constexpr (sizeof(T) == 8) {
+        return 1.0;
+    } else {
+        const int e = ((__double2hiint(er0) >> 20) & 0x7ff) - 1023;
+        return __int_as_float((127 - max(-126, min(126, e >> 1))) << 23);
+    }
+}
+
 // sqrt(sum / er0) < eps: squared away from the boundary
 __device__ __forceinline__ bool sor_done(double sum, double er0, double eps) {
     const double e2 = eps * eps * er0;
@@ -158,7 +174,8 @@ __global__ void __launch_bounds__(SOR_THREADS, 1) k_sor_grid(SorArgs<T> a, Geo g
     __syncthreads();
     const int n = (g.nx >> 1) * g.ny * g.nz, stride = gridDim.x * blockDim.x;
     const int oy = g.sx, oz = g.sx * g.sy;
-    const double er0 = *a.er0;
+    const T sc = sor_scale<T>(*a.er0);
+    const double er0 = *a.er0 * ((double)sc * (double)sc);
     unsigned arrivals = 0, *bar = reinterpret_cast<unsigned *>(a.flag + 3);
     for (int itr = 1; itr <= a.itrmax; ++itr) {
         SorSum<T> s;
@@ -177,7 +194,7 @@ __global__ void __launch_bounds__(SOR_THREADS, 1) k_sor_grid(SorArgs<T> a, Geo g
                 const T p0 = __ldcg(P);
                 const T e = sor_residual(a, __ldcg(P + zm), __ldcg(P + ym), __ldcg(P + xm), p0, __ldcg(P + xp),
                                          __ldcg(P + yp), __ldcg(P + zp), a.R[q]);
-                s.add_sq(e);
+                s.add_sq(e * sc);
                 __stcg(a.Phi + h, sor_update(p0, e, a));
             }
             if (color == 0 && sor_grid_barrier(bar, arrivals, &late)) break;
@@ -287,7 +304,8 @@ __global__ void __launch_bounds__(SOR_CLUSTER_THREADS, 1) k_sor_cluster(SorArgs<
         }
     }
     cluster_barrier();
-    const double er0 = *a.er0;
+    const float sc = sor_scale<float>(*a.er0);
+    const double er0 = *a.er0 * ((double)sc * (double)sc);
     const float above = (float)(a.eps * a.eps * er0) * 1.0001f;
     for (int itr = 1; itr <= a.itrmax; ++itr) {
         SorSum<float> s;
@@ -305,7 +323,7 @@ __global__ void __launch_bounds__(SOR_CLUSTER_THREADS, 1) k_sor_cluster(SorArgs<
                 const float p0 = pv[t][color];
                 const float ym = dn[t] ? at[dn[t]] : p0, yp = up[t] ? at[up[t]] : p0;
                 const float e = sor_residual(a, at[-plane], ym, xm, p0, xp, yp, at[plane], rv[t][color]);
-                s.add_sq(e);
+                s.add_sq(e * sc);
                 const float v = sor_update(p0, e, a);
                 pv[t][color] = v;
                 phi[row_[t] + o * half + ix] = v;

@@ -140,7 +140,7 @@ __device__ __forceinline__ T sor_scale(double er0) {
     }
 }
 
-// sqrt(sum / er0) < eps: squared away from the boundary
+// sqrt(sum / er0) < eps: squared away from the boundary (eps >= 0)
 __device__ __forceinline__ bool sor_done(double sum, double er0, double eps) {
     const double e2 = eps * eps * er0;
     if (sum < e2 * (1.0 - 1.0e-12)) return true;
@@ -411,6 +411,9 @@ inline cudaError_t sor_cluster_size(int *out) {
 // max_cluster > 1 allows the cluster form
 template <typename T>
 inline cudaError_t sor_sweeps(SorArgs<T> a, const Geo &g, int sms, int max_cluster, cudaStream_t s) {
+    // no sum passes a test against a negative or NaN tolerance, nor against zero:
+    // all itrmax sweeps run
+    if (!(a.eps > 0.0)) a.eps = 0.0;
     a.lgx = a.lgy = 0;
     while ((2 << a.lgx) < g.nx) ++a.lgx;
     while ((1 << a.lgy) < g.ny) ++a.lgy;

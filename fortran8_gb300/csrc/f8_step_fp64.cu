@@ -388,8 +388,9 @@ PolyConst poly_const(const Geo &g, const Phys &ph) {
     c.wi = recip(ph.wi);
     c.dc2 = recip(2.0 * ph.newton_dc);
     c.dtwi = ph.dt / ph.wi;
-    c.eps2_lo = ph.newton_eps * ph.newton_eps * (1.0 - 1.0e-12);
-    c.eps2_hi = ph.newton_eps * ph.newton_eps * (1.0 + 1.0e-12);
+    const bool squared = ph.newton_eps > 1.0e-140 && ph.newton_eps < 1.0e140;
+    c.eps2_lo = squared ? ph.newton_eps * ph.newton_eps * (1.0 - 1.0e-12) : 0.0;
+    c.eps2_hi = squared ? ph.newton_eps * ph.newton_eps * (1.0 + 1.0e-12) : INFINITY;
     return c;
 }
 
@@ -413,7 +414,8 @@ GridRecip grid_recip(const Geo &g) {
 
 // The Newton step test sqrt(sr / sx) < eps (fenep.f90:575).  Squared, away from
 // the boundary by more than the rounding of either form; the reference's
-// expression within it (or for NaN).
+// expression within it, for NaN, and for a tolerance that is not positive (all
+// itrmax iterations run then) or whose square is out of range.
 __device__ __forceinline__ bool newton_small(double sr, double sx, double eps, const PolyConst &c) {
     if (sr < sx * c.eps2_lo) return true;
     if (sr > sx * c.eps2_hi) return false;

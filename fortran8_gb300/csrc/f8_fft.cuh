@@ -13,6 +13,7 @@
 #include <type_traits>
 #include "f8_common.cuh"
 #include "f8_df64.cuh"
+#include "f8_recip.cuh"
 
 namespace f8 {
 
@@ -650,8 +651,8 @@ __host__ __device__ inline void wall_coef(const WallSpec &w, int sys, int j, int
 }
 
 // Tables of the Thomas recurrence of every (kx, kz) system: per row and mode
-// P = -b/den and den, in FP64 1/den as the sum of two doubles (Brisebarre, Muller
-// and Raina's division by a known divisor) in the second and third table, in
+// P = -b/den and den, in FP64 1/den as the sum of two doubles (f8_recip.cuh) in
+// the second and third table, in
 // FP32 den itself (an FP32 division is cheap).  Where tdma's guard sets P = Q = 0
 // (fenep_2d.f90:1157-1160): P = 1/den = 0, den = inf.  Layout [row][kz][kx].
 template <typename T>
@@ -670,9 +671,9 @@ __global__ void k_wall_table(T *__restrict__ P, T *__restrict__ rh, T *__restric
         p = guard ? T(0) : -b / den;
         P[o] = p;
         if constexpr (sizeof(T) == 8) {
-            const double r = 1.0 / den;
-            rh[o] = guard ? 0.0 : r;
-            rl[o] = guard ? 0.0 : fma(-den, r, 1.0) / den;
+            const Recip r = guard ? Recip{0.0, 0.0} : recip(den);
+            rh[o] = r.h;
+            rl[o] = r.l;
         } else {
             rh[o] = guard ? __int_as_float(0x7f800000) : den;
         }
@@ -680,7 +681,7 @@ __global__ void k_wall_table(T *__restrict__ P, T *__restrict__ rh, T *__restric
 }
 
 // t / den with those tables
-__device__ __forceinline__ double wall_div(double t, double h, double l) { return __fma_rn(t, h, __dmul_rn(t, l)); }
+__device__ __forceinline__ double wall_div(double t, double h, double l) { return div_by(t, Recip{h, l}); }
 __device__ __forceinline__ float wall_div(float t, float den, float) { return t / den; }
 
 // The wall-normal solves (tdma, fenep_2d.f90:1145-1177) of every mode with

@@ -27,6 +27,7 @@
 #include <algorithm>
 #include "f8_common.cuh"
 #include "f8_df64.cuh"
+#include "f8_recip.cuh"
 
 namespace f8 {
 
@@ -80,7 +81,7 @@ struct SorArgs {
     int *flag;              // [0] converged, [1] iteration, [2] a barrier wait ran out,
                             // [3] arrivals at the grid barrier; zero at launch
     T om, bx, by, bz, b0;   // relaxation, 1/dX^2 ..., the diagonal
-    T b0h, b0l;             // 1/b0 as a sum (FP64)
+    Recip rb0;              // 1/b0 (FP64)
     double eps;
     int itrmax, lgx, lgy;   // log2 of nx / 2 and ny
 };
@@ -103,11 +104,9 @@ __device__ __forceinline__ float sor_residual(const SorArgs<float> &a, float zm,
 __device__ __forceinline__ float sor_update(float phi, float e, const SorArgs<float> &a) {
     return __fadd_rn(phi, __fmul_rn(a.om, e) / a.b0);
 }
-// the division by the known divisor b0 from its two-part reciprocal (2 FP64
-// slots; Brisebarre, Muller and Raina, IEEE Trans. Comput. 53 (2004) 1069)
+// the division by the known divisor b0 from its two-part reciprocal
 __device__ __forceinline__ double sor_update(double phi, double e, const SorArgs<double> &a) {
-    const double t = a.om * e;
-    return phi + __fma_rn(t, a.b0h, __dmul_rn(t, a.b0l));
+    return phi + div_by(a.om * e, a.rb0);
 }
 
 // block sum in thread 0's warp (lane 0 of warp 0 holds it)

@@ -10,6 +10,7 @@
 #include "f8_common.cuh"
 #include "f8_fft.cuh"
 #include "f8_kernels.h"
+#include "f8_recip.cuh"
 #include "f8_sor.cuh"
 
 namespace f8 {
@@ -348,26 +349,6 @@ __global__ void __launch_bounds__(128) k_codes3_exact(const double *__restrict__
 }
 
 // ---------------------------------------------------------------------------
-// Division by a divisor that is known in advance, from its reciprocal as the
-// unevaluated sum h + l of two doubles: RN(x h + RN(x l)) (Brisebarre, Muller and
-// Raina, IEEE Trans. Comput. 53 (2004) 1069).  The sum is within 2^-105 of x/d
-// before its one rounding, so it is the correctly rounded quotient unless x/d
-// lies that close to a rounding boundary (for a given d, a few x at most).  Two
-// FP64 slots where a division takes 7.2 (measured).
-struct Recip {
-    double h, l;
-};
-__host__ __device__ inline Recip recip(double d) {
-    const double h = 1.0 / d;
-    return Recip{h, fma(-d, h, 1.0) / d};
-}
-// on the device the second part only needs a few bits: its division is a product
-__device__ __forceinline__ Recip recip_dev(double d) {
-    const double h = 1.0 / d;
-    return Recip{h, __dmul_rn(__fma_rn(-d, h, 1.0), h)};
-}
-__device__ __forceinline__ double div_by(double x, Recip r) { return __fma_rn(x, r.h, __dmul_rn(x, r.l)); }
-
 // Divisors of the polymer update: the reference's expressions with their
 // divisions by constants.
 struct PolyConst {
@@ -592,8 +573,7 @@ __device__ __forceinline__ bool surely_larger(double a, double b) {
     return (__double2hiint(a) & 0x7fffffff) > (__double2hiint(b) & 0x7fffffff);
 }
 
-// Gauss-Jordan with partial pivoting (fenep.f90:608-643); the pivot row is
-// divided through its reciprocal (div_by)
+// Gauss-Jordan with partial pivoting (fenep.f90:608-643)
 template <int N>
 __device__ inline void gauss(double (&Ah)[N][N + 1], double *x) {
     for (int k = 0; k < N; ++k) {
@@ -608,8 +588,8 @@ __device__ inline void gauss(double (&Ah)[N][N + 1], double *x) {
         }
         if (k != maxidx)
             for (int q = k; q <= N; ++q) { double tmp = Ah[k][q]; Ah[k][q] = Ah[maxidx][q]; Ah[maxidx][q] = tmp; }
-        const Recip piv = recip_dev(Ah[k][k]);
-        for (int q = k + 1; q <= N; ++q) Ah[k][q] = div_by(Ah[k][q], piv);
+        const double piv = Ah[k][k];
+        for (int q = k + 1; q <= N; ++q) Ah[k][q] = Ah[k][q] / piv;
         Ah[k][k] = 1.0;
         for (int r = 0; r < N; ++r) {
             if (r == k) continue;
@@ -623,8 +603,10 @@ __device__ inline void gauss(double (&Ah)[N][N + 1], double *x) {
 
 // The same elimination where every pivot is the diagonal element, as nearly
 // always (the Lyapunov system is dominated by it): in registers, the pivot
-// search as integer comparisons of the high words.  Returns false, with x
-// unusable, when some pivot might be another row's.
+// search as integer comparisons of the high words, the pivot row divided through
+// a reciprocal whose second part only needs a few bits.  Returns false, with x
+// unusable, when some pivot might be another row's or a value is not finite (an
+// infinite or NaN quotient may differ from the division's).
 template <int N>
 __device__ __forceinline__ bool gauss_diagonal(double (&Ah)[N][N + 1], double *x) {
     bool plain = true;
@@ -632,7 +614,8 @@ __device__ __forceinline__ bool gauss_diagonal(double (&Ah)[N][N + 1], double *x
     for (int k = 0; k < N; ++k) {
 #pragma unroll
         for (int r = k + 1; r < N; ++r) plain = plain && surely_larger(Ah[k][k], Ah[r][k]);
-        const Recip piv = recip_dev(Ah[k][k]);
+        const double h = 1.0 / Ah[k][k];
+        const Recip piv{h, __dmul_rn(__fma_rn(-Ah[k][k], h, 1.0), h)};
 #pragma unroll
         for (int q = k + 1; q <= N; ++q) Ah[k][q] = div_by(Ah[k][q], piv);
 #pragma unroll
@@ -644,7 +627,10 @@ __device__ __forceinline__ bool gauss_diagonal(double (&Ah)[N][N + 1], double *x
             }
     }
 #pragma unroll
-    for (int r = 0; r < N; ++r) x[r] = Ah[r][N];
+    for (int r = 0; r < N; ++r) {
+        x[r] = Ah[r][N];
+        plain = plain && (__double2hiint(x[r]) & 0x7ff00000) != 0x7ff00000;
+    }
     return plain && surely_larger(Ah[N - 1][N - 1], 0.0);
 }
 
@@ -1498,8 +1484,7 @@ cudaError_t sor_solve_on(Dev &d, const double *Q, double *Phi, double omega, dou
     a.om = omega;
     a.bx = 1.0 / (g.dx * g.dx); a.by = 1.0 / (g.dy * g.dy); a.bz = g.dim == 3 ? 1.0 / (g.dz * g.dz) : 0.0;
     a.b0 = a.bx + a.bx + a.by + a.by + a.bz + a.bz;
-    const Recip r = recip(a.b0);
-    a.b0h = r.h; a.b0l = r.l;
+    a.rb0 = recip(a.b0);
     a.eps = eps; a.itrmax = itrmax;
     F8_CUDA_RET(sor_sweeps(a, g, device_sm_count(), 1, s));
     int it_host[3] = {0, 0, 0};

@@ -257,8 +257,18 @@ struct f8_ctx {
 
 namespace {
 
+// Every CUDA error of an entry point ends here.  A step that fails between the
+// fork and the join of its side streams leaves kernels on them that write the
+// context's arrays: they have ended when the call returns, so that the next
+// load or step cannot run beside them.  The runtime's own record of the error is
+// cleared, or the next launch check would report it again.
 int fail(f8_ctx *c, cudaError_t e, const char *where) {
-    if (c) c->last_error = std::string(where) + ": " + cudaGetErrorString(e);
+    if (c) {
+        c->last_error = std::string(where) + ": " + cudaGetErrorString(e);
+        for (cudaStream_t q : {c->d.code_side, c->d.aux[0], c->d.aux[1]})
+            if (q) cudaStreamSynchronize(q);
+    }
+    cudaGetLastError();
     return e == cudaErrorMemoryAllocation ? F8_ERR_NOMEM : F8_ERR_CUDA;
 }
 

@@ -216,6 +216,9 @@ inline int kept_segments(double avail, double slot_bytes, double ck_bytes, int K
     return 1;
 }
 
+// a counter that has not reached target; both wrap at 2^32, fewer than 2^31 apart
+__host__ __device__ inline bool behind(unsigned v, unsigned target) { return (int)(target - v) > 0; }
+
 struct StepCounters {
     unsigned long long newton_iters;
     unsigned long long newton_unconverged;

@@ -158,8 +158,8 @@ __device__ __forceinline__ bool sor_grid_barrier(unsigned *bar, unsigned &arriva
         unsigned v;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            if (v < arrivals && clock64() - t0 > SOR_WAIT_CYCLES) { *late = 1; break; }
-        } while (v < arrivals);
+            if (behind(v, arrivals) && clock64() - t0 > SOR_WAIT_CYCLES) { *late = 1; break; }
+        } while (behind(v, arrivals));
     }
     __syncthreads();
     return *late != 0;

@@ -84,6 +84,7 @@ struct SorArgs {
     Recip rb0;              // 1/b0 (FP64)
     double eps;
     int itrmax, lgx, lgy;   // log2 of nx / 2 and ny
+    long long wait = SOR_WAIT_CYCLES;   // limit of each wait of the grid barrier, clock cycles
 };
 
 // the residual, summed in the reference's order (fenep.f90:885-893); FP32: with
@@ -147,7 +148,7 @@ __device__ __forceinline__ bool sor_done(double sum, double er0, double eps) {
 }
 
 // true when the wait ran out
-__device__ __forceinline__ bool sor_grid_barrier(unsigned *bar, unsigned &arrivals, int *late) {
+__device__ __forceinline__ bool sor_grid_barrier(unsigned *bar, unsigned &arrivals, int *late, long long wait) {
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -158,7 +159,7 @@ __device__ __forceinline__ bool sor_grid_barrier(unsigned *bar, unsigned &arriva
         unsigned v;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            if (behind(v, arrivals) && clock64() - t0 > SOR_WAIT_CYCLES) { *late = 1; break; }
+            if (behind(v, arrivals) && clock64() - t0 > wait) { *late = 1; break; }
         } while (behind(v, arrivals));
     }
     __syncthreads();
@@ -196,13 +197,13 @@ __global__ void __launch_bounds__(SOR_THREADS, 1) k_sor_grid(SorArgs<T> a, Geo g
                 s.add_sq(e * sc);
                 __stcg(a.Phi + h, sor_update(p0, e, a));
             }
-            if (color == 0 && sor_grid_barrier(bar, arrivals, &late)) break;
+            if (color == 0 && sor_grid_barrier(bar, arrivals, &late, a.wait)) break;
         }
         // the block's sum, then every block's in the same order
         s = block_sum(s, sh);
         SorSum<T> *part = a.part + (itr & 1) * SOR_MAX_BLOCKS;
         if (threadIdx.x == 0) part[blockIdx.x] = s;
-        if (late || sor_grid_barrier(bar, arrivals, &late)) {
+        if (late || sor_grid_barrier(bar, arrivals, &late, a.wait)) {
             if (threadIdx.x == 0) a.flag[2] = 1;
             return;
         }

@@ -1490,7 +1490,7 @@ cudaError_t sor_solve_on(Dev &d, const double *Q, double *Phi, double omega, dou
     int it_host[3] = {0, 0, 0};
     F8_CUDA_RET(cudaMemcpyAsync(it_host, d.flag, sizeof(it_host), cudaMemcpyDeviceToHost, s));
     F8_CUDA_RET(cudaStreamSynchronize(s));
-    if (it_host[2]) return cudaErrorLaunchTimeout;
+    if (it_host[2]) return cudaErrorTimeout;      // a wait of the grid barrier ran out
     *iters = it_host[0] ? it_host[1] : itrmax + 1;
     F8_CUDA_RET(bc(Phi, g, BC_P, s));
     // zero-mean shift (fenep_2d.f90:577-579)

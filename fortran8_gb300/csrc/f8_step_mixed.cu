@@ -2089,7 +2089,7 @@ cudaError_t sor_solve_m(Dev &d, const StepOpts &o, int *iters, cudaStream_t s) {
     int it_host[3] = {0, 0, 0};
     F8_CUDA_RET(cudaMemcpyAsync(it_host, d.flag, sizeof(it_host), cudaMemcpyDeviceToHost, s));
     F8_CUDA_RET(cudaStreamSynchronize(s));
-    if (it_host[2]) return cudaErrorLaunchTimeout;
+    if (it_host[2]) return cudaErrorTimeout;      // a wait of the grid barrier ran out
     *iters = it_host[0] ? it_host[1] : o.sor_itrmax + 1;
     k_sum_part_f<<<nb, 256, 0, s>>>(d.Phif, d.ni, 1, d.red, g); count_launch();
     k_sum_final<<<1, 256, 0, s>>>(d.red, nb, d.scal, 2, 0); count_launch();

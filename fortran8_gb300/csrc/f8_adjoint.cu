@@ -68,8 +68,8 @@ cudaError_t step_fp64_adjoint(Dev &d, AdjState &A, const TapeStep &t, const doub
         }
         ia.w = drag_w;
         ia.grad = A.grad;
-        ia.d3 = 1;
-        k_ibm_adj<double><<<dim3(g.nz, 3), ibm_adj_block(d.nm), 0, s>>>(ia, g); count_launch();
+        const IbmAdjShape sh = ibm_adj_shape(d.nm);
+        k_ibm_adj<3, double><<<dim3(g.nz, 3, sh.chunks), dim3(32, 3, sh.warps), 0, s>>>(ia, g); count_launch();
     }
     // 2. momentum right-hand side: per-cell sources, then the gather of the
     // velocity, pressure and (with the polymer) C0 / C adjoints
@@ -515,8 +515,8 @@ cudaError_t step_fp64_adjoint2(Dev &d, AdjState &A, const TapeStep &t, const dou
         }
         ia.w = drag_w;
         ia.grad = A.grad;
-        ia.d3 = 0;
-        k_ibm_adj<double><<<dim3(1, 2), ibm_adj_block(d.nm), 0, s>>>(ia, g); count_launch();
+        const IbmAdjShape sh = ibm_adj_shape(d.nm);
+        k_ibm_adj<1, double><<<dim3(1, 2, sh.chunks), dim3(32, 1, sh.warps), 0, s>>>(ia, g); count_launch();
     }
     // 2. momentum right-hand side (the adjoint of U^n starts here; P^n keeps
     // the identity part from P^{n+1})

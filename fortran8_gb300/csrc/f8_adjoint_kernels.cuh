@@ -402,12 +402,11 @@ struct IbmAdjArgs {
     T *lUa[3];               // out: adjoint of Ua (interior cells, scattered)
     const double *w;         // drag weights of this step (ncyl x 3)
     double *grad;            // grad[3 + 2 l], grad[4 + 2 l]: cylinder centre
-    int d3;                  // 0: the 2D step (one marker plane, no z weight, fenep_2d.f90:1726-1819)
 };
 
-// One thread per (marker, plane of its stencil): warps of 32 markers, and a block
-// takes all markers of a (marker plane n, component), IBM_ADJ_CHUNKS warps of
-// them for each of the 3 planes at a time.  Forward: Ub = sum Ua delta dX^3,
+// One thread per (marker, plane of its stencil): a block takes IBM_ADJ_WARPS
+// warps of 32 markers, for each of the PLANES planes (3; in 2D the one that has a
+// weight) of one marker plane n and component.  Forward: Ub = sum Ua delta dX^3,
 // Fc = (Uc - Ub)/dt, drag = -dv sum Fc, f = fold(sum Fc delta dX^3),
 // Q = Ua + dt f - dt B/2.  Marker offsets from the grid points are formed in
 // FP64 (the marker positions are FP64) and the kernel weights in T.  The adjoint
@@ -416,94 +415,93 @@ struct IbmAdjArgs {
 // weights with few warps, and of FP64 additions to the few sums of the cylinder
 // centres, which are formed per warp and per block first: one thread per whole
 // stencil took 18.8 us for 80 markers x 64 planes, this form 14.5 us.
-constexpr int MAX_CYL_SHARED = 64, IBM_ADJ_CHUNKS = 4;
+constexpr int MAX_CYL_SHARED = 64;
 
-template <typename T>
-__global__ void __launch_bounds__(96 * IBM_ADJ_CHUNKS) k_ibm_adj(IbmAdjArgs<T> a, Geo g) {
-    __shared__ T part[IBM_ADJ_CHUNKS][3][32];
+template <int PLANES, typename T>
+__global__ void __launch_bounds__(32 * PLANES * IBM_ADJ_WARPS) k_ibm_adj(IbmAdjArgs<T> a, Geo g) {
+    __shared__ T part[IBM_ADJ_WARPS][PLANES][32];
     __shared__ double gc[2 * MAX_CYL_SHARED];
-    const int kk = threadIdx.y, n = blockIdx.x + 1, comp = blockIdx.y;
-    const int tid = threadIdx.x + 32 * (threadIdx.y + 3 * threadIdx.z), nt = 96 * blockDim.z;
+    const int kk = PLANES == 3 ? threadIdx.y : 1, n = blockIdx.x + 1, comp = blockIdx.y;
+    const int tid = threadIdx.x + 32 * (threadIdx.y + PLANES * threadIdx.z), nt = 32 * PLANES * blockDim.z;
     const bool use_sh = a.ncyl <= MAX_CYL_SHARED;
     if (use_sh)
         for (int q = tid; q < 2 * a.ncyl; q += nt) gc[q] = 0.0;
-    for (int m0 = 0; m0 < a.nm; m0 += 32 * blockDim.z) {
-        __syncthreads();
-        const int m = m0 + 32 * threadIdx.z + threadIdx.x;
-        const bool on = m < a.nm;
-        const int mm = on ? m : 0;
-        const T dt = T(g.dt);
-        const int i0 = a.i0[comp][mm], j0 = a.j0[comp][mm], l = a.mcyl[mm];
-        const T fc = T(a.Fc[comp][(size_t)mm + (size_t)a.nm * (n - 1)]);
-        const T svn = T(a.mvol[mm] * a.idvol);    // spreading: marker volume / (dX dY dZ)
-        const T dvn = T(a.dvn);
-        const int k = n - 1 + kk, fk = wrapz(g, k);
-        const T *lQ = a.lQ[comp], *Ua = a.Ua[comp];
-        // offset of stencil point 0 from the marker in cells: U at (i dX, (j - 1/2) dY), ...
-        const double x0 = (i0 - (comp == 0 ? 0.0 : 0.5)) - a.mx[mm] * a.idx;
-        const double y0 = (j0 - (comp == 1 ? 0.0 : 0.5)) - a.my[mm] * a.idy;
-        // plane k at (k - 1/2) dZ (W: k dZ), the marker plane at (n - 1/4) dZ
-        const T wz = a.d3 ? roma_t(T(kk - 1.25 + (comp == 2 ? 0.5 : 0.0))) : (kk == 1 ? T(1) : T(0));
-        T wxs[3], wys[3], dwx[3], dwy[3], lf[9], u[9];
-        int at[9];
-        T sg[3];
+    const int m = 32 * (blockIdx.z * blockDim.z + threadIdx.z) + threadIdx.x;
+    const bool on = m < a.nm;
+    const int mm = on ? m : 0;
+    const T dt = T(g.dt);
+    const int i0 = a.i0[comp][mm], j0 = a.j0[comp][mm], l = a.mcyl[mm];
+    const T fc = T(a.Fc[comp][(size_t)mm + (size_t)a.nm * (n - 1)]);
+    const T svn = T(a.mvol[mm] * a.idvol);    // spreading: marker volume / (dX dY dZ)
+    const T dvn = T(a.dvn);
+    const int k = n - 1 + kk, fk = wrapz(g, k);
+    const T *lQ = a.lQ[comp], *Ua = a.Ua[comp];
+    // offset of stencil point 0 from the marker in cells: U at (i dX, (j - 1/2) dY), ...
+    const double x0 = (i0 - (comp == 0 ? 0.0 : 0.5)) - a.mx[mm] * a.idx;
+    const double y0 = (j0 - (comp == 1 ? 0.0 : 0.5)) - a.my[mm] * a.idy;
+    // plane k at (k - 1/2) dZ (W: k dZ), the marker plane at (n - 1/4) dZ
+    const T wz = PLANES == 3 ? roma_t(T(kk - 1.25 + (comp == 2 ? 0.5 : 0.0))) : T(1);
+    T wxs[3], wys[3], dwx[3], dwy[3], lf[9], u[9];
+    int at[9];
+    T sg[3];
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const int i = i0 + q % 3, j = j0 + q / 3;
-            const int fj = g.walls ? max(1, min(g.ny, j)) : wrapy(g, j);
-            at[q] = hix(g, wrapx(g, i), fj, fk);
-            lf[q] = g.walls && fj != j ? T(0) : dt * lQ[at[q]];
-            u[q] = Ua[hix(g, i, j, k)];
-        }
+    for (int q = 0; q < 9; ++q) {
+        const int i = i0 + q % 3, j = j0 + q / 3;
+        const int fj = g.walls ? max(1, min(g.ny, j)) : wrapy(g, j);
+        at[q] = hix(g, wrapx(g, i), fj, fk);
+        lf[q] = g.walls && fj != j ? T(0) : dt * lQ[at[q]];
+        u[q] = Ua[hix(g, i, j, k)];
+    }
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            const int j = j0 + q;
-            sg[q] = !g.walls ? T(1) : comp == 1 ? (j == 0 || j >= g.ny ? T(0) : T(1)) : (j == 0 || j == g.ny + 1 ? T(-1) : T(1));
-            const T rx = T(x0 + q), ry = T(y0 + q);
-            wxs[q] = roma_t(rx);
-            wys[q] = roma_t(ry);
-            dwx[q] = -droma_t(rx) * T(a.idx);   // d/dxc
-            dwy[q] = -droma_t(ry) * T(a.idy);
-        }
-        // adjoint of Fc: drag weight + the folded spreading
-        T ls = T(0), gx = T(0), gy = T(0);
+    for (int q = 0; q < 3; ++q) {
+        const int j = j0 + q;
+        sg[q] = !g.walls ? T(1) : comp == 1 ? (j == 0 || j >= g.ny ? T(0) : T(1)) : (j == 0 || j == g.ny + 1 ? T(-1) : T(1));
+        const T rx = T(x0 + q), ry = T(y0 + q);
+        wxs[q] = roma_t(rx);
+        wys[q] = roma_t(ry);
+        dwx[q] = -droma_t(rx) * T(a.idx);   // d/dxc
+        dwy[q] = -droma_t(ry) * T(a.idy);
+    }
+    // adjoint of Fc: drag weight + the folded spreading
+    T ls = T(0), gx = T(0), gy = T(0);
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            ls += lf[q] * (wxs[q % 3] * wys[q / 3]);
-            gx += lf[q] * (dwx[q % 3] * wys[q / 3]);
-            gy += lf[q] * (wxs[q % 3] * dwy[q / 3]);
-        }
-        T (*ps)[32] = part[threadIdx.z];
-        ps[kk][threadIdx.x] = ls * (wz * svn);
-        gx *= fc * svn * wz;
-        gy *= fc * svn * wz;
-        __syncthreads();
-        const T lfc = T(-a.cylvol[l] * a.w[3 * l + comp]) + ps[0][threadIdx.x] + ps[1][threadIdx.x] + ps[2][threadIdx.x];
-        const T lub = -lfc / dt * dvn * wz;
-        T *lUa = a.lUa[comp];
-        T ux = T(0), uy = T(0);
+    for (int q = 0; q < 9; ++q) {
+        ls += lf[q] * (wxs[q % 3] * wys[q / 3]);
+        gx += lf[q] * (dwx[q % 3] * wys[q / 3]);
+        gy += lf[q] * (wxs[q % 3] * dwy[q / 3]);
+    }
+    T (*ps)[32] = part[threadIdx.z];
+    ps[threadIdx.y][threadIdx.x] = ls * (wz * svn);
+    gx *= fc * svn * wz;
+    gy *= fc * svn * wz;
+    __syncthreads();
+    T lfc = T(-a.cylvol[l] * a.w[3 * l + comp]);
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const T v = lub * (wxs[q % 3] * wys[q / 3]) * sg[q / 3];
-            if (on && v != T(0)) atomicAdd(&lUa[at[q]], v);
-            ux += u[q] * (dwx[q % 3] * wys[q / 3]);
-            uy += u[q] * (wxs[q % 3] * dwy[q / 3]);
+    for (int q = 0; q < PLANES; ++q) lfc += ps[q][threadIdx.x];
+    const T lub = -lfc / dt * dvn * wz;
+    T *lUa = a.lUa[comp];
+    T ux = T(0), uy = T(0);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        const T v = lub * (wxs[q % 3] * wys[q / 3]) * sg[q / 3];
+        if (on && v != T(0)) atomicAdd(&lUa[at[q]], v);
+        ux += u[q] * (dwx[q % 3] * wys[q / 3]);
+        uy += u[q] * (wxs[q % 3] * dwy[q / 3]);
+    }
+    const double dx = on ? (double)(gx + lub * ux) : 0.0, dy = on ? (double)(gy + lub * uy) : 0.0;
+    // the warp's sum for each cylinder among its markers (one or two)
+    unsigned todo = 0xffffffffu;
+    while (todo) {
+        const int cl = __shfl_sync(0xffffffffu, l, __ffs(todo) - 1);
+        todo &= ~__ballot_sync(0xffffffffu, l == cl);
+        double sx = l == cl ? dx : 0.0, sy = l == cl ? dy : 0.0;
+        for (int o = 16; o > 0; o >>= 1) {
+            sx += __shfl_down_sync(0xffffffffu, sx, o);
+            sy += __shfl_down_sync(0xffffffffu, sy, o);
         }
-        double dx = on ? (double)(gx + lub * ux) : 0.0, dy = on ? (double)(gy + lub * uy) : 0.0;
-        // the warp's sum for each cylinder among its markers (one or two)
-        unsigned todo = 0xffffffffu;
-        while (todo) {
-            const int cl = __shfl_sync(0xffffffffu, l, __ffs(todo) - 1);
-            todo &= ~__ballot_sync(0xffffffffu, l == cl);
-            double sx = l == cl ? dx : 0.0, sy = l == cl ? dy : 0.0;
-            for (int o = 16; o > 0; o >>= 1) {
-                sx += __shfl_down_sync(0xffffffffu, sx, o);
-                sy += __shfl_down_sync(0xffffffffu, sy, o);
-            }
-            if (threadIdx.x == 0) {
-                atomicAdd(use_sh ? &gc[2 * cl] : &a.grad[3 + 2 * cl], sx);
-                atomicAdd(use_sh ? &gc[2 * cl + 1] : &a.grad[4 + 2 * cl], sy);
-            }
+        if (threadIdx.x == 0) {
+            atomicAdd(use_sh ? &gc[2 * cl] : &a.grad[3 + 2 * cl], sx);
+            atomicAdd(use_sh ? &gc[2 * cl + 1] : &a.grad[4 + 2 * cl], sy);
         }
     }
     if (!use_sh) return;
@@ -1323,7 +1321,6 @@ __global__ void k_take_interior(const T *src, T *dst, Geo g, int n) {
 
 inline dim3 adj_cells(const Geo &g, dim3 b) { return dim3((g.nx + b.x - 1) / b.x, (g.ny + b.y - 1) / b.y, g.nz); }
 // the updated cells: with walls the ghost rows, too
-inline dim3 ibm_adj_block(int nm) { return dim3(32, 3, (unsigned)std::min(IBM_ADJ_CHUNKS, (nm + 31) / 32)); }
 inline dim3 adj_rows(const Geo &g, dim3 b) { return dim3((g.nx + b.x - 1) / b.x, (prows(g) + b.y - 1) / b.y, g.nz); }
 
 }  // namespace

@@ -95,8 +95,8 @@ cudaError_t step_mixed_adjoint(Dev &d, AdjStateF &A, const MixTape &t, const dou
         }
         ia.w = drag_w;
         ia.grad = A.grad;
-        ia.d3 = 1;
-        k_ibm_adj<float><<<dim3(g.nz, 3), ibm_adj_block(d.nm), 0, s>>>(ia, g); count_launch();
+        const IbmAdjShape sh = ibm_adj_shape(d.nm);
+        k_ibm_adj<3, float><<<dim3(g.nz, 3, sh.chunks), dim3(32, 3, sh.warps), 0, s>>>(ia, g); count_launch();
     }
     // 2. momentum right-hand side: per-cell sources, then the gather of the
     // velocity, pressure and (with the polymer) C0 / C adjoints

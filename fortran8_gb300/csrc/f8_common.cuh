@@ -216,6 +216,20 @@ inline int kept_segments(double avail, double slot_bytes, double ck_bytes, int K
     return 1;
 }
 
+// The IBM transpose (k_ibm_adj): a block takes up to IBM_ADJ_WARPS warps of 32
+// markers on one plane of one component, and as many blocks as that takes: one
+// block for all markers of a plane left 2 of 152 SMs to a 2D box (gradient of 6
+// steps of a 512^2 box with 5344 markers 31.1 ms, 18.2 now; 256^2 with 1368 10.6,
+// 7.2; FP64 256x128x4 with 548 7.7, 7.0).
+constexpr int IBM_ADJ_WARPS = 4;
+struct IbmAdjShape {
+    unsigned chunks, warps;
+};
+inline IbmAdjShape ibm_adj_shape(int nm) {
+    const unsigned w = (unsigned)((nm + 31) / 32), bw = w < (unsigned)IBM_ADJ_WARPS ? w : (unsigned)IBM_ADJ_WARPS;
+    return IbmAdjShape{(w + bw - 1) / bw, bw};
+}
+
 // a counter that has not reached target; both wrap at 2^32, fewer than 2^31 apart
 __host__ __device__ inline bool behind(unsigned v, unsigned target) { return (int)(target - v) > 0; }
 

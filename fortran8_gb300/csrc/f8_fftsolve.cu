@@ -83,8 +83,8 @@ cudaError_t set_smem_attrs() {
 
 // Fixed device arrays, one set per GPU: a spectrum of up to 135168 complex
 // values (65 * 64 * 32 = 33 * 64 * 64) and the tables of any grid (twiddles and
-// wavenumbers, N <= 1024).  Both entry points use them, one call at a time
-// (g_solve_mutex): a pair of cudaMalloc / cudaFree takes 62 us on this part, and
+// wavenumbers, N <= 1024).  Both entry points use them, one call at a time on a
+// device (solve_mutex): a pair of cudaMalloc / cudaFree takes 62 us on this part, and
 // two of them were most of a small solve (128 x 128: 239 us with them).
 #define F8_NOALLOC_MAX_SPECTRUM 135168
 #define F8_NOALLOC_MAX_TABLE 8192
@@ -93,8 +93,17 @@ static __device__ __align__(256) double g_noalloc_spectrum[2 * F8_NOALLOC_MAX_SP
 static __device__ __align__(256) double g_noalloc_table[F8_NOALLOC_MAX_TABLE];
 
 namespace {
-std::mutex g_solve_mutex;
+constexpr int kMaxDevices = 64;
+std::mutex g_solve_mutex[kMaxDevices];
+
+// of the current device: calls on other devices have their own arrays
+cudaError_t solve_mutex(std::mutex **m) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    *m = &g_solve_mutex[dev % kMaxDevices];
+    return e;
 }
+}  // namespace
 
 extern "C" int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double lz, const double *q, double *phi,
                             double lhs0, double lhs1) {
@@ -107,7 +116,9 @@ extern "C" int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double
     if (set_smem_attrs() != cudaSuccess) return F8_ERR_CUDA;
     const SolveTables t = make_tables(nx, ny, nz, lx, ly, lz);
     const size_t nspec = (size_t)(nx / 2 + 1) * ny * nz;
-    std::lock_guard<std::mutex> lock(g_solve_mutex);
+    std::mutex *mu = nullptr;
+    if (solve_mutex(&mu) != cudaSuccess) return F8_ERR_CUDA;
+    std::lock_guard<std::mutex> lock(*mu);
     // the arrays of the current device, looked up on every call (a device reset
     // between calls may move them)
     void *tab = nullptr, *fixed = nullptr;
@@ -152,7 +163,7 @@ extern "C" int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double
 //    f8_fft_solve too, and keep the last call's contents; each call overwrites
 //    all it reads (the forward transform fills the whole spectrum and the
 //    tables are rewritten), so nothing has to start at zero; the calls of
-//    several host threads take turns;
+//    several host threads take turns on a device;
 //  * the first call on a device looks up the device addresses of the arrays
 //    (cudaGetSymbolAddress, with that device current); make that first call
 //    before any stream capture on that device.  The addresses are kept for
@@ -166,7 +177,6 @@ struct NoallocPtrs {
     double *tab = nullptr;
 };
 
-constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mutex;
 NoallocPtrs g_noalloc_ptrs[kMaxDevices];
 
@@ -213,7 +223,9 @@ extern "C" int f8_fft_solve_noalloc(int nx, int ny, int nz, double lx, double ly
     if (int st = noalloc_setup(p)) return st;
     const SolveTables t = make_tables(nx, ny, nz, lx, ly, lz);
     if (t.buf.size() > (size_t)F8_NOALLOC_MAX_TABLE) return F8_ERR_TOO_LARGE;
-    std::lock_guard<std::mutex> lock(g_solve_mutex);
+    std::mutex *mu = nullptr;
+    if (solve_mutex(&mu) != cudaSuccess) return F8_ERR_CUDA;
+    std::lock_guard<std::mutex> lock(*mu);
     if (cudaMemcpyAsync(p.tab, t.buf.data(), t.buf.size() * sizeof(double), cudaMemcpyHostToDevice, 0) != cudaSuccess ||
         run_solve(q, phi, p.spec, p.tab, t, nx, ny, nz, lhs0, lhs1, 0) != cudaSuccess ||
         cudaStreamSynchronize(0) != cudaSuccess) {

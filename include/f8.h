@@ -346,7 +346,8 @@ int f8_kernel_timing(f8_ctx *ctx, double *kernel_ms, long long *steps_timed);
  * nz = 1 for a 2D field).  Sizes are powers of two.  FP64.  Grids within the
  * fixed workspace of f8_fft_solve_noalloc use it, larger ones allocate theirs
  * on the device for the duration of the call; runs on the default stream and
- * returns when the result is complete.  Calls from several threads take turns. */
+ * returns when the result is complete.  Calls from several threads take turns
+ * on a device. */
 int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double lz,
                  const double *q, double *phi, double lhs0, double lhs1);
 
@@ -361,7 +362,7 @@ int f8_fft_solve(int nx, int ny, int nz, double lx, double ly, double lz,
  *     F8_ERR_TOO_LARGE;
  *   - every call, of f8_fft_solve too, shares that workspace and leaves its
  *     contents behind; each call overwrites what it reads, and calls from
- *     several threads take turns;
+ *     several threads take turns on a device;
  *   - the first call on a device looks up the workspace address on that
  *     device (the device must be current); make it before any stream capture;
  *   - with CUDA's lazy module loading, the fixed arrays are placed in device

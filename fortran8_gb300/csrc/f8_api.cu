@@ -404,7 +404,6 @@ int setup(f8_ctx *c) {
                            &d.Q[0], &d.Q[1], &d.Q[2]})
             API_CUDA(c, c->alloc(p, ni));
         API_CUDA(c, c->alloc(&d.H, 3 * nspec));
-        API_CUDA(c, c->alloc(&d.H2, (g.walls ? 3 : 1) * nspec));
     } else {
         API_CUDA(c, c->alloc(&d.Cf, cs * d.ncomp));
         for (float **p : {&d.Uf, &d.Vf, &d.Wf, &d.Ul, &d.Vl, &d.Wl, &d.Pf, &d.Pl, &d.Phif, &d.Phil,
@@ -480,7 +479,7 @@ int setup(f8_ctx *c) {
     if (int st = upload(c, &d.ky2, ky2)) return st;
     if (int st = upload(c, &d.kz2, kz2)) return st;
     if (!mixed && g.walls) {
-        for (double *&t : d.walltab) API_CUDA(c, c->alloc(&t, 3 * nxh * (size_t)g.nz * (g.ny + 2)));
+        for (double *&t : d.walltab) API_CUDA(c, c->alloc(&t, wall_table_size<double>(g.ny, (int)nxh, g.nz)));
         API_CUDA(c, wall_tables_fp64(d, c->s));
     }
     if (mixed) {
@@ -499,8 +498,7 @@ int setup(f8_ctx *c) {
         if (g.dim == 2) d.fused_planes = 0;   // 2D: the line transforms and tridiagonal sweeps
         API_CUDA(c, c->alloc(&d.Hf, (d.fused_planes ? 1 : 3) * nspec));
         if (!d.fused_planes && g.walls) {
-            API_CUDA(c, c->alloc(&d.H2f, 3 * nspec));
-            for (float *&t : d.walltabf) API_CUDA(c, c->alloc(&t, 3 * nxh * (size_t)g.nz * (g.ny + 2)));
+            for (float *&t : d.walltabf) API_CUDA(c, c->alloc(&t, wall_table_size<float>(g.ny, (int)nxh, g.nz)));
             API_CUDA(c, wall_tables_mixed(d, c->s));
         }
         // side streams (the V and W Helmholtz solves, the wall ghost rows, the drag)

@@ -216,6 +216,10 @@ inline int kept_segments(double avail, double slot_bytes, double ck_bytes, int K
     return 1;
 }
 
+// values of the Thomas tables of one wall system (k_wall_table; FP32 has no third)
+template <typename T>
+inline size_t wall_table_size(int ny, int nxh, int nz) { return (size_t)(sizeof(T) == 8 ? 3 : 2) * (ny + 2) * nxh * nz; }
+
 // The IBM transpose (k_ibm_adj): a block takes up to IBM_ADJ_WARPS warps of 32
 // markers on one plane of one component, and as many blocks as that takes: one
 // block for all markers of a plane left 2 of 152 SMs to a 2D box (gradient of 6

@@ -595,11 +595,9 @@ inline void fft_solve_passes(int nb, Batch<const TS *> src, T *H, size_t hstride
 
 // ---------------------------------------------------------------------------
 // Wall-normal systems (fenep_2d.f90:1222-1238, 1262-1277, 1318-1332 with
-// NA = 0, NB = NY; x and z periodic).  Input spectrum Hin has rows j = 1..NY
-// (ny rows per plane), output Hout rows j = 0..NY+1 (ny+2 rows per plane).
-// One thread per kx column runs the Thomas recurrence of tdma with the
-// reference's near-zero-pivot guard; the real coefficient recurrence P and the
-// complex right-hand side share shared memory.
+// NA = 0, NB = NY; x and z periodic): rows j = 0..NY+1 of the spectrum, the
+// right-hand side in rows 1..NY, the Thomas recurrence of tdma with the
+// reference's near-zero-pivot guard.
 enum WallSys { SYS_U = 0, SYS_V = 1, SYS_P = 2 };
 
 struct WallSpec {
@@ -652,8 +650,7 @@ __host__ __device__ inline void wall_coef(const WallSpec &w, int sys, int j, int
 
 // Tables of the Thomas recurrence of every (kx, kz) system: per row and mode
 // P = -b/den and den, in FP64 1/den as the sum of two doubles (f8_recip.cuh) in
-// the second and third table, in
-// FP32 den itself (an FP32 division is cheap).  Where tdma's guard sets P = Q = 0
+// the second and third table, in FP32 den itself (an FP32 division is cheap).  Where tdma's guard sets P = Q = 0
 // (fenep_2d.f90:1157-1160): P = 1/den = 0, den = inf.  Layout [row][kz][kx].
 template <typename T>
 __global__ void k_wall_table(T *__restrict__ P, T *__restrict__ rh, T *__restrict__ rl, int ny, int nxh, int nz,
@@ -688,12 +685,11 @@ __device__ __forceinline__ float wall_div(float t, float den, float) { return t 
 // those tables.  A thread runs the recurrence of the real or the imaginary part
 // of one mode (the coefficients are real), neighbouring threads neighbouring
 // values of a row, so the rows stream through without a tile; the forward
-// values wait in the output.  In FP64 the chain is 5 slots a row forward and 2
+// values wait in the rows of the right-hand side.  In FP64 the chain is 5 slots a row forward and 2
 // back, where forming the coefficients and dividing took about 60 in a
 // half-filled warp.
 template <typename T>
-__global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *Hout, size_t hstride, int ny, int nxh,
-                                                  int nz, T inv_nxz, Batch<WallItem<T>> items, Batch<T> off) {
+__global__ void __launch_bounds__(64) k_wall_tdma(T *H, size_t hstride, int ny, int nxh, int nz, T inv_nxz, Batch<WallItem<T>> items, Batch<T> off) {
     const int n = ny + 2;
     const WallItem<T> it = items.p[blockIdx.z];
     const int sys = it.sys;
@@ -704,8 +700,7 @@ __global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *
     const int kz = blockIdx.y;
     if (c >= 2 * nxh) return;
     const size_t mode = (size_t)nxh * kz + (c >> 1);
-    const T *__restrict__ hin = Hin + blockIdx.z * hstride + (size_t)2 * nxh * ny * kz + c;
-    T *hout = Hout + blockIdx.z * hstride + (size_t)2 * nxh * n * kz + c;
+    T *h0 = H + blockIdx.z * hstride + (size_t)2 * nxh * n * kz + c;
     T q = T(0);
     // in groups of 8 rows: the loads do not depend on the recurrence, so a group's
     // are all in flight before its chain begins
@@ -717,7 +712,7 @@ __global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *
             const int j = j0 + u;
             d[u] = h[u] = l[u] = T(0);
             if (j >= n) continue;
-            if (j >= 1 && j <= ny && !(sys == SYS_V && j == ny)) d[u] = hin[(size_t)2 * nxh * (j - 1)] * inv_nxz;
+            if (j >= 1 && j <= ny && !(sys == SYS_V && j == ny)) d[u] = h0[(size_t)2 * nxh * j] * inv_nxz;
             else if (j == n - 1 && mode == 0 && c == 0) d[u] = T(it.top);
             h[u] = rh[(size_t)j * modes + mode];
             if (sizeof(T) == 8) l[u] = rl[(size_t)j * modes + mode];
@@ -730,7 +725,7 @@ __global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *
                                                      : (sys == SYS_V && j >= ny ? T(0) : ci));
             const T t = d[u] - cc * q;
             q = wall_div(t, h[u], l[u]);
-            hout[(size_t)2 * nxh * j] = q;
+            h0[(size_t)2 * nxh * j] = q;
         }
     }
     T x = q;
@@ -742,19 +737,17 @@ __global__ void __launch_bounds__(64) k_wall_tdma(const T *__restrict__ Hin, T *
             p[u] = r[u] = T(0);
             if (j < 0) continue;
             p[u] = P[(size_t)j * modes + mode];
-            r[u] = hout[(size_t)2 * nxh * j];
+            r[u] = h0[(size_t)2 * nxh * j];
         }
 #pragma unroll
         for (int u = 0; u < G; ++u) {
             const int j = j0 - u;
             if (j < 0) continue;
             x = p[u] * x + r[u];
-            hout[(size_t)2 * nxh * j] = x;
+            h0[(size_t)2 * nxh * j] = x;
         }
     }
 }
-
-inline size_t wall_table_size(int ny, int nxh, int nz) { return (size_t)3 * (ny + 2) * nxh * nz; }
 
 template <typename T>
 inline void wall_table(T *tab, int ny, int nxh, int nz, const WallSpec &w, int sys, cudaStream_t s) {
@@ -764,32 +757,32 @@ inline void wall_table(T *tab, int ny, int nxh, int nz, const WallSpec &w, int s
 }
 
 template <typename T>
-inline void wall_tdma(int nb, const T *Hin, T *Hout, size_t hstride, int ny, int nxh, int nz, const WallSpec &w,
+inline void wall_tdma(int nb, T *H, size_t hstride, int ny, int nxh, int nz, const WallSpec &w,
                       Batch<WallItem<T>> items, cudaStream_t s) {
     Batch<T> off{};
     for (int q = 0; q < nb; ++q) {
         T a, b;
         wall_coef<T>(w, items.p[q].sys, 1, ny, 0.0, a, b, off.p[q]);
     }
-    k_wall_tdma<T><<<dim3((2 * nxh + 63) / 64, nz, nb), 64, 0, s>>>(Hin, Hout, hstride, ny, nxh, nz, T(1.0 / w.nxz), items,
-                                                                    off);
+    k_wall_tdma<T><<<dim3((2 * nxh + 63) / 64, nz, nb), 64, 0, s>>>(H, hstride, ny, nxh, nz, T(1.0 / w.nxz), items, off);
     count_launch();
 }
 
 // The wall-bounded solves of nb systems: FFT(x, z) of rows 1..NY, the
 // tridiagonal systems in y over rows 0..NY+1, inverse FFT of all NY+2 rows into
-// the halo rows of out.  H holds nb spectra of ny rows, H2 of ny + 2.
+// the halo rows of out.  H holds nb spectra of ny + 2 rows.
 template <typename T, typename TS, typename Out>
-inline void wall_solve_passes(int nb, Batch<const TS *> src, T *H, T *H2, size_t hstride, Batch<Out> out, const Geo &g,
+inline void wall_solve_passes(int nb, Batch<const TS *> src, T *H, size_t hstride, Batch<Out> out, const Geo &g,
                               const T *twx_r, const T *twx_i, const T *twz_r, const T *twz_i, const WallSpec &w,
                               Batch<WallItem<T>> items, cudaStream_t s) {
     const int nx = g.nx, ny = g.ny, nz = g.nz, nxh = nx / 2 + 1, n = ny + 2;
     const DivideSpec none{};
-    fft_x_fwd<T, TS>(nb, src, H, hstride, nx, ny, 1, ny, ny / 2, nz, twx_r, twx_i, s);
-    if (nz > 1) fft_lines<T>(nb, H, hstride, nz, nxh * ny, nxh, ny, nxh, twz_r, twz_i, -1, 0, none, s);
-    wall_tdma<T>(nb, H, H2, hstride, ny, nxh, nz, w, items, s);
-    if (nz > 1) fft_lines<T>(nb, H2, hstride, nz, nxh * n, nxh, n, nxh, twz_r, twz_i, +1, 0, none, s);
-    fft_x_inv<T, Out>(nb, H2, hstride, out, nx, n, n / 2, nz, 0, g.sx, g.sy, twx_r, twx_i, 0, s);
+    T *H1 = H + (size_t)2 * nxh;      // row 1
+    fft_x_fwd<T, TS>(nb, src, H1, hstride, nx, ny, 1, n, ny / 2, nz, twx_r, twx_i, s);
+    if (nz > 1) fft_lines<T>(nb, H1, hstride, nz, nxh * n, nxh, ny, nxh, twz_r, twz_i, -1, 0, none, s);
+    wall_tdma<T>(nb, H, hstride, ny, nxh, nz, w, items, s);
+    if (nz > 1) fft_lines<T>(nb, H, hstride, nz, nxh * n, nxh, n, nxh, twz_r, twz_i, +1, 0, none, s);
+    fft_x_inv<T, Out>(nb, H, hstride, out, nx, n, n / 2, nz, 0, g.sx, g.sy, twx_r, twx_i, 0, s);
 }
 
 }  // namespace f8

@@ -24,7 +24,7 @@ struct Dev {
     double *Up, *Vp, *Wp, *Ua, *Va, *Wa;   // halo
     double *Bx, *By, *Bz;                  // interior
     double *Q[3];                          // interior right-hand sides
-    double *H, *H2;                        // spectral scratch: up to three spectra of nspec values each
+    double *H;                             // spectral scratch: up to three spectra of nspec values each
     size_t nspec;
     double *walltab[3];                    // FP64 walls: Thomas tables of the U, V, P systems (k_wall_table)
     float *walltabf[3];                    // the same in FP32 (mixed contexts without a fused plane kernel)
@@ -59,7 +59,7 @@ struct Dev {
     float *Qf[3];                          // FP32 right-hand sides dt*(R + f)
     float *Rhf, *Rlf;                      // df64 Poisson right-hand side (interior)
     float *Rdf;                            // Poisson defect (interior)
-    float *Hf, *H2f;                       // FP32 spectra
+    float *Hf;                             // FP32 spectra
     float *HfB[2];                         // spectra of the V and W Helmholtz solves when they run
                                            // beside the U solve (fused spectral path)
     cudaStream_t aux[2];                   // the side streams of those two solves (0: none)

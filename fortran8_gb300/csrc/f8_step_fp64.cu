@@ -1456,7 +1456,7 @@ cudaError_t solve_batch(Dev &d, int nb, const double *const *src, double *const 
                                                 d.twx_i, d.twy_r, d.twy_i, d.twz_r, d.twz_i, d.kx2, d.ky2, d.kz2,
                                                 p ? 0.0 : 1.0, p ? -1.0 : d.ph.dt * d.ph.beta / d.ph.re / 2.0, s);
     } else {
-        wall_solve_passes<double, double, XOutD>(nb, in, d.H, d.H2, d.nspec, out, g, d.twx_r, d.twx_i, d.twz_r, d.twz_i,
+        wall_solve_passes<double, double, XOutD>(nb, in, d.H, d.nspec, out, g, d.twx_r, d.twx_i, d.twz_r, d.twz_i,
                                                  wall_spec(g, d.ph, d.kx2, d.kz2), items, s);
     }
     return cudaGetLastError();

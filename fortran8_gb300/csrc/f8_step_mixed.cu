@@ -1926,7 +1926,7 @@ cudaError_t solve_walls_mp(Dev &d, int nb, Batch<const float *> src, Batch<XOutF
     const Geo &g = d.g;
     Batch<WallItem<float>> items{};
     for (int q = 0; q < nb; ++q) items.p[q] = WallItem<float>{sys[q], d.walltabf[sys[q]], 0.0};
-    wall_solve_passes<float, float, XOutF>(nb, src, d.Hf, d.H2f, d.nspec, out, g, d.twxf_r, d.twxf_i, d.twzf_r, d.twzf_i,
+    wall_solve_passes<float, float, XOutF>(nb, src, d.Hf, d.nspec, out, g, d.twxf_r, d.twxf_i, d.twzf_r, d.twzf_i,
                                            wall_spec(g, d.ph, d.kx2, d.kz2), items, s);
     return cudaGetLastError();
 }

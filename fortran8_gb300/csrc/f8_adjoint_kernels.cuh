@@ -49,12 +49,6 @@ __device__ inline bool adj_inner(const Geo &g, int i, int j, int k) {
     return i >= 1 && i <= g.nx && j >= 1 && j <= g.ny && k >= 1 && k <= g.nz;
 }
 
-// value of an adjoint field at (i, j, k) if that cell is interior, else 0
-template <typename T>
-__device__ inline T lin(const T *A, const Geo &g, int i, int j, int k) {
-    return adj_inner(g, i, j, k) ? A[hix(g, i, j, k)] : T(0);
-}
-
 template <typename T>
 __device__ inline T sgn(T x) { return x > T(0) ? T(1) : (x < T(0) ? T(-1) : T(0)); }
 

@@ -17,18 +17,25 @@
 // Bounds, for a face with mean m, p = |B|^2 / 6 of its deviator B, s = sqrt(p),
 // r = det(B) / (2 s^3), u = sqrt(1 - r) and lambda = m + s 2t(u) (the smallest
 // root of 4t^3 - 3t = r, |t| <= 1):
-//  * double-float p and det(B) carry an absolute error of some 1e-12 of their
-//    scale, which moves lambda by at most 1e-11 s / u;
+//  * the products of p and det(B) in double-float carry an absolute error of some
+//    1e-12 of their scale, given B, which moves lambda by at most 1e-11 s / u;
+//  * B itself: C's components are split to 48 bits before the mean is taken off, and
+//    the differences and means round to as many.  The components of the cell and its
+//    neighbours reach a few M (M = |m| + 2s), so that is up to 10 x 2^-48 M in each
+//    component of B (160 eps M, eps = 2^-52).  It changes s by as much and r by
+//    6 x 160 eps M / s, so lambda by 160 eps M (4 + 2.5 / u);
 //  * the FP32 evaluation of u, 2t(u) (polynomial error 2.2e-7) and the sum moves
 //    it by at most 4e-6 s + 1e-6 |m - m0| (m0 the cell's mean, common to every
 //    face and left out of the comparisons);
 //  * the FP64 formula forms p = a1 - a2^2/3 and q from the unshifted
-//    components, with errors up to ~20 eps M^2 and ~100 eps M^3, M = |m| + 2s;
-//    they move lambda by at most 1e-13 M (M/s) (1 + (M/s)/u) (450 eps, above the
-//    sum of its terms);
+//    components, with errors up to ~20 eps M^2 and ~100 eps M^3; they move lambda
+//    by at most eps M (M/s) (20 + 26 (M/s)/u);
+//  * M/s is at least 2, so this and the error of B together stay below
+//    eps M (M/s) (340 + 126 (M/s)/u): 1e-13 M (M/s) (1 + (M/s)/u), 450 eps, is above;
 //  * the sentinel for repeated roots (|r| >= 1 as FP64 rounds it) can differ
-//    only where 1 - r^2 is within 4e-8 + 4e-13 (M/s)^3 of zero: such faces, and
-//    any that over- or underflow to NaN, are queued.
+//    only where 1 - r^2 is within 4e-8 + 4e-13 (M/s)^3 of zero (1800 eps (M/s)^3: the
+//    FP64 formula's 2 |dr| is 100 eps (M/s)^3 + 60 eps (M/s)^2, B's 1920 eps M/s):
+//    such faces, and any that over- or underflow to NaN, are queued.
 #include <cuda_runtime.h>
 #include "f8_codes_filter.cuh"
 #include "f8_common.cuh"

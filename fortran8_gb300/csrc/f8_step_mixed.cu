@@ -1937,7 +1937,7 @@ inline int x_rows_per_block(int nx) { return 2 * std::max(1, std::min(8, 1024 / 
 inline size_t x_smem(int nx, int rb) { return (size_t)(rb / 2) * 2 * nx * sizeof(float2) + (size_t)(nx / 2 + 1) * (rb + 1) * sizeof(float2); }
 inline int ilog2(int n) { int l = 0; while ((1 << l) < n) ++l; return l; }
 
-// warp-per-row-pair x passes for NX = 32 .. 512; false when NX has no instance
+// x passes in registers for NX = 32 .. 512; false when NX has no instance
 template <typename TS>
 bool xfwd_warp(const Dev &d, const TS *src, float2 *S, int ny, int lj, int joff, cudaStream_t s) {
     const Geo &g = d.g;
@@ -2561,7 +2561,7 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
             // the drag needs only the marker forces: beside the spreading and
             // the solves (joined after the solves)
             const bool want_drag = last && drag_out_dev;
-            if (want_drag && d.aux[1]) {
+            if (want_drag) {
                 F8_CUDA_RET(cudaEventRecord(d.ev_g[4], s));
                 F8_CUDA_RET(cudaStreamWaitEvent(d.aux[1], d.ev_g[4], 0));
                 F8_CUDA_RET(launch_drag(d, drag_out_dev, d.aux[1]));
@@ -2570,7 +2570,6 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
             int maxact = 0;
             for (int c = 0; c < nvc; ++c) maxact = std::max(maxact, d.nact[c]);
             if (maxact > 0) { k_ibm_spread_f<<<dim3((maxact + 127) / 128, g.nz, nvc), 128, 0, s>>>(a, g); count_launch(); }
-            if (want_drag && !d.aux[1]) F8_CUDA_RET(launch_drag(d, drag_out_dev, s));
             if ((e = cudaGetLastError())) return e;
             if (tp && last)
                 for (int c = 0; c < 3; ++c)
@@ -2580,7 +2579,7 @@ cudaError_t step_mixed(Dev &d, const StepOpts &o, double *drag_out_dev, int *sor
         if (r == 0) mark(4);
         // Helmholtz solves for the FP32 increments dU (U* = U^n + dU)
         if ((e = mixed_helmholtz(d, nvc, d.Qf, d.dUf, s))) return e;
-        if (o.ibm && r == repeats - 1 && drag_out_dev && d.aux[1]) F8_CUDA_RET(cudaStreamWaitEvent(s, d.ev_g[5], 0));
+        if (o.ibm && r == repeats - 1 && drag_out_dev) F8_CUDA_RET(cudaStreamWaitEvent(s, d.ev_g[5], 0));
         if (tp) {
             const TapeUp a{{d.Uf, d.Vf, d.Wf}, {d.dUf[0], d.dUf[1], d.dUf[2]}, {tp->Up[0], tp->Up[1], tp->Up[2]}};
             k_tape_up<<<dim3(trow.x, trow.y, 3), tthr, 0, s>>>(a, g); count_launch();

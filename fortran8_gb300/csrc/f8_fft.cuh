@@ -650,8 +650,9 @@ __host__ __device__ inline void wall_coef(const WallSpec &w, int sys, int j, int
 
 // Tables of the Thomas recurrence of every (kx, kz) system: per row and mode
 // P = -b/den and den, in FP64 1/den as the sum of two doubles (f8_recip.cuh) in
-// the second and third table, in FP32 den itself (an FP32 division is cheap).  Where tdma's guard sets P = Q = 0
-// (fenep_2d.f90:1157-1160): P = 1/den = 0, den = inf.  Layout [row][kz][kx].
+// the second and third table, in FP32 den itself (an FP32 division is cheap).
+// Where tdma's guard sets P = Q = 0 (fenep_2d.f90:1157-1160): P = 1/den = 0,
+// den = inf.  Layout [row][kz][kx].
 template <typename T>
 __global__ void k_wall_table(T *__restrict__ P, T *__restrict__ rh, T *__restrict__ rl, int ny, int nxh, int nz,
                              WallSpec w, int sys) {
@@ -685,11 +686,12 @@ __device__ __forceinline__ float wall_div(float t, float den, float) { return t 
 // those tables.  A thread runs the recurrence of the real or the imaginary part
 // of one mode (the coefficients are real), neighbouring threads neighbouring
 // values of a row, so the rows stream through without a tile; the forward
-// values wait in the rows of the right-hand side.  In FP64 the chain is 5 slots a row forward and 2
-// back, where forming the coefficients and dividing took about 60 in a
+// values wait in the rows of the right-hand side.  In FP64 the chain is 5 slots a
+// row forward and 2 back, where forming the coefficients and dividing took about 60 in a
 // half-filled warp.
 template <typename T>
-__global__ void __launch_bounds__(64) k_wall_tdma(T *H, size_t hstride, int ny, int nxh, int nz, T inv_nxz, Batch<WallItem<T>> items, Batch<T> off) {
+__global__ void __launch_bounds__(64) k_wall_tdma(T *H, size_t hstride, int ny, int nxh, int nz, T inv_nxz,
+                                                  Batch<WallItem<T>> items, Batch<T> off) {
     const int n = ny + 2;
     const WallItem<T> it = items.p[blockIdx.z];
     const int sys = it.sys;
